@@ -8,8 +8,13 @@
 //   ADFWI/propagator/acoustic_kernels.py:252-265  alpha / kappa coefficient definitions
 //   ADFWI/propagator/acoustic_kernels.py:268-301  chunked time loop and the record dict
 //
-// One launch advances one time step of all shots (acoustic_tma.cuh, acoustic_vec.cuh):
-// persistent, warp-specialised blocks stream (tile, shot) items through a TMA / mbarrier
+// Float32 solves run on the resident time loop (acoustic_res.cuh) wherever a shot's state fits the
+// shared memory of the blocks that work on it; the per-step kernels below take the rest: FP64,
+// boundary saving, grids too large, receivers on the mirrored row above a free surface, and
+// adjoints driven by dL/d u- or w-records.
+//
+// Per-step kernels: one launch advances one time step of all shots (acoustic_tma.cuh,
+// acoustic_vec.cuh): persistent, warp-specialised blocks stream (tile, shot) items through a TMA / mbarrier
 // pipeline; per item the consumers compute the new pressure on a 16 x 64 tile plus its halo
 // (1 row / column before, 2 after) and then the new u and w on the tile, four adjacent
 // columns per thread, so p, u and w each cross HBM once per step (ping-pong buffers keep the
@@ -28,6 +33,7 @@
 #include <vector>
 
 #include "../../include/adfwi_gb300.h"
+#include "acoustic_geo.cuh"
 #include "common.cuh"
 #include "frames.cuh"
 #include "l2.cuh"
@@ -36,98 +42,6 @@
 
 namespace adfwi {
 namespace ac {
-
-// Explicitly rounded arithmetic (keeps the reference's operation order; no FMA contraction).
-__device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
-
-template <typename T>
-struct Geo {
-  Layout L;
-  int ns, nt, nr;
-  int fs;     // first stencil row of u/w (nabc with a free surface, else 1)
-  int fsurf;  // free surface on / off
-  int zbeg;   // first tiled row (fs-1 with a free surface: rows above never change)
-  int tiles_x;
-  int nabc, nz, nx;
-  T dt;
-  T c1, c2;
-  const int* src_z;          // padded source rows (ns)
-  const int* src_x;          // padded source columns (ns)
-  const int* tile_rcv_beg;   // ntiles+1 offsets into trcv_*
-  const int* trcv_cell;      // (local row << 16) | local column
-  const int* trcv_id;        // receiver index
-  const int* tile_cell_beg;  // ntiles+1 offsets into tcell_*
-  const int* tcell_cell;     // unique receiver cells of a tile, packed like trcv_cell
-  const int* tcell_rbeg;     // ncells+1 offsets into cell_rcv
-  const int* cell_rcv;       // receiver indices grouped by unique cell
-  const int* grp_beg;        // ngroups+1 offsets: shots of each shot group (a group has one model)
-  const int* grp_model;      // model of each shot group
-  // Fused misfit: when fz_tr is set, the dL/d p-records handed to the adjoint are the
-  // normalised L2 misfit's adjoint source, formed from the synthetic records (the p-record
-  // gradient pointer then holds them) and fz_obs with the per-trace factors fz_tr.
-  const T* fz_obs;
-  const l2::TraceFactors<T>* fz_tr;
-  const double* fz_gmul;     // device scale of the source (the objective's gradient w.r.t. the loss)
-  int fz_norm_obs;
-};
-
-// dL/d p-record of shot sh, step t, receiver rid: from the gradient array gp, or formed from the
-// records (gp) and the observed data with the misfit's factors when the misfit is fused. In two
-// parts, the loads (RecPIn) and the value from them, so that a caller handling several
-// receivers issues every load before the arithmetic (the IEEE divisions of the source have an
-// out-of-line slow path, across which later loads are not hoisted).
-// (gmul: the source's scale, read once by the caller with fused_scale)
-template <typename T>
-struct RecPIn {
-  T v, o;
-  l2::TraceFactors<T> f;
-};
-template <typename T>
-__device__ __forceinline__ RecPIn<T> grad_rec_p_load(const Geo<T>& g, const T* gp, int sh, int t, int rid) {
-  RecPIn<T> r;
-  const int64_t o = ((int64_t)sh * g.nt + t) * g.nr + rid;
-  r.v = gp[o];
-  if (g.fz_tr != nullptr) {
-    r.o = g.fz_obs[o];
-    r.f = g.fz_tr[(int64_t)sh * g.nr + rid];
-  }
-  return r;
-}
-template <typename T>
-__device__ __forceinline__ T grad_rec_p_value(const Geo<T>& g, const RecPIn<T>& r, int t, T gmul) {
-  return g.fz_tr == nullptr ? r.v : l2::source(r.f, r.v, r.o, t, g.fz_norm_obs, gmul);
-}
-template <typename T>
-__device__ __forceinline__ T grad_rec_p(const Geo<T>& g, const T* gp, int sh, int t, int rid, T gmul) {
-  return grad_rec_p_value(g, grad_rec_p_load(g, gp, sh, t, rid), t, gmul);
-}
-template <typename T>
-__device__ __forceinline__ T fused_scale(const Geo<T>& g) {
-  return g.fz_gmul != nullptr ? (T)*g.fz_gmul : T(1);
-}
-
-// Update regions of acoustic_kernels.py:115, 139, 151.
-template <typename T>
-__device__ __forceinline__ bool in_p(const Geo<T>& g, int i, int j) {
-  return i >= g.fs + 1 && i <= g.L.nzp - 3 && j >= 2 && j <= g.L.nxp - 3;
-}
-template <typename T>
-__device__ __forceinline__ bool in_u(const Geo<T>& g, int i, int j) {
-  return i >= g.fs && i <= g.L.nzp - 2 && j >= 1 && j <= g.L.nxp - 3;
-}
-template <typename T>
-__device__ __forceinline__ bool in_w(const Geo<T>& g, int i, int j) {
-  return i >= g.fs && i <= g.L.nzp - 3 && j >= 1 && j <= g.L.nxp - 2;
-}
-template <typename T>
-__device__ __forceinline__ bool in_window(const Geo<T>& g, int i, int j) {
-  return i >= g.nabc && i < g.nabc + g.nz && j >= g.nabc && j < g.nabc + g.nx;
-}
 
 // Seed of the reverse pass: lambda = injection of the records of the last step.
 template <typename T>
@@ -211,14 +125,6 @@ __global__ void illum_finalize(Layout L, int groups, int ns, int nabc, int nz, i
   }
 }
 
-// Masked coefficient planes for the branch-free pipelined kernels, computed with the
-// reference's own operations (acoustic_kernels.py:257-265, and 1 - kappa of 115-160):
-//   A1M = alpha1 on the p region, 0 elsewhere;  B1 = 1 - damp*dt on the p region, 1 elsewhere;
-//   A2U / A2W = alpha2 on the u / w regions, 0 elsewhere;
-//   B2 / B3 = 1 - 0.5*(d + d_right)*dt / 1 - 0.5*(d + d_below)*dt on the u / w regions, 1 elsewhere.
-// Ghost cells stay 0. Planes follow the raw a1, a2, damp planes in the coefficient block.
-enum { kA1 = 0, kA2 = 1, kDamp = 2, kA1M = 3, kB1 = 4, kA2U = 5, kA2W = 6, kB2 = 7, kB3 = 8, kNumCoef = 9 };
-
 template <typename T>
 __global__ void mask_coefficients(Geo<T> g, T* cf) {
   const Layout L = g.L;
@@ -239,10 +145,53 @@ __global__ void mask_coefficients(Geo<T> g, T* cf) {
 }
 
 }  // namespace ac
+
+namespace res {
+
+// Gradient of one model from its shots' sums: dst = - (sum over the shots) / alpha on rows from
+// z0 (zero above); a cell whose alpha is zero was summed without the scale.
+__global__ void reduce_scaled(Layout L, int z0, int shots, const float* __restrict__ alpha,
+                              const float* __restrict__ src, float* __restrict__ dst) {
+  const int64_t n = (int64_t)L.nzp * L.nxp;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(e / L.nxp), j = (int)(e - (int64_t)i * L.nxp);
+    const int64_t o = L.off(i, j);
+    float acc = 0.0f;
+    if (i >= z0)
+      for (int s = 0; s < shots; ++s) acc += src[(int64_t)s * L.plane + o];
+    const float al = alpha[o];
+    dst[e] = -acc / (al == 0.0f ? 1.0f : al);
+  }
+}
+
+// The divergence histories written by time_loop hold the stencil's value on every row and column;
+// the per-step adjoint wants zeroes outside the p region: rows above fs + 1 and the last two, the
+// first and last two columns.
+__global__ void zero_outside_p(const __grid_constant__ ac::Geo<float> g, int64_t planes, float* hd) {
+  const Layout L = g.L;
+  const int top = g.fs + 1 - g.zbeg, n = (top + 2) * L.nxp + 4 * (L.nzp - 2 - g.fs - 1);
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < planes * n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t pl = e / n;
+    int k = (int)(e - pl * n), i, j;
+    if (k < (top + 2) * L.nxp) {
+      i = k / L.nxp;
+      j = k - i * L.nxp;
+      i = i < top ? g.zbeg + i : L.nzp - 2 + (i - top);
+    } else {
+      k -= (top + 2) * L.nxp;
+      i = g.fs + 1 + k / 4;
+      j = k % 4 < 2 ? k % 4 : L.nxp - 4 + k % 4;
+    }
+    hd[pl * L.plane + L.off(i, j)] = 0.0f;
+  }
+}
+
+}  // namespace res
 }  // namespace adfwi
 
 #include "acoustic_tma.cuh"
 #include "acoustic_vec.cuh"
+#include "acoustic_res.h"
 #include "bsave.cuh"
 
 // ----------------------------------------------------------------------------------------
@@ -261,10 +210,20 @@ struct Tiling {
   int ncells;
 };
 
+// Launch configuration of the resident time loop (acoustic_res.cuh). G = 0: not taken.
+struct Resident {
+  int glb = 0;                     // strips exchange rows through global memory (else a cluster)
+  int G = 0, S = 0, R = 0, RB = 0, MT = 0, TR = 0, T = 0, CG = 0;
+  int oS = 0, oA1 = 0, oA2 = 0, oPH = 0, oDH = 0, oBox = 0, oInj = 0, injw = 0, injg = 0, oRow = 0, oT = 0, words = 0;
+  int64_t o_sl = 0, o_sb = 0, o_tp = 0, o_ti = 0, o_rb = 0, o_rv = 0;  // tab: strips' receiver cells
+};
+
 struct adfwi_acoustic_plan {
   adfwi_acoustic_desc d;
   int nzp, nxp, fs, zbeg;
   Tiling t2;             // 16 x 64 tiles of the pipelined forward and adjoint steps
+  Resident rf, ra;       // the resident time loop, forward and adjoint, where the grid allows it
+  int64_t o_sm = 0;      // tab: the model of each shot
   int K, nseg;           // snapshot interval and number of segments (gradient mode)
   int last_chunk_start;  // first step of the reference's last checkpoint chunk
   int elem;              // bytes per element
@@ -285,7 +244,7 @@ struct adfwi_acoustic_plan {
 namespace {
 
 struct Carve {
-  int64_t coef, fa, fb, ilp, ilu, tab, flag;  // forward
+  int64_t coef, fa, fb, ilp, ilu, tab, flag, box;  // forward
   int64_t snap, snap_scale, bsv, hp, hd, la, lb, g1, g2;  // gradient extras
   int64_t mst, mpk, mnorm, mfac;                     // fused misfit: trace stats, gather peaks, norms, factors
   int64_t total;
@@ -293,11 +252,14 @@ struct Carve {
 
 int64_t align256(int64_t x) { return (x + 255) / 256 * 256; }
 
+int64_t res_box_bytes(const Resident& r);
+
 // A gradient plan in boundary-saving mode (with a single step there is nothing to rebuild: the
 // history of that step is kept).
 bool boundary_saving(const adfwi_acoustic_plan* p) { return p->bsave && p->d.nt > 1; }
 
-Carve carve(const adfwi_acoustic_plan* p, bool grad, int K) {
+// (box: with the inboxes of the resident loop's strips)
+Carve carve(const adfwi_acoustic_plan* p, bool grad, int K, bool box = true) {
   Carve c{};
   const int64_t pl = p->L.plane * p->elem;
   const int64_t ns = p->d.ns;
@@ -310,6 +272,7 @@ Carve carve(const adfwi_acoustic_plan* p, bool grad, int K) {
   c.ilu = take((int64_t)p->t2.ngroups * pl);
   c.tab = take((int64_t)p->tab.size() * 4);
   c.flag = take(256);
+  if (box) c.box = take(std::max(res_box_bytes(p->rf), grad ? res_box_bytes(p->ra) : (int64_t)0));
   if (grad) {
     const int nseg = (p->d.nt + K - 1) / K;
     const bool bs = boundary_saving(p);
@@ -399,10 +362,11 @@ int grid_blocks(int64_t n) { return (int)std::min<int64_t>(std::max<int64_t>((n 
 
 template <typename T>
 int setup_common(const adfwi_acoustic_plan* p, unsigned char* ws, const Carve& c, const void* alpha1,
-                 const void* alpha2, const void* damp, cudaStream_t st) {
+                 const void* alpha2, const void* damp, bool clear_fields, cudaStream_t st) {
   const int64_t pl = p->L.plane * p->elem;
-  // Zero coefficient planes (ghosts), field buffers and illumination partials.
-  ADFWI_CUDA_TRY(cudaMemsetAsync(ws + c.coef, 0, c.tab - c.coef, st));
+  // Zero coefficient planes (ghosts) and, where they are read before they are written, field
+  // buffers and illumination partials.
+  ADFWI_CUDA_TRY(cudaMemsetAsync(ws + c.coef, 0, (clear_fields ? c.tab : c.fa) - c.coef, st));
   ADFWI_CUDA_TRY(cudaMemsetAsync(ws + c.flag, 0, 256, st));
   ADFWI_CUDA_TRY(cudaMemcpyAsync(ws + c.tab, p->tab_pin.ptr, p->tab.size() * 4, cudaMemcpyHostToDevice, st));
   const int64_t n = (int64_t)p->nzp * p->nxp;
@@ -562,19 +526,217 @@ int set_smem_limits() {
   return kOk;
 }
 
+// ---------------------------------------------------------------- resident time loop (host)
+using res::ResKernel;
+ResKernel res_kernel(const Resident& r, bool adj, bool sums) {
+  return adj ? res::adjoint_kernel(r.RB, r.MT, r.glb) : res::forward_kernel(r.RB, r.MT, sums, r.glb);
+}
+
+// Shared memory above 48 KB and clusters of more than 8 blocks are properties of the kernel in one
+// device's context: opted into once per (device, kernel), to the most that any configuration
+// takes, since solves run from several threads.
+std::mutex g_res_mu;
+std::vector<std::pair<int, ResKernel>> g_res_done;
+cudaError_t res_prepare(ResKernel k) {
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(g_res_mu);
+  for (const auto& d : g_res_done)
+    if (d.first == dev && d.second == k) return cudaSuccess;
+  e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) g_res_done.push_back({dev, k});
+  return e;
+}
+
+// A cluster per shot, or a cooperative launch (strips that wait for one another through global
+// memory are resident together).
+void res_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const Resident& r, cudaStream_t st) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3((unsigned)(r.G * r.S));
+  cfg->blockDim = dim3((unsigned)r.T);
+  cfg->dynamicSmemBytes = (size_t)r.words * 4;
+  cfg->stream = st;
+  if (r.glb) {
+    attr->id = cudaLaunchAttributeCooperative;
+    attr->val.cooperative = 1;
+  } else {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)r.G;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  }
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+}
+
+int64_t res_box_bytes(const Resident& r) {
+  return r.glb ? (int64_t)2 * r.G * r.S * res::kBoxRows * r.CG * 32 : 0;
+}
+
+res::ResArgs res_args(const adfwi_acoustic_plan* p, const Resident& r, unsigned char* ws, const Carve& c) {
+  res::ResArgs a;
+  memset(&a, 0, sizeof(a));
+  a.G = r.G;
+  a.S = r.S;
+  a.z0 = p->d.free_surface ? p->fs : 0;
+  a.NR = p->nzp - a.z0;
+  a.R = r.R;
+  a.TR = r.TR;
+  a.CG = r.CG;
+  a.oS = r.oS;
+  a.oA1 = r.oA1;
+  a.oA2 = r.oA2;
+  a.oPH = r.oPH;
+  a.oDH = r.oDH;
+  a.oBox = r.oBox;
+  a.oInj = r.oInj;
+  a.injw = r.injw;
+  a.injg = r.injg;
+  a.oRow = r.oRow;
+  a.oT = r.oT;
+  a.cf = reinterpret_cast<const float*>(ws + c.coef);
+  a.cf_stride = (int64_t)ac::kNumCoef * p->L.plane;
+  const int32_t* tb = reinterpret_cast<const int32_t*>(ws + c.tab);
+  a.shot_model = tb + p->o_sm;
+  a.row_slot = tb + r.o_sl;
+  a.strip_beg = tb + r.o_sb;
+  a.tpos = tb + r.o_tp;
+  a.trid = tb + r.o_ti;
+  a.srbeg = tb + r.o_rb;
+  a.srcv = tb + r.o_rv;
+  a.box = reinterpret_cast<unsigned long long*>(ws + c.box);
+  a.flag = reinterpret_cast<int*>(ws + c.flag);
+  a.nz = 0x8000000080000000ull;
+  return a;
+}
+
+// Steps t0 .. t1-1 (the adjoint downwards) in launches of at most about a tenth of a second (6 us
+// per step and wave of shots): blocks that wait for their neighbours are then never held up for
+// long by another stream's launch. Between launches the state and the sums are in s1, acc0 and
+// acc1; a launch's split changes no result.
+int res_launch(const adfwi_acoustic_plan* p, const Resident& r, bool adj, bool sums, const ac::Geo<float>& g,
+               res::ResArgs a, int t0, int t1, cudaStream_t st) {
+  ResKernel k = res_kernel(r, adj, sums);
+  ADFWI_CUDA_TRY(res_prepare(k));
+  const int waves = r.glb ? (p->d.ns + r.S - 1) / r.S : (p->d.ns * r.G + 151) / 152;
+  const int most = std::max(64, 16000 / waves);
+  for (int done = 0; done < t1 - t0; done += most) {
+    const int n = std::min(most, t1 - t0 - done);
+    a.t0 = adj ? t1 - done - n : t0 + done;
+    a.t1 = a.t0 + n;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    res_config(&cfg, attr, r, st);
+    if (r.glb) ADFWI_CUDA_TRY(cudaMemsetAsync(a.box, 0, res_box_bytes(r), st));
+    ADFWI_LAUNCH(adj ? kAcAdjStep : kAcFwdStep, st, ADFWI_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, g, a)));
+    a.s0 = a.s1;
+    a.first = 0;
+  }
+  return kOk;
+}
+
+// The forward solve on the resident time loop: one launch, or one per snapshot interval. The
+// state lives in fa between launches and the per-shot illumination sums in fb (3 ns planes each;
+// the per-step kernels' ping-pong buffers).
+int forward_resident(const adfwi_acoustic_plan* p, unsigned char* ws, const Carve& c, const float* wav, float* rec_p,
+                     float* rec_u, float* rec_w, bool grad, int K, cudaStream_t st) {
+  const int nt = p->d.nt, ns = p->d.ns;
+  const int64_t pl = p->L.plane;
+  const bool full = grad && K >= nt;
+  const ac::Geo<float> g = make_geo<float>(p, ws, c, p->t2);
+  res::ResArgs a = res_args(p, p->rf, ws, c);
+  float* fa = reinterpret_cast<float*>(ws + c.fa);
+  float* fb = reinterpret_cast<float*>(ws + c.fb);
+  a.wav = wav;
+  a.rec_p = rec_p;
+  a.rec_u = rec_u;
+  a.rec_w = rec_w;
+  a.accum_u = p->last_chunk_start;
+  a.acc0 = fb;
+  a.acc1 = fb + ns * pl;
+  a.s1 = fa;
+  if (full) {
+    a.hp = reinterpret_cast<float*>(ws + c.hp);
+    a.hd = reinterpret_cast<float*>(ws + c.hd);
+  }
+  const int step = grad && !full ? K : nt;
+  for (int t0 = 0; t0 < nt; t0 += step) {
+    if (grad && !full) {
+      const int rc = snapshot_store<float>(p->d.snapshot_precision, fa, 3 * (int64_t)ns, pl, ws + c.snap,
+                                           ws + c.snap_scale, (int64_t)(t0 / K) * 3 * ns, st);
+      if (rc) return rc;
+    }
+    a.s0 = t0 == 0 ? nullptr : fa;
+    a.first = t0 == 0;
+    const int rc = res_launch(p, p->rf, false, true, g, a, t0, std::min(nt, t0 + step), st);
+    if (rc) return rc;
+  }
+  return kOk;
+}
+
+// Steps t0 .. t1-1 again from the state in fa, keeping their histories (slot 0 is step t0).
+int recompute_resident(const adfwi_acoustic_plan* p, unsigned char* ws, const Carve& c, const float* wav, int t0, int t1,
+                       cudaStream_t st) {
+  const ac::Geo<float> g = make_geo<float>(p, ws, c, p->t2);
+  res::ResArgs a = res_args(p, p->rf, ws, c);
+  a.wav = wav;
+  a.s0 = a.s1 = reinterpret_cast<float*>(ws + c.fa);
+  a.hp = reinterpret_cast<float*>(ws + c.hp);
+  a.hd = reinterpret_cast<float*>(ws + c.hd);
+  a.h0 = t0;
+  return res_launch(p, p->rf, false, false, g, a, t0, t1, st);
+}
+
+// What the per-step adjoint expects of the divergence history of a resident forward.
+int mask_divergence(const ac::Geo<float>& g, int64_t planes, float* hd, cudaStream_t st) {
+  ADFWI_LAUNCH(kAux, st, (res::zero_outside_p<<<152 * 8, 256, 0, st>>>(g, planes, hd)));
+  ADFWI_CUDA_TRY(cudaGetLastError());
+  return kOk;
+}
+
+// Reverse steps t1-1 .. t0 on the histories of a segment that begins at step h0. grec_p: dL/d
+// p-records of rnt steps per shot from step r0. The adjoint state lives in la between launches
+// and the per-shot gradient sums in lb (3 ns planes each).
+int adjoint_resident(const adfwi_acoustic_plan* p, unsigned char* ws, const Carve& c, const float* grec_p, int r0, int rnt,
+                     int t0, int t1, int h0, bool first, cudaStream_t st) {
+  const ac::Geo<float> g = make_geo<float>(p, ws, c, p->t2);
+  res::ResArgs a = res_args(p, p->ra, ws, c);
+  float* la = reinterpret_cast<float*>(ws + c.la);
+  float* lb = reinterpret_cast<float*>(ws + c.lb);
+  a.s0 = first ? nullptr : la;
+  a.s1 = la;
+  a.first = first;
+  a.hp = reinterpret_cast<float*>(ws + c.hp);
+  a.hd = reinterpret_cast<float*>(ws + c.hd);
+  a.rec_p = const_cast<float*>(grec_p);
+  a.r0 = r0;
+  a.rnt = rnt;
+  a.acc0 = lb;
+  a.acc1 = lb + p->d.ns * p->L.plane;
+  a.h0 = h0;
+  return res_launch(p, p->ra, true, true, g, a, t0, t1, st);
+}
+
 template <typename T>
 int forward_impl(const adfwi_acoustic_plan* p, const void* alpha1, const void* alpha2, const void* damp,
                  const void* wavelet, void* rec_p, void* rec_u, void* rec_w, void* fw_p, void* fw_u,
-                 void* fw_w, bool grad, unsigned char* ws, int64_t ws_bytes, cudaStream_t st) {
+                 void* fw_w, bool grad, unsigned char* ws, int64_t ws_bytes, cudaStream_t st, bool box = true) {
   int rc = set_smem_limits<T>();
   if (rc) return rc;
   const int K = grad ? p->K : 1;
-  Carve c = carve(p, grad, K);
+  Carve c = carve(p, grad, K, box);
   if (ws_bytes < c.total) {
     set_error("workspace too small: %lld bytes given, %lld needed", (long long)ws_bytes, (long long)c.total);
     return kWorkspaceTooSmall;
   }
-  rc = setup_common<T>(p, ws, c, alpha1, alpha2, damp, st);
+  const bool bs = grad && boundary_saving(p);
+  const bool full = grad && !bs && K >= p->d.nt;
+  bool resident = false;
+  if constexpr (sizeof(T) == 4) resident = p->rf.G > 0 && (box || !p->rf.glb);
+  // (the resident loop starts from zeroes of its own; the first snapshot is the zero state)
+  rc = setup_common<T>(p, ws, c, alpha1, alpha2, damp, !resident || (grad && !full), st);
   if (rc) return rc;
   ac::Geo<T> g = make_geo<T>(p, ws, c, p->t2);
   const int64_t pl = p->L.plane;
@@ -586,11 +748,9 @@ int forward_impl(const adfwi_acoustic_plan* p, const void* alpha1, const void* a
   T* ilu = reinterpret_cast<T*>(ws + c.ilu);
   int* flag = reinterpret_cast<int*>(ws + c.flag);
   const T* wav = static_cast<const T*>(wavelet);
-  const bool bs = grad && boundary_saving(p);
-  const bool full = grad && !bs && K >= p->d.nt;
   T* hp = grad ? reinterpret_cast<T*>(ws + c.hp) : nullptr;
   T* hd = grad ? reinterpret_cast<T*>(ws + c.hd) : nullptr;
-  if (full) {
+  if (full && !resident) {
     // the pressure history is read with its halo (as the next step's input and by the adjoint)
     rc = zero_frames<T>(hp, (int64_t)K * ns, p->L, st);
     if (rc) return rc;
@@ -598,7 +758,16 @@ int forward_impl(const adfwi_acoustic_plan* p, const void* alpha1, const void* a
   T* cur = fa;
   T* nxt = fb;
   const int64_t bslot = (int64_t)3 * ns * p->nframe;  // elements of one boundary-saving slot
-  for (int it = 0; it < p->d.nt; ++it) {
+  if constexpr (sizeof(T) == 4) {
+    if (resident) {
+      rc = forward_resident(p, ws, c, wav, static_cast<T*>(rec_p), static_cast<T*>(rec_u), static_cast<T*>(rec_w),
+                            grad, K, st);
+      if (rc) return rc;
+      ilp = fb;  // one partial plane per shot
+      ilu = fb + ns * pl;
+    }
+  }
+  for (int it = resident ? p->d.nt : 0; it < p->d.nt; ++it) {
     if (grad && !full && !bs && it % K == 0) {
       rc = snapshot_store<T>(p->d.snapshot_precision, cur, 3 * ns, pl, ws + c.snap, ws + c.snap_scale,
                              (int64_t)(it / K) * 3 * ns, st);
@@ -631,9 +800,10 @@ int forward_impl(const adfwi_acoustic_plan* p, const void* alpha1, const void* a
     const int64_t n = (int64_t)p->d.nz * p->d.nx;
     auto at = [&](void* f, int m) { return f ? static_cast<T*>(f) + (int64_t)m * n : nullptr; };
     for (int m = 0; m < p->nm; ++m) {  // model m: its groups' partial planes and its shots' last w
-      const int g0 = p->model_grp_beg[m], s0 = p->model_shot_beg[m];
+      const int s0 = p->model_shot_beg[m], g0 = resident ? s0 : p->model_grp_beg[m];
+      const int ng = (resident ? p->model_shot_beg[m + 1] : p->model_grp_beg[m + 1]) - g0;
       ADFWI_LAUNCH(kAux, st, (ac::illum_finalize<T><<<grid_blocks(n), 256, 0, st>>>(
-                                  p->L, p->model_grp_beg[m + 1] - g0, p->model_shot_beg[m + 1] - s0, p->d.nabc,
+                                  p->L, ng, p->model_shot_beg[m + 1] - s0, p->d.nabc,
                                   p->d.nz, p->d.nx, ilp + (int64_t)g0 * pl, ilu + (int64_t)g0 * pl,
                                   cur + 2 * ns * pl + (int64_t)s0 * pl, at(fw_p, m), at(fw_u, m), at(fw_w, m))));
     }
@@ -690,12 +860,58 @@ int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void*
   const T* gw = static_cast<const T*>(grw);
 
   ADFWI_CUDA_TRY(cudaMemsetAsync(la, 0, 3 * ns * pl * sizeof(T), st));
+  if constexpr (sizeof(T) == 4) {
+    // the resident adjoint takes dL/d p-records; dL/d u- and w-records go through the per-step
+    // kernels. A fused misfit's records are formed a stretch of steps at a time in fb, which the
+    // adjoint does not use.
+    const int64_t stretch = fz == nullptr ? nt : 3 * pl / p->d.nr;
+    if (p->ra.G > 0 && gu == nullptr && gw == nullptr && stretch > 0) {
+      const int nseg = full ? 1 : (nt + K - 1) / K;
+      for (int seg = nseg - 1; seg >= 0; --seg) {
+        const int t0 = seg * K, t1 = std::min(nt, t0 + K);
+        if (!full) {
+          rc = snapshot_load<T>(p->d.snapshot_precision, fa, 3 * ns, pl, ws + c.snap, ws + c.snap_scale,
+                                (int64_t)seg * 3 * ns, st);
+          if (!rc) rc = recompute_resident(p, ws, c, wav, t0, t1, st);
+          if (rc) return rc;
+        }
+        for (int e1 = t1; e1 > t0;) {
+          const int e0 = (int)std::max<int64_t>(t0, e1 - stretch);
+          if (fz != nullptr)
+            ADFWI_LAUNCH(kAux, st, (l2::sources<T><<<l2::grid((int)ns, p->d.nr), l2::block(), 0, st>>>(
+                                       (int)ns, nt, p->d.nr, e0, e1, fz->norm_obs, gp, static_cast<const T*>(fz->obs),
+                                       g2.fz_tr, fz->gmul, fb)));
+          rc = adjoint_resident(p, ws, c, fz != nullptr ? fb : gp, fz != nullptr ? e0 : 0, fz != nullptr ? e1 - e0 : nt,
+                                e0, e1, t0, e1 == nt, st);
+          if (rc) return rc;
+          e1 = e0;
+        }
+      }
+      const int64_t n = (int64_t)p->nzp * p->nxp;
+      for (int m = 0; m < p->nm; ++m) {  // model m's gradients: the sums over its shots
+        const int s0 = p->model_shot_beg[m], nm = p->model_shot_beg[m + 1] - s0;
+        const T* cm = cf + (int64_t)m * ac::kNumCoef * pl;
+        ADFWI_LAUNCH(kAux, st, (res::reduce_scaled<<<grid_blocks(n), 256, 0, st>>>(
+                                    p->L, p->d.free_surface ? p->fs : 0, nm, cm + ac::kA1 * pl, lb + (int64_t)s0 * pl,
+                                    static_cast<T*>(ga1) + m * n)));
+        ADFWI_LAUNCH(kAux, st, (res::reduce_scaled<<<grid_blocks(n), 256, 0, st>>>(
+                                    p->L, p->d.free_surface ? p->fs : 0, nm, cm + ac::kA2 * pl, lb + (ns + s0) * pl,
+                                    static_cast<T*>(ga2) + m * n)));
+      }
+      ADFWI_CUDA_TRY(cudaGetLastError());
+      return kOk;
+    }
+  }
   ADFWI_CUDA_TRY(cudaMemsetAsync(lb, 0, 3 * ns * pl * sizeof(T), st));
   ADFWI_CUDA_TRY(cudaMemsetAsync(g1p, 0, (size_t)p->t2.ngroups * pl * sizeof(T), st));
   ADFWI_CUDA_TRY(cudaMemsetAsync(g2p, 0, (size_t)p->t2.ngroups * pl * sizeof(T), st));
-  if (!full) {
-    // the recomputed pressure history is read with its halo by the next step and the adjoint
+  if (!full || p->rf.G > 0) {
+    // the recomputed pressure history is read with its halo by the next step and the adjoint (the
+    // resident forward leaves the frames of a whole history as they were)
     rc = zero_frames<T>(hp, (int64_t)K * ns, p->L, st);
+    if constexpr (sizeof(T) == 4) {
+      if (!rc && full && p->rf.G > 0) rc = mask_divergence(g2, (int64_t)nt * ns, hd, st);
+    }
     if (rc) return rc;
   }
   if (gp || gu || gw) {
@@ -742,7 +958,14 @@ int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void*
       if (rc) return rc;
       T* cur = fa;
       T* nxt = fb;
-      for (int it = t0; it < t1; ++it) {
+      bool resident = false;
+      if constexpr (sizeof(T) == 4) {
+        resident = p->rf.G > 0;
+        if (resident) rc = recompute_resident(p, ws, c, wav, t0, t1, st);
+        if (!rc && resident) rc = mask_divergence(g2, (int64_t)(t1 - t0) * ns, hd, st);
+        if (rc) return rc;
+      }
+      for (int it = resident ? t1 : t0; it < t1; ++it) {
         const T* p0 = it == t0 ? fa : hp + (int64_t)(it - 1 - t0) * ns * pl;
         rc = launch_fwd<T>(p, g2, it, 0, cf, wav, p0, cur + ns * pl, cur + 2 * ns * pl,
                            hp + (int64_t)(it - t0) * ns * pl, nxt + ns * pl, nxt + 2 * ns * pl,
@@ -817,7 +1040,7 @@ int l2_sources_impl(const adfwi_acoustic_plan* p, const void* syn, const void* o
   const int ns = p->d.ns, nt = p->d.nt, nr = p->d.nr;
   const auto* fac = reinterpret_cast<const l2::TraceFactors<T>*>(ws + c.mfac);
   ADFWI_LAUNCH(kAux, st, (l2::sources<T><<<l2::grid(ns, nr), l2::block(), 0, st>>>(
-                             ns, nt, nr, flags & 1, static_cast<const T*>(syn), static_cast<const T*>(obs), fac, gmul,
+                             ns, nt, nr, 0, nt, flags & 1, static_cast<const T*>(syn), static_cast<const T*>(obs), fac, gmul,
                              static_cast<T*>(adj))));
   ADFWI_CUDA_TRY(cudaGetLastError());
   return kOk;
@@ -963,6 +1186,222 @@ void build_tiling(adfwi_acoustic_plan* p, Tiling* tl, int tz, int tx, const std:
   t.insert(t.end(), cr.begin(), cr.end());
 }
 
+// Shared memory of a configuration, in words.
+// (most, most_rows: receiver cells, and rows holding any, of the strip that has the most)
+void res_layout(Resident* r, bool adj, int kept, bool tables, int most, int most_rows) {
+  const int w4 = 4 * r->CG, R = r->R, sb = res::kGrp * (r->CG + 1);
+  int o = res::kHeadWords;
+  r->oS = o;
+  o += (R + 4) * sb + res::kGrp;
+  r->oA1 = kept >= 1 ? o : 0;
+  if (kept >= 1) o += R * w4;
+  r->oA2 = kept >= 2 ? o : 0;
+  if (kept >= 2) o += R * w4;
+  r->oPH = r->oDH = 0;
+  if (adj) {
+    r->oPH = o;
+    o += (R + 3) * w4 + 4;
+    r->oDH = o;
+    o += R * w4;
+  }
+  r->oBox = o;
+  if (!r->glb && r->G > 1) o += res::kBoxRows * r->CG * 8;
+  // dL/d records of the step and of the next: one row lies in the unused U slots of rows R and R+1
+  r->injg = most_rows <= 1 ? res::kGrp : 4;
+  r->injw = most_rows <= 1 ? sb : most_rows * w4;
+  r->oInj = most_rows <= 1 ? r->oS + (R + 2) * sb + res::kGrp : o;
+  if (adj && most_rows > 1) o += 2 * r->injw;
+  r->oRow = o;
+  if (adj) o += R;
+  r->oT = tables ? o : 0;
+  r->words = o + (tables ? 2 * most : 0);
+}
+
+// Blocks of a variant that an SM holds: MT threads of 65536 / MT registers, and the shared memory.
+int res_per_sm(const Resident& r) {
+  const int regs = 65536 / r.MT / 8 * 8;
+  return std::min(65536 / (regs * r.T), 233472 / (r.words * 4 + 1024));
+}
+
+// Clusters of C blocks that are resident at a time when an SM holds n such blocks: asked of the
+// runtime once per (device, C, n), since it depends on how the SMs are grouped.
+std::mutex g_cluster_mu;
+std::vector<std::vector<int>> g_clusters;  // per device: C x n, -1 unknown
+int resident_clusters(const Resident& r, int n, int dev, ResKernel k) {
+  constexpr int kN = 32;
+  n = std::min(n, kN - 1);
+  std::lock_guard<std::mutex> lk(g_cluster_mu);
+  if ((int)g_clusters.size() <= dev) g_clusters.resize(dev + 1);
+  std::vector<int>& t = g_clusters[dev];
+  if (t.empty()) t.assign((res::kMaxCluster + 1) * kN, -1);
+  int& v = t[r.G * kN + n];
+  if (v < 0) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    res_config(&cfg, attr, r, nullptr);
+    if (res_prepare(k) != cudaSuccess || cudaOccupancyMaxActiveClusters(&v, k, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      v = 0;
+    }
+  }
+  return v;
+}
+
+// The configuration with the least estimated time per step of all shots: waves of shots x (what
+// the exchange between strips costs + the 128-cell units of an SM x the variant's time per unit).
+// In us, from sweeps of G and of the variants with per-launch times (300 x 700 padded with 10 and
+// 30 shots, 148 x 260 with 40, 200 x 200 with 10, 600 x 1600 with 8):
+//   exchange: 1.6 through global memory, 0.7 in a cluster (whose shared memory is next door, but
+//     only 7 clusters of 16 blocks, 13 of 10 or 23 of 6 fit the GPU at a time);
+//   per unit, forward / adjoint: 0.065 / 0.09 for 3 rows per thread and 128 registers; the adjoint
+//     loses a third at 80 registers (spills), and more rows per thread leave fewer warps;
+//   several blocks per SM run 15 % slower than one that does the same work.
+// For example 300 x 700 with 30 shots, us per step: forward 29.2 with 25 strips of 12 rows and
+// 3 rows per thread (35.4 with 6, 43.5 with 38 strips of 8), adjoint 40.8 with 25 strips and 6
+// rows per thread (45.8 with 4, 46.9 with 3, 52.6 with 50 strips of 6).
+Resident res_choose(const adfwi_acoustic_plan* p, bool adj, const std::vector<std::pair<int64_t, int>>& rc, int max_smem,
+                    int sms, int dev) {
+  const int z0 = p->d.free_surface ? p->fs : 0;
+  const int NR = p->nzp - z0, CG = (p->nxp + 3) / 4, ns = p->d.ns;
+  std::vector<int> cells(NR + 1, 0);  // receiver cells of the rows before each row
+  for (size_t q = 0; q < rc.size(); ++q)
+    if (q == 0 || rc[q].first != rc[q - 1].first) cells[(rc[q].first >> 16) + 1]++;
+  std::vector<int> held(NR + 1, 0);   // rows before each row that hold any
+  for (int r = 0; r < NR; ++r) {
+    held[r + 1] = held[r] + (cells[r + 1] > 0);
+    cells[r + 1] += cells[r];
+  }
+  Resident best;
+  double best_cost = 1e30;
+  for (int glb = 0; glb < 2; ++glb) {
+    for (int G = glb ? 2 : 1; G <= (glb ? 2 * sms : res::kMaxCluster); ++G) {
+      const int least = NR / G;
+      if (least < 4) break;
+      int most = 0, most_rows = 0;
+      for (int k = 0; k < G; ++k) {
+        const int b = (int)((int64_t)k * NR / G), e = (int)((int64_t)(k + 1) * NR / G);
+        most = std::max(most, cells[e] - cells[b]);
+        most_rows = std::max(most_rows, held[e] - held[b]);
+      }
+      Resident r;
+      r.glb = glb;
+      r.G = G;
+      r.R = (NR + G - 1) / G;
+      r.CG = CG;
+      for (const int* v : res::kVariants) {
+        r.RB = v[0];
+        r.MT = v[1];
+        r.TR = (r.R + r.RB - 1) / r.RB;
+        if (least / r.TR < 2) continue;  // the boundary threads own both rows that cross
+        r.T = (r.TR * CG + 31) / 32 * 32;
+        if (r.T > r.MT) continue;
+        for (int kept = 2; kept >= -1; --kept) {  // alpha1, alpha2 kept; -1: not even the receiver tables
+          res_layout(&r, adj, std::max(0, kept), kept >= 0, most, most_rows);
+          if (r.words * 4 > max_smem) continue;
+          const int n = res_per_sm(r);
+          if (n < 1) continue;
+          r.S = 1;
+          const int cap = glb ? n * sms / G : resident_clusters(r, n, dev, res_kernel(r, adj, true));
+          if (cap < 1) continue;
+          r.S = glb ? std::min(ns, cap) : ns;
+          const int waves = (ns + cap - 1) / cap;
+          const double load = (double)std::min(ns, cap) * G / sms;
+          const double units = r.R * CG / 32.0 * (load > 1.0 ? 1.15 * load : 1.0);
+          const double per_unit = adj ? (r.RB == 3 ? (r.MT == 512 ? 0.09 : 0.12) : r.RB == 4 ? (r.MT == 512 ? 0.105 : 0.115) : 0.1)
+                                      : (r.RB == 3 ? 0.065 : r.RB == 4 ? (r.MT == 512 ? 0.09 : 0.076) : 0.084);
+          const double cost = waves * ((glb ? 1.6 : 0.7) + per_unit * units) * (1.0 - 0.01 * kept);
+          if (cost < best_cost) {
+            best_cost = cost;
+            best = r;
+          }
+          break;
+        }
+      }
+    }
+  }
+  if (best.G > 0 && best.glb) {  // what the runtime says of the chosen one decides
+    int occ = 0;
+    ResKernel k = res_kernel(best, adj, true);
+    if (res_prepare(k) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, best.T, (size_t)best.words * 4) != cudaSuccess)
+      cudaGetLastError();
+    best.S = std::min(ns, occ * sms / best.G);
+    if (best.S < 1) best = Resident();
+  }
+  return best;
+}
+
+// Configurations of the resident time loop for this plan's grid and shots, and their tables
+// (appended to p->tab). They stay empty where the state does not fit.
+void plan_resident(adfwi_acoustic_plan* p, const int32_t* rcv_z, const int32_t* rcv_x) {
+  const adfwi_acoustic_desc& d = p->d;
+  if (p->elem != 4 || p->bsave) return;
+  int dev = 0, max_smem = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return;  // no device: plans made for their sizes only
+  }
+  // receivers in (row, column) order; receivers on the mirrored row above a free surface stay with
+  // the per-step kernels (their dL/d records fold into the interior)
+  const int z0 = d.free_surface ? p->fs : 0;
+  std::vector<std::pair<int64_t, int>> rc(d.nr);
+  bool above = false;
+  for (int r = 0; r < d.nr; ++r) {
+    const int z = rcv_z[r] + d.nabc - z0, x = rcv_x[r] + d.nabc;
+    rc[r] = {((int64_t)z << 16) | x, r};
+    above = above || z < 0;
+  }
+  if (above) return;
+  std::stable_sort(rc.begin(), rc.end(), [](const std::pair<int64_t, int>& a, const std::pair<int64_t, int>& b) {
+    return a.first < b.first;
+  });
+  p->rf = res_choose(p, false, rc, max_smem, sms, dev);
+  if (p->rf.G > 0) p->ra = res_choose(p, true, rc, max_smem, sms, dev);
+  std::vector<int32_t>& t = p->tab;
+  p->o_sm = t.size();
+  for (int m = 0; m < p->nm; ++m)
+    for (int s = p->model_shot_beg[m]; s < p->model_shot_beg[m + 1]; ++s) t.push_back(m);
+  const int64_t NR = p->nzp - z0;
+  for (Resident* r : {&p->rf, &p->ra}) {
+    if (r->G == 0) continue;
+    std::vector<int32_t> beg(r->G + 1, 0), slot(NR, 0), pos, rid, rbeg, rcv;
+    const int sb = res::kGrp * (r->CG + 1);
+    int strip = 0, last = -1, nslot = 0;
+    for (size_t q = 0; q < rc.size(); ++q) {
+      const int z = (int)(rc[q].first >> 16), x = (int)(rc[q].first & 0xffff);
+      while (z >= (int)((int64_t)(strip + 1) * NR / r->G)) ++strip, nslot = 0;
+      if (z != last) slot[z] = ++nslot;
+      last = z;
+      if (q == 0 || rc[q].first != rc[q - 1].first) {
+        beg[strip + 1]++;
+        const int row = z - (int)((int64_t)strip * NR / r->G);
+        pos.push_back(r == &p->ra ? ((slot[z] - 1) * r->CG + x / 4) * r->injg + x % 4 : row * sb + res::kGrp * (x / 4) + x % 4);
+        rid.push_back(rc[q].second);
+        rbeg.push_back((int32_t)rcv.size());
+      } else {
+        rid.back() = -(int32_t)rid.size();  // -1 - cell: several receivers
+      }
+      rcv.push_back(rc[q].second);
+    }
+    rbeg.push_back((int32_t)rcv.size());
+    for (int q = 0; q < r->G; ++q) beg[q + 1] += beg[q];
+    r->o_sl = t.size();
+    t.insert(t.end(), slot.begin(), slot.end());
+    r->o_sb = t.size();
+    t.insert(t.end(), beg.begin(), beg.end());
+    r->o_tp = t.size();
+    t.insert(t.end(), pos.begin(), pos.end());
+    r->o_ti = t.size();
+    t.insert(t.end(), rid.begin(), rid.end());
+    r->o_rb = t.size();
+    t.insert(t.end(), rbeg.begin(), rbeg.end());
+    r->o_rv = t.size();
+    t.insert(t.end(), rcv.begin(), rcv.end());
+  }
+}
+
 // ----------------------------------------------------------------------------------------
 // Forward solve for callers that cannot allocate device memory.
 //
@@ -1006,7 +1445,10 @@ int adfwi_acoustic_forward_noalloc(const adfwi_acoustic_plan* p, const void* alp
   ADFWI_CHECK_ARG(p && alpha1 && alpha2 && damp && wavelet, "null argument");
   ADFWI_CHECK_ARG((rec_p && rec_u && rec_w) || (!rec_p && !rec_u && !rec_w), "records: give all three or none");
   ADFWI_CHECK_ARG(p->d.nr > 0 || rec_p == nullptr, "records requested without receivers");
-  const int64_t need = carve(p, false, 1).total;
+  // strips that exchange rows through global memory need inboxes: without the room for them the
+  // per-step kernels solve (the same records)
+  const bool box = carve(p, false, 1).total <= kStaticScratchBytes;
+  const int64_t need = carve(p, false, 1, box).total;
   if (need > kStaticScratchBytes) {
     set_error("adfwi_acoustic_forward_noalloc: this solve needs %lld bytes of scratch but the static scratch "
               "array holds %lld bytes (64 MiB); use adfwi_acoustic_forward with a caller-provided workspace",
@@ -1023,14 +1465,14 @@ int adfwi_acoustic_forward_noalloc(const adfwi_acoustic_plan* p, const void* alp
   // in the shared array do not leak into this one.
   if (p->d.dtype == ADFWI_F64)
     return forward_impl<double>(p, alpha1, alpha2, damp, wavelet, rec_p, rec_u, rec_w, fw_p, fw_u, fw_w, false, w,
-                                kStaticScratchBytes, st);
+                                kStaticScratchBytes, st, box);
   return forward_impl<float>(p, alpha1, alpha2, damp, wavelet, rec_p, rec_u, rec_w, fw_p, fw_u, fw_w, false, w,
-                             kStaticScratchBytes, st);
+                             kStaticScratchBytes, st, box);
 }
 
 int adfwi_acoustic_noalloc_status(const adfwi_acoustic_plan* p, int32_t* status, void* stream) {
   ADFWI_CHECK_ARG(p && status, "null argument");
-  const Carve c = carve(p, false, 1);
+  const Carve c = carve(p, false, 1, false);
   ADFWI_CHECK_ARG(c.total <= kStaticScratchBytes, "this plan's forward does not fit the static scratch array");
   void* ws = nullptr;
   int rc = static_scratch_address(&ws);
@@ -1169,6 +1611,7 @@ int plan_create_impl(const adfwi_acoustic_desc* desc, const int32_t* src_z, cons
     p->t2.blocks = std::max(1, std::min(run_blocks, p->t2.ntiles * p->t2.ngroups));
     p->t2.fwd_blocks = std::max(1, std::min(run_fblocks, p->t2.ntiles * p->t2.ngroups));
   }
+  plan_resident(p, rcv_z, rcv_x);
   if (t.empty()) t.push_back(0);
 
   if (!p->tab_pin.assign(p->tab.data(), p->tab.size() * 4)) {

@@ -208,9 +208,10 @@ __global__ void __launch_bounds__(kThreads) factors(int ns, int nt, int nr, doub
   norms[tr] = n;
 }
 
-// The adjoint source of every sample, times *gmul when gmul is given.
+// The adjoint source of the samples t0 .. t1-1 (adj: ns x (t1 - t0) x nr), times *gmul when gmul is
+// given.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) sources(int ns, int nt, int nr, int normalise_obs,
+__global__ void __launch_bounds__(kThreads) sources(int ns, int nt, int nr, int t0, int t1, int normalise_obs,
                                                     const T* __restrict__ syn, const T* __restrict__ obs,
                                                     const TraceFactors<T>* __restrict__ fac,
                                                     const double* __restrict__ gmul, T* __restrict__ adj) {
@@ -219,11 +220,11 @@ __global__ void __launch_bounds__(kThreads) sources(int ns, int nt, int nr, int 
   if (r >= nr) return;
   const TraceFactors<T> f = fac[(int64_t)s * nr + r];
   const T gm = gmul != nullptr ? (T)*gmul : T(1);
-  const int64_t base = (int64_t)s * nt * nr + r;
+  const int64_t base = (int64_t)s * nt * nr + r, out = ((int64_t)s * (t1 - t0) - t0) * nr + r;
 #pragma unroll 4
-  for (int t = y; t < nt; t += kPhases) {
+  for (int t = t0 + y; t < t1; t += kPhases) {
     const int64_t o = base + (int64_t)t * nr;
-    adj[o] = source(f, syn[o], obs[o], t, normalise_obs, gm);
+    adj[out + (int64_t)t * nr] = source(f, syn[o], obs[o], t, normalise_obs, gm);
   }
 }
 

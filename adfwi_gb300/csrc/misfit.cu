@@ -65,7 +65,7 @@ int run(int32_t ns, int32_t nt, int32_t nr, double dt, double silent_rel, int32_
   ADFWI_LAUNCH(kAux, st, (peaks<T><<<grid(ns, nr), block(), 0, st>>>(ns, nt, nr, sy, ob, stats, gsyn, gobs)));
   ADFWI_LAUNCH(kAux, st, (factors<T><<<grid(ns, nr), block(), 0, st>>>(ns, nt, nr, dt, silent_rel, nob, sy, ob, stats,
                                                                          gsyn, gobs, fac, norms)));
-  ADFWI_LAUNCH(kAux, st, (sources<T><<<grid(ns, nr), block(), 0, st>>>(ns, nt, nr, nob, sy, ob, fac, nullptr,
+  ADFWI_LAUNCH(kAux, st, (sources<T><<<grid(ns, nr), block(), 0, st>>>(ns, nt, nr, 0, nt, nob, sy, ob, fac, nullptr,
                                                                          static_cast<T*>(adj))));
   ADFWI_LAUNCH(kAux, st, (sum_norms<<<1, kThreads, 0, st>>>((int64_t)ns * nr, norms, loss)));
   ADFWI_CUDA_TRY(cudaGetLastError());
