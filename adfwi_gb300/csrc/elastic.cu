@@ -263,20 +263,106 @@ struct StagedZ {
   __device__ __forceinline__ T operator()(int ii, int jj) const { return s[(ii - i0 + 3) * kTileX + (jj - j0)]; }
 };
 
-// ======================================================================= forward, PML
-// Split-field update of a cell and its totals in one pass (elastic_kernels.py:351-402); the rows
-// whose totals read other rows (free surface) are left to the *_fs_rows kernels that follow.
 template <typename T>
-__device__ __forceinline__ bool stress_fs_row(const Geo<T>& g, int i) {
-  return g.fsurf && i >= g.h - 3 && i <= g.h - 1;
+__device__ __forceinline__ int tile_count(const Geo<T>& g) {
+  return ((g.L.nxp + kTileX - 1) / kTileX) * ((g.L.nzp + kTileZ - 1) / kTileZ);
 }
+
+// The velocity rows above a free surface (elastic_kernels.py:395-402) from the totals of rows h-1
+// and h: vz[h-3] = vz[h-2] = vz[h-1] and vx[h-2] from vz[h-1] and vx[h], on columns J; zero
+// elsewhere. The stress update reads them through this function (vx, vz: a shot's planes), so they
+// need no pass of their own before it.
+template <typename T>
+__device__ __forceinline__ T vel_above(const Geo<T>& g, const T* vx, const T* vz, bool x, int r, int j) {
+  const int h = g.h;
+  if (r >= h - 1) return (x ? vx : vz)[g.L.off(r, j)];
+  if (j < g.jlo || j > g.jhi || r < h - 3) return T(0);
+  const T up = vz[g.L.off(h - 1, j)];
+  if (!x) return up;
+  if (r == h - 3) return T(0);
+  const T right = vz[g.L.off(h - 1, j + 1)];
+  return radd(rsub(radd(rsub(j + 1 <= g.jhi ? right : T(0), up), right), up), vx[g.L.off(h, j)]);
+}
+// Receiver records taken by extra blocks of the step kernels (elastic_kernels.py:407-411): the
+// blocks of a launch after its tiles gather `ncomp` components of step `it` from fields that the
+// launch only reads, so recording costs no launch of its own. src: the first component's planes;
+// c0: its index in the record array; rows_above: the velocity rows above the free surface are not
+// in `src` (a receiver there reads vel_above).
+template <typename T>
+__device__ __forceinline__ void record_block(const Geo<T>& g, int tiles, int shots, int it, const T* src, int ncomp, int c0,
+                                             T* rec, bool rows_above = false) {
+  const int r = ((int)blockIdx.x - tiles) * (int)blockDim.x + (int)threadIdx.x;
+  if (r >= g.nr) return;
+  const int64_t NSP = (int64_t)g.ns * g.L.plane, RS = (int64_t)g.ns * g.nt * g.nr;
+  const int i = g.rcv_z[r], j = g.rcv_x[r];
+  const int64_t oc = g.L.off(i, j);
+  rows_above = rows_above && g.fsurf && i < g.h - 1;
+  for (int q = 0; q < shots; ++q) {
+    const int s = (int)blockIdx.y * shots + q;
+    if (s >= g.ns) break;
+    const int64_t o = (int64_t)s * g.L.plane + oc, e = ((int64_t)s * g.nt + it) * g.nr + r;
+    if (rows_above) {
+      const T *vx = src + o - oc, *vz = vx + NSP;
+      rec[c0 * RS + e] = vel_above(g, vx, vz, true, i, j);
+      rec[(c0 + 1) * RS + e] = vel_above(g, vx, vz, false, i, j);
+      continue;
+    }
+    for (int c = 0; c < ncomp; ++c) rec[(c0 + c) * RS + e] = src[c * NSP + o];
+  }
+}
+template <int NN, typename T>
+__device__ __forceinline__ T dzb_above(const Geo<T>& g, const T* vx, const T* vz, bool x, int i, int j) {
+  auto a = [&](int r) { return vel_above(g, vx, vz, x, r, j); };
+  T r = rmul(g.f0, rsub(a(i), a(i - 1)));
+  r = radd(r, rmul(g.f1, rsub(a(i + 1), a(i - 2))));
+  if (NN == 3) r = radd(r, rmul(g.f2, rsub(a(i + 2), a(i - 3))));
+  return r;
+}
+template <int NN, typename T>
+__device__ __forceinline__ T dzf_above(const Geo<T>& g, const T* vx, const T* vz, bool x, int i, int j) {
+  auto a = [&](int r) { return vel_above(g, vx, vz, x, r, j); };
+  T r = rmul(g.f0, rsub(a(i + 1), a(i)));
+  r = radd(r, rmul(g.f1, rsub(a(i + 2), a(i - 1))));
+  if (NN == 3) r = radd(r, rmul(g.f2, rsub(a(i + 3), a(i - 2))));
+  return r;
+}
+
+// Stress totals of a cell (offset o) with the free-surface rows h-3 .. h-1 (elastic_kernels.py:
+// 375-384): tzz[h-1] = 0, tzz[h-2] = -tzz[h], txz[h-2] = -txz[h-1], txz[h-3] = -txz[h]. The cells of
+// rows h-1 and h write the mirrored values; the cells they mirror to leave theirs out.
+template <typename T>
+__device__ __forceinline__ void store_stress(const Geo<T>& g, int i, int64_t o, int64_t NSP, T xx, T zz, T xz, T* tt) {
+  const int64_t P = g.L.pitch;
+  const int h = g.h;
+  tt[TXX * NSP + o] = xx;
+  if (!g.fsurf || i > h || i < h - 3) {
+    tt[TZZ * NSP + o] = zz;
+    tt[TXZ * NSP + o] = xz;
+    return;
+  }
+  if (i == h - 1) zz = T(0);
+  if (i != h - 2) tt[TZZ * NSP + o] = zz;
+  if (i >= h - 1) tt[TXZ * NSP + o] = xz;
+  if (i == h - 1) tt[TXZ * NSP + o - P] = -xz;
+  if (i == h) {
+    tt[TZZ * NSP + o - 2 * P] = -zz;
+    tt[TXZ * NSP + o - 3 * P] = -xz;
+  }
+}
+
+// ======================================================================= forward, PML
+// Split-field update of a cell and its totals in one pass (elastic_kernels.py:351-402), two launches
+// per step: the stress rows that mirror others at the free surface are written by the cells they
+// mirror, the velocity rows above it by the next stress update, which reads them as vel_above.
+// With a pass for each kind of surface rows and one for the records, five launches, a step of one
+// shot on a 122 x 140 grid took 18.9 us; it takes 15.2.
 template <typename T>
 __device__ __forceinline__ bool vel_fs_row(const Geo<T>& g, int i, int j) {
   return g.fsurf && j >= g.jlo && j <= g.jhi && (i == g.h - 2 || i == g.h - 3);
 }
 
 // Cells that keep split fields: inside the update region, where a PML factor differs from 1,
-// and in the rows the free-surface kernels rebuild from split parts (h-3 .. h) plus one. Every
+// and in the surface rows that mirror others or are mirrored (h-3 .. h) plus one. Every
 // other cell of the update region advances its totals directly: there the split update is
 // x' = x + a, z' = z + b, total = x' + z' (the factors are exactly 1), so the unsplit
 // t' = (t + a) + b differs only by one rounding of the sum and moves half the bytes.
@@ -286,13 +372,18 @@ __device__ __forceinline__ bool keeps_split(const Geo<T>& g, int i, T bcx, T bcz
 }
 
 // tprev: stress totals at the start of the step (tt itself when the totals advance in place);
-// tt: where the new totals go.
+// tt: where the new totals go; rec: the velocity records of step it - 1 are taken (null: none).
 template <typename T, int NN>
-__global__ void stress_pml_tot(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ v,
-                               T* __restrict__ ts, T* tt, const T* tprev, const T* __restrict__ wav) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
+__global__ void stress_pml_tot(Geo<T> g, int it, const T* __restrict__ cf, T* __restrict__ v, T* __restrict__ ts, T* tt,
+                               const T* tprev, const T* __restrict__ wav, T* __restrict__ rec) {
+  griddep_wait();  // launched with programmatic serialisation in the time loops
   griddep_launch_dependents();
+  if (const int tiles = tile_count(g); (int)blockIdx.x >= tiles) {
+    record_block(g, tiles, kCellShots, it - 1, (const T*)v, 2, 3, rec, true);
+    return;
+  }
   EL_CELL_SHOTS
+  const bool above = g.fsurf && i <= g.h + NN - 2;  // the vertical differences reach rows above the surface
   const bool inside = in_I(g, i, j);
   bool split = true;
   T pxn = T(0), pzn = T(0), pxi = T(0), pzi = T(0);
@@ -348,9 +439,27 @@ __global__ void stress_pml_tot(Geo<T> g, int it, const T* __restrict__ cf, const
       const T* vx = v;
       const T* vz = v + NSP;
       const T dxbm_vx = dxb<NN>(g, vx, o), dxbm_vz = dxb<NN>(g, vz, o);
-      const T dzbm_vx = dzb<NN>(g, vx, o), dzbm_vz = dzb<NN>(g, vz, o);
-      const T dxfm_vx = dxf<NN>(g, vx, o), dzfm_vx = dzf<NN>(g, vx, o);
-      const T dxfm_vz = dxf<NN>(g, vz, o), dzfm_vz = dzf<NN>(g, vz, o);
+      const T dxfm_vx = dxf<NN>(g, vx, o), dxfm_vz = dxf<NN>(g, vz, o);
+      T dzbm_vx, dzbm_vz, dzfm_vx, dzfm_vz;
+      if (above) {
+        const T *ux = vx + (int64_t)s * PL, *uz = vz + (int64_t)s * PL;
+        dzbm_vx = dzb_above<NN>(g, ux, uz, true, i, j);
+        dzbm_vz = dzb_above<NN>(g, ux, uz, false, i, j);
+        dzfm_vx = dzf_above<NN>(g, ux, uz, true, i, j);
+        dzfm_vz = dzf_above<NN>(g, ux, uz, false, i, j);
+        if (i == g.h - 1) {  // the rows above, for whoever reads the velocities later
+#pragma unroll
+          for (int r = 2; r <= 3; ++r) {
+            v[VX * NSP + o - (r - 1) * (int64_t)g.L.pitch] = vel_above(g, ux, uz, true, g.h - r, j);
+            v[VZ * NSP + o - (r - 1) * (int64_t)g.L.pitch] = vel_above(g, ux, uz, false, g.h - r, j);
+          }
+        }
+      } else {
+        dzbm_vx = dzb<NN>(g, vx, o);
+        dzbm_vz = dzb<NN>(g, vz, o);
+        dzfm_vx = dzf<NN>(g, vx, o);
+        dzfm_vz = dzf<NN>(g, vz, o);
+      }
       sp[TXX_X] = rmul(radd(rmul(pxn, sp[TXX_X]), rmul(g.dt_dx, radd(rmul(c11, dxbm_vx), rmul(c15, dxbm_vz)))), pxi);
       sp[TXX_Z] = rmul(radd(rmul(pzn, sp[TXX_Z]), rmul(g.dt_dz, radd(rmul(c15, dzbm_vx), rmul(c13, dzbm_vz)))), pzi);
       sp[TZZ_X] = rmul(radd(rmul(pxn, sp[TZZ_X]), rmul(g.dt_dx, radd(rmul(c13, dxbm_vx), rmul(c35, dxbm_vz)))), pxi);
@@ -370,42 +479,21 @@ __global__ void stress_pml_tot(Geo<T> g, int it, const T* __restrict__ cf, const
     }
 #pragma unroll
     for (int k = 0; k < 6; ++k) ts[k * NSP + o] = sp[k];
-    if (!stress_fs_row(g, i)) {
-      tt[TXX * NSP + o] = radd(sp[TXX_X], sp[TXX_Z]);
-      tt[TZZ * NSP + o] = radd(sp[TZZ_X], sp[TZZ_Z]);
-      tt[TXZ * NSP + o] = radd(sp[TXZ_X], sp[TXZ_Z]);
-    }
+    store_stress(g, i, o, NSP, radd(sp[TXX_X], sp[TXX_Z]), radd(sp[TZZ_X], sp[TZZ_Z]), radd(sp[TXZ_X], sp[TXZ_Z]), tt);
   }
 }
 
-// Stress totals of the free-surface rows h-3 .. h-1 (elastic_kernels.py:375-384).
-template <typename T>
-__global__ void stress_fs_rows_pml(Geo<T> g, const T* __restrict__ ts, T* __restrict__ tt) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
-  griddep_launch_dependents();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= g.L.nxp) return;
-  const int i = g.h - 3 + (int)blockIdx.z, s = blockIdx.y;
-  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL, P = g.L.pitch;
-  const int64_t o = (int64_t)s * PL + g.L.off(i, j);
-  auto sum = [&](int f, int64_t oo) { return radd(ts[(2 * f) * NSP + oo], ts[(2 * f + 1) * NSP + oo]); };
-  T xx = sum(TXX, o), zz = sum(TZZ, o), xz = sum(TXZ, o);
-  const int h = g.h;
-  if (i == h - 1) zz = T(0);
-  if (i == h - 2) zz = -sum(TZZ, o + 2 * P);
-  if (i == h - 2) xz = -sum(TXZ, o + P);
-  if (i == h - 3) xz = -sum(TXZ, o + 3 * P);
-  tt[TXX * NSP + o] = xx;
-  tt[TZZ * NSP + o] = zz;
-  tt[TXZ * NSP + o] = xz;
-}
-
-// vprev: velocity totals at the start of the step (v itself when they advance in place).
+// vprev: velocity totals at the start of the step (v itself when they advance in place); rec: the
+// stress records of step it are taken (null: none).
 template <typename T, int NN>
-__global__ void vel_pml_tot(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ tt, T* __restrict__ vs,
-                            T* v, const T* vprev) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
+__global__ void vel_pml_tot(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ tt, T* __restrict__ vs,
+                            T* v, const T* vprev, T* __restrict__ rec) {
+  griddep_wait();  // launched with programmatic serialisation in the time loops
   griddep_launch_dependents();
+  if (const int tiles = tile_count(g); (int)blockIdx.x >= tiles) {
+    record_block(g, tiles, kCellShots, it, tt, 3, 0, rec);
+    return;
+  }
   EL_CELL_SHOTS
   const bool inside = in_I(g, i, j);
   bool split = true;
@@ -458,39 +546,24 @@ __global__ void vel_pml_tot(Geo<T> g, const T* __restrict__ cf, const T* __restr
   }
 }
 
-// Velocity totals of the free-surface rows h-3, h-2 (elastic_kernels.py:395-402), from the
-// split velocities of all rows.
-template <typename T>
-__global__ void vel_fs_rows_pml(Geo<T> g, const T* __restrict__ vs, T* __restrict__ v) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
-  griddep_launch_dependents();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < g.jlo || j > g.jhi || j >= g.L.nxp) return;
-  const int i = g.h - 3 + (int)blockIdx.z, s = blockIdx.y;
-  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL, P = g.L.pitch;
-  const int64_t o = (int64_t)s * PL + g.L.off(i, j);
-  auto vxs = [&](int64_t oo) { return radd(vs[VX_X * NSP + oo], vs[VX_Z * NSP + oo]); };
-  auto vzs = [&](int64_t oo) { return radd(vs[VZ_X * NSP + oo], vs[VZ_Z * NSP + oo]); };
-  T vx = vxs(o), vz = vzs(o);
-  const int h = g.h;
-  if (i == h - 2) {
-    const T vz_up = vzs(o + P);
-    const T vzn_r = (j + 1 <= g.jhi) ? vzs(o + P + 1) : vzs(o + 1);
-    vz = vz_up;
-    vx = radd(rsub(radd(rsub(vzn_r, vz_up), vzs(o + P + 1)), vz_up), vxs(o + 2 * P));
-  } else {
-    vz = vzs(o + 2 * P);
-  }
-  v[VX * NSP + o] = vx;
-  v[VZ * NSP + o] = vz;
-}
-
 // ======================================================================= forward, absorbing layer
+// The step out of place (tprev -> ts, v -> vout) or in place; the free-surface stress rows
+// (elastic_kernels.py:738-742) are written by the cells they mirror, as with the PML. Four launches a
+// step with a free surface (the velocity rows above it are inputs of the damping) and two without,
+// programmatically serialised; the reverse step takes six and four. A gradient step pair of 4 shots
+// on a 151 x 207 grid without one took 84 us as nine plain launches and two copies; it takes 50.
 template <typename T, int NN>
-__global__ void stress_abl(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ v, T* __restrict__ ts,
-                           const T* __restrict__ wav) {
+__global__ void stress_abl(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ v, T* ts, const T* tprev,
+                           const T* __restrict__ wav, T* __restrict__ rec) {
+  griddep_wait();
+  griddep_launch_dependents();
+  if (const int tiles = tile_count(g); (int)blockIdx.x >= tiles) {
+    record_block(g, tiles, 1, it - 1, v, 2, 3, rec);
+    return;
+  }
   EL_CELL_SHOT
   const int64_t occ = g.L.off(i, j);
+  T xx = tprev[TXX * NSP + o], zz = tprev[TZZ * NSP + o], xz = tprev[TXZ * NSP + o];
   if (in_I(g, i, j)) {
     const T* vx = v;
     const T* vz = v + NSP;
@@ -500,60 +573,59 @@ __global__ void stress_abl(Geo<T> g, int it, const T* __restrict__ cf, const T* 
     const T dxfm_vz = dxf<NN>(g, vz, o), dzfm_vz = dzf<NN>(g, vz, o);
     const T c11 = cf[C11 * PL + occ], c13 = cf[C13 * PL + occ], c15 = cf[C15 * PL + occ];
     const T c33 = cf[C33 * PL + occ], c35 = cf[C35 * PL + occ], c55 = cf[C55 * PL + occ];
-    T* f;
-    f = ts + TXX * NSP + o;
-    *f = radd(*f, rmul(g.dt, radd(rdiv(radd(rmul(c11, dxbm_vx), rmul(c15, dxbm_vz)), g.dx),
+    xx = radd(xx, rmul(g.dt, radd(rdiv(radd(rmul(c11, dxbm_vx), rmul(c15, dxbm_vz)), g.dx),
                                   rdiv(radd(rmul(c15, dzbm_vx), rmul(c13, dzbm_vz)), g.dz))));
-    f = ts + TZZ * NSP + o;
-    *f = radd(*f, rmul(g.dt, radd(rdiv(radd(rmul(c13, dxbm_vx), rmul(c35, dxbm_vz)), g.dx),
+    zz = radd(zz, rmul(g.dt, radd(rdiv(radd(rmul(c13, dxbm_vx), rmul(c35, dxbm_vz)), g.dx),
                                   rdiv(radd(rmul(c35, dzbm_vx), rmul(c33, dzbm_vz)), g.dz))));
-    f = ts + TXZ * NSP + o;
-    *f = radd(*f, rmul(g.dt, radd(rdiv(radd(rmul(c15, dxfm_vx), rmul(c55, dxfm_vz)), g.dx),
+    xz = radd(xz, rmul(g.dt, radd(rdiv(radd(rmul(c15, dxfm_vx), rmul(c55, dxfm_vz)), g.dx),
                                   rdiv(radd(rmul(c55, dzfm_vx), rmul(c35, dzfm_vz)), g.dz))));
   }
   if (i == g.src_z[s] && j == g.src_x[s]) {
     const T w = wav[(int64_t)s * g.nt + it];
-    ts[TXX * NSP + o] = radd(ts[TXX * NSP + o], rmul(g.src_m[3 * s + 0], w));
-    ts[TZZ * NSP + o] = radd(ts[TZZ * NSP + o], rmul(g.src_m[3 * s + 1], w));
-    ts[TXZ * NSP + o] = radd(ts[TXZ * NSP + o], rmul(g.src_m[3 * s + 2], w));
+    xx = radd(xx, rmul(g.src_m[3 * s + 0], w));
+    zz = radd(zz, rmul(g.src_m[3 * s + 1], w));
+    xz = radd(xz, rmul(g.src_m[3 * s + 2], w));
   }
+  store_stress(g, i, o, NSP, xx, zz, xz, ts);
 }
 
-// Free-surface stress rows in place (elastic_kernels.py:738-742); one thread per column.
-template <typename T>
-__global__ void stress_fs_abl(Geo<T> g, T* __restrict__ ts) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= g.L.nxp) return;
-  const int s = blockIdx.y, h = g.h;
-  const int64_t NSP = (int64_t)g.ns * g.L.plane, so = (int64_t)s * g.L.plane;
-  T* zz = ts + TZZ * NSP + so;
-  T* xz = ts + TXZ * NSP + so;
-  zz[g.L.off(h - 1, j)] = T(0);
-  zz[g.L.off(h - 2, j)] = -zz[g.L.off(h, j)];
-  xz[g.L.off(h - 2, j)] = -xz[g.L.off(h - 1, j)];
-  xz[g.L.off(h - 3, j)] = -xz[g.L.off(h, j)];
-}
-
+// Without a free surface the damping is applied here; with one it follows the surface rows.
 template <typename T, int NN>
-__global__ void vel_abl(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ tt, T* __restrict__ v) {
+__global__ void vel_abl(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ tt, T* v, const T* vprev,
+                        T* __restrict__ rec) {
+  griddep_wait();
+  griddep_launch_dependents();
+  if (const int tiles = tile_count(g); (int)blockIdx.x >= tiles) {
+    record_block(g, tiles, 1, it, tt, 3, 0, rec);
+    return;
+  }
   EL_CELL_SHOT
-  if (!in_I(g, i, j)) return;
   const int64_t occ = g.L.off(i, j);
-  const T dxfm_txx = dxf<NN>(g, tt + TXX * NSP, o);
-  const T dzbm_txz = dzb<NN>(g, tt + TXZ * NSP, o);
-  const T dxbm_txz = dxb<NN>(g, tt + TXZ * NSP, o);
-  const T dzfm_tzz = dzf<NN>(g, tt + TZZ * NSP, o);
-  const T bx = cf[BX * PL + occ], bz = cf[BZ * PL + occ];
-  T* f = v + VX * NSP + o;
-  *f = radd(*f, rmul(rmul(g.dt, bx), radd(rdiv(dxfm_txx, g.dx), rdiv(dzbm_txz, g.dz))));
-  f = v + VZ * NSP + o;
-  *f = radd(*f, rmul(rmul(g.dt, bz), radd(rdiv(dxbm_txz, g.dx), rdiv(dzfm_tzz, g.dz))));
+  T vx = vprev[VX * NSP + o], vz = vprev[VZ * NSP + o];
+  if (in_I(g, i, j)) {
+    const T dxfm_txx = dxf<NN>(g, tt + TXX * NSP, o);
+    const T dzbm_txz = dzb<NN>(g, tt + TXZ * NSP, o);
+    const T dxbm_txz = dxb<NN>(g, tt + TXZ * NSP, o);
+    const T dzfm_tzz = dzf<NN>(g, tt + TZZ * NSP, o);
+    const T bx = cf[BX * PL + occ], bz = cf[BZ * PL + occ];
+    vx = radd(vx, rmul(rmul(g.dt, bx), radd(rdiv(dxfm_txx, g.dx), rdiv(dzbm_txz, g.dz))));
+    vz = radd(vz, rmul(rmul(g.dt, bz), radd(rdiv(dxbm_txz, g.dx), rdiv(dzfm_tzz, g.dz))));
+  }
+  if (!g.fsurf) {
+    const T d = cf[DAMP * PL + occ];
+    vx = rmul(vx, d);
+    vz = rmul(vz, d);
+  }
+  v[VX * NSP + o] = vx;
+  v[VZ * NSP + o] = vz;
 }
 
 // Free-surface velocity rows in place (elastic_kernels.py:753-756); one thread per column in J.
 // Reads only rows h-1, h and the cell (h-2, jhi+1), none of which any thread writes.
 template <typename T>
 __global__ void vel_fs_abl(Geo<T> g, T* __restrict__ v) {
+  griddep_wait();
+  griddep_launch_dependents();
   const int j = g.jlo + blockIdx.x * blockDim.x + threadIdx.x;
   if (j > g.jhi) return;
   const int s = blockIdx.y, h = g.h;
@@ -571,29 +643,21 @@ __global__ void vel_fs_abl(Geo<T> g, T* __restrict__ v) {
 
 template <typename T>
 __global__ void damp_v(Geo<T> g, const T* __restrict__ cf, T* __restrict__ v) {
+  griddep_wait();
+  griddep_launch_dependents();
   EL_CELL_SHOT
   const T d = cf[DAMP * PL + g.L.off(i, j)];
   v[VX * NSP + o] = rmul(v[VX * NSP + o], d);
   v[VZ * NSP + o] = rmul(v[VZ * NSP + o], d);
 }
 
-// Receivers: txx, tzz, txz, vx, vz totals at each receiver (elastic_kernels.py:407-411).
+// The velocity records of step it, after the last step (the stress update of the next one would
+// have taken them).
 template <typename T>
-__global__ void record(Geo<T> g, int it, const T* __restrict__ tt, const T* __restrict__ v, T* rec) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
+__global__ void record_v(Geo<T> g, int it, const T* __restrict__ v, T* __restrict__ rec, bool rows_above) {
+  griddep_wait();
   griddep_launch_dependents();
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= g.nr) return;
-  const int s = blockIdx.y;
-  const int64_t NSP = (int64_t)g.ns * g.L.plane;
-  const int64_t o = (int64_t)s * g.L.plane + g.L.off(g.rcv_z[r], g.rcv_x[r]);
-  const int64_t RS = (int64_t)g.ns * g.nt * g.nr;
-  const int64_t q = ((int64_t)s * g.nt + it) * g.nr + r;
-  rec[0 * RS + q] = tt[TXX * NSP + o];
-  rec[1 * RS + q] = tt[TZZ * NSP + o];
-  rec[2 * RS + q] = tt[TXZ * NSP + o];
-  rec[3 * RS + q] = v[VX * NSP + o];
-  rec[4 * RS + q] = v[VZ * NSP + o];
+  record_block(g, 0, 1, it, v, 2, 3, rec, rows_above);
 }
 
 // forward_wavefield_* += sum_s X^2 of the last step of a chunk (elastic_kernels.py:414-418, 1016-1021).
@@ -729,35 +793,6 @@ struct PlaneQ {
   Layout L;
   __device__ __forceinline__ T operator()(int ii, int jj) const { return base[L.off(ii, jj)]; }
 };
-
-// (B3q) the velocity update's adjoint sources, once per cell and shot (zero outside I):
-// q = lambda(v split) * dt * b / (d * pml_d) for (vx_x, vx_z, vz_x, vz_z); PMLM = 0 uses the
-// absorbing-layer velocities (no pml_d).
-template <typename T, bool PMLM>
-__global__ void adj_tq(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lvv, T* __restrict__ q4) {
-  EL_CELL_SHOT
-  T a = T(0), b = T(0), c = T(0), d = T(0);
-  if (in_I(g, i, j)) {
-    const int64_t c0 = g.L.off(i, j);
-    const T bx = cf[BX * PL + c0], bz = cf[BZ * PL + c0];
-    if (PMLM) {
-      const Pml<T> p = pml_at(g, cf, c0, PL);
-      a = lvv[VX_X * NSP + o] * (g.dt * bx) / (g.dx * p.xd);
-      b = lvv[VX_Z * NSP + o] * (g.dt * bx) / (g.dz * p.zd);
-      c = lvv[VZ_X * NSP + o] * (g.dt * bz) / (g.dx * p.xd);
-      d = lvv[VZ_Z * NSP + o] * (g.dt * bz) / (g.dz * p.zd);
-    } else {
-      a = lvv[VX * NSP + o] * (g.dt * bx) / g.dx;
-      b = lvv[VX * NSP + o] * (g.dt * bx) / g.dz;
-      c = lvv[VZ * NSP + o] * (g.dt * bz) / g.dx;
-      d = lvv[VZ * NSP + o] * (g.dt * bz) / g.dz;
-    }
-  }
-  q4[0 * NSP + o] = a;
-  q4[1 * NSP + o] = b;
-  q4[2 * NSP + o] = c;
-  q4[3 * NSP + o] = d;
-}
 
 // (B4 + B3a) per shot group: the split velocities' lambda after the step (the velocity
 // free-surface adjoint, then S * lambda + lambda of the totals; read from lvs_in, written to
@@ -978,7 +1013,7 @@ __device__ __forceinline__ void stress_k(const Geo<T>& g, const T* __restrict__ 
   }
 }
 template <typename T, bool PMLM>
-__device__ __forceinline__ StressQ<T> stress_q(const T* __restrict__ lts, int64_t oo, int64_t NSP, T kx, T kz) {
+__device__ __forceinline__ StressQ<T> stress_q(const T* lts, int64_t oo, int64_t NSP, T kx, T kz) {
   StressQ<T> r;
   if (PMLM) {
     r.a = lts[TXX_X * NSP + oo] * kx;
@@ -998,11 +1033,12 @@ __device__ __forceinline__ StressQ<T> stress_q(const T* __restrict__ lts, int64_
   return r;
 }
 
-// (B1q) the stress update's adjoint sources for the velocity transposes, once per cell and
-// shot (zero outside I): sx_b, sx_zb, sx_f, sx_zf, sz_b, sz_zb, sz_f, sz_zf.
+// (B1q) the stress update's adjoint sources for the velocity transposes at a cell (c0) of one shot
+// (o), zero outside I: sx_b, sx_zb, sx_f, sx_zf, sz_b, sz_zb, sz_f, sz_zf.
 template <typename T, bool PMLM>
-__global__ void adj_vq(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lts, T* __restrict__ q8) {
-  EL_CELL_SHOT
+__device__ __forceinline__ void stress_sources(const Geo<T>& g, const T* __restrict__ cf, const T* lts, int i, int j,
+                                               int64_t o, T* __restrict__ q8) {
+  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL;
   T v[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] = T(0);
@@ -1024,6 +1060,13 @@ __global__ void adj_vq(Geo<T> g, const T* __restrict__ cf, const T* __restrict__
   }
 #pragma unroll
   for (int k = 0; k < 8; ++k) q8[k * NSP + o] = v[k];
+}
+template <typename T, bool PMLM>
+__global__ void adj_vq(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lts, T* __restrict__ q8) {
+  griddep_wait();
+  griddep_launch_dependents();
+  EL_CELL_SHOT
+  stress_sources<T, PMLM>(g, cf, lts, i, j, o, q8);
 }
 
 // (B1a) lambda of the velocity totals at the start of the step (overwrite) and the C gradients.
@@ -1367,12 +1410,14 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(T) == 4 ? 3 : 1)
   }
 }
 
-// ABL (reverse of v *= damp and the free-surface velocity rows): lv_out = FS^T(damp * lv_in).
+// ABL (reverse of v *= damp and the free-surface velocity rows): lv_out = FS^T(damp * lv_in), and
+// the velocity update's adjoint sources q4 (vx_x, vx_z, vz_x, vz_z) at the cell, zero outside I.
 template <typename T>
-__global__ void adj_vfs_abl(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lv_in, T* lv_out,
-                            T* scratch) {
+__global__ void adj_vfs_abl(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lv_in, T* __restrict__ lv_out,
+                            T* __restrict__ q4) {
+  griddep_wait();
+  griddep_launch_dependents();
   EL_CELL_SHOT
-  (void)scratch;
   // damp-weighted lambda at the cells the free-surface adjoint reads
   auto dl = [&](int comp, int64_t oo, int ii, int jj) { return cf[DAMP * PL + g.L.off(ii, jj)] * lv_in[comp * NSP + oo]; };
   T ax = dl(VX, o, i, j), az = dl(VZ, o, i, j);
@@ -1402,12 +1447,22 @@ __global__ void adj_vfs_abl(Geo<T> g, const T* __restrict__ cf, const T* __restr
   }
   lv_out[VX * NSP + o] = ax;
   lv_out[VZ * NSP + o] = az;
+  const bool inside = in_I(g, i, j);
+  const int64_t c0 = g.L.off(i, j);
+  const T bx = inside ? g.dt * cf[BX * PL + c0] : T(0), bz = inside ? g.dt * cf[BZ * PL + c0] : T(0);
+  q4[0 * NSP + o] = inside ? ax * bx / g.dx : T(0);
+  q4[1 * NSP + o] = inside ? ax * bx / g.dz : T(0);
+  q4[2 * NSP + o] = inside ? az * bz / g.dx : T(0);
+  q4[3 * NSP + o] = inside ? az * bz / g.dz : T(0);
 }
 
-// ABL: lt += transposes of the velocity update's stress differences; bx, bz gradients.
+// ABL: lt += transposes of the velocity update's stress differences; bx, bz gradients; without a
+// free surface also the stress update's adjoint sources q8 (with one they follow its rows).
 template <typename T, int NN>
-__global__ void adj_t_abl(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lv,
-                          const T* __restrict__ qv, T* lt, const T* __restrict__ tt_hist, T* gpart, int eg) {
+__global__ void adj_t_abl(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lv, const T* __restrict__ qv, T* lt,
+                          const T* __restrict__ tt_hist, T* gpart, int eg, T* __restrict__ q8) {
+  griddep_wait();
+  griddep_launch_dependents();
   EL_CELL
   EL_SHOT_GROUP
   T* gbx = gbase + 6 * PL;
@@ -1421,6 +1476,7 @@ __global__ void adj_t_abl(Geo<T> g, const T* __restrict__ cf, const T* __restric
     lt[TXX * NSP + o] += dxf_t<NN>(g, q1, i, j);
     lt[TXZ * NSP + o] += dzb_t<NN>(g, q2, i, j) + dxb_t<NN>(g, q3, i, j);
     lt[TZZ * NSP + o] += dzf_t<NN>(g, q4, i, j);
+    if (!g.fsurf) stress_sources<T, false>(g, cf, lt, i, j, o, q8);
     if (in_I(g, i, j)) {
       const T* th = tt_hist;
       gx += lv[VX * NSP + o] * g.dt * (dxf<NN>(g, th + TXX * NSP, o) / g.dx + dzb<NN>(g, th + TXZ * NSP, o) / g.dz);
@@ -1436,6 +1492,8 @@ __global__ void adj_t_abl(Geo<T> g, const T* __restrict__ cf, const T* __restric
 // ABL: stress free-surface adjoint in place, one thread per column.
 template <typename T>
 __global__ void adj_tfs_abl(Geo<T> g, T* lt) {
+  griddep_wait();
+  griddep_launch_dependents();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= g.L.nxp) return;
   const int s = blockIdx.y, h = g.h;
@@ -1544,14 +1602,12 @@ ECarve ecarve(const adfwi_elastic_plan* p, bool grad, int K) {
   const int64_t pl = p->L.plane * p->elem, ns = p->d.ns;
   int64_t o = 0;
   auto take = [&](int64_t b) { int64_t at = o; o += al256(b); return at; };
-  const int nsplit = p->d.pml ? 10 : 3;  // fields updated in place (split stresses+velocities | stresses)
   c.coef = take(ncoef(p) * pl);
-  c.st = take((int64_t)(p->d.pml ? 10 : 3) * ns * pl);  // PML: 6 split stresses + 4 split velocities
-  c.tt = take(3 * ns * pl);                               // stress totals (PML) | unused (ABL)
-  c.vtmp = take(2 * ns * pl);                             // velocity totals / ABL velocities
+  c.st = take((int64_t)(p->d.pml ? 10 : 0) * ns * pl);  // PML: 6 split stresses + 4 split velocities
+  c.tt = take(3 * ns * pl);                               // stress totals
+  c.vtmp = take(2 * ns * pl);                             // velocity totals
   c.srcm = take(ns * 3 * p->elem);
   c.tab = take((int64_t)p->tab.size() * 4);
-  (void)nsplit;
   if (grad) {
     const bool full = K >= p->d.nt;
     const int nseg = (p->d.nt + K - 1) / K;
@@ -1564,12 +1620,12 @@ ECarve ecarve(const adfwi_elastic_plan* p, bool grad, int K) {
     // lambda of the split stresses (6) and of the split velocities (4), twice each (a reverse
     // step reads one copy and writes the other)
     c.lst = take((int64_t)(p->d.pml ? 20 : 3) * ns * pl);
-    c.lt = take(3 * ns * pl);
+    c.lt = take((p->d.pml ? 3 : 0) * ns * pl);
     c.lv = take(2 * ns * pl);
     c.lv2 = take(2 * ns * pl);
-    // adjoint sources of the absorbing-layer step transposes (8 planes per shot; the PML kernels
-    // form theirs in shared memory)
-    c.qsrc = take(p->d.pml ? 0 : 8 * ns * pl);
+    // adjoint sources of the absorbing-layer step transposes (8 + 4 planes per shot; the PML
+    // kernels form theirs in shared memory)
+    c.qsrc = take(p->d.pml ? 0 : 12 * ns * pl);
     c.gc = take(8 * pl * egroups(p));
   }
   c.total = o;
@@ -1662,39 +1718,34 @@ int esetup(const adfwi_elastic_plan* p, unsigned char* ws, const ECarve& c, cons
   return kOk;
 }
 
-// One forward step. vin: velocity totals at the start of the step; vout: where the new
-// totals go; tt: where the stress totals go (PML). ABL keeps v in vin (= vout) in place.
+// One forward step. vin, tprev: velocity and stress totals at the start of the step; vout, tt:
+// where the new totals go (the same memory when they advance in place). rec: records, or null: the
+// velocity records of the step before and the stress records of this one are taken.
+// Programmatically serialised launches: each kernel waits for the previous one's data.
 template <typename T, int NN>
 void estep(const adfwi_elastic_plan* p, const el::Geo<T>& g, int it, const T* cf, const T* wav, T* st, T* tt,
-           const T* tprev, const T* vin, T* vout, cudaStream_t s) {
-  const dim3 gc = cells_grid(p, p->d.ns), b(el::kTileThreads);
+           const T* tprev, T* vin, T* vout, T* rec, cudaStream_t s) {
+  const dim3 b(el::kTileThreads);
   const int64_t NSP = (int64_t)p->d.ns * p->L.plane;
+  const int shots = p->d.pml ? el::kCellShots : 1;
+  const dim3 gc = cells_grid(p, (p->d.ns + shots - 1) / shots);
+  const unsigned rb = rec != nullptr && p->d.nr > 0 ? (p->d.nr + el::kTileThreads - 1) / el::kTileThreads : 0;
+  const dim3 gs(gc.x + (it > 0 ? rb : 0), gc.y), gv(gc.x + rb, gc.y);
   if (p->d.pml) {
-    T* ts = st;
-    T* vs = st + 6 * NSP;
-    const dim3 gcs = cells_grid(p, (p->d.ns + el::kCellShots - 1) / el::kCellShots);
-    // programmatically serialised launches: each kernel waits for the previous one's data
-    ADFWI_LAUNCH(kElFwdStep, s,
-                 (void)launch_pdl_kernel(el::stress_pml_tot<T, NN>, gcs, b, 0, s, g, it, cf, vin, ts, tt, tprev, wav));
-    if (p->d.free_surface) {
-      const dim3 gfs((unsigned)((p->nxp + 127) / 128), p->d.ns, 3);
-      ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::stress_fs_rows_pml<T>, gfs, dim3(128), 0, s, g, ts, tt));
-    }
-    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_pml_tot<T, NN>, gcs, b, 0, s, g, cf, tt, vs, vout, vin));
-    if (p->d.free_surface) {
-      const dim3 gfs((unsigned)((p->nxp + 127) / 128), p->d.ns, 2);
-      ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_fs_rows_pml<T>, gfs, dim3(128), 0, s, g, vs, vout));
-    }
+    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::stress_pml_tot<T, NN>, gs, b, 0, s, g, it, cf, vin, st, tt,
+                                                        tprev, wav, rec));
+    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_pml_tot<T, NN>, gv, b, 0, s, g, it, cf, (const T*)tt,
+                                                        st + 6 * NSP, vout, (const T*)vin, rec));
   } else {
-    // ABL: stresses live in `tt`, velocities in place in vin (== vout)
-    T* v = vout;
-    if (vin != vout) cudaMemcpyAsync(v, vin, 2 * NSP * sizeof(T), cudaMemcpyDeviceToDevice, s);
     const dim3 gcol((unsigned)((p->nxp + 127) / 128), p->d.ns);
-    ADFWI_LAUNCH(kElFwdStep, s, (el::stress_abl<T, NN><<<gc, b, 0, s>>>(g, it, cf, v, tt, wav)));
-    if (p->d.free_surface) ADFWI_LAUNCH(kElFwdStep, s, (el::stress_fs_abl<T><<<gcol, 128, 0, s>>>(g, tt)));
-    ADFWI_LAUNCH(kElFwdStep, s, (el::vel_abl<T, NN><<<gc, b, 0, s>>>(g, cf, tt, v)));
-    if (p->d.free_surface) ADFWI_LAUNCH(kElFwdStep, s, (el::vel_fs_abl<T><<<gcol, 128, 0, s>>>(g, v)));
-    ADFWI_LAUNCH(kElFwdStep, s, (el::damp_v<T><<<gc, b, 0, s>>>(g, cf, v)));
+    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::stress_abl<T, NN>, gs, b, 0, s, g, it, cf, (const T*)vin, tt,
+                                                        tprev, wav, rec));
+    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_abl<T, NN>, gv, b, 0, s, g, it, cf, (const T*)tt, vout,
+                                                        (const T*)vin, rec));
+    if (p->d.free_surface) {
+      ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_fs_abl<T>, gcol, dim3(128), 0, s, g, vout));
+      ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::damp_v<T>, gc, b, 0, s, g, cf, vout));
+    }
   }
 }
 
@@ -1746,7 +1797,7 @@ int eforward(const adfwi_elastic_plan* p, const void* const* coef, const int32_t
   if (full) {
     // the histories double as the state and are read with their halos
     int rc0 = zero_frames<T>(hv, (int64_t)K * 2 * p->d.ns, p->L, s);
-    if (!rc0 && p->d.pml) rc0 = zero_frames<T>(ht, (int64_t)K * 3 * p->d.ns, p->L, s);
+    if (!rc0) rc0 = zero_frames<T>(ht, (int64_t)K * 3 * p->d.ns, p->L, s);
     if (rc0) return rc0;
   }
   size_t chunk = 0;
@@ -1768,18 +1819,14 @@ int eforward(const adfwi_elastic_plan* p, const void* const* coef, const int32_t
       vout = it + 1 < nt ? hv + (int64_t)(it + 1) * 2 * NSP : v0;
       if (it == 0) ADFWI_CUDA_TRY(cudaMemsetAsync(hv, 0, 2 * NSP * sizeof(T), s));
       if (it == 0) vin = hv;
-      tt = p->d.pml ? ht + (int64_t)it * 3 * NSP : tt0;
-      if (p->d.pml && it > 0) tprev = ht + (int64_t)(it - 1) * 3 * NSP;
+      tt = ht + (int64_t)it * 3 * NSP;
+      if (it > 0) tprev = ht + (int64_t)(it - 1) * 3 * NSP;
     }
-    estep<T, NN>(p, g, it, cf, wav, stt, tt, tprev, vin, vout, s);
-    if (full && !p->d.pml) {
-      // ABL: stresses evolve in tt0; keep a copy of this step's stresses for the adjoint
-      ADFWI_CUDA_TRY(cudaMemcpyAsync(ht + (int64_t)it * 3 * NSP, tt0, 3 * NSP * sizeof(T), cudaMemcpyDeviceToDevice, s));
-    }
-    if (rec && p->d.nr > 0) {
+    estep<T, NN>(p, g, it, cf, wav, stt, tt, tprev, vin, vout, static_cast<T*>(rec), s);
+    if (rec && p->d.nr > 0 && it + 1 == nt) {
       dim3 gr((unsigned)((p->d.nr + 127) / 128), p->d.ns);
-      ADFWI_LAUNCH(kAux, s, (void)launch_pdl_kernel(el::record<T>, gr, dim3(128), 0, s, g, it, (const T*)tt, (const T*)vout,
-                                                    static_cast<T*>(rec)));
+      ADFWI_LAUNCH(kAux, s, (void)launch_pdl_kernel(el::record_v<T>, gr, dim3(128), 0, s, g, it, (const T*)vout,
+                                                    static_cast<T*>(rec), p->d.pml != 0));
     }
     if (fw && chunk < p->chunk_end.size() && it == p->chunk_end[chunk]) {
       const int64_t n = (int64_t)p->d.nz * p->d.nx;
@@ -1820,20 +1867,20 @@ int ebackward(const adfwi_elastic_plan* p, const void* wavelet, const void* grec
   const T* gr = static_cast<const T*>(grec);
   const int nsf = p->d.pml ? 20 : 3;
   ADFWI_CUDA_TRY(cudaMemsetAsync(lst, 0, nsf * NSP * sizeof(T), s));
-  ADFWI_CUDA_TRY(cudaMemsetAsync(lt, 0, 3 * NSP * sizeof(T), s));
+  if (p->d.pml) ADFWI_CUDA_TRY(cudaMemsetAsync(lt, 0, 3 * NSP * sizeof(T), s));
   ADFWI_CUDA_TRY(cudaMemsetAsync(lv, 0, 2 * NSP * sizeof(T), s));
   const int egr = egroups(p), eg = eshots_per_group(p);
   ADFWI_CUDA_TRY(cudaMemsetAsync(gcp, 0, (int64_t)egr * 8 * PL * sizeof(T), s));
   if (!p->d.pml) {
     // the source planes are read with their halos by the transposed stencils
-    int rc0 = zero_frames<T>(qsrc, (int64_t)8 * ns, p->L, s);
+    int rc0 = zero_frames<T>(qsrc, (int64_t)12 * ns, p->L, s);
     if (rc0) return rc0;
   }
   ADFWI_CUDA_TRY(cudaMemsetAsync(lv2, 0, 2 * NSP * sizeof(T), s));
   if (!full) {
     // recomputed histories are read with their halos
     int rc0 = zero_frames<T>(hv, (int64_t)K * 2 * ns, p->L, s);
-    if (!rc0 && p->d.pml) rc0 = zero_frames<T>(ht, (int64_t)K * 3 * ns, p->L, s);
+    if (!rc0) rc0 = zero_frames<T>(ht, (int64_t)K * 3 * ns, p->L, s);
     if (rc0) return rc0;
   }
   const dim3 gcs = cells_grid(p, ns), gcg = cells_grid(p, egroups(p)), b(el::kTileThreads);
@@ -1861,11 +1908,9 @@ int ebackward(const adfwi_elastic_plan* p, const void* wavelet, const void* grec
         const int k = it - t0;
         T* vin = hv + (int64_t)k * 2 * NSP;
         T* vout = k + 1 < K && it + 1 < t1 ? hv + (int64_t)(k + 1) * 2 * NSP : v0;
-        T* tt = p->d.pml ? ht + (int64_t)k * 3 * NSP : tt0;
-        const T* tprev = p->d.pml && k > 0 ? ht + (int64_t)(k - 1) * 3 * NSP : tt0;
-        if (!p->d.pml && vout != vin) ADFWI_CUDA_TRY(cudaMemcpyAsync(vout, vin, 2 * NSP * sizeof(T), cudaMemcpyDeviceToDevice, s));
-        estep<T, NN>(p, g, it, cf, wav, stt, tt, tprev, p->d.pml ? vin : vout, vout, s);
-        if (!p->d.pml) ADFWI_CUDA_TRY(cudaMemcpyAsync(ht + (int64_t)k * 3 * NSP, tt0, 3 * NSP * sizeof(T), cudaMemcpyDeviceToDevice, s));
+        T* tt = ht + (int64_t)k * 3 * NSP;
+        const T* tprev = k > 0 ? ht + (int64_t)(k - 1) * 3 * NSP : tt0;
+        estep<T, NN>(p, g, it, cf, wav, stt, tt, tprev, vin, vout, (T*)nullptr, s);
       }
     }
     for (int it = t1 - 1; it >= t0; --it) {
@@ -1890,14 +1935,18 @@ int ebackward(const adfwi_elastic_plan* p, const void* wavelet, const void* grec
         ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_v_pml<T, NN>, gcg, b, (size_t)smem_vp, s, g, cf,
                                                             (const T*)lt, (const T*)lts_in, lts_out, lv, vh, gcp, eg));
       } else {
-        if (gr) ADFWI_LAUNCH(kAux, s, (el::adj_inject<T><<<ginj, 128, 0, s>>>(g, it, gr, lst, lv, 3)));
-        ADFWI_LAUNCH(kElAdjStep, s, (el::adj_vfs_abl<T><<<gcs, b, 0, s>>>(g, cf, lv, lv2, nullptr)));
+        T* q4 = qsrc + 8 * NSP;
+        if (gr) ADFWI_LAUNCH(kAux, s, (void)launch_pdl_kernel(el::adj_inject<T>, ginj, dim3(128), 0, s, g, it, gr, lst, lv, 3));
+        ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_vfs_abl<T>, gcs, b, 0, s, g, cf, (const T*)lv, lv2, q4));
         std::swap(lv, lv2);
-        ADFWI_LAUNCH(kElAdjStep, s, (el::adj_tq<T, false><<<gcs, b, 0, s>>>(g, cf, lv, qsrc)));
-        ADFWI_LAUNCH(kElAdjStep, s, (el::adj_t_abl<T, NN><<<gcg, b, 0, s>>>(g, cf, lv, qsrc, lst, th, gcp, eg)));
-        if (p->d.free_surface) ADFWI_LAUNCH(kElAdjStep, s, (el::adj_tfs_abl<T><<<gcol, 128, 0, s>>>(g, lst)));
-        ADFWI_LAUNCH(kElAdjStep, s, (el::adj_vq<T, false><<<gcs, b, 0, s>>>(g, cf, lst, qsrc)));
-        ADFWI_LAUNCH(kElAdjStep, s, (el::adj_v<T, NN, false><<<gcg, b, smem_va, s>>>(g, cf, lst, qsrc, lv, vh, gcp, eg)));
+        ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_t_abl<T, NN>, gcg, b, 0, s, g, cf, (const T*)lv,
+                                                            (const T*)q4, lst, th, gcp, eg, qsrc));
+        if (p->d.free_surface) {
+          ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_tfs_abl<T>, gcol, dim3(128), 0, s, g, lst));
+          ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_vq<T, false>, gcs, b, 0, s, g, cf, (const T*)lst, qsrc));
+        }
+        ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_v<T, NN, false>, gcg, b, (size_t)smem_va, s, g, cf,
+                                                            (const T*)lst, (const T*)qsrc, lv, vh, gcp, eg));
       }
     }
     ADFWI_CUDA_TRY(cudaGetLastError());
