@@ -37,11 +37,9 @@ namespace el {
 __device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float rdiv(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double rdiv(double a, double b) { return __ddiv_rn(a, b); }
 
 // Field indices inside the state blocks (each field = ns consecutive planes).
 enum { TXX_X = 0, TXX_Z, TZZ_X, TZZ_Z, TXZ_X, TXZ_Z };  // split stresses (PML)
@@ -160,24 +158,14 @@ constexpr int kTileX = 32, kTileZ = 8, kTileThreads = kTileX * kTileZ;
   const int64_t o = (int64_t)s * PL + g.L.off(i, j);                                 \
   (void)NSP;
 
-// Per-cell kernels that take several shots of one cell per thread (blockIdx.y picks a block of
-// kCellShots consecutive shots): the cell's coefficients and PML factors are loaded and formed
-// once, and the shots' field loads are independent, so more of them are in flight.
-#ifndef ADFWI_EL_CELL_SHOTS
-#define ADFWI_EL_CELL_SHOTS 2
-#endif
-constexpr int kCellShots = ADFWI_EL_CELL_SHOTS;
-#define EL_CELL_SHOTS                                                                \
-  EL_TILE_IJ                                                                         \
-  const int s_lo = blockIdx.y * kCellShots;                                          \
-  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL;                            \
-  const int64_t occ = g.L.off(i, j);
-
-// x / d where d is a PML denominator 1 + dt/2 d(x): exactly x wherever d is 1 (outside the
-// absorbing frame), so the division runs only inside the frame.
+// 1 / d of a PML denominator d = 1 + dt/2 d(x): exactly 1 where d is (outside the absorbing frame),
+// so the division runs only inside the frame. Only coefficients are divided: where a wave has not
+// arrived a field is zero or subnormal, and a division of such a value takes a slow path of tens of
+// instructions (two launches of 20 shots on a 242 x 480 grid: 82 us with four divisions of fields a
+// cell, 61 with products).
 template <typename T>
-__device__ __forceinline__ T rdiv_pml(T x, T d) {
-  return d == T(1) ? x : rdiv(x, d);
+__device__ __forceinline__ T pml_inv(T d) {
+  return d == T(1) ? T(1) : T(1) / d;
 }
 
 #define EL_CELL                                                                      \
@@ -263,10 +251,69 @@ struct StagedZ {
   __device__ __forceinline__ T operator()(int ii, int jj) const { return s[(ii - i0 + 3) * kTileX + (jj - j0)]; }
 };
 
+// ---- forward kernels: a thread takes kVW consecutive columns of a row, read and written as 16-byte
+// vectors (columns start at a multiple of kVW, planes at multiples of 128 bytes with a ghost frame of
+// 4 columns, so every vector is aligned). A warp covers 32 columns of 4 rows (2 in double precision)
+// and a block of 128 threads 32 columns of 4 kVW rows.
+constexpr int kVecThreads = 128, kVecX = 32;
 template <typename T>
-__device__ __forceinline__ int tile_count(const Geo<T>& g) {
-  return ((g.L.nxp + kTileX - 1) / kTileX) * ((g.L.nzp + kTileZ - 1) / kTileZ);
+constexpr int kVW = 16 / (int)sizeof(T);
+template <typename T>
+constexpr int kVecRows = kVecThreads * kVW<T> / kVecX;
+template <typename T>
+struct Vec {
+  T v[kVW<T>];
+};
+template <typename T>
+__device__ __forceinline__ Vec<T> ldv(const T* p) {
+  Vec<T> r;
+  *reinterpret_cast<int4*>(r.v) = *reinterpret_cast<const int4*>(p);
+  return r;
 }
+template <typename T>
+__device__ __forceinline__ void stv(T* p, const Vec<T>& x) {
+  *reinterpret_cast<int4*>(p) = *reinterpret_cast<const int4*>(x.v);
+}
+// The vector at p of a row with the whole vectors that hold its NN neighbours on each side.
+template <typename T, int NN>
+struct Row {
+  static constexpr int H = (NN + kVW<T> - 1) / kVW<T> * kVW<T>;
+  T v[kVW<T> + 2 * H];
+  __device__ __forceinline__ explicit Row(const T* p) {
+#pragma unroll
+    for (int k = 0; k < kVW<T> + 2 * H; k += kVW<T>)
+      *reinterpret_cast<int4*>(v + k) = *reinterpret_cast<const int4*>(p - H + k);
+  }
+  __device__ __forceinline__ T operator()(int k) const { return v[H + k]; }
+};
+// Half-cell difference times `scale` (dt / dx or dt / dz; elastic_kernels.py:66-108): `at(m)` is the
+// value m cells from the lower of the two middle ones. Differences, coefficient products and sums
+// of the forward kernels are fused multiply-adds, and one sum is added to a total.
+template <typename T>
+struct Fd {
+  T f0, f1, f2;
+  __device__ __forceinline__ Fd(const Geo<T>& g, T scale) : f0(g.f0 * scale), f1(g.f1 * scale), f2(g.f2 * scale) {}
+  template <int NN, typename A>
+  __device__ __forceinline__ T diff(const A& at) const {
+    T r = f0 * (at(1) - at(0)) + f1 * (at(2) - at(-1));
+    if (NN == 3) r += f2 * (at(3) - at(-2));
+    return r;
+  }
+};
+template <typename T>
+__host__ __device__ __forceinline__ int vec_tiles(const Layout& L) {
+  return ((L.nxp + kVecX - 1) / kVecX) * ((L.nzp + kVecRows<T> - 1) / kVecRows<T>);
+}
+// this thread's row i and first column j
+#define EL_VEC_IJ                                                               \
+  constexpr int W = kVW<T>;                                                     \
+  const int tiles_x_ = (g.L.nxp + kVecX - 1) / kVecX;                           \
+  const int ti_ = (int)blockIdx.x / tiles_x_, tj_ = (int)blockIdx.x - ti_ * tiles_x_; \
+  const int i = ti_ * kVecRows<T> + (int)threadIdx.x / (kVecX / W);             \
+  const int j = tj_ * kVecX + (int)threadIdx.x % (kVecX / W) * W;               \
+  if (i >= g.L.nzp || j >= g.L.nxp) return;                                     \
+  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL, P = g.L.pitch;        \
+  const int64_t occ = g.L.off(i, j);
 
 // The velocity rows above a free surface (elastic_kernels.py:395-402) from the totals of rows h-1
 // and h: vz[h-3] = vz[h-2] = vz[h-1] and vx[h-2] from vz[h-1] and vx[h], on columns J; zero
@@ -289,7 +336,7 @@ __device__ __forceinline__ T vel_above(const Geo<T>& g, const T* vx, const T* vz
 // c0: its index in the record array; rows_above: the velocity rows above the free surface are not
 // in `src` (a receiver there reads vel_above).
 template <typename T>
-__device__ __forceinline__ void record_block(const Geo<T>& g, int tiles, int shots, int it, const T* src, int ncomp, int c0,
+__device__ __forceinline__ void record_block(const Geo<T>& g, int tiles, int it, const T* src, int ncomp, int c0,
                                              T* rec, bool rows_above = false) {
   const int r = ((int)blockIdx.x - tiles) * (int)blockDim.x + (int)threadIdx.x;
   if (r >= g.nr) return;
@@ -297,75 +344,68 @@ __device__ __forceinline__ void record_block(const Geo<T>& g, int tiles, int sho
   const int i = g.rcv_z[r], j = g.rcv_x[r];
   const int64_t oc = g.L.off(i, j);
   rows_above = rows_above && g.fsurf && i < g.h - 1;
-  for (int q = 0; q < shots; ++q) {
-    const int s = (int)blockIdx.y * shots + q;
-    if (s >= g.ns) break;
-    const int64_t o = (int64_t)s * g.L.plane + oc, e = ((int64_t)s * g.nt + it) * g.nr + r;
-    if (rows_above) {
-      const T *vx = src + o - oc, *vz = vx + NSP;
-      rec[c0 * RS + e] = vel_above(g, vx, vz, true, i, j);
-      rec[(c0 + 1) * RS + e] = vel_above(g, vx, vz, false, i, j);
-      continue;
-    }
-    for (int c = 0; c < ncomp; ++c) rec[(c0 + c) * RS + e] = src[c * NSP + o];
-  }
-}
-template <int NN, typename T>
-__device__ __forceinline__ T dzb_above(const Geo<T>& g, const T* vx, const T* vz, bool x, int i, int j) {
-  auto a = [&](int r) { return vel_above(g, vx, vz, x, r, j); };
-  T r = rmul(g.f0, rsub(a(i), a(i - 1)));
-  r = radd(r, rmul(g.f1, rsub(a(i + 1), a(i - 2))));
-  if (NN == 3) r = radd(r, rmul(g.f2, rsub(a(i + 2), a(i - 3))));
-  return r;
-}
-template <int NN, typename T>
-__device__ __forceinline__ T dzf_above(const Geo<T>& g, const T* vx, const T* vz, bool x, int i, int j) {
-  auto a = [&](int r) { return vel_above(g, vx, vz, x, r, j); };
-  T r = rmul(g.f0, rsub(a(i + 1), a(i)));
-  r = radd(r, rmul(g.f1, rsub(a(i + 2), a(i - 1))));
-  if (NN == 3) r = radd(r, rmul(g.f2, rsub(a(i + 3), a(i - 2))));
-  return r;
-}
-
-// Stress totals of a cell (offset o) with the free-surface rows h-3 .. h-1 (elastic_kernels.py:
-// 375-384): tzz[h-1] = 0, tzz[h-2] = -tzz[h], txz[h-2] = -txz[h-1], txz[h-3] = -txz[h]. The cells of
-// rows h-1 and h write the mirrored values; the cells they mirror to leave theirs out.
-template <typename T>
-__device__ __forceinline__ void store_stress(const Geo<T>& g, int i, int64_t o, int64_t NSP, T xx, T zz, T xz, T* tt) {
-  const int64_t P = g.L.pitch;
-  const int h = g.h;
-  tt[TXX * NSP + o] = xx;
-  if (!g.fsurf || i > h || i < h - 3) {
-    tt[TZZ * NSP + o] = zz;
-    tt[TXZ * NSP + o] = xz;
+  const int s = blockIdx.y;
+  const int64_t o = (int64_t)s * g.L.plane + oc, e = ((int64_t)s * g.nt + it) * g.nr + r;
+  if (rows_above) {
+    const T *vx = src + o - oc, *vz = vx + NSP;
+    rec[c0 * RS + e] = vel_above(g, vx, vz, true, i, j);
+    rec[(c0 + 1) * RS + e] = vel_above(g, vx, vz, false, i, j);
     return;
   }
-  if (i == h - 1) zz = T(0);
-  if (i != h - 2) tt[TZZ * NSP + o] = zz;
-  if (i >= h - 1) tt[TXZ * NSP + o] = xz;
-  if (i == h - 1) tt[TXZ * NSP + o - P] = -xz;
+  for (int c = 0; c < ncomp; ++c) rec[(c0 + c) * RS + e] = src[c * NSP + o];
+}
+
+// Stress totals of a vector (offset o, row i) with the free-surface rows h-3 .. h-1
+// (elastic_kernels.py:375-384, 738-742): tzz[h-1] = 0, tzz[h-2] = -tzz[h], txz[h-2] = -txz[h-1],
+// txz[h-3] = -txz[h]. Rows h-1 and h write the mirrored values; the rows they mirror to leave
+// theirs out.
+template <typename T>
+__device__ __forceinline__ void store_stress(const Geo<T>& g, int i, int64_t o, int64_t NSP, const Vec<T>& xx, Vec<T> zz,
+                                             const Vec<T>& xz, T* tt) {
+  const int64_t P = g.L.pitch;
+  const int h = g.h;
+  stv(tt + TXX * NSP + o, xx);
+  if (!g.fsurf || i > h || i < h - 3) {
+    stv(tt + TZZ * NSP + o, zz);
+    stv(tt + TXZ * NSP + o, xz);
+    return;
+  }
+  Vec<T> nz, nx;
+#pragma unroll
+  for (int e = 0; e < kVW<T>; ++e) {
+    if (i == h - 1) zz.v[e] = T(0);
+    nz.v[e] = -zz.v[e];
+    nx.v[e] = -xz.v[e];
+  }
+  if (i != h - 2) stv(tt + TZZ * NSP + o, zz);
+  if (i >= h - 1) stv(tt + TXZ * NSP + o, xz);
+  if (i == h - 1) stv(tt + TXZ * NSP + o - P, nx);
   if (i == h) {
-    tt[TZZ * NSP + o - 2 * P] = -zz;
-    tt[TXZ * NSP + o - 3 * P] = -xz;
+    stv(tt + TZZ * NSP + o - 2 * P, nz);
+    stv(tt + TXZ * NSP + o - 3 * P, nx);
   }
 }
 
-// ======================================================================= forward, PML
-// Split-field update of a cell and its totals in one pass (elastic_kernels.py:351-402), two launches
-// per step: the stress rows that mirror others at the free surface are written by the cells they
-// mirror, the velocity rows above it by the next stress update, which reads them as vel_above.
-// With a pass for each kind of surface rows and one for the records, five launches, a step of one
-// shot on a 122 x 140 grid took 18.9 us; it takes 15.2.
-template <typename T>
-__device__ __forceinline__ bool vel_fs_row(const Geo<T>& g, int i, int j) {
-  return g.fsurf && j >= g.jlo && j <= g.jhi && (i == g.h - 2 || i == g.h - 3);
-}
-
-// Cells that keep split fields: inside the update region, where a PML factor differs from 1,
-// and in the surface rows that mirror others or are mirrored (h-3 .. h) plus one. Every
-// other cell of the update region advances its totals directly: there the split update is
-// x' = x + a, z' = z + b, total = x' + z' (the factors are exactly 1), so the unsplit
-// t' = (t + a) + b differs only by one rounding of the sum and moves half the bytes.
+// ======================================================================= forward
+// Split-field update with PML (elastic_kernels.py:351-402) or unsplit update with an absorbing
+// layer (:733-774), fields and totals in one pass, two launches per step: the stress rows that
+// mirror others at the free surface are written by the rows they mirror; with PML the velocity rows
+// above it are formed and written by the next stress update (with an absorbing layer they are inputs
+// of the damping and take two small launches).
+//
+// What bounds them is latency: a thread's chain of loads from L2 and the launch boundary, not L2 or
+// DRAM bandwidth (30 % of either) nor issue slots (32 %). So a thread takes four columns as 16-byte
+// vectors with all its loads in flight at once (160 registers, three blocks per SM; four blocks with
+// spills, two shots per thread and 64-column tiles measured 3 to 20 % slower), and reads what the
+// launch before does not write ahead of that launch's end. 300 steps of one shot on a 122 x 140 grid:
+// 4.56 -> 3.47 ms; 200 steps of 20 shots on a 242 x 480 grid: 16.3 -> 12.7 ms, against one cell and
+// two shots per thread with scalar loads and exact divisions by dx.
+//
+// Cells that keep split fields: outside the update region, where a PML factor differs from 1,
+// and in the surface rows that mirror others or are mirrored (h-3 .. h) plus one. Every other cell
+// advances its totals directly: there the split update is x' = x + a, z' = z + b, total = x' + z'
+// (the factors are exactly 1), so the unsplit t' = (t + a) + b differs only by one rounding of the
+// sum and moves half the bytes.
 template <typename T>
 __device__ __forceinline__ bool keeps_split(const Geo<T>& g, int i, T bcx, T bcz) {
   return bcx != T(0) || bcz != T(0) || (g.fsurf && i <= g.h + 1);
@@ -373,251 +413,258 @@ __device__ __forceinline__ bool keeps_split(const Geo<T>& g, int i, T bcx, T bcz
 
 // tprev: stress totals at the start of the step (tt itself when the totals advance in place);
 // tt: where the new totals go; rec: the velocity records of step it - 1 are taken (null: none).
-template <typename T, int NN>
-__global__ void stress_pml_tot(Geo<T> g, int it, const T* __restrict__ cf, T* __restrict__ v, T* __restrict__ ts, T* tt,
-                               const T* tprev, const T* __restrict__ wav, T* __restrict__ rec) {
-  griddep_wait();  // launched with programmatic serialisation in the time loops
-  griddep_launch_dependents();
-  if (const int tiles = tile_count(g); (int)blockIdx.x >= tiles) {
-    record_block(g, tiles, kCellShots, it - 1, (const T*)v, 2, 3, rec, true);
+template <typename T, int NN, bool PML>
+__global__ void __launch_bounds__(kVecThreads, 3)
+    stress_step(Geo<T> g, int it, const T* __restrict__ cf, T* __restrict__ v, T* __restrict__ ts, T* tt, const T* tprev,
+                const T* __restrict__ wav, T* __restrict__ rec) {
+  if (const int tiles = vec_tiles<T>(g.L); (int)blockIdx.x >= tiles) {
+    griddep_wait();
+    griddep_launch_dependents();
+    record_block(g, tiles, it - 1, (const T*)v, 2, 3, rec, PML);
     return;
   }
-  EL_CELL_SHOTS
-  const bool above = g.fsurf && i <= g.h + NN - 2;  // the vertical differences reach rows above the surface
-  const bool inside = in_I(g, i, j);
-  bool split = true;
-  T pxn = T(0), pzn = T(0), pxi = T(0), pzi = T(0);
-  T c11 = T(0), c13 = T(0), c15 = T(0), c33 = T(0), c35 = T(0), c55 = T(0);
-  if (inside) {
-    const T bcx = cf[BCX * PL + occ], bcz = cf[BCZ * PL + occ];
-    split = keeps_split(g, i, bcx, bcz);
-    const T pxd = radd(T(1), rmul(g.hdt, bcx)), pzd = radd(T(1), rmul(g.hdt, bcz));
-    pxn = rsub(T(1), rmul(g.hdt, bcx));
-    pzn = rsub(T(1), rmul(g.hdt, bcz));
-    pxi = rdiv_pml(T(1), pxd);
-    pzi = rdiv_pml(T(1), pzd);
-    c11 = cf[C11 * PL + occ];
-    c13 = cf[C13 * PL + occ];
-    c15 = cf[C15 * PL + occ];
-    c33 = cf[C33 * PL + occ];
-    c35 = cf[C35 * PL + occ];
-    c55 = cf[C55 * PL + occ];
+  EL_VEC_IJ
+  const int s = blockIdx.y;
+  const int64_t so = (int64_t)s * PL, o = so + occ;
+  const int src_row = g.src_z[s], src_col = g.src_x[s];
+  // What the launch before this one (the velocity update) does not write is read ahead of its end.
+  Vec<T> c[6], bcx, bcz, t[3], px[3], pz[3];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) c[k] = ldv(cf + (C11 + k) * PL + occ);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) t[k] = ldv(tprev + k * NSP + o);
+  bool in[W], sp[W], any = false;
+  if (PML) {
+    bcx = ldv(cf + BCX * PL + occ);
+    bcz = ldv(cf + BCZ * PL + occ);
   }
 #pragma unroll
-  for (int q = 0; q < kCellShots; ++q) {
-    const int s = s_lo + q;
-    if (s >= g.ns) break;
-    const int64_t o = (int64_t)s * PL + occ;
-    if (!split) {
-      const T* vx = v;
-      const T* vz = v + NSP;
-      const T dxbm_vx = dxb<NN>(g, vx, o), dxbm_vz = dxb<NN>(g, vz, o);
-      const T dzbm_vx = dzb<NN>(g, vx, o), dzbm_vz = dzb<NN>(g, vz, o);
-      const T dxfm_vx = dxf<NN>(g, vx, o), dzfm_vx = dzf<NN>(g, vx, o);
-      const T dxfm_vz = dxf<NN>(g, vz, o), dzfm_vz = dzf<NN>(g, vz, o);
-      T xx = radd(radd(tprev[TXX * NSP + o], rmul(g.dt_dx, radd(rmul(c11, dxbm_vx), rmul(c15, dxbm_vz)))),
-                  rmul(g.dt_dz, radd(rmul(c15, dzbm_vx), rmul(c13, dzbm_vz))));
-      T zz = radd(radd(tprev[TZZ * NSP + o], rmul(g.dt_dx, radd(rmul(c13, dxbm_vx), rmul(c35, dxbm_vz)))),
-                  rmul(g.dt_dz, radd(rmul(c35, dzbm_vx), rmul(c33, dzbm_vz))));
-      T xz = radd(radd(tprev[TXZ * NSP + o], rmul(g.dt_dx, radd(rmul(c15, dxfm_vx), rmul(c55, dxfm_vz)))),
-                  rmul(g.dt_dz, radd(rmul(c55, dzfm_vx), rmul(c35, dzfm_vz))));
-      if (i == g.src_z[s] && j == g.src_x[s]) {  // -MT/2 w on both split parts: twice on the total
-        const T w = wav[(int64_t)s * g.nt + it];
-        xx = radd(xx, rmul(T(2), rmul(g.src_m[3 * s + 0], w)));
-        zz = radd(zz, rmul(T(2), rmul(g.src_m[3 * s + 1], w)));
-        xz = radd(xz, rmul(T(2), rmul(g.src_m[3 * s + 2], w)));
+  for (int e = 0; e < W; ++e) {
+    in[e] = in_I(g, i, j + e);
+    sp[e] = PML && (!in[e] || keeps_split(g, i, bcx.v[e], bcz.v[e]));
+    any = any || sp[e];
+  }
+  griddep_wait();  // launched with programmatic serialisation in the time loops
+  griddep_launch_dependents();
+  {
+    const Row<T, NN> x(v + VX * NSP + o), z(v + VZ * NSP + o);
+    Vec<T> rx[2 * NN + 1], rz[2 * NN + 1];  // rows i - NN .. i + NN
+#pragma unroll
+    for (int k = 0; k <= 2 * NN; ++k)
+      if (k != NN) {
+        rx[k] = ldv(v + VX * NSP + o + (k - NN) * P);
+        rz[k] = ldv(v + VZ * NSP + o + (k - NN) * P);
       }
-      tt[TXX * NSP + o] = xx;
-      tt[TZZ * NSP + o] = zz;
-      tt[TXZ * NSP + o] = xz;
-      continue;
+    if (any) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        px[k] = ldv(ts + (2 * k) * NSP + o);
+        pz[k] = ldv(ts + (2 * k + 1) * NSP + o);
+      }
     }
-    T sp[6];
+    // source of the step on the cell of this vector that holds it
+    T w[3] = {T(0), T(0), T(0)};
+    const int se = i == src_row ? src_col - j : -1;
+    const bool has_src = se >= 0 && se < W;
+    if (has_src) {
+      const T wv = wav[(int64_t)s * g.nt + it];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) sp[k] = ts[k * NSP + o];
-    if (inside) {
-      const T* vx = v;
-      const T* vz = v + NSP;
-      const T dxbm_vx = dxb<NN>(g, vx, o), dxbm_vz = dxb<NN>(g, vz, o);
-      const T dxfm_vx = dxf<NN>(g, vx, o), dxfm_vz = dxf<NN>(g, vz, o);
-      T dzbm_vx, dzbm_vz, dzfm_vx, dzfm_vz;
-      if (above) {
-        const T *ux = vx + (int64_t)s * PL, *uz = vz + (int64_t)s * PL;
-        dzbm_vx = dzb_above<NN>(g, ux, uz, true, i, j);
-        dzbm_vz = dzb_above<NN>(g, ux, uz, false, i, j);
-        dzfm_vx = dzf_above<NN>(g, ux, uz, true, i, j);
-        dzfm_vz = dzf_above<NN>(g, ux, uz, false, i, j);
-        if (i == g.h - 1) {  // the rows above, for whoever reads the velocities later
+      for (int k = 0; k < 3; ++k) w[k] = rmul(g.src_m[3 * s + k], wv);
+    }
+    if (PML && g.fsurf && i <= g.h + NN - 2) {  // rows above the surface are read: form them
+      Vec<T> ax, az;
 #pragma unroll
-          for (int r = 2; r <= 3; ++r) {
-            v[VX * NSP + o - (r - 1) * (int64_t)g.L.pitch] = vel_above(g, ux, uz, true, g.h - r, j);
-            v[VZ * NSP + o - (r - 1) * (int64_t)g.L.pitch] = vel_above(g, ux, uz, false, g.h - r, j);
-          }
+      for (int e = 0; e < W; ++e) {
+        ax.v[e] = vel_above(g, v + VX * NSP + so, v + VZ * NSP + so, true, g.h - 2, j + e);
+        az.v[e] = vel_above(g, v + VX * NSP + so, v + VZ * NSP + so, false, g.h - 2, j + e);
+      }
+#pragma unroll
+      for (int k = 0; k < NN; ++k) {
+        const int r = i + k - NN;
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          if (r < g.h - 1) rx[k].v[e] = r == g.h - 2 ? ax.v[e] : T(0);
+          if (r < g.h - 1) rz[k].v[e] = r >= g.h - 3 ? az.v[e] : T(0);
         }
-      } else {
-        dzbm_vx = dzb<NN>(g, vx, o);
-        dzbm_vz = dzb<NN>(g, vz, o);
-        dzfm_vx = dzf<NN>(g, vx, o);
-        dzfm_vz = dzf<NN>(g, vz, o);
       }
-      sp[TXX_X] = rmul(radd(rmul(pxn, sp[TXX_X]), rmul(g.dt_dx, radd(rmul(c11, dxbm_vx), rmul(c15, dxbm_vz)))), pxi);
-      sp[TXX_Z] = rmul(radd(rmul(pzn, sp[TXX_Z]), rmul(g.dt_dz, radd(rmul(c15, dzbm_vx), rmul(c13, dzbm_vz)))), pzi);
-      sp[TZZ_X] = rmul(radd(rmul(pxn, sp[TZZ_X]), rmul(g.dt_dx, radd(rmul(c13, dxbm_vx), rmul(c35, dxbm_vz)))), pxi);
-      sp[TZZ_Z] = rmul(radd(rmul(pzn, sp[TZZ_Z]), rmul(g.dt_dz, radd(rmul(c35, dzbm_vx), rmul(c33, dzbm_vz)))), pzi);
-      sp[TXZ_X] = rmul(radd(rmul(pxn, sp[TXZ_X]), rmul(g.dt_dx, radd(rmul(c15, dxfm_vx), rmul(c55, dxfm_vz)))), pxi);
-      sp[TXZ_Z] = rmul(radd(rmul(pzn, sp[TXZ_Z]), rmul(g.dt_dz, radd(rmul(c55, dzfm_vx), rmul(c35, dzfm_vz)))), pzi);
-    }
-    if (i == g.src_z[s] && j == g.src_x[s]) {
-      const T w = wav[(int64_t)s * g.nt + it];
-      const T axx = rmul(g.src_m[3 * s + 0], w), azz = rmul(g.src_m[3 * s + 1], w), axz = rmul(g.src_m[3 * s + 2], w);
-      sp[TXX_X] = radd(sp[TXX_X], axx);
-      sp[TXX_Z] = radd(sp[TXX_Z], axx);
-      sp[TZZ_X] = radd(sp[TZZ_X], azz);
-      sp[TZZ_Z] = radd(sp[TZZ_Z], azz);
-      sp[TXZ_X] = radd(sp[TXZ_X], axz);
-      sp[TXZ_Z] = radd(sp[TXZ_Z], axz);
-    }
+      if (i == g.h - 1) {  // and kept for whoever reads the velocities later
+        stv(v + VX * NSP + o - P, ax);
+        stv(v + VZ * NSP + o - P, az);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) ts[k * NSP + o] = sp[k];
-    store_stress(g, i, o, NSP, radd(sp[TXX_X], sp[TXX_Z]), radd(sp[TZZ_X], sp[TZZ_Z]), radd(sp[TXZ_X], sp[TXZ_Z]), tt);
+        for (int e = 0; e < W; ++e) ax.v[e] = T(0);
+        stv(v + VX * NSP + o - 2 * P, ax);
+        stv(v + VZ * NSP + o - 2 * P, az);
+      }
+    }
+    const Fd<T> fx(g, g.dt_dx), fz(g, g.dt_dz);
+    Vec<T> a[6];  // the increments of the split parts xx_x, xx_z, zz_x, zz_z, xz_x, xz_z
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      auto zx = [&](int m) { return m == 0 ? x(e) : rx[NN + m].v[e]; };
+      auto zz = [&](int m) { return m == 0 ? z(e) : rz[NN + m].v[e]; };
+      const T dxbm_vx = fx.template diff<NN>([&](int m) { return x(e - 1 + m); });
+      const T dxbm_vz = fx.template diff<NN>([&](int m) { return z(e - 1 + m); });
+      const T dzbm_vx = fz.template diff<NN>([&](int m) { return zx(m - 1); });
+      const T dzbm_vz = fz.template diff<NN>([&](int m) { return zz(m - 1); });
+      const T dxfm_vx = fx.template diff<NN>([&](int m) { return x(e + m); });
+      const T dxfm_vz = fx.template diff<NN>([&](int m) { return z(e + m); });
+      const T dzfm_vx = fz.template diff<NN>(zx);
+      const T dzfm_vz = fz.template diff<NN>(zz);
+      const T c11 = c[0].v[e], c13 = c[1].v[e], c15 = c[2].v[e], c33 = c[3].v[e], c35 = c[4].v[e], c55 = c[5].v[e];
+      a[0].v[e] = c11 * dxbm_vx + c15 * dxbm_vz;
+      a[1].v[e] = c15 * dzbm_vx + c13 * dzbm_vz;
+      a[2].v[e] = c13 * dxbm_vx + c35 * dxbm_vz;
+      a[3].v[e] = c35 * dzbm_vx + c33 * dzbm_vz;
+      a[4].v[e] = c15 * dxfm_vx + c55 * dxfm_vz;
+      a[5].v[e] = c55 * dzfm_vx + c35 * dzfm_vz;
+    }
+    if (!PML) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          if (in[e]) t[k].v[e] += a[2 * k].v[e] + a[2 * k + 1].v[e];
+          if (has_src && e == se) t[k].v[e] += w[k];
+        }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int e = 0; e < W; ++e)
+          if (!sp[e]) {
+            t[k].v[e] += a[2 * k].v[e] + a[2 * k + 1].v[e];
+            if (has_src && e == se) t[k].v[e] += T(2) * w[k];  // -MT/2 w on both split parts
+          }
+      if (any) {
+        T pxn[W], pxi[W], pzn[W], pzi[W];
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          pxn[e] = T(1) - g.hdt * bcx.v[e];
+          pzn[e] = T(1) - g.hdt * bcz.v[e];
+          pxi[e] = pml_inv(T(1) + g.hdt * bcx.v[e]);
+          pzi[e] = pml_inv(T(1) + g.hdt * bcz.v[e]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+#pragma unroll
+          for (int e = 0; e < W; ++e)
+            if (sp[e]) {
+              if (in[e]) {
+                px[k].v[e] = (pxn[e] * px[k].v[e] + a[2 * k].v[e]) * pxi[e];
+                pz[k].v[e] = (pzn[e] * pz[k].v[e] + a[2 * k + 1].v[e]) * pzi[e];
+              }
+              if (has_src && e == se) {
+                px[k].v[e] += w[k];
+                pz[k].v[e] += w[k];
+              }
+              t[k].v[e] = px[k].v[e] + pz[k].v[e];
+            }
+          stv(ts + (2 * k) * NSP + o, px[k]);
+          stv(ts + (2 * k + 1) * NSP + o, pz[k]);
+        }
+      }
+    }
+    store_stress(g, i, o, NSP, t[TXX], t[TZZ], t[TXZ], tt);
   }
 }
 
 // vprev: velocity totals at the start of the step (v itself when they advance in place); rec: the
-// stress records of step it are taken (null: none).
-template <typename T, int NN>
-__global__ void vel_pml_tot(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ tt, T* __restrict__ vs,
-                            T* v, const T* vprev, T* __restrict__ rec) {
+// stress records of step it are taken (null: none). Without a free surface the absorbing layer's
+// damping is applied here; with one it follows the surface rows.
+template <typename T, int NN, bool PML>
+__global__ void __launch_bounds__(kVecThreads, 3)
+    vel_step(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ tt, T* __restrict__ vs, T* v,
+             const T* vprev, T* __restrict__ rec) {
+  if (const int tiles = vec_tiles<T>(g.L); (int)blockIdx.x >= tiles) {
+    griddep_wait();
+    griddep_launch_dependents();
+    record_block(g, tiles, it, tt, 3, 0, rec);
+    return;
+  }
+  EL_VEC_IJ
+  const int64_t o = (int64_t)blockIdx.y * PL + occ;
+  // What the launch before this one (the stress update) does not write is read ahead of its end.
+  const Vec<T> bx = ldv(cf + BX * PL + occ), bz = ldv(cf + BZ * PL + occ);
+  Vec<T> nx = ldv(vprev + VX * NSP + o), nz = ldv(vprev + VZ * NSP + o);
+  Vec<T> bcx, bcz, damp, f[4];
+  if (PML) {
+    bcx = ldv(cf + BCX * PL + occ);
+    bcz = ldv(cf + BCZ * PL + occ);
+  } else {
+    damp = ldv(cf + DAMP * PL + occ);
+  }
+  bool in[W], sp[W], any = false;
+#pragma unroll
+  for (int e = 0; e < W; ++e) {
+    in[e] = in_I(g, i, j + e);
+    sp[e] = PML && (!in[e] || keeps_split(g, i, bcx.v[e], bcz.v[e]));
+    any = any || sp[e];
+  }
   griddep_wait();  // launched with programmatic serialisation in the time loops
   griddep_launch_dependents();
-  if (const int tiles = tile_count(g); (int)blockIdx.x >= tiles) {
-    record_block(g, tiles, kCellShots, it, tt, 3, 0, rec);
-    return;
-  }
-  EL_CELL_SHOTS
-  const bool inside = in_I(g, i, j);
-  bool split = true;
-  T pxd = T(1), pxn = T(0), pzd = T(1), pzn = T(0), dbx = T(0), dbz = T(0);
-  if (inside) {
-    const T bcx = cf[BCX * PL + occ], bcz = cf[BCZ * PL + occ];
-    split = keeps_split(g, i, bcx, bcz);
-    pxd = radd(T(1), rmul(g.hdt, bcx));
-    pxn = rsub(T(1), rmul(g.hdt, bcx));
-    pzd = radd(T(1), rmul(g.hdt, bcz));
-    pzn = rsub(T(1), rmul(g.hdt, bcz));
-    dbx = rmul(g.dt, cf[BX * PL + occ]);
-    dbz = rmul(g.dt, cf[BZ * PL + occ]);
-  }
+  {
+    const Row<T, NN> xx(tt + TXX * NSP + o), xz(tt + TXZ * NSP + o);
+    Vec<T> rxz[2 * NN], rzz[2 * NN];  // rows i - NN .. i + NN - 1 of txz, i - NN + 1 .. i + NN of tzz
 #pragma unroll
-  for (int q = 0; q < kCellShots; ++q) {
-    const int s = s_lo + q;
-    if (s >= g.ns) break;
-    const int64_t o = (int64_t)s * PL + occ;
-    if (!split) {
-      const T dxfm_txx = dxf<NN>(g, tt + TXX * NSP, o);
-      const T dzbm_txz = dzb<NN>(g, tt + TXZ * NSP, o);
-      const T dxbm_txz = dxb<NN>(g, tt + TXZ * NSP, o);
-      const T dzfm_tzz = dzf<NN>(g, tt + TZZ * NSP, o);
-      const T vx = radd(radd(vprev[VX * NSP + o], rdiv(rmul(dbx, dxfm_txx), g.dx)), rdiv(rmul(dbx, dzbm_txz), g.dz));
-      const T vz = radd(radd(vprev[VZ * NSP + o], rdiv(rmul(dbz, dxbm_txz), g.dx)), rdiv(rmul(dbz, dzfm_tzz), g.dz));
-      v[VX * NSP + o] = vx;
-      v[VZ * NSP + o] = vz;
-      continue;
+    for (int k = 0; k < 2 * NN; ++k) {
+      if (k != NN) rxz[k] = ldv(tt + TXZ * NSP + o + (k - NN) * P);
+      rzz[k] = ldv(tt + TZZ * NSP + o + (k - NN + 1) * P);
     }
-    T sv[4];
+    if (any) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) sv[k] = vs[k * NSP + o];
-    if (inside) {
-      const T dxfm_txx = dxf<NN>(g, tt + TXX * NSP, o);
-      const T dzbm_txz = dzb<NN>(g, tt + TXZ * NSP, o);
-      const T dxbm_txz = dxb<NN>(g, tt + TXZ * NSP, o);
-      const T dzfm_tzz = dzf<NN>(g, tt + TZZ * NSP, o);
-      sv[VX_X] = rdiv_pml(radd(rmul(pxn, sv[VX_X]), rdiv(rmul(dbx, dxfm_txx), g.dx)), pxd);
-      sv[VX_Z] = rdiv_pml(radd(rmul(pzn, sv[VX_Z]), rdiv(rmul(dbx, dzbm_txz), g.dz)), pzd);
-      sv[VZ_X] = rdiv_pml(radd(rmul(pxn, sv[VZ_X]), rdiv(rmul(dbz, dxbm_txz), g.dx)), pxd);
-      sv[VZ_Z] = rdiv_pml(radd(rmul(pzn, sv[VZ_Z]), rdiv(rmul(dbz, dzfm_tzz), g.dz)), pzd);
+      for (int k = 0; k < 4; ++k) f[k] = ldv(vs + k * NSP + o);
+    }
+    const Fd<T> fx(g, g.dt_dx), fz(g, g.dt_dz);
+    Vec<T> a[4];  // the increments of the split parts vx_x, vx_z, vz_x, vz_z
 #pragma unroll
-      for (int k = 0; k < 4; ++k) vs[k * NSP + o] = sv[k];
+    for (int e = 0; e < W; ++e) {
+      a[0].v[e] = bx.v[e] * fx.template diff<NN>([&](int m) { return xx(e + m); });
+      a[1].v[e] = bx.v[e] * fz.template diff<NN>([&](int m) { return m == 1 ? xz(e) : rxz[NN + m - 1].v[e]; });
+      a[2].v[e] = bz.v[e] * fx.template diff<NN>([&](int m) { return xz(e - 1 + m); });
+      a[3].v[e] = bz.v[e] * fz.template diff<NN>([&](int m) { return rzz[NN + m - 1].v[e]; });
     }
-    if (!vel_fs_row(g, i, j)) {
-      v[VX * NSP + o] = radd(sv[VX_X], sv[VX_Z]);
-      v[VZ * NSP + o] = radd(sv[VZ_X], sv[VZ_Z]);
+    if (!PML) {
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        if (in[e]) {
+          nx.v[e] += a[0].v[e] + a[1].v[e];
+          nz.v[e] += a[2].v[e] + a[3].v[e];
+        }
+        if (!g.fsurf) {
+          nx.v[e] *= damp.v[e];
+          nz.v[e] *= damp.v[e];
+        }
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        if (!sp[e]) {
+          nx.v[e] += a[0].v[e] + a[1].v[e];
+          nz.v[e] += a[2].v[e] + a[3].v[e];
+        }
+      }
+      if (any) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const Vec<T>& bc = k & 1 ? bcz : bcx;
+#pragma unroll
+          for (int e = 0; e < W; ++e)
+            if (sp[e] && in[e])
+              f[k].v[e] = ((T(1) - g.hdt * bc.v[e]) * f[k].v[e] + a[k].v[e]) * pml_inv(T(1) + g.hdt * bc.v[e]);
+          stv(vs + k * NSP + o, f[k]);
+        }
+#pragma unroll
+        for (int e = 0; e < W; ++e)
+          if (sp[e]) {
+            nx.v[e] = f[VX_X].v[e] + f[VX_Z].v[e];
+            nz.v[e] = f[VZ_X].v[e] + f[VZ_Z].v[e];
+          }
+      }
+      if (g.fsurf && (i == g.h - 2 || i == g.h - 3)) return;  // the next stress update's
     }
+    stv(v + VX * NSP + o, nx);
+    stv(v + VZ * NSP + o, nz);
   }
-}
-
-// ======================================================================= forward, absorbing layer
-// The step out of place (tprev -> ts, v -> vout) or in place; the free-surface stress rows
-// (elastic_kernels.py:738-742) are written by the cells they mirror, as with the PML. Four launches a
-// step with a free surface (the velocity rows above it are inputs of the damping) and two without,
-// programmatically serialised; the reverse step takes six and four. A gradient step pair of 4 shots
-// on a 151 x 207 grid without one took 84 us as nine plain launches and two copies; it takes 50.
-template <typename T, int NN>
-__global__ void stress_abl(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ v, T* ts, const T* tprev,
-                           const T* __restrict__ wav, T* __restrict__ rec) {
-  griddep_wait();
-  griddep_launch_dependents();
-  if (const int tiles = tile_count(g); (int)blockIdx.x >= tiles) {
-    record_block(g, tiles, 1, it - 1, v, 2, 3, rec);
-    return;
-  }
-  EL_CELL_SHOT
-  const int64_t occ = g.L.off(i, j);
-  T xx = tprev[TXX * NSP + o], zz = tprev[TZZ * NSP + o], xz = tprev[TXZ * NSP + o];
-  if (in_I(g, i, j)) {
-    const T* vx = v;
-    const T* vz = v + NSP;
-    const T dxbm_vx = dxb<NN>(g, vx, o), dxbm_vz = dxb<NN>(g, vz, o);
-    const T dzbm_vx = dzb<NN>(g, vx, o), dzbm_vz = dzb<NN>(g, vz, o);
-    const T dxfm_vx = dxf<NN>(g, vx, o), dzfm_vx = dzf<NN>(g, vx, o);
-    const T dxfm_vz = dxf<NN>(g, vz, o), dzfm_vz = dzf<NN>(g, vz, o);
-    const T c11 = cf[C11 * PL + occ], c13 = cf[C13 * PL + occ], c15 = cf[C15 * PL + occ];
-    const T c33 = cf[C33 * PL + occ], c35 = cf[C35 * PL + occ], c55 = cf[C55 * PL + occ];
-    xx = radd(xx, rmul(g.dt, radd(rdiv(radd(rmul(c11, dxbm_vx), rmul(c15, dxbm_vz)), g.dx),
-                                  rdiv(radd(rmul(c15, dzbm_vx), rmul(c13, dzbm_vz)), g.dz))));
-    zz = radd(zz, rmul(g.dt, radd(rdiv(radd(rmul(c13, dxbm_vx), rmul(c35, dxbm_vz)), g.dx),
-                                  rdiv(radd(rmul(c35, dzbm_vx), rmul(c33, dzbm_vz)), g.dz))));
-    xz = radd(xz, rmul(g.dt, radd(rdiv(radd(rmul(c15, dxfm_vx), rmul(c55, dxfm_vz)), g.dx),
-                                  rdiv(radd(rmul(c55, dzfm_vx), rmul(c35, dzfm_vz)), g.dz))));
-  }
-  if (i == g.src_z[s] && j == g.src_x[s]) {
-    const T w = wav[(int64_t)s * g.nt + it];
-    xx = radd(xx, rmul(g.src_m[3 * s + 0], w));
-    zz = radd(zz, rmul(g.src_m[3 * s + 1], w));
-    xz = radd(xz, rmul(g.src_m[3 * s + 2], w));
-  }
-  store_stress(g, i, o, NSP, xx, zz, xz, ts);
-}
-
-// Without a free surface the damping is applied here; with one it follows the surface rows.
-template <typename T, int NN>
-__global__ void vel_abl(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ tt, T* v, const T* vprev,
-                        T* __restrict__ rec) {
-  griddep_wait();
-  griddep_launch_dependents();
-  if (const int tiles = tile_count(g); (int)blockIdx.x >= tiles) {
-    record_block(g, tiles, 1, it, tt, 3, 0, rec);
-    return;
-  }
-  EL_CELL_SHOT
-  const int64_t occ = g.L.off(i, j);
-  T vx = vprev[VX * NSP + o], vz = vprev[VZ * NSP + o];
-  if (in_I(g, i, j)) {
-    const T dxfm_txx = dxf<NN>(g, tt + TXX * NSP, o);
-    const T dzbm_txz = dzb<NN>(g, tt + TXZ * NSP, o);
-    const T dxbm_txz = dxb<NN>(g, tt + TXZ * NSP, o);
-    const T dzfm_tzz = dzf<NN>(g, tt + TZZ * NSP, o);
-    const T bx = cf[BX * PL + occ], bz = cf[BZ * PL + occ];
-    vx = radd(vx, rmul(rmul(g.dt, bx), radd(rdiv(dxfm_txx, g.dx), rdiv(dzbm_txz, g.dz))));
-    vz = radd(vz, rmul(rmul(g.dt, bz), radd(rdiv(dxbm_txz, g.dx), rdiv(dzfm_tzz, g.dz))));
-  }
-  if (!g.fsurf) {
-    const T d = cf[DAMP * PL + occ];
-    vx = rmul(vx, d);
-    vz = rmul(vz, d);
-  }
-  v[VX * NSP + o] = vx;
-  v[VZ * NSP + o] = vz;
 }
 
 // Free-surface velocity rows in place (elastic_kernels.py:753-756); one thread per column in J.
@@ -657,7 +704,7 @@ template <typename T>
 __global__ void record_v(Geo<T> g, int it, const T* __restrict__ v, T* __restrict__ rec, bool rows_above) {
   griddep_wait();
   griddep_launch_dependents();
-  record_block(g, 0, 1, it, v, 2, 3, rec, rows_above);
+  record_block(g, 0, it, v, 2, 3, rec, rows_above);
 }
 
 // forward_wavefield_* += sum_s X^2 of the last step of a chunk (elastic_kernels.py:414-418, 1016-1021).
@@ -1449,11 +1496,11 @@ __global__ void adj_vfs_abl(Geo<T> g, const T* __restrict__ cf, const T* __restr
   lv_out[VZ * NSP + o] = az;
   const bool inside = in_I(g, i, j);
   const int64_t c0 = g.L.off(i, j);
-  const T bx = inside ? g.dt * cf[BX * PL + c0] : T(0), bz = inside ? g.dt * cf[BZ * PL + c0] : T(0);
-  q4[0 * NSP + o] = inside ? ax * bx / g.dx : T(0);
-  q4[1 * NSP + o] = inside ? ax * bx / g.dz : T(0);
-  q4[2 * NSP + o] = inside ? az * bz / g.dx : T(0);
-  q4[3 * NSP + o] = inside ? az * bz / g.dz : T(0);
+  const T bx = inside ? cf[BX * PL + c0] : T(0), bz = inside ? cf[BZ * PL + c0] : T(0);
+  q4[0 * NSP + o] = ax * bx * g.dt_dx;
+  q4[1 * NSP + o] = ax * bx * g.dt_dz;
+  q4[2 * NSP + o] = az * bz * g.dt_dx;
+  q4[3 * NSP + o] = az * bz * g.dt_dz;
 }
 
 // ABL: lt += transposes of the velocity update's stress differences; bx, bz gradients; without a
@@ -1479,8 +1526,8 @@ __global__ void adj_t_abl(Geo<T> g, const T* __restrict__ cf, const T* __restric
     if (!g.fsurf) stress_sources<T, false>(g, cf, lt, i, j, o, q8);
     if (in_I(g, i, j)) {
       const T* th = tt_hist;
-      gx += lv[VX * NSP + o] * g.dt * (dxf<NN>(g, th + TXX * NSP, o) / g.dx + dzb<NN>(g, th + TXZ * NSP, o) / g.dz);
-      gz += lv[VZ * NSP + o] * g.dt * (dxb<NN>(g, th + TXZ * NSP, o) / g.dx + dzf<NN>(g, th + TZZ * NSP, o) / g.dz);
+      gx += lv[VX * NSP + o] * (dxf<NN>(g, th + TXX * NSP, o) * g.dt_dx + dzb<NN>(g, th + TXZ * NSP, o) * g.dt_dz);
+      gz += lv[VZ * NSP + o] * (dxb<NN>(g, th + TXZ * NSP, o) * g.dt_dx + dzf<NN>(g, th + TZZ * NSP, o) * g.dt_dz);
     }
   }
   if (in_I(g, i, j)) {
@@ -1725,27 +1772,21 @@ int esetup(const adfwi_elastic_plan* p, unsigned char* ws, const ECarve& c, cons
 template <typename T, int NN>
 void estep(const adfwi_elastic_plan* p, const el::Geo<T>& g, int it, const T* cf, const T* wav, T* st, T* tt,
            const T* tprev, T* vin, T* vout, T* rec, cudaStream_t s) {
-  const dim3 b(el::kTileThreads);
+  const dim3 b(el::kVecThreads);
   const int64_t NSP = (int64_t)p->d.ns * p->L.plane;
-  const int shots = p->d.pml ? el::kCellShots : 1;
-  const dim3 gc = cells_grid(p, (p->d.ns + shots - 1) / shots);
-  const unsigned rb = rec != nullptr && p->d.nr > 0 ? (p->d.nr + el::kTileThreads - 1) / el::kTileThreads : 0;
-  const dim3 gs(gc.x + (it > 0 ? rb : 0), gc.y), gv(gc.x + rb, gc.y);
-  if (p->d.pml) {
-    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::stress_pml_tot<T, NN>, gs, b, 0, s, g, it, cf, vin, st, tt,
-                                                        tprev, wav, rec));
-    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_pml_tot<T, NN>, gv, b, 0, s, g, it, cf, (const T*)tt,
-                                                        st + 6 * NSP, vout, (const T*)vin, rec));
-  } else {
+  const unsigned tiles = el::vec_tiles<T>(p->L), gy = p->d.ns;
+  const unsigned rb = rec != nullptr && p->d.nr > 0 ? (p->d.nr + el::kVecThreads - 1) / el::kVecThreads : 0;
+  const dim3 gs(tiles + (it > 0 ? rb : 0), gy), gv(tiles + rb, gy);
+  auto stress = p->d.pml ? el::stress_step<T, NN, true> : el::stress_step<T, NN, false>;
+  auto vel = p->d.pml ? el::vel_step<T, NN, true> : el::vel_step<T, NN, false>;
+  ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(stress, gs, b, 0, s, g, it, cf, vin, st, tt, tprev, wav, rec));
+  ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(vel, gv, b, 0, s, g, it, cf, (const T*)tt,
+                                                      p->d.pml ? st + 6 * NSP : nullptr, vout, (const T*)vin, rec));
+  if (!p->d.pml && p->d.free_surface) {
     const dim3 gcol((unsigned)((p->nxp + 127) / 128), p->d.ns);
-    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::stress_abl<T, NN>, gs, b, 0, s, g, it, cf, (const T*)vin, tt,
-                                                        tprev, wav, rec));
-    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_abl<T, NN>, gv, b, 0, s, g, it, cf, (const T*)tt, vout,
-                                                        (const T*)vin, rec));
-    if (p->d.free_surface) {
-      ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_fs_abl<T>, gcol, dim3(128), 0, s, g, vout));
-      ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::damp_v<T>, gc, b, 0, s, g, cf, vout));
-    }
+    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::vel_fs_abl<T>, gcol, dim3(128), 0, s, g, vout));
+    ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(el::damp_v<T>, cells_grid(p, p->d.ns), dim3(el::kTileThreads), 0,
+                                                        s, g, cf, vout));
   }
 }
 
@@ -1884,7 +1925,6 @@ int ebackward(const adfwi_elastic_plan* p, const void* wavelet, const void* grec
     if (rc0) return rc0;
   }
   const dim3 gcs = cells_grid(p, ns), gcg = cells_grid(p, egroups(p)), b(el::kTileThreads);
-  const dim3 gcm = cells_grid(p, (ns + el::kCellShots - 1) / el::kCellShots);
   // shared memory of the staged gradient kernels (above the 48 KB default in double precision)
   const int smem_t = el::kAdjTElems * (int)sizeof(T);
   const int smem_vp = el::kAdjVPmlElems * (int)sizeof(T);
