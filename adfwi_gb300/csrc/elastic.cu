@@ -28,7 +28,6 @@
 
 #include "../../include/adfwi_gb300.h"
 #include "common.cuh"
-#include "frames.cuh"
 #include "snapshot.cuh"
 
 namespace adfwi {
@@ -57,6 +56,7 @@ struct Geo {
   int top, nabc, nz, nx;       // energy window
   T dt, dx, dz, dt_dx, dt_dz, hdt;
   T f0, f1, f2;                // staggered coefficients
+  T fx[3], fz[3];              // the same times dt / dx and dt / dz, rounded once
   const int* src_z;
   const int* src_x;
   const T* src_m;              // ns x 3 source weights (xx, zz, xz) already scaled for the mode
@@ -65,79 +65,13 @@ struct Geo {
   const int* ucell_zx;         // unique receiver cells (i << 16 | j)
   const int* ucell_beg;        // ncells+1 offsets into ucell_rcv
   const int* ucell_rcv;
+  const int* tile_beg;         // first unique receiver cell of each tile of the reverse kernels, and the end
   int ncells;
 };
 
 template <typename T>
 __device__ __forceinline__ bool in_I(const Geo<T>& g, int i, int j) {
   return i >= g.ilo && i <= g.ihi && j >= g.jlo && j <= g.jhi;
-}
-
-// ---- half-cell differences (elastic_kernels.py:66-108): f_k (a[+1+k] - a[-k]) etc.
-template <int NN, typename T>
-__device__ __forceinline__ T dxf(const Geo<T>& g, const T* a, int64_t o) {
-  T r = rmul(g.f0, rsub(a[o + 1], a[o]));
-  r = radd(r, rmul(g.f1, rsub(a[o + 2], a[o - 1])));
-  if (NN == 3) r = radd(r, rmul(g.f2, rsub(a[o + 3], a[o - 2])));
-  return r;
-}
-template <int NN, typename T>
-__device__ __forceinline__ T dxb(const Geo<T>& g, const T* a, int64_t o) {
-  T r = rmul(g.f0, rsub(a[o], a[o - 1]));
-  r = radd(r, rmul(g.f1, rsub(a[o + 1], a[o - 2])));
-  if (NN == 3) r = radd(r, rmul(g.f2, rsub(a[o + 2], a[o - 3])));
-  return r;
-}
-template <int NN, typename T>
-__device__ __forceinline__ T dzf(const Geo<T>& g, const T* a, int64_t o, int64_t P) {
-  T r = rmul(g.f0, rsub(a[o + P], a[o]));
-  r = radd(r, rmul(g.f1, rsub(a[o + 2 * P], a[o - P])));
-  if (NN == 3) r = radd(r, rmul(g.f2, rsub(a[o + 3 * P], a[o - 2 * P])));
-  return r;
-}
-template <int NN, typename T>
-__device__ __forceinline__ T dzb(const Geo<T>& g, const T* a, int64_t o, int64_t P) {
-  T r = rmul(g.f0, rsub(a[o], a[o - P]));
-  r = radd(r, rmul(g.f1, rsub(a[o + P], a[o - 2 * P])));
-  if (NN == 3) r = radd(r, rmul(g.f2, rsub(a[o + 2 * P], a[o - 3 * P])));
-  return r;
-}
-// planes in global memory (row pitch of the layout)
-template <int NN, typename T>
-__device__ __forceinline__ T dzf(const Geo<T>& g, const T* a, int64_t o) {
-  return dzf<NN>(g, a, o, (int64_t)g.L.pitch);
-}
-template <int NN, typename T>
-__device__ __forceinline__ T dzb(const Geo<T>& g, const T* a, int64_t o) {
-  return dzb<NN>(g, a, o, (int64_t)g.L.pitch);
-}
-
-// ---- transposes in gather form: contribution to cell (i, j) of q placed at the cells that
-// read (i, j). q(i', j') must be zero outside the update region.
-//   Dxf^T q (j) = sum_k f_k (q[j-1-k] - q[j+k]);   Dxb^T q (j) = sum_k f_k (q[j-k] - q[j+1+k])
-template <int NN, typename T, typename Q>
-__device__ __forceinline__ T dxf_t(const Geo<T>& g, const Q& q, int i, int j) {
-  T r = g.f0 * (q(i, j - 1) - q(i, j)) + g.f1 * (q(i, j - 2) - q(i, j + 1));
-  if (NN == 3) r += g.f2 * (q(i, j - 3) - q(i, j + 2));
-  return r;
-}
-template <int NN, typename T, typename Q>
-__device__ __forceinline__ T dxb_t(const Geo<T>& g, const Q& q, int i, int j) {
-  T r = g.f0 * (q(i, j) - q(i, j + 1)) + g.f1 * (q(i, j - 1) - q(i, j + 2));
-  if (NN == 3) r += g.f2 * (q(i, j - 2) - q(i, j + 3));
-  return r;
-}
-template <int NN, typename T, typename Q>
-__device__ __forceinline__ T dzf_t(const Geo<T>& g, const Q& q, int i, int j) {
-  T r = g.f0 * (q(i - 1, j) - q(i, j)) + g.f1 * (q(i - 2, j) - q(i + 1, j));
-  if (NN == 3) r += g.f2 * (q(i - 3, j) - q(i + 2, j));
-  return r;
-}
-template <int NN, typename T, typename Q>
-__device__ __forceinline__ T dzb_t(const Geo<T>& g, const Q& q, int i, int j) {
-  T r = g.f0 * (q(i, j) - q(i + 1, j)) + g.f1 * (q(i - 1, j) - q(i + 2, j));
-  if (NN == 3) r += g.f2 * (q(i - 2, j) - q(i + 3, j));
-  return r;
 }
 
 // The cell of this thread in the per-cell kernels: a block of 256 threads covers a tile of
@@ -168,11 +102,6 @@ __device__ __forceinline__ T pml_inv(T d) {
   return d == T(1) ? T(1) : T(1) / d;
 }
 
-#define EL_CELL                                                                      \
-  EL_TILE_IJ                                                                         \
-  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL;                            \
-  const int64_t oc = g.L.off(i, j);
-
 // Gradient kernels: blockIdx.y picks a group of `eg` consecutive shots; the group's gradient
 // partials (8 planes) start at gpart + blockIdx.y * 8 * PL and are summed over the groups in a
 // fixed order at the end of the backward pass (deterministic).
@@ -180,84 +109,27 @@ __device__ __forceinline__ T pml_inv(T d) {
   const int s_beg = blockIdx.y * eg, s_end = min(g.ns, s_beg + eg);                  \
   T* gbase = gpart + (int64_t)blockIdx.y * 8 * PL;
 
-// Staging of the shot-group gradient kernels. Per shot, a block copies the 32 x 8 tile of every
-// plane it reads into shared memory with 16-byte asynchronous copies, with the halo its
-// stencils need (4 columns each side for x differences, 3 rows each side for z differences,
-// none for pointwise reads), then evaluates its cells there: each staged element is fetched
-// once per block instead of once per reading thread.
-constexpr int kSW = kTileX + 8;     // staged row: columns j0-4 .. j0+kTileX+3
-constexpr int kSZ = kTileZ + 6;     // staged rows: i0-3 .. i0+kTileZ+2
-constexpr int kSPlane = kSW * kSZ;  // elements of one staged plane
-constexpr int kSC = 3 * kSW + 4;    // staged index of the tile's cell (i0, j0)
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Queue the copies of rows i0-zh .. i0+kTileZ+zh-1 and columns j0-xh .. j0+kTileX+xh-1 (xh 0 or
-// 4, zh 0 or 3) of `plane` into the staged plane `dst`. Every copy starts on a 16-byte boundary
-// (j0 is a multiple of 32, rows are 128-byte multiples, the ghost frame is 4 columns wide), and
-// every row and column read lies in the plane's allocation: the layout keeps 4 ghost rows and
-// columns before the grid and a 16-row / 64-column margin after it.
-template <typename T>
-__device__ __forceinline__ void stage(T* dst, const T* plane, const Layout& L, int i0, int j0, int zh, int xh) {
-  constexpr int E = 16 / (int)sizeof(T);
-  const int cols = (kTileX + 2 * xh) / E, rows = kTileZ + 2 * zh;
-  for (int t = threadIdx.x; t < rows * cols; t += kTileThreads) {
-    const int r = t / cols, c = t - r * cols;
-    cp_async16(dst + (r - zh + 3) * kSW + (c * E - xh + 4), plane + L.off(i0 - zh + r, j0 - xh + c * E));
-  }
-}
-
-// A staged plane read at grid cells (ii, jj) of the block's tile.
-template <typename T>
-struct StagedQ {
-  const T* s;
-  int i0, j0;
-  __device__ __forceinline__ T operator()(int ii, int jj) const { return s[(ii - i0 + 3) * kSW + (jj - j0 + 4)]; }
-};
-
-// Compact staged planes: an x plane holds only the tile rows with the x halo (kTileZ x kSW), a z
-// plane only the tile columns with the z halo (kSZ x kTileX).
-constexpr int kXPlane = kTileZ * kSW, kZPlane = kSZ * kTileX;
-template <typename T>
-__device__ __forceinline__ void stage_x(T* dst, const T* plane, const Layout& L, int i0, int j0) {
-  constexpr int E = 16 / (int)sizeof(T), cols = kSW / E;
-  for (int t = threadIdx.x; t < kTileZ * cols; t += kTileThreads) {
-    const int r = t / cols, c = t - r * cols;
-    cp_async16(dst + r * kSW + c * E, plane + L.off(i0 + r, j0 - 4 + c * E));
-  }
-}
-template <typename T>
-__device__ __forceinline__ void stage_z(T* dst, const T* plane, const Layout& L, int i0, int j0) {
-  constexpr int E = 16 / (int)sizeof(T), cols = kTileX / E;
-  for (int t = threadIdx.x; t < kSZ * cols; t += kTileThreads) {
-    const int r = t / cols, c = t - r * cols;
-    cp_async16(dst + r * kTileX + c * E, plane + L.off(i0 - 3 + r, j0 + c * E));
-  }
-}
-template <typename T>
-struct StagedX {
-  const T* s;
-  int i0, j0;
-  __device__ __forceinline__ T operator()(int ii, int jj) const { return s[(ii - i0) * kSW + (jj - j0 + 4)]; }
-};
-template <typename T>
-struct StagedZ {
-  const T* s;
-  int i0, j0;
-  __device__ __forceinline__ T operator()(int ii, int jj) const { return s[(ii - i0 + 3) * kTileX + (jj - j0)]; }
-};
-
-// ---- forward kernels: a thread takes kVW consecutive columns of a row, read and written as 16-byte
-// vectors (columns start at a multiple of kVW, planes at multiples of 128 bytes with a ghost frame of
-// 4 columns, so every vector is aligned). A warp covers 32 columns of 4 rows (2 in double precision)
-// and a block of 128 threads 32 columns of 4 kVW rows.
+// ---- a thread takes kVW consecutive columns of a row, read and written as one vector of 8 bytes (16
+// in double precision; columns start at a multiple of kVW, planes at multiples of 128 bytes with a
+// ghost frame of 4 columns, so every vector is aligned). In the forward kernels a warp covers 32
+// columns of 2 rows and a block of 128 threads 32 columns of 8 rows. One column per thread moves the
+// same bytes with twice the instructions, four leave too few warps: 12.1, 10.5 and 12.7 ms for 200
+// forward steps of 20 shots on a 242 x 480 grid with 1, 2 and 4.
 constexpr int kVecThreads = 128, kVecX = 32;
 template <typename T>
-constexpr int kVW = 16 / (int)sizeof(T);
+constexpr int kVW = 2;
+template <int B>
+struct Bytes;
+template <>
+struct Bytes<8> {
+  using t = int2;
+};
+template <>
+struct Bytes<16> {
+  using t = int4;
+};
+template <typename T>
+using VecBits = typename Bytes<kVW<T> * (int)sizeof(T)>::t;
 template <typename T>
 constexpr int kVecRows = kVecThreads * kVW<T> / kVecX;
 template <typename T>
@@ -267,12 +139,12 @@ struct Vec {
 template <typename T>
 __device__ __forceinline__ Vec<T> ldv(const T* p) {
   Vec<T> r;
-  *reinterpret_cast<int4*>(r.v) = *reinterpret_cast<const int4*>(p);
+  *reinterpret_cast<VecBits<T>*>(r.v) = *reinterpret_cast<const VecBits<T>*>(p);
   return r;
 }
 template <typename T>
 __device__ __forceinline__ void stv(T* p, const Vec<T>& x) {
-  *reinterpret_cast<int4*>(p) = *reinterpret_cast<const int4*>(x.v);
+  *reinterpret_cast<VecBits<T>*>(p) = *reinterpret_cast<const VecBits<T>*>(x.v);
 }
 // The vector at p of a row with the whole vectors that hold its NN neighbours on each side.
 template <typename T, int NN>
@@ -282,17 +154,16 @@ struct Row {
   __device__ __forceinline__ explicit Row(const T* p) {
 #pragma unroll
     for (int k = 0; k < kVW<T> + 2 * H; k += kVW<T>)
-      *reinterpret_cast<int4*>(v + k) = *reinterpret_cast<const int4*>(p - H + k);
+      *reinterpret_cast<VecBits<T>*>(v + k) = *reinterpret_cast<const VecBits<T>*>(p - H + k);
   }
   __device__ __forceinline__ T operator()(int k) const { return v[H + k]; }
 };
-// Half-cell difference times `scale` (dt / dx or dt / dz; elastic_kernels.py:66-108): `at(m)` is the
+// Half-cell difference (elastic_kernels.py:66-108), the coefficients with or without dt / dx: `at(m)` is the
 // value m cells from the lower of the two middle ones. Differences, coefficient products and sums
 // of the forward kernels are fused multiply-adds, and one sum is added to a total.
 template <typename T>
 struct Fd {
   T f0, f1, f2;
-  __device__ __forceinline__ Fd(const Geo<T>& g, T scale) : f0(g.f0 * scale), f1(g.f1 * scale), f2(g.f2 * scale) {}
   template <int NN, typename A>
   __device__ __forceinline__ T diff(const A& at) const {
     T r = f0 * (at(1) - at(0)) + f1 * (at(2) - at(-1));
@@ -394,12 +265,12 @@ __device__ __forceinline__ void store_stress(const Geo<T>& g, int i, int64_t o, 
 // of the damping and take two small launches).
 //
 // What bounds them is latency: a thread's chain of loads from L2 and the launch boundary, not L2 or
-// DRAM bandwidth (30 % of either) nor issue slots (32 %). So a thread takes four columns as 16-byte
-// vectors with all its loads in flight at once (160 registers, three blocks per SM; four blocks with
-// spills, two shots per thread and 64-column tiles measured 3 to 20 % slower), and reads what the
-// launch before does not write ahead of that launch's end. 300 steps of one shot on a 122 x 140 grid:
-// 4.56 -> 3.47 ms; 200 steps of 20 shots on a 242 x 480 grid: 16.3 -> 12.7 ms, against one cell and
-// two shots per thread with scalar loads and exact divisions by dx.
+// DRAM bandwidth (30 % of either) nor issue slots (32 %). So a thread has all its loads in flight at
+// once and reads what the launch before does not write ahead of that launch's end; with two columns a
+// thread that takes 96 registers, five blocks per SM (six and eight spill and measured 7 and 30 %
+// slower). 300 steps of one shot on a 122 x 140 grid: 4.56 -> 3.0 ms; 200 steps of 20 shots on a
+// 242 x 480 grid: 16.3 -> 10.5 ms, against one cell and two shots per thread with scalar loads and
+// exact divisions by dx.
 //
 // Cells that keep split fields: outside the update region, where a PML factor differs from 1,
 // and in the surface rows that mirror others or are mirrored (h-3 .. h) plus one. Every other cell
@@ -414,7 +285,7 @@ __device__ __forceinline__ bool keeps_split(const Geo<T>& g, int i, T bcx, T bcz
 // tprev: stress totals at the start of the step (tt itself when the totals advance in place);
 // tt: where the new totals go; rec: the velocity records of step it - 1 are taken (null: none).
 template <typename T, int NN, bool PML>
-__global__ void __launch_bounds__(kVecThreads, 3)
+__global__ void __launch_bounds__(kVecThreads, 5)
     stress_step(Geo<T> g, int it, const T* __restrict__ cf, T* __restrict__ v, T* __restrict__ ts, T* tt, const T* tprev,
                 const T* __restrict__ wav, T* __restrict__ rec) {
   if (const int tiles = vec_tiles<T>(g.L); (int)blockIdx.x >= tiles) {
@@ -496,7 +367,7 @@ __global__ void __launch_bounds__(kVecThreads, 3)
         stv(v + VZ * NSP + o - 2 * P, az);
       }
     }
-    const Fd<T> fx(g, g.dt_dx), fz(g, g.dt_dz);
+    const Fd<T> fx{g.fx[0], g.fx[1], g.fx[2]}, fz{g.fz[0], g.fz[1], g.fz[2]};
     Vec<T> a[6];  // the increments of the split parts xx_x, xx_z, zz_x, zz_z, xz_x, xz_z
 #pragma unroll
     for (int e = 0; e < W; ++e) {
@@ -572,7 +443,7 @@ __global__ void __launch_bounds__(kVecThreads, 3)
 // stress records of step it are taken (null: none). Without a free surface the absorbing layer's
 // damping is applied here; with one it follows the surface rows.
 template <typename T, int NN, bool PML>
-__global__ void __launch_bounds__(kVecThreads, 3)
+__global__ void __launch_bounds__(kVecThreads, 5)
     vel_step(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ tt, T* __restrict__ vs, T* v,
              const T* vprev, T* __restrict__ rec) {
   if (const int tiles = vec_tiles<T>(g.L); (int)blockIdx.x >= tiles) {
@@ -614,7 +485,7 @@ __global__ void __launch_bounds__(kVecThreads, 3)
 #pragma unroll
       for (int k = 0; k < 4; ++k) f[k] = ldv(vs + k * NSP + o);
     }
-    const Fd<T> fx(g, g.dt_dx), fz(g, g.dt_dz);
+    const Fd<T> fx{g.fx[0], g.fx[1], g.fx[2]}, fz{g.fz[0], g.fz[1], g.fz[2]};
     Vec<T> a[4];  // the increments of the split parts vx_x, vx_z, vz_x, vz_z
 #pragma unroll
     for (int e = 0; e < W; ++e) {
@@ -727,48 +598,31 @@ __global__ void energy(Geo<T> g, const T* __restrict__ tt, const T* __restrict__
 }
 
 // ======================================================================= adjoint
-// Receiver residuals of step `it` into the adjoint stress totals lt (overwritten: zero + injection)
-// and added to the adjoint velocity totals lv. One thread per (unique receiver cell, shot).
+// dL/d velocity records of step it added to lv, before the first reverse step (each adj_v_step adds
+// those of the step before its own). One thread per (unique receiver cell, shot).
 template <typename T>
-__global__ void adj_inject(Geo<T> g, int it, const T* __restrict__ grec, T* lt, T* lv, int parts) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
-  griddep_launch_dependents();
+__global__ void adj_inject(Geo<T> g, int it, const T* __restrict__ grec, T* lv) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= g.ncells) return;
   const int s = blockIdx.y;
   const int64_t NSP = (int64_t)g.ns * g.L.plane;
   const int cell = g.ucell_zx[q];
   const int64_t o = (int64_t)s * g.L.plane + g.L.off(cell >> 16, cell & 0xffff);
-  const int64_t RS = (int64_t)g.ns * g.nt * g.nr;
-  const int64_t base = ((int64_t)s * g.nt + it) * g.nr;
-  T a[5] = {T(0), T(0), T(0), T(0), T(0)};
-  for (int m = g.ucell_beg[q]; m < g.ucell_beg[q + 1]; ++m) {
-    const int64_t qq = base + g.ucell_rcv[m];
-    for (int c = 0; c < 5; ++c) a[c] += grec[c * RS + qq];
-  }
-  if (parts & 2) {  // stresses
-    lt[TXX * NSP + o] += a[0];
-    lt[TZZ * NSP + o] += a[1];
-    lt[TXZ * NSP + o] += a[2];
-  }
-  if (parts & 1) {  // velocities
-    lv[VX * NSP + o] += a[3];
-    lv[VZ * NSP + o] += a[4];
+  const int64_t RS = (int64_t)g.ns * g.nt * g.nr, base = ((int64_t)s * g.nt + it) * g.nr;
+  for (int c = 0; c < 2; ++c) {
+    T a = T(0);
+    for (int m = g.ucell_beg[q]; m < g.ucell_beg[q + 1]; ++m) a += grec[(3 + c) * RS + base + g.ucell_rcv[m]];
+    lv[c * NSP + o] += a;
   }
 }
 
-// Adjoint of the free-surface velocity rows: lambda of the velocity totals BEFORE the rows
-// h-3 / h-2 were overwritten (reverse of elastic_kernels.py:400-402), at cell (i, j).
-template <typename T>
-__device__ __forceinline__ void vfs_adjoint(const Geo<T>& g, const T* lvx, const T* lvz, int i, int j, int64_t o,
-                                            T& ax, T& az) {
-  const int64_t P = g.L.pitch;
-  ax = lvx[o];
-  az = lvz[o];
-  if (!g.fsurf) return;
+// Adjoint of the free-surface velocity rows (reverse of elastic_kernels.py:400-402, 753-756): lambda
+// of the velocities BEFORE the rows h-3 / h-2 were overwritten, at cell (i, j). l(comp, ii, jj) is
+// the lambda after; ax, az hold l at (i, j) on entry.
+template <typename T, typename F>
+__device__ __forceinline__ void vfs_adjoint(const Geo<T>& g, int i, int j, const F& l, T& ax, T& az) {
   const int h = g.h;
   auto inJ = [&](int m) { return m >= g.jlo && m <= g.jhi; };
-  auto A = [&](int m, int64_t om) { return inJ(m) ? lvx[om] : T(0); };  // lambda vx[h-2, m] (om: offset of (h-2, m))
   if (i == h - 3) {
     if (inJ(j)) az = T(0);
   } else if (i == h - 2) {
@@ -776,32 +630,23 @@ __device__ __forceinline__ void vfs_adjoint(const Geo<T>& g, const T* lvx, const
       ax = T(0);
       az = T(0);
     } else if (inJ(j - 1)) {
-      az = lvz[o] + lvx[o - 1];
+      az += l(VX, i, j - 1);
     }
   } else if (i == h - 1) {
-    const int64_t o2 = o - P;  // (h-2, j)
-    T a_l = inJ(j - 1) ? lvx[o2 - 1] : T(0);
-    T a_c = A(j, o2);
-    T r = lvz[o] + a_l - a_c;
-    if (inJ(j)) {
-      const T b = lvz[o2 - P];  // lambda vz[h-3, j]
-      const T cval = lvz[o2] + b + a_l - a_c;
-      r += cval;
-    }
+    const T a_l = inJ(j - 1) ? l(VX, h - 2, j - 1) : T(0);
+    const T a_c = inJ(j) ? l(VX, h - 2, j) : T(0);
+    T r = az + a_l - a_c;
+    if (inJ(j)) r += l(VZ, h - 2, j) + l(VZ, h - 3, j) + a_l - a_c;
     az = r;
   } else if (i == h) {
-    if (inJ(j)) ax = lvx[o] + lvx[o - 2 * P];
+    if (inJ(j)) ax += l(VX, h - 2, j);
   }
 }
 
-// Adjoint of the free-surface stress rows (reverse of elastic_kernels.py:381-384).
+// Adjoint of the free-surface stress rows (reverse of elastic_kernels.py:381-384) at a cell of row i:
+// azz, axz hold the lambda there on entry, lzz and lxz point to it in planes of pitch P.
 template <typename T>
-__device__ __forceinline__ void tfs_adjoint(const Geo<T>& g, const T* lzz, const T* lxz, int i, int64_t o, T& azz,
-                                            T& axz) {
-  const int64_t P = g.L.pitch;
-  azz = lzz[o];
-  axz = lxz[o];
-  if (!g.fsurf) return;
+__device__ __forceinline__ void tfs_adjoint(const Geo<T>& g, const T* lzz, const T* lxz, int i, int P, T& azz, T& axz) {
   const int h = g.h;
   if (i == h - 3) axz = T(0);
   if (i == h - 2) {
@@ -810,729 +655,675 @@ __device__ __forceinline__ void tfs_adjoint(const Geo<T>& g, const T* lzz, const
   }
   if (i == h - 1) {
     azz = T(0);
-    axz = lxz[o] - lxz[o - P];
+    axz -= lxz[-P];
   }
   if (i == h) {
-    azz = lzz[o] - lzz[o - 2 * P];
-    axz = lxz[o] - lxz[o - 3 * P];
+    azz -= lzz[-2 * P];
+    axz -= lxz[-3 * P];
   }
 }
 
+// The reverse step is two launches. Each takes a group of shots per block, a tile of kAR rows x 32
+// columns with a vector of kVW columns per thread, and per shot: forms in shared memory the adjoint
+// sources of the update that it reverses (lambda after the step times coefficient times dt/dx or
+// dt/dz, zero outside I) on the tile and on the NN rows or 4 columns around it that the transposed
+// differences read, then applies the transposes and adds to the gradients in registers.
+//
+// Cells that keep split fields in the forward step have a lambda per split part, advanced here as
+// S * lambda + lambda of the total (read from one copy and written to the other, so that no block
+// reads a halo cell another block has already advanced), and the transposes overwrite the lambda
+// of the totals. In every other cell both parts of a field have the same lambda for all time (S = 1 and
+// equal increments): only its running sum is kept, in the plane of the total, to which the transposes
+// add. That is the case of all cells with an absorbing layer, whose update is unsplit.
+//
+// dL/d records: stresses are added by adj_t_step after its transposes, the velocities of the step
+// before by adj_v_step after its own.
+//
+// What bounds them is the latency of a shot's chain: copies, sources, barrier, transposes. All that a
+// shot reads is copied to shared memory while the shot before is evaluated (loads into registers
+// instead were moved to their uses by the compiler: 66 and 75 us a launch for 20 shots on a 282 x 480
+// grid, with copies 50 and 57); histories and records are copied ahead of the end of the launch
+// before. Shared memory (75 and 91 KB) and registers (80 and 128) allow three and two blocks of 256
+// threads per SM; with 3 shots per block and more the copies of all but the first shot are hidden.
+// 400 gradient steps of 20 shots on a 242 x 480 grid take 62 ms (75 with a lambda per split part in
+// every cell, tiles of 8 rows, and two launches for the dL/d records).
+constexpr int kAR = 16;
 template <typename T>
-struct Pml {
-  T xd, xn, zd, zn;
-};
-template <typename T>
-__device__ __forceinline__ Pml<T> pml_at(const Geo<T>& g, const T* cf, int64_t oc, int64_t PL) {
-  const T bcx = cf[BCX * PL + oc], bcz = cf[BCZ * PL + oc];
-  Pml<T> p;
-  p.xd = T(1) + g.hdt * bcx;
-  p.xn = T(1) - g.hdt * bcx;
-  p.zd = T(1) + g.hdt * bcz;
-  p.zn = T(1) - g.hdt * bcz;
-  return p;
-}
+constexpr int kAdjThreads = kAR * kVecX / kVW<T>;
+constexpr int kAXW = kVecX + 8;                             // an x plane's row: columns j0-4 .. j0+35
+constexpr int kAX = kAR * kAXW, kAZ = (kAR + 6) * kVecX;  // x plane: tile rows; z plane: rows i0-3 ..
+constexpr int kAH = (kAR + 6) * kAXW;                       // a history plane: z plane's rows, x plane's columns
+constexpr int kAI = kAR * kVecX;                            // a plane of the tile alone
+// one of two buffers (split lambda, then sources; lambda of the totals; history; lambda to add to), and
+// all shared memory (two buffers, dL/d records)
+constexpr int kAdjTBuf = 2 * kAX + 2 * kAZ + 2 * kAH + 3 * kAH + 3 * kAI, kAdjT = 2 * kAdjTBuf + 3 * kAI;
+constexpr int kAdjVBuf = 4 * kAX + 4 * kAZ + 3 * kAH + 2 * kAH + 2 * kAI, kAdjV = 2 * kAdjVBuf + 2 * kAI;
 
-// One plane of a (field, shot) block read at grid cells; the block's ghost frame is zero.
-template <typename T>
-struct PlaneQ {
-  const T* base;
-  Layout L;
-  __device__ __forceinline__ T operator()(int ii, int jj) const { return base[L.off(ii, jj)]; }
-};
-
-// (B4 + B3a) per shot group: the split velocities' lambda after the step (the velocity
-// free-surface adjoint, then S * lambda + lambda of the totals; read from lvs_in, written to
-// lvs_out, so that no block reads a halo cell another block has already advanced), lt = the
-// transposes of the velocity update's stress differences (the dL/d stress records of the step
-// are added after it, by adj_inject), and the bx, bz gradients. The update's adjoint sources q
-// (lambda of the split velocities times dt b / (d pml_d), zero outside I) are formed in shared
-// memory where the transposes read them. Per block the tile's factors are formed once with the
-// halo (S and dt b / (d pml_d); x factors on compact x planes, z factors on compact z planes).
-// Per shot, the lambda of the four split velocities (x parts on compact x planes, z parts on
-// compact z planes), the lambda of the velocity totals and txx, txz, tzz of the forward history
-// (full planes) are staged into one of two buffers -- the next shot's copies are in flight while
-// a shot is evaluated. Each thread then advances the lambda of its own cell (kept in registers
-// for the gradients, stored for the next step) and of at most one halo cell, and turns the
-// staged lambda into q in place; the transposes and gradients follow. 43.9 KB of shared memory
-// in single precision.
-constexpr int kAdjTShot = 2 * kXPlane + 2 * kZPlane + 5 * kSPlane;     // one shot's staged planes
-constexpr int kAdjTElems = 3 * kXPlane + 3 * kZPlane + 2 * kAdjTShot;  // factors; two shot buffers
-constexpr int kXHalo = kTileZ * 8, kZHalo = 6 * kTileX;  // halo cells of the compact x / z planes
-static_assert(kXHalo + kZHalo == kTileThreads, "one halo cell per thread");
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-#ifndef ADFWI_EL_ADJT_MINB
-#define ADFWI_EL_ADJT_MINB 5
-#endif
-template <typename T, int NN>
-__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 4 ? ADFWI_EL_ADJT_MINB : 2)
-    adj_t_pml(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lv, const T* __restrict__ lvs_in,
-              T* __restrict__ lvs_out, T* __restrict__ lt, const T* __restrict__ tt_hist, T* __restrict__ gpart,
-              int eg) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
-  griddep_launch_dependents();
-  extern __shared__ __align__(16) unsigned char el_smem[];
-  T* sFx = reinterpret_cast<T*>(el_smem);  // S_x, dt bx / (dx pml_xd), dt bz / (dx pml_xd) (x planes)
-  T* sFz = sFx + 3 * kXPlane;              // S_z, dt bx / (dz pml_zd), dt bz / (dz pml_zd) (z planes)
-  T* sB = sFz + 3 * kZPlane;               // two shot buffers
-  // a shot buffer: lambda vx_x, vz_x (x planes; q_vxx, q_vzx once formed), lambda vx_z, vz_z (z
-  // planes; q_vxz, q_vzz), lambda of the totals vx, vz, txx, txz, tzz (full planes)
-  constexpr int oLz = 2 * kXPlane, oV = oLz + 2 * kZPlane, oT = oV + 2 * kSPlane;
-  const int tiles_x = (g.L.nxp + kTileX - 1) / kTileX;
-  const int i0 = ((int)blockIdx.x / tiles_x) * kTileZ, j0 = ((int)blockIdx.x % tiles_x) * kTileX;
-  const int ty = (int)threadIdx.x / kTileX, tx = (int)threadIdx.x % kTileX;
-  const int i = i0 + ty, j = j0 + tx;
-  const bool valid = i < g.L.nzp && j < g.L.nxp, inside = valid && in_I(g, i, j);
-  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL, oc = g.L.off(i, j);
-  const int sc = kSC + ty * kSW + tx, cx = ty * kSW + tx + 4, cz = (ty + 3) * kTileX + tx;
-  // this thread's halo cell: x-plane columns j0-4 .. j0-1 and j0+32 .. j0+35, or z-plane rows
-  // i0-3 .. i0-1 and i0+8 .. i0+10
-  const bool hx = (int)threadIdx.x < kXHalo;
-  int hr, hc;  // the halo cell's row and column relative to (i0, j0)
-  if (hx) {
-    const int c8 = (int)threadIdx.x & 7;
-    hr = (int)threadIdx.x >> 3;
-    hc = c8 < 4 ? c8 - 4 : c8 + kTileX - 4;
-  } else {
-    const int t = (int)threadIdx.x - kXHalo, r6 = t / kTileX;
-    hr = r6 < 3 ? r6 - 3 : r6 + kTileZ - 3;
-    hc = t - r6 * kTileX;
-  }
-  const int hi = i0 + hr, hj = j0 + hc;
-  const bool hvalid = hi >= 0 && hi < g.L.nzp && hj >= 0 && hj < g.L.nxp;
-  const int hs = hx ? hr * kSW + hc + 4 : (hr + 3) * kTileX + hc;  // in its compact plane
-  const int hf = (hr + 3) * kSW + hc + 4;                            // in a full plane
-  EL_SHOT_GROUP
-  T* gbx = gbase + 6 * PL;
-  T* gbz = gbase + 7 * PL;
-  const T* lvx = lv + VX * NSP;
-  const T* lvz = lv + VZ * NSP;
-  auto issue = [&](int s, T* B) {
-    const int64_t so = (int64_t)s * PL;
-    stage_x(B, lvs_in + VX_X * NSP + so, g.L, i0, j0);
-    stage_x(B + kXPlane, lvs_in + VZ_X * NSP + so, g.L, i0, j0);
-    stage_z(B + oLz, lvs_in + VX_Z * NSP + so, g.L, i0, j0);
-    stage_z(B + oLz + kZPlane, lvs_in + VZ_Z * NSP + so, g.L, i0, j0);
-    stage(B + oV, lvx + so, g.L, i0, j0, 3, 4);
-    stage(B + oV + kSPlane, lvz + so, g.L, i0, j0, 3, 4);
-    stage(B + oT, tt_hist + TXX * NSP + so, g.L, i0, j0, 0, 4);
-    stage(B + oT + kSPlane, tt_hist + TXZ * NSP + so, g.L, i0, j0, 3, 4);
-    stage(B + oT + 2 * kSPlane, tt_hist + TZZ * NSP + so, g.L, i0, j0, 3, 0);
-    cp_async_commit();
-  };
-  if (s_beg < s_end) issue(s_beg, sB);
-  // the factors, formed as the per-cell adjoint forms them (S = 1 and the source factors zero
-  // outside I), while the first shot's copies land
-  for (int t = threadIdx.x; t < kXPlane; t += kTileThreads) {
-    const int ii = i0 + t / kSW, jj = j0 - 4 + t % kSW;
-    T sx = T(1), fx = T(0), fz = T(0);
-    if (in_I(g, ii, jj)) {
-      const int64_t c0 = g.L.off(ii, jj);
-      const Pml<T> p = pml_at(g, cf, c0, PL);
-      const T ix = T(1) / p.xd, kx = g.dt_dx * ix;
-      sx = p.xn * ix;
-      fx = cf[BX * PL + c0] * kx;
-      fz = cf[BZ * PL + c0] * kx;
-    }
-    sFx[t] = sx;
-    sFx[kXPlane + t] = fx;
-    sFx[2 * kXPlane + t] = fz;
-  }
-  for (int t = threadIdx.x; t < kZPlane; t += kTileThreads) {
-    const int ii = i0 - 3 + t / kTileX, jj = j0 + t % kTileX;
-    T sz = T(1), fx = T(0), fz = T(0);
-    if (in_I(g, ii, jj)) {
-      const int64_t c0 = g.L.off(ii, jj);
-      const Pml<T> p = pml_at(g, cf, c0, PL);
-      const T iz = T(1) / p.zd, kz = g.dt_dz * iz;
-      sz = p.zn * iz;
-      fx = cf[BX * PL + c0] * kz;
-      fz = cf[BZ * PL + c0] * kz;
-    }
-    sFz[t] = sz;
-    sFz[kZPlane + t] = fx;
-    sFz[2 * kZPlane + t] = fz;
-  }
-  // (the barrier after the first shot's copies orders these writes before their reads)
-  // d(v_x')/d(bx) = dt * D(T) / (d * pml_d), likewise for bz: the cell's factors dt / (d pml_d)
-  T kx = T(0), kz = T(0), gx = T(0), gz = T(0);
-  if (inside) {
-    const Pml<T> p = pml_at(g, cf, oc, PL);
-    kx = g.dt / (g.dx * p.xd);
-    kz = g.dt / (g.dz * p.zd);
-  }
-  // rows whose totals' lambda the velocity free-surface adjoint combines across cells
-  const int fs_lo = g.fsurf ? g.h - 3 : 1 << 30, fs_hi = g.fsurf ? g.h : -1;
-  auto q_of = [](T v, T f) { return f != T(0) ? v * f : T(0); };
-  for (int s = s_beg; s < s_end; ++s) {
-    T* B = sB + ((s - s_beg) & 1) * kAdjTShot;
-    if (s + 1 < s_end) {
-      issue(s + 1, sB + ((s + 1 - s_beg) & 1) * kAdjTShot);  // into the buffer the previous shot used
-      cp_async_wait_group<1>();
-    } else {
-      cp_async_wait_group<0>();
-    }
-    __syncthreads();
-    const int64_t so = (int64_t)s * PL;
-    T* sLx = B;
-    T* sLz = B + oLz;
-    // own cell: lambda after the step (cells outside the grid keep their zero), stored; q
-    T vxx = sLx[cx], vzx = sLx[kXPlane + cx], vxz = sLz[cz], vzz = sLz[kZPlane + cz];
-    if (valid) {
-      const int64_t o = so + oc;
-      T ax = B[oV + sc], az = B[oV + kSPlane + sc];
-      if (i >= fs_lo && i <= fs_hi) vfs_adjoint(g, lvx, lvz, i, j, o, ax, az);
-      const T sx = sFx[cx], sz = sFz[cz];
-      vxx = sx * vxx + ax;
-      vzx = sx * vzx + az;
-      vxz = sz * vxz + ax;
-      vzz = sz * vzz + az;
-      lvs_out[VX_X * NSP + o] = vxx;
-      lvs_out[VZ_X * NSP + o] = vzx;
-      lvs_out[VX_Z * NSP + o] = vxz;
-      lvs_out[VZ_Z * NSP + o] = vzz;
-    }
-    sLx[cx] = q_of(vxx, sFx[kXPlane + cx]);
-    sLx[kXPlane + cx] = q_of(vzx, sFx[2 * kXPlane + cx]);
-    sLz[cz] = q_of(vxz, sFz[kZPlane + cz]);
-    sLz[kZPlane + cz] = q_of(vzz, sFz[2 * kZPlane + cz]);
-    // halo cell: lambda after the step (not stored: another block owns the cell); q
-    {
-      T* hl = hx ? sLx + hs : sLz + hs;
-      const int HP = hx ? kXPlane : kZPlane;
-      const T* hF = hx ? sFx + hs : sFz + hs;
-      T va = hl[0], vb = hl[HP];
-      if (hvalid) {
-        T ax = B[oV + hf], az = B[oV + kSPlane + hf];
-        if (hi >= fs_lo && hi <= fs_hi) vfs_adjoint(g, lvx, lvz, hi, hj, so + g.L.off(hi, hj), ax, az);
-        const T sh = hF[0];
-        va = sh * va + ax;
-        vb = sh * vb + az;
-      }
-      hl[0] = q_of(va, hF[HP]);
-      hl[HP] = q_of(vb, hF[2 * HP]);
-    }
-    __syncthreads();
-    if (valid) {
-      const StagedX<T> q_vxx{sLx, i0, j0}, q_vzx{sLx + kXPlane, i0, j0};
-      const StagedZ<T> q_vxz{sLz, i0, j0}, q_vzz{sLz + kZPlane, i0, j0};
-      const T* sT = B + oT;
-      const int64_t o = so + oc;
-      lt[TXX * NSP + o] = dxf_t<NN>(g, q_vxx, i, j);
-      lt[TXZ * NSP + o] = dzb_t<NN>(g, q_vxz, i, j) + dxb_t<NN>(g, q_vzx, i, j);
-      lt[TZZ * NSP + o] = dzf_t<NN>(g, q_vzz, i, j);
-      if (inside) {
-        gx += vxx * dxf<NN>(g, sT, sc) * kx + vxz * dzb<NN>(g, sT + kSPlane, sc, kSW) * kz;
-        gz += vzx * dxb<NN>(g, sT + kSPlane, sc) * kx + vzz * dzf<NN>(g, sT + 2 * kSPlane, sc, kSW) * kz;
-      }
-    }
-    __syncthreads();  // this buffer is refilled by the copies of the shot after next
-  }
-  if (inside) {
-    gbx[oc] += gx;
-    gbz[oc] += gz;
-  }
-}
-
-// Coefficient-weighted adjoint sources of the stress update at cell (ii, jj):
-// q[0..5] = lambda of txx_x, txx_z, tzz_x, tzz_z, txz_x, txz_z times their d(update)/d(C D v).
-template <typename T>
-struct StressQ {
-  T a, b, c, d, e, f;  // xx_x, xx_z, zz_x, zz_z, xz_x, xz_z
-};
-
-// Coefficient-weighted adjoint sources of the stress update at cell (i, j) of one shot.
-// The cell's factors: dt/dx / pml_xd and dt/dz / pml_zd (PML form), dt/dx and dt/dz (ABL form).
-template <typename T, bool PMLM>
-__device__ __forceinline__ void stress_k(const Geo<T>& g, const T* __restrict__ cf, int64_t c0, int64_t PL, T& kx,
-                                         T& kz) {
-  if (PMLM) {
-    const Pml<T> p = pml_at(g, cf, c0, PL);
-    kx = g.dt_dx / p.xd;
-    kz = g.dt_dz / p.zd;
-  } else {
-    kx = g.dt / g.dx;
-    kz = g.dt / g.dz;
-  }
-}
-template <typename T, bool PMLM>
-__device__ __forceinline__ StressQ<T> stress_q(const T* lts, int64_t oo, int64_t NSP, T kx, T kz) {
-  StressQ<T> r;
-  if (PMLM) {
-    r.a = lts[TXX_X * NSP + oo] * kx;
-    r.b = lts[TXX_Z * NSP + oo] * kz;
-    r.c = lts[TZZ_X * NSP + oo] * kx;
-    r.d = lts[TZZ_Z * NSP + oo] * kz;
-    r.e = lts[TXZ_X * NSP + oo] * kx;
-    r.f = lts[TXZ_Z * NSP + oo] * kz;
-  } else {
-    r.a = lts[TXX * NSP + oo] * kx;
-    r.b = lts[TXX * NSP + oo] * kz;
-    r.c = lts[TZZ * NSP + oo] * kx;
-    r.d = lts[TZZ * NSP + oo] * kz;
-    r.e = lts[TXZ * NSP + oo] * kx;
-    r.f = lts[TXZ * NSP + oo] * kz;
-  }
+// f_k (q[-k] - q[1+k]): a transposed half-cell difference (gather form); `at(m)` as in Fd
+template <int NN, typename T, typename A>
+__device__ __forceinline__ T diff_t(const Geo<T>& g, const A& at) {
+  T r = g.f0 * (at(0) - at(1)) + g.f1 * (at(-1) - at(2));
+  if (NN == 3) r += g.f2 * (at(-2) - at(3));
   return r;
 }
 
-// (B1q) the stress update's adjoint sources for the velocity transposes at a cell (c0) of one shot
-// (o), zero outside I: sx_b, sx_zb, sx_f, sx_zf, sz_b, sz_zb, sz_f, sz_zf.
-template <typename T, bool PMLM>
-__device__ __forceinline__ void stress_sources(const Geo<T>& g, const T* __restrict__ cf, const T* lts, int i, int j,
-                                               int64_t o, T* __restrict__ q8) {
-  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL;
-  T v[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = T(0);
-  if (in_I(g, i, j)) {
-    const int64_t c0 = g.L.off(i, j);
-    T kx, kz;
-    stress_k<T, PMLM>(g, cf, c0, PL, kx, kz);
-    const StressQ<T> r = stress_q<T, PMLM>(lts, o, NSP, kx, kz);
-    const T c11 = cf[C11 * PL + c0], c13 = cf[C13 * PL + c0], c15 = cf[C15 * PL + c0];
-    const T c33 = cf[C33 * PL + c0], c35 = cf[C35 * PL + c0], c55 = cf[C55 * PL + c0];
-    v[0] = c11 * r.a + c13 * r.c;
-    v[1] = c15 * r.b + c35 * r.d;
-    v[2] = c15 * r.e;
-    v[3] = c55 * r.f;
-    v[4] = c15 * r.a + c35 * r.c;
-    v[5] = c13 * r.b + c33 * r.d;
-    v[6] = c55 * r.e;
-    v[7] = c35 * r.f;
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) q8[k * NSP + o] = v[k];
-}
-template <typename T, bool PMLM>
-__global__ void adj_vq(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lts, T* __restrict__ q8) {
-  griddep_wait();
-  griddep_launch_dependents();
-  EL_CELL_SHOT
-  stress_sources<T, PMLM>(g, cf, lts, i, j, o, q8);
-}
-
-// (B1a) lambda of the velocity totals at the start of the step (overwrite) and the C gradients.
-// pml = 1: split-field update; pml = 0: absorbing-layer update (lts then holds txx, tzz, txz,
-// and lv is accumulated instead of overwritten because v' = v + ...).
-// Staged planes per shot: 0-7 the stress update's adjoint sources (sx_b x, sx_zb z, sx_f x,
-// sx_zf z, sz_b x, sz_zb z, sz_f x, sz_zf z), 8-9 vx, vz of the forward history (x, z),
-// 10.. lambda of the (split) stresses (6 with the PML, 3 without).
-template <bool PMLM>
-constexpr int adj_v_planes() {
-  return PMLM ? 16 : 13;
-}
-template <typename T, int NN, bool PMLM>
-__global__ void __launch_bounds__(kTileThreads)
-    adj_v(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lts, const T* __restrict__ q8,
-          T* __restrict__ lv, const T* __restrict__ v_hist, T* __restrict__ gpart, int eg) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
-  griddep_launch_dependents();
-  extern __shared__ __align__(16) unsigned char el_smem[];
-  T* sm = reinterpret_cast<T*>(el_smem);
-  const int tiles_x = (g.L.nxp + kTileX - 1) / kTileX;
-  const int i0 = ((int)blockIdx.x / tiles_x) * kTileZ, j0 = ((int)blockIdx.x % tiles_x) * kTileX;
-  const int ty = (int)threadIdx.x / kTileX, tx = (int)threadIdx.x % kTileX;
-  const int i = i0 + ty, j = j0 + tx;
-  const bool valid = i < g.L.nzp && j < g.L.nxp, inside = valid && in_I(g, i, j);
-  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL, oc = g.L.off(i, j);
-  const int sc = kSC + ty * kSW + tx;
-  EL_SHOT_GROUP
-  T* gc = gbase;
-  T g11 = T(0), g13 = T(0), g15 = T(0), g33 = T(0), g35 = T(0), g55 = T(0);
-  T kx = T(0), kz = T(0);
-  if (inside) stress_k<T, PMLM>(g, cf, oc, PL, kx, kz);
-  constexpr int nst = PMLM ? 6 : 3;
-  for (int s = s_beg; s < s_end; ++s) {
-    const int64_t so = (int64_t)s * PL;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      stage(sm + k * kSPlane, q8 + k * NSP + so, g.L, i0, j0, (k & 1) ? 3 : 0, (k & 1) ? 0 : 4);
-    stage(sm + 8 * kSPlane, v_hist + VX * NSP + so, g.L, i0, j0, 3, 4);
-    stage(sm + 9 * kSPlane, v_hist + VZ * NSP + so, g.L, i0, j0, 3, 4);
-#pragma unroll
-    for (int k = 0; k < nst; ++k) stage(sm + (10 + k) * kSPlane, lts + k * NSP + so, g.L, i0, j0, 0, 0);
-    cp_async_wait_all();
-    __syncthreads();
-    if (valid) {
-      const StagedQ<T> q0{sm, i0, j0}, q1{sm + kSPlane, i0, j0}, q2{sm + 2 * kSPlane, i0, j0},
-          q3{sm + 3 * kSPlane, i0, j0}, q4{sm + 4 * kSPlane, i0, j0}, q5{sm + 5 * kSPlane, i0, j0},
-          q6{sm + 6 * kSPlane, i0, j0}, q7{sm + 7 * kSPlane, i0, j0};
-      const T avx = dxb_t<NN>(g, q0, i, j) + dzb_t<NN>(g, q1, i, j) + dxf_t<NN>(g, q2, i, j) + dzf_t<NN>(g, q3, i, j);
-      const T avz = dxb_t<NN>(g, q4, i, j) + dzb_t<NN>(g, q5, i, j) + dxf_t<NN>(g, q6, i, j) + dzf_t<NN>(g, q7, i, j);
-      const int64_t o = so + oc;
-      if (PMLM) {
-        lv[VX * NSP + o] = avx;
-        lv[VZ * NSP + o] = avz;
-      } else {
-        lv[VX * NSP + o] += avx;
-        lv[VZ * NSP + o] += avz;
-      }
-      if (inside) {
-        const StressQ<T> r = stress_q<T, PMLM>(sm + 10 * kSPlane + sc, 0, kSPlane, kx, kz);
-        const T* vx = sm + 8 * kSPlane;
-        const T* vz = sm + 9 * kSPlane;
-        const T dxb_vx = dxb<NN>(g, vx, sc), dxb_vz = dxb<NN>(g, vz, sc);
-        const T dzb_vx = dzb<NN>(g, vx, sc, kSW), dzb_vz = dzb<NN>(g, vz, sc, kSW);
-        const T dxf_vx = dxf<NN>(g, vx, sc), dxf_vz = dxf<NN>(g, vz, sc);
-        const T dzf_vx = dzf<NN>(g, vx, sc, kSW), dzf_vz = dzf<NN>(g, vz, sc, kSW);
-        g11 += r.a * dxb_vx;
-        g13 += r.b * dzb_vz + r.c * dxb_vx;
-        g15 += r.a * dxb_vz + r.b * dzb_vx + r.e * dxf_vx;
-        g33 += r.d * dzb_vz;
-        g35 += r.c * dxb_vz + r.d * dzb_vx + r.f * dzf_vz;
-        g55 += r.e * dxf_vz + r.f * dzf_vx;
-      }
-    }
-    __syncthreads();  // the next shot's copies overwrite the staged planes
-  }
-  if (inside) {
-    gc[C11 * PL + oc] += g11;
-    gc[C13 * PL + oc] += g13;
-    gc[C15 * PL + oc] += g15;
-    gc[C33 * PL + oc] += g33;
-    gc[C35 * PL + oc] += g35;
-    gc[C55 * PL + oc] += g55;
-  }
-}
-
-// (B2 + B1a, PML) per shot group: the split stresses' lambda after the step (the stress
-// free-surface adjoint, then S * lambda + lambda of the totals; read from lts_in, written to
-// lts_out, so that no block reads a halo cell another block has already advanced), lambda of the
-// velocity totals at the start of the step (overwrite) and the C gradients, with the stress
-// update's adjoint sources formed in shared memory. Per block the tile's cell coefficients
-// C11 .. C55 (full planes, with the halo) are staged once and the factors S_x and dt/dx / pml_xd
-// (compact x planes), S_z and dt/dz / pml_zd (compact z planes; S = 1 and the source factors zero
-// outside I) formed once. Per shot the lambda of the six split stresses (x parts on compact x
-// planes, z parts on compact z planes), the lambda of the stress totals and vx, vz of the
-// forward history (full planes) are staged into one of two buffers -- the next shot's copies
-// are in flight while a shot is evaluated. Each thread then advances the lambda of its own cell
-// (stored for the next step; its weighted lambda kept for the gradients) and of at most one
-// halo cell and forms their eight sources q (sx_b, sx_zb, sx_f, sx_zf, sz_b, sz_zb, sz_f, sz_zf:
-// coefficient-weighted lambda, zero outside I), three of each four over the lambda they are
-// formed from; the transposes and gradients follow. 63.5 KB of shared memory in single
-// precision.
-constexpr int kAdjVShot = 3 * kXPlane + 3 * kZPlane + 5 * kSPlane;  // one shot's staged planes
-constexpr int kAdjVPmlElems = 6 * kSPlane + 3 * kXPlane + 3 * kZPlane + 2 * kAdjVShot;  // C, factors, q; buffers
+// A thread's vector of the tile and the vector of the tile's halo that it also forms sources for.
 template <typename T, int NN>
-__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 4 ? 3 : 1)
-    adj_v_pml(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lt, const T* __restrict__ lts_in,
-              T* __restrict__ lts_out, T* __restrict__ lv, const T* __restrict__ v_hist, T* __restrict__ gpart,
-              int eg) {
-  griddep_wait();  // launched with programmatic serialisation in the PML time loops
-  griddep_launch_dependents();
-  extern __shared__ __align__(16) unsigned char el_smem[];
-  T* sC = reinterpret_cast<T*>(el_smem);  // 6 full planes
-  T* sKx = sC + 6 * kSPlane;              // S_x, dt/dx / pml_xd (x planes)
-  T* sKz = sKx + 2 * kXPlane;             // S_z, dt/dz / pml_zd (z planes)
-  T* sQx = sKz + 2 * kZPlane;             // the fourth x source q6 (x plane)
-  T* sQz = sQx + kXPlane;                 // the fourth z source q7 (z plane)
-  T* sB = sQz + kZPlane;                  // two shot buffers
-  // a shot buffer: lambda txx_x, tzz_x, txz_x (x planes; then q0, q2, q4), lambda txx_z, tzz_z,
-  // txz_z (z planes; then q1, q3, q5), lambda of txx, tzz, txz, and vx, vz (full planes)
-  constexpr int oLz = 3 * kXPlane, oA = oLz + 3 * kZPlane, oV = oA + 3 * kSPlane;
-  const int tiles_x = (g.L.nxp + kTileX - 1) / kTileX;
-  const int i0 = ((int)blockIdx.x / tiles_x) * kTileZ, j0 = ((int)blockIdx.x % tiles_x) * kTileX;
-  const int ty = (int)threadIdx.x / kTileX, tx = (int)threadIdx.x % kTileX;
-  const int i = i0 + ty, j = j0 + tx;
-  const bool valid = i < g.L.nzp && j < g.L.nxp, inside = valid && in_I(g, i, j);
-  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL, oc = g.L.off(i, j);
-  const int sc = kSC + ty * kSW + tx, cx = ty * kSW + tx + 4, cz = (ty + 3) * kTileX + tx;
-  // this thread's halo cell: x-plane columns j0-4 .. j0-1 and j0+32 .. j0+35, or z-plane rows
-  // i0-3 .. i0-1 and i0+8 .. i0+10
-  const bool hx = (int)threadIdx.x < kXHalo;
-  int hr, hc;  // the halo cell's row and column relative to (i0, j0)
-  if (hx) {
-    const int c8 = (int)threadIdx.x & 7;
-    hr = (int)threadIdx.x >> 3;
-    hc = c8 < 4 ? c8 - 4 : c8 + kTileX - 4;
-  } else {
-    const int t = (int)threadIdx.x - kXHalo, r6 = t / kTileX;
-    hr = r6 < 3 ? r6 - 3 : r6 + kTileZ - 3;
-    hc = t - r6 * kTileX;
-  }
-  const int hi = i0 + hr, hj = j0 + hc;
-  const bool hvalid = hi >= 0 && hi < g.L.nzp && hj >= 0 && hj < g.L.nxp;
-  const int hs = hx ? hr * kSW + hc + 4 : (hr + 3) * kTileX + hc;  // in its compact plane
-  const int hf = (hr + 3) * kSW + hc + 4;                            // in a full plane
-  EL_SHOT_GROUP
-  T* gc = gbase;
-  const T* lxx = lt + TXX * NSP;
-  const T* lzz = lt + TZZ * NSP;
-  const T* lxz = lt + TXZ * NSP;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) stage(sC + k * kSPlane, cf + (C11 + k) * PL, g.L, i0, j0, 3, 4);
-  cp_async_commit();
-  auto issue = [&](int s, T* B) {
-    const int64_t so = (int64_t)s * PL;
-    // the x parts of the split stresses feed the sources of x differences, the z parts those of
-    // z differences
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      stage_x(B + k * kXPlane, lts_in + (2 * k) * NSP + so, g.L, i0, j0);
-      stage_z(B + oLz + k * kZPlane, lts_in + (2 * k + 1) * NSP + so, g.L, i0, j0);
-    }
-    stage(B + oA, lxx + so, g.L, i0, j0, 3, 4);
-    stage(B + oA + kSPlane, lzz + so, g.L, i0, j0, 3, 4);
-    stage(B + oA + 2 * kSPlane, lxz + so, g.L, i0, j0, 3, 4);
-    stage(B + oV, v_hist + VX * NSP + so, g.L, i0, j0, 3, 4);
-    stage(B + oV + kSPlane, v_hist + VZ * NSP + so, g.L, i0, j0, 3, 4);
-    cp_async_commit();
-  };
-  if (s_beg < s_end) issue(s_beg, sB);
-  // the factors, formed as the per-cell adjoint forms them, while the first copies land
-  for (int t = threadIdx.x; t < kXPlane; t += kTileThreads) {
-    const int ii = i0 + t / kSW, jj = j0 - 4 + t % kSW;
-    T sx = T(1), kx = T(0);
-    if (in_I(g, ii, jj)) {
-      const int64_t c0 = g.L.off(ii, jj);
-      const Pml<T> p = pml_at(g, cf, c0, PL);
-      sx = p.xn * (T(1) / p.xd);
-      kx = g.dt_dx / (T(1) + g.hdt * cf[BCX * PL + c0]);
-    }
-    sKx[t] = sx;
-    sKx[kXPlane + t] = kx;
-  }
-  for (int t = threadIdx.x; t < kZPlane; t += kTileThreads) {
-    const int ii = i0 - 3 + t / kTileX, jj = j0 + t % kTileX;
-    T sz = T(1), kz = T(0);
-    if (in_I(g, ii, jj)) {
-      const int64_t c0 = g.L.off(ii, jj);
-      const Pml<T> p = pml_at(g, cf, c0, PL);
-      sz = p.zn * (T(1) / p.zd);
-      kz = g.dt_dz / (T(1) + g.hdt * cf[BCZ * PL + c0]);
-    }
-    sKz[t] = sz;
-    sKz[kZPlane + t] = kz;
-  }
-  // (the barrier after the first shot's copies orders these writes before their reads)
-  // rows whose totals' lambda the stress free-surface adjoint combines across cells
-  const int fs_lo = g.fsurf ? g.h - 3 : 1 << 30, fs_hi = g.fsurf ? g.h : -1;
-  T g11 = T(0), g13 = T(0), g15 = T(0), g33 = T(0), g35 = T(0), g55 = T(0);
-  for (int s = s_beg; s < s_end; ++s) {
-    T* B = sB + ((s - s_beg) & 1) * kAdjVShot;
-    if (s + 1 < s_end) {
-      issue(s + 1, sB + ((s + 1 - s_beg) & 1) * kAdjVShot);  // into the buffer the previous shot used
-      cp_async_wait_group<1>();
+struct AdjTile {
+  static constexpr int W = kVW<T>, NX = kAR * 8 / W, NZ = 2 * NN * kVecX / W;  // halo vectors beside, above and below
+  static_assert(NX + NZ <= kAdjThreads<T>, "one halo vector per thread");
+  int i0, j0;            // the tile's first cell
+  int i, j, px, pz, ph, pi;  // own vector; its place in an x, a z and a history plane and in the tile
+  int hi, hj, hp, hph;   // halo vector, its place (x plane if hx, else z plane) and in a history plane
+  bool valid, halo, hx;  // on the grid; has a halo vector on the grid or beside it
+  __device__ __forceinline__ explicit AdjTile(const Layout& L) {
+    const int tiles_x = (L.nxp + kVecX - 1) / kVecX, t = threadIdx.x;
+    i0 = ((int)blockIdx.x / tiles_x) * kAR;
+    j0 = ((int)blockIdx.x % tiles_x) * kVecX;
+    const int r = t / (kVecX / W), c = t % (kVecX / W) * W;
+    i = i0 + r;
+    j = j0 + c;
+    px = r * kAXW + c + 4;
+    pz = (r + 3) * kVecX + c;
+    ph = (r + 3) * kAXW + c + 4;
+    pi = r * kVecX + c;
+    valid = i < L.nzp && j < L.nxp;
+    hx = t < NX;
+    halo = t < NX + NZ;
+    if (hx) {
+      const int hr = t / (8 / W), k = t % (8 / W) * W;
+      hi = i0 + hr;
+      hj = j0 + (k < 4 ? k - 4 : kVecX + k - 4);
+      hp = hr * kAXW + hj - j0 + 4;
     } else {
-      cp_async_wait_group<0>();
+      const int u = t - NX, k = u / (kVecX / W);
+      const int hr = k < NN ? k - NN : kAR + k - NN;
+      hi = i0 + hr;
+      hj = j0 + u % (kVecX / W) * W;
+      hp = (hr + 3) * kVecX + hj - j0;
     }
-    __syncthreads();
+    hph = (hi - i0 + 3) * kAXW + hj - j0 + 4;
+  }
+};
+
+// Copies of N planes (`stride` apart) around the tile into shared memory planes of ROWS rows and COLS
+// columns, from row i0 - ZH and column j0 - XH, left in flight. Every copy is 16 bytes on a 16-byte
+// boundary (j0 is a multiple of 32, rows start at multiples of 128 bytes, the ghost frame is 4 columns
+// wide) and lies in the plane's allocation, which keeps 4 rows and columns before the grid and 20 rows
+// and 64 columns after it.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+template <int N, int ROWS, int COLS, int ZH, int XH, typename T>
+__device__ __forceinline__ void stage(const Geo<T>& g, T* dst, const T* src, int64_t stride, int i0, int j0) {
+  constexpr int E = 16 / (int)sizeof(T), C = COLS / E;
+#pragma unroll
+  for (int t0 = 0; t0 < ROWS * C; t0 += kAdjThreads<T>) {
+    const int t = t0 + (int)threadIdx.x;
+    if (t >= ROWS * C) break;
+    const int r = t / C, c = t % C * E;
+    const T* from = src + g.L.off(i0 - ZH + r, j0 - XH + c);
+#pragma unroll
+    for (int k = 0; k < N; ++k) cp_async16(dst + k * (ROWS * COLS) + r * COLS + c, from + k * stride);
+  }
+}
+template <int N, typename T>
+__device__ __forceinline__ void stage_full(const Geo<T>& g, T* dst, const T* src, int64_t stride, int i0, int j0) {
+  stage<N, kAR + 6, kAXW, 3, 4>(g, dst, src, stride, i0, j0);
+}
+
+// The factors of a vector: 1 + dt/2 d inverted times dt/dx (k) and the decay S of a split lambda.
+// unit: bit e set where cell e keeps no split fields (only cells of I can); in: cells of I.
+template <typename T, bool PML>
+struct AdjFactors {
+  T kx[kVW<T>], kz[kVW<T>], sx[kVW<T>], sz[kVW<T>];
+  unsigned in = 0, unit = 0;
+  __device__ __forceinline__ AdjFactors(const Geo<T>& g, const T* cf, int i, int j) {
+    Vec<T> bx, bz;
+    const bool near = i >= g.ilo && i <= g.ihi && j + kVW<T> > g.jlo && j <= g.jhi;
+    if (PML && near) {
+      bx = ldv(cf + BCX * g.L.plane + g.L.off(i, j));
+      bz = ldv(cf + BCZ * g.L.plane + g.L.off(i, j));
+    }
+#pragma unroll
+    for (int e = 0; e < kVW<T>; ++e) {
+      const bool ok = in_I(g, i, j + e);
+      kx[e] = ok ? g.dt_dx : T(0);
+      kz[e] = ok ? g.dt_dz : T(0);
+      sx[e] = sz[e] = T(1);
+      if (ok) in |= 1u << e;
+      if (PML && ok) {
+        const T ix = pml_inv(T(1) + g.hdt * bx.v[e]), iz = pml_inv(T(1) + g.hdt * bz.v[e]);
+        kx[e] *= ix;
+        kz[e] *= iz;
+        sx[e] = (T(1) - g.hdt * bx.v[e]) * ix;
+        sz[e] = (T(1) - g.hdt * bz.v[e]) * iz;
+        if (!keeps_split(g, i, bx.v[e], bz.v[e])) unit |= 1u << e;
+      }
+    }
+    if (!PML) unit = (1u << kVW<T>) - 1u;
+  }
+  __device__ __forceinline__ bool split() const { return PML && (in & ~unit) != 0u; }
+};
+
+// Lambda of the velocities of the vector at (i, j) (place ph in the staged planes l, j0 the tile's first
+// column) with the reverse of the damping (d) and of the free-surface rows, which lie in the first
+// row of tiles.
+template <typename T, bool PML>
+__device__ __forceinline__ void adj_vel_totals(const Geo<T>& g, const T* cf, const T* l, int ph, int j0, const Vec<T>& d,
+                                               int i, int j, Vec<T>& ax, Vec<T>& az) {
+  ax = ldv(l + VX * kAH + ph);
+  az = ldv(l + VZ * kAH + ph);
+  if (!PML) {
+#pragma unroll
+    for (int e = 0; e < kVW<T>; ++e) {
+      ax.v[e] *= d.v[e];
+      az.v[e] *= d.v[e];
+    }
+  }
+  if (g.fsurf && i >= g.h - 3 && i <= g.h) {
+    auto at = [&](int comp, int ii, int jj) {
+      const T v = l[comp * kAH + (ii + 3) * kAXW + max(jj - j0 + 4, 0)];
+      return PML ? v : cf[DAMP * g.L.plane + g.L.off(ii, jj)] * v;
+    };
+#pragma unroll
+    for (int e = 0; e < kVW<T>; ++e) vfs_adjoint(g, i, j + e, at, ax.v[e], az.v[e]);
+  }
+}
+
+// dL/d records of one step at the receivers of this block's tile, NC components of them: each thread
+// takes a receiver cell (unique cells, so no two threads share one), reads its traces ahead of their
+// use and leaves their sum in shared memory planes of the tile's cells, from which the owner of the
+// cell adds it to its lambda. Read where they were needed, they were a chain of five dependent loads
+// that every shot of a tile with receivers waited for (12 us of a launch of one shot).
+template <typename T, int NC>
+struct Inject {
+  int beg, end, cell = 0, m0 = 0, m1 = 0;
+  const T* grec;  // the first component's records of the step, shot 0
+  T a[NC] = {};
+  __device__ __forceinline__ Inject(const Geo<T>& g, const T* gr, int c0, int it) : beg((int)threadIdx.x), end(0) {
+    if (gr == nullptr || it < 0) return;
+    grec = gr + ((int64_t)c0 * g.ns * g.nt + it) * g.nr;
+    beg = g.tile_beg[blockIdx.x] + (int)threadIdx.x;
+    end = g.tile_beg[blockIdx.x + 1];
+    if (beg < end) take(g, beg);
+  }
+  __device__ __forceinline__ void take(const Geo<T>& g, int q) {
+    const int zx = g.ucell_zx[q];
+    cell = (zx >> 16) % kAR * kVecX + (zx & 0xffff) % kVecX;
+    m0 = g.ucell_beg[q];
+    m1 = g.ucell_beg[q + 1];
+  }
+  // whether the tile has receivers (uniform over the block)
+  __device__ __forceinline__ bool any() const { return end - beg + (int)threadIdx.x > 0; }
+  __device__ __forceinline__ void fetch(const Geo<T>& g, int s) {
+    if (beg >= end) return;
+    const int64_t RS = (int64_t)g.ns * g.nt * g.nr;
+    const T* e = grec + (int64_t)s * g.nt * g.nr;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) a[c] = T(0);
+    for (int m = m0; m < m1; ++m) {
+      const int r = g.ucell_rcv[m];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) a[c] += e[c * RS + r];
+    }
+  }
+  // the fetched sums into the planes; a tile with more receiver cells than threads reads the rest here
+  __device__ __forceinline__ void put(const Geo<T>& g, int s, T* planes) {
+    for (int q = beg; q < end;) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) planes[c * kAI + cell] = a[c];
+      q += kAdjThreads<T>;
+      if (q < end) take(g, q), fetch(g, s);
+    }
+    if (end - beg > kAdjThreads<T>) take(g, beg);
+  }
+};
+
+// Reverse of the velocity update: lambda of the (split) velocities after the step (lvs_in -> lvs_out
+// with PML; lv -> lv_out with an absorbing layer), lt from the transposes of its stress differences,
+// dL/d stress records of step it, and the bx, bz gradients.
+template <typename T, int NN, bool PML>
+__global__ void __launch_bounds__(kAdjThreads<T>, sizeof(T) == 4 ? (PML ? 3 : 2) : 1)
+    adj_t_step(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ lv, T* __restrict__ lv_out,
+               const T* __restrict__ lvs_in, T* __restrict__ lvs_out, T* lt, const T* __restrict__ tt_hist,
+               const T* __restrict__ grec, T* gpart, int eg) {
+  extern __shared__ __align__(16) unsigned char el_smem[];
+  constexpr int W = kVW<T>;
+  const AdjTile<T, NN> p(g.L);
+  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL;
+  const int64_t oc = g.L.off(p.i, p.j), oh = g.L.off(p.hi, p.hj);
+  EL_SHOT_GROUP
+  // coefficients are not written by the launches before
+  const AdjFactors<T, PML> f(g, cf, p.i, p.j), fh(g, cf, p.halo ? p.hi : -1, p.hj);
+  Vec<T> bx{}, bz{}, hbx{}, hbz{};
+  if (f.in) {
+    bx = ldv(cf + BX * PL + oc);
+    bz = ldv(cf + BZ * PL + oc);
+  }
+  if (fh.in) {
+    hbx = ldv(cf + BX * PL + oh);
+    hbz = ldv(cf + BZ * PL + oh);
+  }
+  Vec<T> gx{}, gz{};
+  Vec<T> damp{}, hdamp{};
+  if (!PML) {
+    if (p.valid) damp = ldv(cf + DAMP * PL + oc);
+    if (fh.in) hdamp = ldv(cf + DAMP * PL + oh);
+  }
+  auto buffer = [&](int s) { return reinterpret_cast<T*>(el_smem) + ((s - s_beg) & 1) * kAdjTBuf; };
+  const bool any_split = PML && __syncthreads_or(f.split() || fh.split());
+  const bool any_unit = !PML || __syncthreads_or(f.unit);
+  auto stage_shot = [&](int s) {
+    T* b = buffer(s);
     const int64_t so = (int64_t)s * PL;
-    T* sLx = B;
-    T* sLz = B + oLz;
-    const T* sA = B + oA;
-    // own cell: lambda after the step (stored), the stress update's sources at the cell
-    // (stress_q's PML form), then q
-    StressQ<T> r;
-    {
-      T lxx_x = sLx[cx], lzz_x = sLx[kXPlane + cx], lxz_x = sLx[2 * kXPlane + cx];
-      T lxx_z = sLz[cz], lzz_z = sLz[kZPlane + cz], lxz_z = sLz[2 * kZPlane + cz];
-      if (valid) {
-        const int64_t o = so + oc;
-        const T axx = sA[sc];
-        T azz = sA[kSPlane + sc], axz = sA[2 * kSPlane + sc];
-        if (i >= fs_lo && i <= fs_hi) tfs_adjoint(g, lzz, lxz, i, o, azz, axz);
-        const T sx = sKx[cx], sz = sKz[cz];
-        lxx_x = sx * lxx_x + axx;
-        lxx_z = sz * lxx_z + axx;
-        lzz_x = sx * lzz_x + azz;
-        lzz_z = sz * lzz_z + azz;
-        lxz_x = sx * lxz_x + axz;
-        lxz_z = sz * lxz_z + axz;
-        lts_out[TXX_X * NSP + o] = lxx_x;
-        lts_out[TXX_Z * NSP + o] = lxx_z;
-        lts_out[TZZ_X * NSP + o] = lzz_x;
-        lts_out[TZZ_Z * NSP + o] = lzz_z;
-        lts_out[TXZ_X * NSP + o] = lxz_x;
-        lts_out[TXZ_Z * NSP + o] = lxz_z;
-      }
-      const T kx = sKx[kXPlane + cx], kz = sKz[kZPlane + cz];
-      r.a = lxx_x * kx;
-      r.c = lzz_x * kx;
-      r.e = lxz_x * kx;
-      r.b = lxx_z * kz;
-      r.d = lzz_z * kz;
-      r.f = lxz_z * kz;
-      const T c11 = sC[sc], c13 = sC[kSPlane + sc], c15 = sC[2 * kSPlane + sc];
-      const T c33 = sC[3 * kSPlane + sc], c35 = sC[4 * kSPlane + sc], c55 = sC[5 * kSPlane + sc];
-      T a = T(0), b = T(0), c = T(0), d = T(0);
-      if (kx != T(0)) {  // inside I (the factor is positive there)
-        a = c11 * r.a + c13 * r.c;
-        b = c15 * r.e;
-        c = c15 * r.a + c35 * r.c;
-        d = c55 * r.e;
-      }
-      sLx[cx] = a;
-      sLx[kXPlane + cx] = b;
-      sLx[2 * kXPlane + cx] = c;
-      sQx[cx] = d;
-      a = b = c = d = T(0);
-      if (kz != T(0)) {
-        a = c15 * r.b + c35 * r.d;
-        b = c55 * r.f;
-        c = c13 * r.b + c33 * r.d;
-        d = c35 * r.f;
-      }
-      sLz[cz] = a;
-      sLz[kZPlane + cz] = b;
-      sLz[2 * kZPlane + cz] = c;
-      sQz[cz] = d;
+    if (any_split) {
+      stage<2, kAR, kAXW, 0, 4>(g, b, lvs_in + VX_X * NSP + so, (VZ_X - VX_X) * NSP, p.i0, p.j0);
+      stage<2, kAR + 6, kVecX, 3, 0>(g, b + 2 * kAX, lvs_in + VX_Z * NSP + so, (VZ_Z - VX_Z) * NSP, p.i0, p.j0);
     }
-    // halo cell: lambda after the step (not stored: another block owns the cell), its sources
-    {
-      T* hl = hx ? sLx + hs : sLz + hs;
-      const int HP = hx ? kXPlane : kZPlane;
-      const T* hK = hx ? sKx + hs : sKz + hs;
-      T l0 = hl[0], l1 = hl[HP], l2 = hl[2 * HP];  // lambda of the txx, tzz, txz part
-      if (hvalid) {
-        const T axx = sA[hf];
-        T azz = sA[kSPlane + hf], axz = sA[2 * kSPlane + hf];
-        if (hi >= fs_lo && hi <= fs_hi) tfs_adjoint(g, lzz, lxz, hi, so + g.L.off(hi, hj), azz, axz);
-        const T sh = hK[0];
-        l0 = sh * l0 + axx;
-        l1 = sh * l1 + azz;
-        l2 = sh * l2 + axz;
+    b += 2 * kAX + 2 * kAZ;
+    stage_full<2>(g, b, lv + so, NSP, p.i0, p.j0);
+    if (any_unit) stage<3, kAR, kVecX, 0, 0>(g, b + 5 * kAH, (const T*)lt + so, NSP, p.i0, p.j0);
+  };
+  auto stage_history = [&](int s) {
+    stage_full<3>(g, buffer(s) + 2 * kAX + 2 * kAZ + 2 * kAH, tt_hist + (int64_t)s * PL, NSP, p.i0, p.j0);
+  };
+  T* sI = reinterpret_cast<T*>(el_smem) + 2 * kAdjTBuf;
+  Inject<T, 3> inj(g, grec, 0, it);
+  if (inj.any()) {
+    for (int t = threadIdx.x; t < 3 * kAI; t += kAdjThreads<T>) sI[t] = T(0);
+    inj.fetch(g, s_beg);
+  }
+  stage_history(s_beg);  // nor are the histories
+  griddep_wait();  // launched with programmatic serialisation
+  griddep_launch_dependents();
+  stage_shot(s_beg);
+  for (int s = s_beg; s < s_end; ++s) {
+    T* sX = buffer(s);
+    T* sZ = sX + 2 * kAX;
+    const T* sV = sZ + 2 * kAZ;
+    const T* sH = sV + 2 * kAH + p.ph;
+    const T* sO = sV + 5 * kAH + p.pi;
+    cp_async_wait_all();
+    __syncthreads();  // the copies of all threads; the other buffer's readers
+    if (s + 1 < s_end) {
+      stage_shot(s + 1);
+      stage_history(s + 1);
+    }
+    const int64_t so = (int64_t)s * PL, o = so + oc;
+    Vec<T> vx_x{}, vz_x{}, vx_z{}, vz_z{};  // lambda after the step times k
+    if (p.valid) {
+      Vec<T> ax, az;
+      adj_vel_totals<T, PML>(g, cf, sV, p.ph, p.j0, damp, p.i, p.j, ax, az);
+      if (!PML) {
+        stv(lv_out + VX * NSP + o, ax);
+        stv(lv_out + VZ * NSP + o, az);
       }
-      const T k = hK[HP];
-      T a = T(0), b = T(0), c = T(0), d = T(0);
-      if (k != T(0)) {
-        const T r0 = l0 * k, r1 = l1 * k, r2 = l2 * k;
-        if (hx) {  // ra, rc, re
-          const T c15 = sC[2 * kSPlane + hf];
-          a = sC[hf] * r0 + sC[kSPlane + hf] * r1;
-          b = c15 * r2;
-          c = c15 * r0 + sC[4 * kSPlane + hf] * r1;
-          d = sC[5 * kSPlane + hf] * r2;
-        } else {  // rb, rd, rf
-          const T c35 = sC[4 * kSPlane + hf];
-          a = sC[2 * kSPlane + hf] * r0 + c35 * r1;
-          b = sC[5 * kSPlane + hf] * r2;
-          c = sC[kSPlane + hf] * r0 + sC[3 * kSPlane + hf] * r1;
-          d = c35 * r2;
+      vx_x = vx_z = ax;
+      vz_x = vz_z = az;
+      if (f.split()) {
+        Vec<T> sp[4];
+        sp[VX_X] = ldv(sX + p.px);
+        sp[VZ_X] = ldv(sX + kAX + p.px);
+        sp[VX_Z] = ldv(sZ + p.pz);
+        sp[VZ_Z] = ldv(sZ + kAZ + p.pz);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+#pragma unroll
+          for (int e = 0; e < W; ++e) {
+            const T n = ((k & 1) ? f.sz[e] : f.sx[e]) * sp[k].v[e] + (k < 2 ? ax.v[e] : az.v[e]);
+            (k == VX_X ? vx_x : k == VX_Z ? vx_z : k == VZ_X ? vz_x : vz_z).v[e] = n;
+            sp[k].v[e] = (f.unit >> e & 1u) ? T(0) : n;
+          }
+          stv(lvs_out + k * NSP + o, sp[k]);
         }
       }
-      hl[0] = a;
-      hl[HP] = b;
-      hl[2 * HP] = c;
-      (hx ? sQx : sQz)[hs] = d;
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        vx_x.v[e] = f.in >> e & 1u ? vx_x.v[e] * f.kx[e] : T(0);
+        vz_x.v[e] = f.in >> e & 1u ? vz_x.v[e] * f.kx[e] : T(0);
+        vx_z.v[e] = f.in >> e & 1u ? vx_z.v[e] * f.kz[e] : T(0);
+        vz_z.v[e] = f.in >> e & 1u ? vz_z.v[e] * f.kz[e] : T(0);
+      }
     }
+    {
+      Vec<T> q[4];
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        q[0].v[e] = vx_x.v[e] * bx.v[e];
+        q[1].v[e] = vz_x.v[e] * bz.v[e];
+        q[2].v[e] = vx_z.v[e] * bx.v[e];
+        q[3].v[e] = vz_z.v[e] * bz.v[e];
+      }
+      stv(sX + p.px, q[0]);
+      stv(sX + kAX + p.px, q[1]);
+      stv(sZ + p.pz, q[2]);
+      stv(sZ + kAZ + p.pz, q[3]);
+    }
+    if (p.halo) {
+      Vec<T> q0{}, q1{};
+      if (fh.in) {
+        Vec<T> ax, az, l0{}, l1{};
+        adj_vel_totals<T, PML>(g, cf, sV, p.hph, p.j0, hdamp, p.hi, p.hj, ax, az);
+        if (fh.split()) {
+          l0 = ldv((p.hx ? sX : sZ) + p.hp);
+          l1 = ldv((p.hx ? sX + kAX : sZ + kAZ) + p.hp);
+        }
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          const T sh = p.hx ? fh.sx[e] : fh.sz[e], k = p.hx ? fh.kx[e] : fh.kz[e];
+          q0.v[e] = fh.in >> e & 1u ? (sh * l0.v[e] + ax.v[e]) * k * hbx.v[e] : T(0);
+          q1.v[e] = fh.in >> e & 1u ? (sh * l1.v[e] + az.v[e]) * k * hbz.v[e] : T(0);
+        }
+      }
+      stv((p.hx ? sX : sZ) + p.hp, q0);
+      stv((p.hx ? sX + kAX : sZ + kAZ) + p.hp, q1);
+    }
+    if (inj.any()) inj.put(g, s, sI);
     __syncthreads();
-    if (valid) {
-      const StagedX<T> q0{sLx, i0, j0}, q2{sLx + kXPlane, i0, j0}, q4{sLx + 2 * kXPlane, i0, j0}, q6{sQx, i0, j0};
-      const StagedZ<T> q1{sLz, i0, j0}, q3{sLz + kZPlane, i0, j0}, q5{sLz + 2 * kZPlane, i0, j0}, q7{sQz, i0, j0};
-      const T avx = dxb_t<NN>(g, q0, i, j) + dzb_t<NN>(g, q1, i, j) + dxf_t<NN>(g, q2, i, j) + dzf_t<NN>(g, q3, i, j);
-      const T avz = dxb_t<NN>(g, q4, i, j) + dzb_t<NN>(g, q5, i, j) + dxf_t<NN>(g, q6, i, j) + dzf_t<NN>(g, q7, i, j);
-      const int64_t o = so + oc;
-      lv[VX * NSP + o] = avx;
-      lv[VZ * NSP + o] = avz;
-      if (inside) {
-        const T* vx = B + oV;
-        const T* vz = B + oV + kSPlane;
-        const T dxb_vx = dxb<NN>(g, vx, sc), dxb_vz = dxb<NN>(g, vz, sc);
-        const T dzb_vx = dzb<NN>(g, vx, sc, kSW), dzb_vz = dzb<NN>(g, vz, sc, kSW);
-        const T dxf_vx = dxf<NN>(g, vx, sc), dxf_vz = dxf<NN>(g, vz, sc);
-        const T dzf_vx = dzf<NN>(g, vx, sc, kSW), dzf_vz = dzf<NN>(g, vz, sc, kSW);
-        g11 += r.a * dxb_vx;
-        g13 += r.b * dzb_vz + r.c * dxb_vx;
-        g15 += r.a * dxb_vz + r.b * dzb_vx + r.e * dxf_vx;
-        g33 += r.d * dzb_vz;
-        g35 += r.c * dxb_vz + r.d * dzb_vx + r.f * dzf_vz;
-        g55 += r.e * dxf_vz + r.f * dzf_vx;
+    if (s + 1 < s_end) inj.fetch(g, s + 1);
+    if (p.valid) {
+      Vec<T> n[3];
+      {
+        const Row<T, NN> qx(sX + p.px), qz(sX + kAX + p.px);
+        Vec<T> rx[2 * NN + 1], rz[2 * NN + 1];
+#pragma unroll
+        for (int k = 0; k <= 2 * NN; ++k) {
+          rx[k] = ldv(sZ + p.pz + (k - NN) * kVecX);
+          rz[k] = ldv(sZ + kAZ + p.pz + (k - NN) * kVecX);
+        }
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          n[TXX].v[e] = diff_t<NN>(g, [&](int m) { return qx(e - 1 + m); });
+          n[TXZ].v[e] = diff_t<NN>(g, [&](int m) { return rx[NN + m].v[e]; }) +
+                        diff_t<NN>(g, [&](int m) { return qz(e + m); });
+          n[TZZ].v[e] = diff_t<NN>(g, [&](int m) { return rz[NN + m - 1].v[e]; });
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if (f.unit) {
+          const Vec<T> old = ldv(sO + c * kAI);
+#pragma unroll
+          for (int e = 0; e < W; ++e)
+            if (f.unit >> e & 1u) n[c].v[e] += old.v[e];
+        }
+        if (inj.any()) {
+          const Vec<T> a = ldv(sI + c * kAI + p.pi);
+#pragma unroll
+          for (int e = 0; e < W; ++e) n[c].v[e] += a.v[e];
+        }
+        stv(lt + c * NSP + o, n[c]);
+      }
+      if (f.in) {
+        const Row<T, NN> xx(sH + TXX * kAH), xz(sH + TXZ * kAH);
+        Vec<T> rxz[2 * NN], rzz[2 * NN];
+#pragma unroll
+        for (int k = 0; k < 2 * NN; ++k) {
+          if (k != NN) rxz[k] = ldv(sH + TXZ * kAH + (k - NN) * kAXW);
+          rzz[k] = ldv(sH + TZZ * kAH + (k - NN + 1) * kAXW);
+        }
+        const Fd<T> fd{g.f0, g.f1, g.f2};
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          gx.v[e] += vx_x.v[e] * fd.template diff<NN>([&](int m) { return xx(e + m); }) +
+                     vx_z.v[e] * fd.template diff<NN>([&](int m) { return m == 1 ? xz(e) : rxz[NN + m - 1].v[e]; });
+          gz.v[e] += vz_x.v[e] * fd.template diff<NN>([&](int m) { return xz(e - 1 + m); }) +
+                     vz_z.v[e] * fd.template diff<NN>([&](int m) { return rzz[NN + m - 1].v[e]; });
+        }
       }
     }
-    __syncthreads();  // this buffer is refilled by the copies of the shot after next
   }
-  if (inside) {
-    gc[C11 * PL + oc] += g11;
-    gc[C13 * PL + oc] += g13;
-    gc[C15 * PL + oc] += g15;
-    gc[C33 * PL + oc] += g33;
-    gc[C35 * PL + oc] += g35;
-    gc[C55 * PL + oc] += g55;
+  if (p.valid && f.in) {
+    Vec<T> a = ldv(gbase + 6 * PL + oc), b = ldv(gbase + 7 * PL + oc);
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      if (f.in >> e & 1u) a.v[e] += gx.v[e];
+      if (f.in >> e & 1u) b.v[e] += gz.v[e];
+    }
+    stv(gbase + 6 * PL + oc, a);
+    stv(gbase + 7 * PL + oc, b);
   }
 }
 
-// ABL (reverse of v *= damp and the free-surface velocity rows): lv_out = FS^T(damp * lv_in), and
-// the velocity update's adjoint sources q4 (vx_x, vx_z, vz_x, vz_z) at the cell, zero outside I.
-template <typename T>
-__global__ void adj_vfs_abl(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lv_in, T* __restrict__ lv_out,
-                            T* __restrict__ q4) {
-  griddep_wait();
-  griddep_launch_dependents();
-  EL_CELL_SHOT
-  // damp-weighted lambda at the cells the free-surface adjoint reads
-  auto dl = [&](int comp, int64_t oo, int ii, int jj) { return cf[DAMP * PL + g.L.off(ii, jj)] * lv_in[comp * NSP + oo]; };
-  T ax = dl(VX, o, i, j), az = dl(VZ, o, i, j);
-  if (g.fsurf) {
-    const int h = g.h;
-    const int64_t P = g.L.pitch;
-    auto inJ = [&](int m) { return m >= g.jlo && m <= g.jhi; };
-    if (i == h - 3) {
-      if (inJ(j)) az = T(0);
-    } else if (i == h - 2) {
-      if (inJ(j)) {
-        ax = T(0);
-        az = T(0);
-      } else if (inJ(j - 1)) {
-        az += dl(VX, o - 1, i, j - 1);
-      }
-    } else if (i == h - 1) {
-      const int64_t o2 = o - P;
-      const T a_l = inJ(j - 1) ? dl(VX, o2 - 1, i - 1, j - 1) : T(0);
-      const T a_c = inJ(j) ? dl(VX, o2, i - 1, j) : T(0);
-      T r = az + a_l - a_c;
-      if (inJ(j)) r += dl(VZ, o2, i - 1, j) + dl(VZ, o2 - P, i - 2, j) + a_l - a_c;
-      az = r;
-    } else if (i == h) {
-      if (inJ(j)) ax += dl(VX, o - 2 * P, i - 2, j);
-    }
-  }
-  lv_out[VX * NSP + o] = ax;
-  lv_out[VZ * NSP + o] = az;
-  const bool inside = in_I(g, i, j);
-  const int64_t c0 = g.L.off(i, j);
-  const T bx = inside ? cf[BX * PL + c0] : T(0), bz = inside ? cf[BZ * PL + c0] : T(0);
-  q4[0 * NSP + o] = ax * bx * g.dt_dx;
-  q4[1 * NSP + o] = ax * bx * g.dt_dz;
-  q4[2 * NSP + o] = az * bz * g.dt_dx;
-  q4[3 * NSP + o] = az * bz * g.dt_dz;
-}
-
-// ABL: lt += transposes of the velocity update's stress differences; bx, bz gradients; without a
-// free surface also the stress update's adjoint sources q8 (with one they follow its rows).
-template <typename T, int NN>
-__global__ void adj_t_abl(Geo<T> g, const T* __restrict__ cf, const T* __restrict__ lv, const T* __restrict__ qv, T* lt,
-                          const T* __restrict__ tt_hist, T* gpart, int eg, T* __restrict__ q8) {
-  griddep_wait();
-  griddep_launch_dependents();
-  EL_CELL
+// Reverse of the stress update: lambda of the (split) stresses after the step (lts_in -> lts_out with
+// PML), lv from the transposes of its velocity differences, dL/d velocity records of step it - 1, and
+// the C gradients.
+template <typename T, int NN, bool PML>
+__global__ void __launch_bounds__(kAdjThreads<T>, sizeof(T) == 4 ? 2 : 1)
+    adj_v_step(Geo<T> g, int it, const T* __restrict__ cf, const T* __restrict__ lt, const T* __restrict__ lts_in,
+               T* __restrict__ lts_out, T* lv, const T* __restrict__ v_hist, const T* __restrict__ grec, T* gpart,
+               int eg) {
+  extern __shared__ __align__(16) unsigned char el_smem[];
+  constexpr int W = kVW<T>;
+  const AdjTile<T, NN> p(g.L);
+  const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL;
+  const int64_t oc = g.L.off(p.i, p.j), oh = g.L.off(p.hi, p.hj);
   EL_SHOT_GROUP
-  T* gbx = gbase + 6 * PL;
-  T* gbz = gbase + 7 * PL;
-  T gx = T(0), gz = T(0);
-  for (int s = s_beg; s < s_end; ++s) {
+  const AdjFactors<T, PML> f(g, cf, p.i, p.j), fh(g, cf, p.halo ? p.hi : -1, p.hj);
+  Vec<T> c[6] = {}, hc[6] = {};
+  if (f.in) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) c[k] = ldv(cf + (C11 + k) * PL + oc);
+  }
+  if (fh.in) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) hc[k] = ldv(cf + (C11 + k) * PL + oh);
+  }
+  constexpr int k11 = 0, k13 = 1, k15 = 2, k33 = 3, k35 = 4, k55 = 5;
+  static_assert(C13 == C11 + 1 && C15 == C11 + 2 && C33 == C11 + 3 && C35 == C11 + 4 && C55 == C11 + 5, "order of C");
+  Vec<T> gc[6] = {};
+  auto buffer = [&](int s) { return reinterpret_cast<T*>(el_smem) + ((s - s_beg) & 1) * kAdjVBuf; };
+  const bool any_split = PML && __syncthreads_or(f.split() || fh.split());
+  const bool any_unit = !PML || __syncthreads_or(f.unit);
+  auto stage_shot = [&](int s) {
+    T* b = buffer(s);
     const int64_t so = (int64_t)s * PL;
-    const PlaneQ<T> q1{qv + 0 * NSP + so, g.L}, q2{qv + 1 * NSP + so, g.L};
-    const PlaneQ<T> q3{qv + 2 * NSP + so, g.L}, q4{qv + 3 * NSP + so, g.L};
-    const int64_t o = so + oc;
-    lt[TXX * NSP + o] += dxf_t<NN>(g, q1, i, j);
-    lt[TXZ * NSP + o] += dzb_t<NN>(g, q2, i, j) + dxb_t<NN>(g, q3, i, j);
-    lt[TZZ * NSP + o] += dzf_t<NN>(g, q4, i, j);
-    if (!g.fsurf) stress_sources<T, false>(g, cf, lt, i, j, o, q8);
-    if (in_I(g, i, j)) {
-      const T* th = tt_hist;
-      gx += lv[VX * NSP + o] * (dxf<NN>(g, th + TXX * NSP, o) * g.dt_dx + dzb<NN>(g, th + TXZ * NSP, o) * g.dt_dz);
-      gz += lv[VZ * NSP + o] * (dxb<NN>(g, th + TXZ * NSP, o) * g.dt_dx + dzf<NN>(g, th + TZZ * NSP, o) * g.dt_dz);
+    if (any_split) {
+      stage<3, kAR, kAXW, 0, 4>(g, b, lts_in + so, 2 * NSP, p.i0, p.j0);
+      stage<3, kAR + 6, kVecX, 3, 0>(g, b + 4 * kAX, lts_in + NSP + so, 2 * NSP, p.i0, p.j0);
+    }
+    b += 4 * kAX + 4 * kAZ;
+    stage_full<3>(g, b, lt + so, NSP, p.i0, p.j0);
+    if (any_unit) stage<2, kAR, kVecX, 0, 0>(g, b + 5 * kAH, (const T*)lv + so, NSP, p.i0, p.j0);
+  };
+  auto stage_history = [&](int s) {
+    stage_full<2>(g, buffer(s) + 4 * kAX + 4 * kAZ + 3 * kAH, v_hist + (int64_t)s * PL, NSP, p.i0, p.j0);
+  };
+  T* sI = reinterpret_cast<T*>(el_smem) + 2 * kAdjVBuf;
+  Inject<T, 2> inj(g, grec, 3, it - 1);
+  if (inj.any()) {
+    for (int t = threadIdx.x; t < 2 * kAI; t += kAdjThreads<T>) sI[t] = T(0);
+    inj.fetch(g, s_beg);
+  }
+  stage_history(s_beg);
+  griddep_wait();  // launched with programmatic serialisation
+  griddep_launch_dependents();
+  stage_shot(s_beg);
+  for (int s = s_beg; s < s_end; ++s) {
+    T* sX = buffer(s);
+    T* sZ = sX + 4 * kAX;
+    const T* sL = sZ + 4 * kAZ;
+    const T* sH = sL + 3 * kAH + p.ph;
+    const T* sO = sL + 5 * kAH + p.pi;
+    cp_async_wait_all();
+    __syncthreads();  // the copies of all threads; the other buffer's readers
+    if (s + 1 < s_end) {
+      stage_shot(s + 1);
+      stage_history(s + 1);
+    }
+    const int64_t so = (int64_t)s * PL, o = so + oc;
+    Vec<T> lx[3] = {}, lz[3] = {};  // lambda of txx, tzz, txz after the step times k: x parts, z parts
+    if (f.in) {
+      Vec<T> l[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) l[k] = ldv(sL + k * kAH + p.ph);
+      if (PML && g.fsurf && p.i <= g.h) {
+#pragma unroll
+        for (int e = 0; e < W; ++e)
+          tfs_adjoint(g, sL + TZZ * kAH + p.ph + e, sL + TXZ * kAH + p.ph + e, p.i, kAXW, l[TZZ].v[e], l[TXZ].v[e]);
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) lx[k] = lz[k] = l[k];
+      if (f.split()) {
+        Vec<T> sp[6];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          sp[2 * k] = ldv(sX + k * kAX + p.px);
+          sp[2 * k + 1] = ldv(sZ + k * kAZ + p.pz);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          Vec<T>&sx = sp[2 * k], &sz = sp[2 * k + 1];
+#pragma unroll
+          for (int e = 0; e < W; ++e) {
+            lx[k].v[e] = f.sx[e] * sx.v[e] + l[k].v[e];
+            lz[k].v[e] = f.sz[e] * sz.v[e] + l[k].v[e];
+            const bool u = f.unit >> e & 1u;
+            sx.v[e] = u ? T(0) : lx[k].v[e];
+            sz.v[e] = u ? T(0) : lz[k].v[e];
+          }
+          stv(lts_out + (2 * k) * NSP + o, sx);
+          stv(lts_out + (2 * k + 1) * NSP + o, sz);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          lx[k].v[e] = f.in >> e & 1u ? lx[k].v[e] * f.kx[e] : T(0);
+          lz[k].v[e] = f.in >> e & 1u ? lz[k].v[e] * f.kz[e] : T(0);
+        }
+    }
+    // sources of the x differences (of vx backward, forward; of vz backward, forward) and of the z ones
+    auto put_x = [&](const Vec<T>* C, const Vec<T>* l, T* at) {
+      Vec<T> q[4];
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        q[0].v[e] = C[k11].v[e] * l[TXX].v[e] + C[k13].v[e] * l[TZZ].v[e];
+        q[1].v[e] = C[k15].v[e] * l[TXZ].v[e];
+        q[2].v[e] = C[k15].v[e] * l[TXX].v[e] + C[k35].v[e] * l[TZZ].v[e];
+        q[3].v[e] = C[k55].v[e] * l[TXZ].v[e];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) stv(at + k * kAX, q[k]);
+    };
+    auto put_z = [&](const Vec<T>* C, const Vec<T>* l, T* at) {
+      Vec<T> q[4];
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        q[0].v[e] = C[k15].v[e] * l[TXX].v[e] + C[k35].v[e] * l[TZZ].v[e];
+        q[1].v[e] = C[k55].v[e] * l[TXZ].v[e];
+        q[2].v[e] = C[k13].v[e] * l[TXX].v[e] + C[k33].v[e] * l[TZZ].v[e];
+        q[3].v[e] = C[k35].v[e] * l[TXZ].v[e];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) stv(at + k * kAZ, q[k]);
+    };
+    put_x(c, lx, sX + p.px);
+    put_z(c, lz, sZ + p.pz);
+    if (p.halo) {
+      Vec<T> l[3] = {};
+      if (fh.in) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) l[k] = ldv(sL + k * kAH + p.hph);
+        if (PML && g.fsurf && p.hi <= g.h) {
+#pragma unroll
+          for (int e = 0; e < W; ++e)
+            tfs_adjoint(g, sL + TZZ * kAH + p.hph + e, sL + TXZ * kAH + p.hph + e, p.hi, kAXW, l[TZZ].v[e], l[TXZ].v[e]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          Vec<T> sp{};
+          if (fh.split()) sp = ldv((p.hx ? sX + k * kAX : sZ + k * kAZ) + p.hp);
+#pragma unroll
+          for (int e = 0; e < W; ++e) {
+            const T sh = p.hx ? fh.sx[e] : fh.sz[e], kk = p.hx ? fh.kx[e] : fh.kz[e];
+            l[k].v[e] = fh.in >> e & 1u ? (sh * sp.v[e] + l[k].v[e]) * kk : T(0);
+          }
+        }
+      }
+      if (p.hx)
+        put_x(hc, l, sX + p.hp);
+      else
+        put_z(hc, l, sZ + p.hp);
+    }
+    if (inj.any()) inj.put(g, s, sI);
+    __syncthreads();
+    if (s + 1 < s_end) inj.fetch(g, s + 1);
+    if (p.valid) {
+      Vec<T> n[2];
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const Row<T, NN> qb(sX + 2 * v * kAX + p.px), qf(sX + (2 * v + 1) * kAX + p.px);
+        Vec<T> rb[2 * NN], rf[2 * NN];  // rows i - NN + 1 .. i + NN of the backward, i - NN .. of the forward
+#pragma unroll
+        for (int k = 0; k < 2 * NN; ++k) {
+          rb[k] = ldv(sZ + 2 * v * kAZ + p.pz + (k - NN + 1) * kVecX);
+          rf[k] = ldv(sZ + (2 * v + 1) * kAZ + p.pz + (k - NN) * kVecX);
+        }
+#pragma unroll
+        for (int e = 0; e < W; ++e)
+          n[v].v[e] = diff_t<NN>(g, [&](int m) { return qb(e + m); }) +
+                      diff_t<NN>(g, [&](int m) { return rb[NN + m - 1].v[e]; }) +
+                      diff_t<NN>(g, [&](int m) { return qf(e - 1 + m); }) +
+                      diff_t<NN>(g, [&](int m) { return rf[NN + m - 1].v[e]; });
+        if (f.unit) {
+          const Vec<T> old = ldv(sO + v * kAI);
+#pragma unroll
+          for (int e = 0; e < W; ++e)
+            if (f.unit >> e & 1u) n[v].v[e] += old.v[e];
+        }
+        if (inj.any()) {
+          const Vec<T> a = ldv(sI + v * kAI + p.pi);
+#pragma unroll
+          for (int e = 0; e < W; ++e) n[v].v[e] += a.v[e];
+        }
+        stv(lv + v * NSP + o, n[v]);
+      }
+      if (f.in) {
+        const Row<T, NN> x(sH + VX * kAH), z(sH + VZ * kAH);
+        Vec<T> rx[2 * NN + 1], rz[2 * NN + 1];
+#pragma unroll
+        for (int k = 0; k <= 2 * NN; ++k)
+          if (k != NN) {
+            rx[k] = ldv(sH + VX * kAH + (k - NN) * kAXW);
+            rz[k] = ldv(sH + VZ * kAH + (k - NN) * kAXW);
+          }
+        const Fd<T> fd{g.f0, g.f1, g.f2};
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          auto zx = [&](int m) { return m == 0 ? x(e) : rx[NN + m].v[e]; };
+          auto zz = [&](int m) { return m == 0 ? z(e) : rz[NN + m].v[e]; };
+          const T dxb_vx = fd.template diff<NN>([&](int m) { return x(e - 1 + m); });
+          const T dxb_vz = fd.template diff<NN>([&](int m) { return z(e - 1 + m); });
+          const T dzb_vx = fd.template diff<NN>([&](int m) { return zx(m - 1); });
+          const T dzb_vz = fd.template diff<NN>([&](int m) { return zz(m - 1); });
+          const T dxf_vx = fd.template diff<NN>([&](int m) { return x(e + m); });
+          const T dxf_vz = fd.template diff<NN>([&](int m) { return z(e + m); });
+          const T dzf_vx = fd.template diff<NN>(zx);
+          const T dzf_vz = fd.template diff<NN>(zz);
+          gc[k11].v[e] += lx[TXX].v[e] * dxb_vx;
+          gc[k13].v[e] += lz[TXX].v[e] * dzb_vz + lx[TZZ].v[e] * dxb_vx;
+          gc[k15].v[e] += lx[TXX].v[e] * dxb_vz + lz[TXX].v[e] * dzb_vx + lx[TXZ].v[e] * dxf_vx;
+          gc[k33].v[e] += lz[TZZ].v[e] * dzb_vz;
+          gc[k35].v[e] += lx[TZZ].v[e] * dxb_vz + lz[TZZ].v[e] * dzb_vx + lz[TXZ].v[e] * dzf_vz;
+          gc[k55].v[e] += lx[TXZ].v[e] * dxf_vz + lz[TXZ].v[e] * dzf_vx;
+        }
+      }
     }
   }
-  if (in_I(g, i, j)) {
-    gbx[oc] += gx;
-    gbz[oc] += gz;
+  if (p.valid && f.in) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      Vec<T> a = ldv(gbase + k * PL + oc);
+#pragma unroll
+      for (int e = 0; e < W; ++e)
+        if (f.in >> e & 1u) a.v[e] += gc[k].v[e];
+      stv(gbase + k * PL + oc, a);
+    }
   }
 }
 
@@ -1609,7 +1400,7 @@ struct adfwi_elastic_plan {
   std::vector<int32_t> tab;
   std::vector<unsigned char> srcm;  // ns x 3 source weights (xx, zz, xz) in the solve's dtype
   PinnedBytes tab_pin, srcm_pin;    // page-locked copies of tab and srcm, the sources of each upload
-  int64_t o_srcz, o_srcx, o_rcvz, o_rcvx, o_uzx, o_ubeg, o_urcv;
+  int64_t o_srcz, o_srcx, o_rcvz, o_rcvx, o_uzx, o_ubeg, o_urcv, o_tbeg;
   int ncells;
   std::vector<int> chunk_end;  // last step of each reference checkpoint chunk
 };
@@ -1620,22 +1411,23 @@ int64_t al256(int64_t x) { return (x + 255) / 256 * 256; }
 
 struct ECarve {
   int64_t coef, st, tt, vtmp, srcm, tab;       // forward
-  int64_t snap, snap_scale, hv, ht, lst, lt, lv, lv2, qsrc, gc;  // gradient
+  int64_t snap, snap_scale, hv, ht, lst, lt, lv, lv2, gc;  // gradient
   int64_t total;
 };
 
 // Coefficient planes: C11 C13 C15 C33 C35 C55 bx bz + (bcx bcz | damp)
 int ncoef(const adfwi_elastic_plan* p) { return p->d.pml ? 10 : 9; }
 
-// Shot groups of the gradient kernels: enough (cell, group) threads to fill the GPU (about
-// 300 k), at most one group per shot.
+// Tiles of the reverse kernels (one block each per shot group).
+int adj_tiles(const adfwi_elastic_plan* p) {
+  return ((p->nzp + el::kAR - 1) / el::kAR) * ((p->nxp + el::kVecX - 1) / el::kVecX);
+}
+// Shot groups of the reverse kernels: about two waves of two blocks per SM, at most one group per shot.
+// More groups split the shots' copies and add gradient planes: 64.4, 65.6 and 71.3 ms for 400 steps of
+// 20 shots on a 242 x 480 grid with 600, 900 and 1800 blocks.
 int egroups(const adfwi_elastic_plan* p) {
-  const int64_t cells = (int64_t)p->nzp * p->nxp;
-#ifndef ADFWI_EL_THREADS
-#define ADFWI_EL_THREADS 300000
-#endif
-  const int64_t want = ((int64_t)ADFWI_EL_THREADS + cells - 1) / cells;
-  const int g = (int)std::max<int64_t>(1, std::min<int64_t>(p->d.ns, want));
+  const int tiles = adj_tiles(p);
+  const int g = std::max(1, std::min(p->d.ns, (600 + tiles - 1) / tiles));
   const int eg = (p->d.ns + g - 1) / g;
   return (p->d.ns + eg - 1) / eg;
 }
@@ -1666,13 +1458,10 @@ ECarve ecarve(const adfwi_elastic_plan* p, bool grad, int K) {
     c.ht = take((int64_t)K * 3 * ns * pl);  // stress totals after each step's free surface
     // lambda of the split stresses (6) and of the split velocities (4), twice each (a reverse
     // step reads one copy and writes the other)
-    c.lst = take((int64_t)(p->d.pml ? 20 : 3) * ns * pl);
-    c.lt = take((p->d.pml ? 3 : 0) * ns * pl);
+    c.lst = take((int64_t)(p->d.pml ? 20 : 0) * ns * pl);
+    c.lt = take(3 * ns * pl);
     c.lv = take(2 * ns * pl);
-    c.lv2 = take(2 * ns * pl);
-    // adjoint sources of the absorbing-layer step transposes (8 + 4 planes per shot; the PML
-    // kernels form theirs in shared memory)
-    c.qsrc = take(p->d.pml ? 0 : 12 * ns * pl);
+    c.lv2 = take((p->d.pml ? 0 : 2) * ns * pl);  // with an absorbing layer lambda of the velocities has two copies
     c.gc = take(8 * pl * egroups(p));
   }
   c.total = o;
@@ -1724,6 +1513,11 @@ el::Geo<T> egeo(const adfwi_elastic_plan* p, const unsigned char* ws, const ECar
   g.f0 = (T)d.fdc[0];
   g.f1 = (T)d.fdc[1];
   g.f2 = (T)(p->NN == 3 ? d.fdc[2] : 0.0);
+  for (int k = 0; k < 3; ++k) {
+    const double f = k < p->NN ? d.fdc[k] : 0.0;
+    g.fx[k] = (T)(f * d.dt / d.dx);
+    g.fz[k] = (T)(f * d.dt / d.dz);
+  }
   const int32_t* tb = reinterpret_cast<const int32_t*>(ws + c.tab);
   g.src_z = tb + p->o_srcz;
   g.src_x = tb + p->o_srcx;
@@ -1733,6 +1527,7 @@ el::Geo<T> egeo(const adfwi_elastic_plan* p, const unsigned char* ws, const ECar
   g.ucell_zx = tb + p->o_uzx;
   g.ucell_beg = tb + p->o_ubeg;
   g.ucell_rcv = tb + p->o_urcv;
+  g.tile_beg = tb + p->o_tbeg;
   g.ncells = p->ncells;
   return g;
 }
@@ -1835,12 +1630,6 @@ int eforward(const adfwi_elastic_plan* p, const void* const* coef, const int32_t
   T* ht = grad ? reinterpret_cast<T*>(ws + c.ht) : nullptr;
   const int nt = p->d.nt;
   if (fw) ADFWI_CUDA_TRY(cudaMemsetAsync(fw, 0, 5 * (int64_t)p->d.nz * p->d.nx * sizeof(T), s));
-  if (full) {
-    // the histories double as the state and are read with their halos
-    int rc0 = zero_frames<T>(hv, (int64_t)K * 2 * p->d.ns, p->L, s);
-    if (!rc0) rc0 = zero_frames<T>(ht, (int64_t)K * 3 * p->d.ns, p->L, s);
-    if (rc0) return rc0;
-  }
   size_t chunk = 0;
   for (int it = 0; it < nt; ++it) {
     if (grad && !full && it % K == 0) {
@@ -1904,36 +1693,23 @@ int ebackward(const adfwi_elastic_plan* p, const void* wavelet, const void* grec
   T* lv = reinterpret_cast<T*>(ws + c.lv);
   T* lv2 = reinterpret_cast<T*>(ws + c.lv2);
   T* gcp = reinterpret_cast<T*>(ws + c.gc);
-  T* qsrc = reinterpret_cast<T*>(ws + c.qsrc);
   const T* gr = static_cast<const T*>(grec);
-  const int nsf = p->d.pml ? 20 : 3;
-  ADFWI_CUDA_TRY(cudaMemsetAsync(lst, 0, nsf * NSP * sizeof(T), s));
-  if (p->d.pml) ADFWI_CUDA_TRY(cudaMemsetAsync(lt, 0, 3 * NSP * sizeof(T), s));
+  if (p->d.pml) ADFWI_CUDA_TRY(cudaMemsetAsync(lst, 0, 20 * NSP * sizeof(T), s));
+  ADFWI_CUDA_TRY(cudaMemsetAsync(lt, 0, 3 * NSP * sizeof(T), s));
   ADFWI_CUDA_TRY(cudaMemsetAsync(lv, 0, 2 * NSP * sizeof(T), s));
   const int egr = egroups(p), eg = eshots_per_group(p);
   ADFWI_CUDA_TRY(cudaMemsetAsync(gcp, 0, (int64_t)egr * 8 * PL * sizeof(T), s));
-  if (!p->d.pml) {
-    // the source planes are read with their halos by the transposed stencils
-    int rc0 = zero_frames<T>(qsrc, (int64_t)12 * ns, p->L, s);
-    if (rc0) return rc0;
-  }
-  ADFWI_CUDA_TRY(cudaMemsetAsync(lv2, 0, 2 * NSP * sizeof(T), s));
-  if (!full) {
-    // recomputed histories are read with their halos
-    int rc0 = zero_frames<T>(hv, (int64_t)K * 2 * ns, p->L, s);
-    if (!rc0) rc0 = zero_frames<T>(ht, (int64_t)K * 3 * ns, p->L, s);
-    if (rc0) return rc0;
-  }
-  const dim3 gcs = cells_grid(p, ns), gcg = cells_grid(p, egroups(p)), b(el::kTileThreads);
-  // shared memory of the staged gradient kernels (above the 48 KB default in double precision)
-  const int smem_t = el::kAdjTElems * (int)sizeof(T);
-  const int smem_vp = el::kAdjVPmlElems * (int)sizeof(T);
-  const int smem_va = el::adj_v_planes<false>() * el::kSPlane * (int)sizeof(T);
-  ADFWI_CUDA_TRY(cudaFuncSetAttribute(el::adj_t_pml<T, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
-  ADFWI_CUDA_TRY(cudaFuncSetAttribute(el::adj_v_pml<T, NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_vp));
-  ADFWI_CUDA_TRY(cudaFuncSetAttribute(el::adj_v<T, NN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_va));
+  if (!p->d.pml) ADFWI_CUDA_TRY(cudaMemsetAsync(lv2, 0, 2 * NSP * sizeof(T), s));
+  const dim3 ga(adj_tiles(p), egr), ba(el::kAdjThreads<T>);
+  auto adj_t = p->d.pml ? el::adj_t_step<T, NN, true> : el::adj_t_step<T, NN, false>;
+  auto adj_v = p->d.pml ? el::adj_v_step<T, NN, true> : el::adj_v_step<T, NN, false>;
+  // shared memory of the reverse kernels (above the 48 KB default in double precision)
+  const int smem_t = el::kAdjT * (int)sizeof(T), smem_v = el::kAdjV * (int)sizeof(T);
+  ADFWI_CUDA_TRY(cudaFuncSetAttribute(adj_t, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
+  ADFWI_CUDA_TRY(cudaFuncSetAttribute(adj_v, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_v));
   const dim3 gcol((unsigned)((p->nxp + 127) / 128), ns);
-  const dim3 ginj((unsigned)std::max(1, (p->ncells + 127) / 128), ns);
+  if (gr && p->ncells > 0)
+    ADFWI_LAUNCH(kAux, s, (el::adj_inject<T><<<dim3((unsigned)((p->ncells + 127) / 128), ns), 128, 0, s>>>(g, nt - 1, gr, lv)));
   const int nseg = full ? 1 : (nt + K - 1) / K;
   int flip = 0;  // which copy of the split velocities' lambda the next reverse step reads
   for (int seg = nseg - 1; seg >= 0; --seg) {
@@ -1957,37 +1733,24 @@ int ebackward(const adfwi_elastic_plan* p, const void* wavelet, const void* grec
       const int k = it - t0;
       const T* vh = hv + (int64_t)k * 2 * NSP;  // velocity totals at the start of step it
       const T* th = ht + (int64_t)k * 3 * NSP;  // stress totals of step it
-      if (p->d.pml) {
-        // one stream of programmatically serialised launches per reverse step; lt is
-        // overwritten by adj_t_pml before the stress-record gradients are added to it
-        if (gr) ADFWI_LAUNCH(kAux, s, (void)launch_pdl_kernel(el::adj_inject<T>, ginj, dim3(128), 0, s, g, it, gr, lt, lv, 1));
-        // lambda of the split stresses: planes 0-5 / 6-11 of lst, of the split velocities 12-15 /
-        // 16-19; each reverse step reads one copy and writes the other
-        const int f = flip;
-        flip ^= 1;
-        T* lvs_in = lst + (12 + 4 * f) * NSP;
-        T* lvs_out = lst + (16 - 4 * f) * NSP;
-        T* lts_in = lst + (6 * f) * NSP;
-        T* lts_out = lst + (6 - 6 * f) * NSP;
-        ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_t_pml<T, NN>, gcg, b, (size_t)smem_t, s, g, cf,
-                                                            (const T*)lv, (const T*)lvs_in, lvs_out, lt, th, gcp, eg));
-        if (gr) ADFWI_LAUNCH(kAux, s, (void)launch_pdl_kernel(el::adj_inject<T>, ginj, dim3(128), 0, s, g, it, gr, lt, lv, 2));
-        ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_v_pml<T, NN>, gcg, b, (size_t)smem_vp, s, g, cf,
-                                                            (const T*)lt, (const T*)lts_in, lts_out, lv, vh, gcp, eg));
-      } else {
-        T* q4 = qsrc + 8 * NSP;
-        if (gr) ADFWI_LAUNCH(kAux, s, (void)launch_pdl_kernel(el::adj_inject<T>, ginj, dim3(128), 0, s, g, it, gr, lst, lv, 3));
-        ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_vfs_abl<T>, gcs, b, 0, s, g, cf, (const T*)lv, lv2, q4));
+      // lambda of the split stresses: planes 0-5 / 6-11 of lst, of the split velocities 12-15 /
+      // 16-19; each reverse step reads one copy and writes the other
+      const int f = flip;
+      flip ^= 1;
+      const T* lvs_in = lst + (12 + 4 * f) * NSP;
+      T* lvs_out = lst + (16 - 4 * f) * NSP;
+      const T* lts_in = lst + (6 * f) * NSP;
+      T* lts_out = lst + (6 - 6 * f) * NSP;
+      // programmatically serialised launches
+      ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(adj_t, ga, ba, (size_t)smem_t, s, g, it, cf, (const T*)lv, lv2,
+                                                          lvs_in, lvs_out, lt, th, gr, gcp, eg));
+      if (!p->d.pml) {
         std::swap(lv, lv2);
-        ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_t_abl<T, NN>, gcg, b, 0, s, g, cf, (const T*)lv,
-                                                            (const T*)q4, lst, th, gcp, eg, qsrc));
-        if (p->d.free_surface) {
-          ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_tfs_abl<T>, gcol, dim3(128), 0, s, g, lst));
-          ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_vq<T, false>, gcs, b, 0, s, g, cf, (const T*)lst, qsrc));
-        }
-        ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_v<T, NN, false>, gcg, b, (size_t)smem_va, s, g, cf,
-                                                            (const T*)lst, (const T*)qsrc, lv, vh, gcp, eg));
+        if (p->d.free_surface)
+          ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(el::adj_tfs_abl<T>, gcol, dim3(128), 0, s, g, lt));
       }
+      ADFWI_LAUNCH(kElAdjStep, s, (void)launch_pdl_kernel(adj_v, ga, ba, (size_t)smem_v, s, g, it, cf, (const T*)lt,
+                                                          lts_in, lts_out, lv, vh, gr, gcp, eg));
     }
     ADFWI_CUDA_TRY(cudaGetLastError());
   }
@@ -2083,17 +1846,28 @@ int adfwi_elastic_plan_create(const adfwi_elastic_desc* desc, const int32_t* src
   p->o_rcvx = t.size();
   for (int r = 0; r < d.nr; ++r) t.push_back(rcv_x[r] + d.nabc);
   // unique receiver cells
-  std::vector<std::pair<int, int>> cells(d.nr);
-  for (int r = 0; r < d.nr; ++r) cells[r] = {((rcv_z[r] + p->top) << 16) | (rcv_x[r] + d.nabc), r};
-  std::stable_sort(cells.begin(), cells.end());
-  std::vector<int32_t> uzx, ubeg, urcv;
-  for (int q = 0; q < d.nr; ++q) {
-    if (q == 0 || cells[q].first != cells[q - 1].first) {
-      uzx.push_back(cells[q].first);
-      ubeg.push_back((int32_t)urcv.size());
-    }
-    urcv.push_back(cells[q].second);
+  // in the order of the reverse kernels' tiles
+  struct Cell {
+    int tile, zx, r;
+    bool operator<(const Cell& o) const { return tile != o.tile ? tile < o.tile : zx < o.zx; }
+  };
+  const int tiles_x = (p->nxp + el::kVecX - 1) / el::kVecX, tiles = adj_tiles(p);
+  std::vector<Cell> cells(d.nr);
+  for (int r = 0; r < d.nr; ++r) {
+    const int z = rcv_z[r] + p->top, x = rcv_x[r] + d.nabc;
+    cells[r] = {z / el::kAR * tiles_x + x / el::kVecX, (z << 16) | x, r};
   }
+  std::stable_sort(cells.begin(), cells.end());
+  std::vector<int32_t> uzx, ubeg, urcv, tbeg(tiles + 1, 0);
+  for (int q = 0; q < d.nr; ++q) {
+    if (q == 0 || cells[q].zx != cells[q - 1].zx) {
+      uzx.push_back(cells[q].zx);
+      ubeg.push_back((int32_t)urcv.size());
+      ++tbeg[cells[q].tile + 1];
+    }
+    urcv.push_back(cells[q].r);
+  }
+  for (int t = 0; t < tiles; ++t) tbeg[t + 1] += tbeg[t];
   ubeg.push_back((int32_t)urcv.size());
   p->ncells = (int)uzx.size();
   p->o_uzx = t.size();
@@ -2102,6 +1876,8 @@ int adfwi_elastic_plan_create(const adfwi_elastic_desc* desc, const int32_t* src
   t.insert(t.end(), ubeg.begin(), ubeg.end());
   p->o_urcv = t.size();
   t.insert(t.end(), urcv.begin(), urcv.end());
+  p->o_tbeg = t.size();
+  t.insert(t.end(), tbeg.begin(), tbeg.end());
   if (t.empty()) t.push_back(0);
   // torch.chunk(wavelet, checkpoint_segments): the energy maps keep the last step of each chunk
   const int chunk = (d.nt + d.checkpoint_segments - 1) / d.checkpoint_segments;

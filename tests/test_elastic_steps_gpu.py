@@ -1,7 +1,8 @@
 """Elastic step kernels at the edges of their launches, against the CPU oracle (GPU tests).
 
 Receivers on the rows above the free surface (whose velocities the next stress update forms from
-the rows below), more receivers than one block of threads, an odd number of shots, one and two
+the rows below), more receivers than one block of threads, more receiver cells in one tile of the
+reverse kernels than a block has threads, an odd number of shots, one and two
 steps (the velocity records of the last step are taken after it), grids of a partial tile, and
 recomputed segments. In float64 the two sides round differently a few times per step and cell, so
 records stay within steps x 1e-14 < 1e-12 relative L2, and gradients, which sum products of two
@@ -28,6 +29,7 @@ def close(a, b, tol):
     (45, 3, 300, 21, 30, 4, "PML", True, 0),
     (45, 2, 40, 24, 41, 6, "PML", True, 11),
     (45, 3, 256, 16, 25, 4, "PML", False, 0),
+    (45, 2, 600, 21, 30, 6, "PML", True, 0),
     (1, 2, 5, 12, 20, 4, "gerjan", False, 0),
     (45, 3, 300, 21, 30, 6, "gerjan", False, 0),
     (45, 2, 40, 24, 41, 4, "gerjan", True, 11),
