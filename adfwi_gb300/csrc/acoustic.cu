@@ -191,6 +191,7 @@ __global__ void zero_outside_p(const __grid_constant__ ac::Geo<float> g, int64_t
 
 #include "acoustic_tma.cuh"
 #include "acoustic_vec.cuh"
+#include "acoustic_f64.cuh"
 #include "acoustic_res.h"
 #include "bsave.cuh"
 
@@ -224,6 +225,7 @@ struct adfwi_acoustic_plan {
   Tiling t2;             // 16 x 64 tiles of the pipelined forward and adjoint steps
   Resident rf, ra;       // the resident time loop, forward and adjoint, where the grid allows it
   int64_t o_sm = 0;      // tab: the model of each shot
+  int64_t o_rij = 0, o_cij = 0;  // tab: padded cells of the receivers and of the unique receiver cells (FP64)
   int K, nseg;           // snapshot interval and number of segments (gradient mode)
   int last_chunk_start;  // first step of the reference's last checkpoint chunk
   int elem;              // bytes per element
@@ -385,38 +387,22 @@ int setup_common(const adfwi_acoustic_plan* p, unsigned char* ws, const Carve& c
   return kOk;
 }
 
-// Stages of the TMA ring of each variant (deep: the FP32 variants compiled for VDEEP blocks per
-// SM; FP64 has one variant).
-template <typename T>
-int vec_adj_stages(bool deep) {
-  return sizeof(T) == 8 ? 2 : ((deep ? ac2::VDEEP : ac2::VAMINB) >= 3 ? 2 : 3);
+// Stages of the TMA ring of each variant of the FP32 step kernels (deep: those compiled for VDEEP
+// blocks per SM).
+int vec_adj_stages(bool deep) { return (deep ? ac2::VDEEP : ac2::VAMINB) >= 3 ? 2 : 3; }
+int vec_stages(bool deep) { return (deep ? ac2::VDEEP : ac2::VMINB) >= 3 ? 3 : 4; }
+using StepKernel = void (*)(ac2::Maps, ac::Geo<float>, ac2::StepArgs<float>);
+StepKernel fwd_kernel(bool deep) {
+  return deep ? ac2::fwd_step_vec<float, ac2::VDEEP> : ac2::fwd_step_vec<float, ac2::VMINB>;
 }
-template <typename T>
-int vec_stages(bool deep) {
-  return sizeof(T) == 8 ? 2 : ((deep ? ac2::VDEEP : ac2::VMINB) >= 3 ? 3 : 4);
-}
-template <typename T>
-using StepKernel = void (*)(ac2::Maps, ac::Geo<T>, ac2::StepArgs<T>);
-template <typename T>
-StepKernel<T> fwd_kernel(bool deep) {
-  if constexpr (sizeof(T) == 4) {
-    if (deep) return ac2::fwd_step_vec<T, ac2::VDEEP>;
-  }
-  return ac2::fwd_step_vec<T, ac2::VMINB>;
-}
-template <typename T>
-StepKernel<T> adj_kernel(bool deep) {
-  if constexpr (sizeof(T) == 4) {
-    if (deep) return ac2::adj_step_vec<T, ac2::VDEEP>;
-  }
-  return ac2::adj_step_vec<T, ac2::VAMINB>;
+StepKernel adj_kernel(bool deep) {
+  return deep ? ac2::adj_step_vec<float, ac2::VDEEP> : ac2::adj_step_vec<float, ac2::VAMINB>;
 }
 
 // Launch of a persistent step kernel with programmatic stream serialisation (the kernel
 // calls griddepcontrol.wait before touching data of the previous launch).
-template <typename T>
-cudaError_t launch_pdl(void (*kernel)(ac2::Maps, ac::Geo<T>, ac2::StepArgs<T>), int blocks, int smem, cudaStream_t st,
-                       const ac2::Maps& maps, const ac::Geo<T>& g, const ac2::StepArgs<T>& a) {
+cudaError_t launch_pdl(StepKernel kernel, int blocks, int smem, cudaStream_t st, const ac2::Maps& maps,
+                       const ac::Geo<float>& g, const ac2::StepArgs<float>& a) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3(ac2::VTHREADS);
@@ -430,9 +416,8 @@ cudaError_t launch_pdl(void (*kernel)(ac2::Maps, ac::Geo<T>, ac2::StepArgs<T>), 
   return cudaLaunchKernelEx(&cfg, kernel, maps, g, a);
 }
 
-template <typename T>
-ac2::StepArgs<T> step_args(const adfwi_acoustic_plan* p, int it, const T* cf, int* flag) {
-  ac2::StepArgs<T> a;
+ac2::StepArgs<float> step_args(const adfwi_acoustic_plan* p, int it, const float* cf, int* flag) {
+  ac2::StepArgs<float> a;
   memset(&a, 0, sizeof(a));
   a.it = it;
   a.G = p->t2.G;
@@ -444,19 +429,18 @@ ac2::StepArgs<T> step_args(const adfwi_acoustic_plan* p, int it, const T* cf, in
   return a;
 }
 
-template <typename T>
-int launch_fwd(const adfwi_acoustic_plan* p, const ac::Geo<T>& g, int it, int accum_u, const T* cf,
-               const T* wav, const T* p0, const T* u0, const T* w0, T* p1, T* u1, T* w1, T* d1, T* rp, T* ru,
-               T* rw, T* ilp, T* ilu, int* flag, cudaStream_t st) {
+int launch_fwd(const adfwi_acoustic_plan* p, const ac::Geo<float>& g, int it, int accum_u, const float* cf,
+               const float* wav, const float* p0, const float* u0, const float* w0, float* p1, float* u1, float* w1, float* d1, float* rp, float* ru,
+               float* rw, float* ilp, float* ilu, int* flag, cudaStream_t st) {
   const int64_t ns = p->d.ns;
   ac2::Maps maps;
-  int rc = make_plane_map(&maps.a, u0, sizeof(T), p->L, ns, ac2::BOXX, ac2::EZ);
-  if (!rc) rc = make_plane_map(&maps.b, w0, sizeof(T), p->L, ns, ac2::BOXX, ac2::WZ);
-  if (!rc) rc = make_plane_map(&maps.c, p0, sizeof(T), p->L, ns, ac2::BOXX, ac2::EZ);
+  int rc = make_plane_map(&maps.a, u0, sizeof(float), p->L, ns, ac2::BOXX, ac2::EZ);
+  if (!rc) rc = make_plane_map(&maps.b, w0, sizeof(float), p->L, ns, ac2::BOXX, ac2::WZ);
+  if (!rc) rc = make_plane_map(&maps.c, p0, sizeof(float), p->L, ns, ac2::BOXX, ac2::EZ);
   if (rc) return rc;
-  ac2::StepArgs<T> a = step_args<T>(p, it, cf, flag);
+  ac2::StepArgs<float> a = step_args(p, it, cf, flag);
   a.accum_u = accum_u;
-  a.stages = vec_stages<T>(p->deep);
+  a.stages = vec_stages(p->deep);
   a.wav = wav;
   a.o0 = p1;
   a.o1 = u1;
@@ -467,26 +451,25 @@ int launch_fwd(const adfwi_acoustic_plan* p, const ac::Geo<T>& g, int it, int ac
   a.rec_w = rw;
   a.acc0 = ilp;
   a.acc1 = ilu;
-  const int smem = ac2::VecFwdLayout<T>::bytes(a.stages);
+  const int smem = ac2::VecFwdLayout<float>::bytes(a.stages);
   ADFWI_LAUNCH(kAcFwdStep, st,
-               ADFWI_CUDA_TRY(launch_pdl(fwd_kernel<T>(p->deep), p->t2.fwd_blocks, smem, st, maps, g, a)));
+               ADFWI_CUDA_TRY(launch_pdl(fwd_kernel(p->deep), p->t2.fwd_blocks, smem, st, maps, g, a)));
   return kOk;
 }
 
-template <typename T>
-int launch_adj(const adfwi_acoustic_plan* p, const ac::Geo<T>& g, int it, const T* cf, const T* lp0, const T* lu0,
-               const T* lw0, T* lp1, T* lu1, T* lw1, const T* ph, const T* dh, const T* gp, const T* gu, const T* gw,
-               T* g1, T* g2, int* flag, cudaStream_t st) {
+int launch_adj(const adfwi_acoustic_plan* p, const ac::Geo<float>& g, int it, const float* cf, const float* lp0, const float* lu0,
+               const float* lw0, float* lp1, float* lu1, float* lw1, const float* ph, const float* dh, const float* gp, const float* gu, const float* gw,
+               float* g1, float* g2, int* flag, cudaStream_t st) {
   const int64_t ns = p->d.ns;
   ac2::Maps maps;
-  int rc = make_plane_map(&maps.a, lu0, sizeof(T), p->L, ns, ac2::BOXX, ac2::EZ);
-  if (!rc) rc = make_plane_map(&maps.b, lw0, sizeof(T), p->L, ns, ac2::BOXX, ac2::WZ);
-  if (!rc) rc = make_plane_map(&maps.c, lp0, sizeof(T), p->L, ns, ac2::BOXX, ac2::EZ);
-  if (!rc) rc = make_plane_map(&maps.d, ph, sizeof(T), p->L, ns, ac2::BOXX, ac2::EZ);
-  if (!rc) rc = make_plane_map(&maps.e, dh, sizeof(T), p->L, ns, ac2::BOXX, ac2::EZ);
+  int rc = make_plane_map(&maps.a, lu0, sizeof(float), p->L, ns, ac2::BOXX, ac2::EZ);
+  if (!rc) rc = make_plane_map(&maps.b, lw0, sizeof(float), p->L, ns, ac2::BOXX, ac2::WZ);
+  if (!rc) rc = make_plane_map(&maps.c, lp0, sizeof(float), p->L, ns, ac2::BOXX, ac2::EZ);
+  if (!rc) rc = make_plane_map(&maps.d, ph, sizeof(float), p->L, ns, ac2::BOXX, ac2::EZ);
+  if (!rc) rc = make_plane_map(&maps.e, dh, sizeof(float), p->L, ns, ac2::BOXX, ac2::EZ);
   if (rc) return rc;
-  ac2::StepArgs<T> a = step_args<T>(p, it, cf, flag);
-  a.stages = vec_adj_stages<T>(p->deep);
+  ac2::StepArgs<float> a = step_args(p, it, cf, flag);
+  a.stages = vec_adj_stages(p->deep);
   a.o0 = lp1;
   a.o1 = lu1;
   a.o2 = lw1;
@@ -495,33 +478,80 @@ int launch_adj(const adfwi_acoustic_plan* p, const ac::Geo<T>& g, int it, const 
   a.rec_w = gw;
   a.acc0 = g1;
   a.acc1 = g2;
-  const int smem = ac2::VecAdjLayout<T>::bytes(a.stages);
+  const int smem = ac2::VecAdjLayout<float>::bytes(a.stages);
   ADFWI_LAUNCH(kAcAdjStep, st,
-               ADFWI_CUDA_TRY(launch_pdl(adj_kernel<T>(p->deep), p->t2.blocks, smem, st, maps, g, a)));
+               ADFWI_CUDA_TRY(launch_pdl(adj_kernel(p->deep), p->t2.blocks, smem, st, maps, g, a)));
+  return kOk;
+}
+
+// The double-precision step (acoustic_f64.cuh): the same arguments.
+ac3::Cells f64_cells(const adfwi_acoustic_plan* p, const ac::Geo<double>& g) {
+  const int32_t* tb = g.src_z - p->o_srcz;
+  return {tb + p->o_rij, tb + p->o_cij, p->t2.ncells};
+}
+unsigned f64_blocks(int64_t n) { return (unsigned)((n + ac3::kThreads - 1) / ac3::kThreads); }
+
+int launch_fwd(const adfwi_acoustic_plan* p, const ac::Geo<double>& g, int it, int accum_u, const double* cf,
+               const double* wav, const double* p0, const double* u0, const double* w0, double* p1, double* u1,
+               double* w1, double* d1, double* rp, double* ru, double* rw, double* ilp, double* ilu, int*,
+               cudaStream_t st) {
+  const ac3::Cells cells = f64_cells(p, g);
+  const int64_t cfs = (int64_t)ac::kNumCoef * p->L.plane;
+  const unsigned nt = ac3::tiles(p->L, p->zbeg), gy = p->t2.ngroups;
+  const unsigned rb = rp != nullptr && p->d.nr > 0 ? f64_blocks(p->d.nr) : 0;
+  const dim3 b(ac3::kThreads);
+  ADFWI_LAUNCH(kAcFwdStep, st,
+               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::p_step, dim3(nt + (it > 0 ? rb : 0), gy), b, 0, st, g, cells, (int)nt,
+                                                it, cf, cfs, p0, u0, w0, p1, d1, wav, ilp, ru, rw)));
+  ADFWI_LAUNCH(kAcFwdStep, st,
+               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::uw_step, dim3(nt + rb, gy), b, 0, st, g, cells, (int)nt, it, cf, cfs,
+                                                (const double*)p1, u0, w0, u1, w1, accum_u ? ilu : nullptr, rp)));
+  if (rb && it + 1 == p->d.nt)
+    ADFWI_LAUNCH(kAux, st, ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::record_uw, dim3(rb, gy), b, 0, st, g, cells, it,
+                                                            (const double*)u1, (const double*)w1, ru, rw)));
+  return kOk;
+}
+
+// (lambda_u and lambda_w advance in place; qp: one scratch plane per shot, zero above the tiled rows)
+int launch_adj_f64(const adfwi_acoustic_plan* p, const ac::Geo<double>& g, int it, const double* cf, const double* lp0,
+                   double* lp1, double* lu, double* lw, double* qp, const double* ph, const double* dh, const double* gp,
+                   const double* gu, const double* gw, double* g1, double* g2, cudaStream_t st) {
+  const ac3::Cells cells = f64_cells(p, g);
+  const int64_t cfs = (int64_t)ac::kNumCoef * p->L.plane;
+  const unsigned nt = ac3::tiles(p->L, p->zbeg), gy = p->t2.ngroups, cb = f64_blocks(cells.ncells);
+  const dim3 b(ac3::kThreads);
+  ADFWI_LAUNCH(kAcAdjStep, st,
+               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::adj_p_step, dim3(nt, gy), b, 0, st, g, cf, cfs, lp0, (const double*)lu,
+                                                (const double*)lw, lp1, qp, dh, g1)));
+  ADFWI_LAUNCH(kAcAdjStep, st,
+               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::adj_uw_step, dim3(nt + (gp && it >= 1 ? cb : 0), gy), b, 0, st, g, cells,
+                                                (int)nt, it, cf, cfs, (const double*)qp, lu, lw, ph, g2, gp, lp1)));
+  if ((gu || gw) && it >= 1 && cells.ncells > 0) {
+    ADFWI_LAUNCH(kAux, st, (ac3::adj_inject_uw<<<dim3(cb, p->d.ns), b, 0, st>>>(g, cells, it - 1, gu, gw, lu, lw)));
+    ADFWI_CUDA_TRY(cudaGetLastError());
+  }
   return kOk;
 }
 
 // The opt-in above 48 KB of dynamic shared memory is a property of the kernel in one device's
-// context, so it is set once per device ordinal (and per element type), under a mutex: the
+// context, so it is set once per device ordinal, under a mutex: the
 // serving workers call solves from several threads, and a process may drive more than one GPU.
 std::mutex g_smem_mu;
-std::vector<unsigned char> g_smem_done;  // bit 0: float kernels, bit 1: double kernels, per device
+std::vector<unsigned char> g_smem_done;  // per device
 
-template <typename T>
 int set_smem_limits() {
   int dev = 0;
   ADFWI_CUDA_TRY(cudaGetDevice(&dev));
-  const unsigned char bit = sizeof(T) == 8 ? 2 : 1;
   std::lock_guard<std::mutex> lk(g_smem_mu);
   if ((int)g_smem_done.size() <= dev) g_smem_done.resize(dev + 1, 0);
-  if (!(g_smem_done[dev] & bit)) {
-    for (int deep = 0; deep < (sizeof(T) == 4 ? 2 : 1); ++deep) {
-      ADFWI_CUDA_TRY(cudaFuncSetAttribute(fwd_kernel<T>(deep), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          ac2::VecFwdLayout<T>::bytes(vec_stages<T>(deep))));
-      ADFWI_CUDA_TRY(cudaFuncSetAttribute(adj_kernel<T>(deep), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          ac2::VecAdjLayout<T>::bytes(vec_adj_stages<T>(deep))));
+  if (!g_smem_done[dev]) {
+    for (int deep = 0; deep < 2; ++deep) {
+      ADFWI_CUDA_TRY(cudaFuncSetAttribute(fwd_kernel(deep), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          ac2::VecFwdLayout<float>::bytes(vec_stages(deep))));
+      ADFWI_CUDA_TRY(cudaFuncSetAttribute(adj_kernel(deep), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          ac2::VecAdjLayout<float>::bytes(vec_adj_stages(deep))));
     }
-    g_smem_done[dev] |= bit;
+    g_smem_done[dev] = 1;
   }
   return kOk;
 }
@@ -723,7 +753,7 @@ template <typename T>
 int forward_impl(const adfwi_acoustic_plan* p, const void* alpha1, const void* alpha2, const void* damp,
                  const void* wavelet, void* rec_p, void* rec_u, void* rec_w, void* fw_p, void* fw_u,
                  void* fw_w, bool grad, unsigned char* ws, int64_t ws_bytes, cudaStream_t st, bool box = true) {
-  int rc = set_smem_limits<T>();
+  int rc = sizeof(T) == 4 ? set_smem_limits() : kOk;
   if (rc) return rc;
   const int K = grad ? p->K : 1;
   Carve c = carve(p, grad, K, box);
@@ -782,7 +812,7 @@ int forward_impl(const adfwi_acoustic_plan* p, const void* alpha1, const void* a
       p1 = hp + (int64_t)it * ns * pl;
       d1 = hd + (int64_t)it * ns * pl;
     }
-    rc = launch_fwd<T>(p, g, it, it >= p->last_chunk_start ? 1 : 0, cf, wav, p0, cur + ns * pl, cur + 2 * ns * pl,
+    rc = launch_fwd(p, g, it, it >= p->last_chunk_start ? 1 : 0, cf, wav, p0, cur + ns * pl, cur + 2 * ns * pl,
                        p1, nxt + ns * pl, nxt + 2 * ns * pl, d1, static_cast<T*>(rec_p), static_cast<T*>(rec_u),
                        static_cast<T*>(rec_w), ilp, ilu, flag, st);
     if (rc) return rc;
@@ -825,7 +855,7 @@ template <typename T>
 int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void* grp, const void* gru,
                   const void* grw, void* ga1, void* ga2, unsigned char* ws, int64_t ws_bytes, cudaStream_t st,
                   const FusedL2* fz = nullptr) {
-  int rc = set_smem_limits<T>();
+  int rc = sizeof(T) == 4 ? set_smem_limits() : kOk;
   if (rc) return rc;
   const int K = p->K;
   Carve c = carve(p, true, K);
@@ -921,6 +951,19 @@ int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void*
   }
   T* lcur = la;
   T* lnxt = lb;
+  // reverse step it on p after it and its divergence
+  auto reverse = [&](int it, const T* ph, const T* dh) {
+    int e;
+    if constexpr (sizeof(T) == 8) {  // lambda_u, lambda_w in place in la; q in lb
+      e = launch_adj_f64(p, g2, it, cf, lcur, lnxt, la + ns * pl, la + 2 * ns * pl, lb + ns * pl, ph, dh, gp, gu, gw, g1p,
+                         g2p, st);
+    } else {
+      e = launch_adj(p, g2, it, cf, lcur, lcur + ns * pl, lcur + 2 * ns * pl, lnxt, lnxt + ns * pl, lnxt + 2 * ns * pl, ph,
+                     dh, gp, gu, gw, g1p, g2p, flag, st);
+    }
+    std::swap(lcur, lnxt);
+    return e;
+  };
   if (boundary_saving(p)) {
     // The forward left its last state in fa (nt even) or fb; rebuild the states backwards, the
     // pressure ping-ponging between the two buffers' p planes, u and w in place.
@@ -939,10 +982,8 @@ int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void*
                                                                       p->nframe)));
       ADFWI_LAUNCH(kAux, st, (ac::bs_reverse_p<T><<<gr, gb, 0, st>>>(g2, p->bbox, it, fidx, cf, pcur, u, w, poth, hd,
                                                                      slot, p->nframe, wav)));
-      rc = launch_adj<T>(p, g2, it, cf, lcur, lcur + ns * pl, lcur + 2 * ns * pl, lnxt, lnxt + ns * pl,
-                         lnxt + 2 * ns * pl, pcur, hd, gp, gu, gw, g1p, g2p, flag, st);
+      rc = reverse(it, pcur, hd);
       if (rc) return rc;
-      std::swap(lcur, lnxt);
       std::swap(pcur, poth);
     }
     ADFWI_CUDA_TRY(cudaGetLastError());
@@ -967,7 +1008,7 @@ int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void*
       }
       for (int it = resident ? t1 : t0; it < t1; ++it) {
         const T* p0 = it == t0 ? fa : hp + (int64_t)(it - 1 - t0) * ns * pl;
-        rc = launch_fwd<T>(p, g2, it, 0, cf, wav, p0, cur + ns * pl, cur + 2 * ns * pl,
+        rc = launch_fwd(p, g2, it, 0, cf, wav, p0, cur + ns * pl, cur + 2 * ns * pl,
                            hp + (int64_t)(it - t0) * ns * pl, nxt + ns * pl, nxt + 2 * ns * pl,
                            hd + (int64_t)(it - t0) * ns * pl, nullptr, nullptr, nullptr, nullptr, nullptr, flag, st);
         if (rc) return rc;
@@ -975,11 +1016,8 @@ int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void*
       }
     }
     for (int it = t1 - 1; it >= t0; --it) {
-      rc = launch_adj<T>(p, g2, it, cf, lcur, lcur + ns * pl, lcur + 2 * ns * pl, lnxt, lnxt + ns * pl,
-                         lnxt + 2 * ns * pl, hp + (int64_t)(it - t0) * ns * pl, hd + (int64_t)(it - t0) * ns * pl, gp,
-                         gu, gw, g1p, g2p, flag, st);
+      rc = reverse(it, hp + (int64_t)(it - t0) * ns * pl, hd + (int64_t)(it - t0) * ns * pl);
       if (rc) return rc;
-      std::swap(lcur, lnxt);
     }
     ADFWI_CUDA_TRY(cudaGetLastError());
   }
@@ -1063,15 +1101,13 @@ int resident_blocks(K kernel, int threads, int smem, int fallback) {
   return sms * occ;
 }
 
-template <typename T>
 int resident_adj_blocks(bool deep) {
-  return resident_blocks(adj_kernel<T>(deep), ac2::VTHREADS, ac2::VecAdjLayout<T>::bytes(vec_adj_stages<T>(deep)),
-                         sizeof(T) == 8 ? 1 : (deep ? ac2::VDEEP : ac2::VAMINB));
+  return resident_blocks(adj_kernel(deep), ac2::VTHREADS, ac2::VecAdjLayout<float>::bytes(vec_adj_stages(deep)),
+                         deep ? ac2::VDEEP : ac2::VAMINB);
 }
-template <typename T>
 int resident_fwd_blocks(bool deep) {
-  return resident_blocks(fwd_kernel<T>(deep), ac2::VTHREADS, ac2::VecFwdLayout<T>::bytes(vec_stages<T>(deep)),
-                         sizeof(T) == 8 ? 1 : (deep ? ac2::VDEEP : ac2::VMINB));
+  return resident_blocks(fwd_kernel(deep), ac2::VTHREADS, ac2::VecFwdLayout<float>::bytes(vec_stages(deep)),
+                         deep ? ac2::VDEEP : ac2::VMINB);
 }
 
 // Padded grids at least this wide run the deep-ring variants (one more stage, 2 blocks per SM).
@@ -1185,6 +1221,11 @@ void build_tiling(adfwi_acoustic_plan* p, Tiling* tl, int tz, int tx, const std:
   tl->o_cr = t.size();
   t.insert(t.end(), cr.begin(), cr.end());
 }
+
+// Shots per group of the double-precision steps: one while that gives at most 16 blocks of 128 threads
+// per SM (more blocks than are resident), then as many as keep to that; a group has one partial plane
+// per sum.
+int f64_group_shots(int ns, int tiles) { return std::max(1, (int)((int64_t)ns * tiles / (152 * 16))); }
 
 // Shared memory of a configuration, in words.
 // (most, most_rows: receiver cells, and rows holding any, of the strip that has the most)
@@ -1595,21 +1636,33 @@ int plan_create_impl(const adfwi_acoustic_desc* desc, const int32_t* src_z, cons
     const int ntiles = ((p->nxp + ac2::TX - 1) / ac2::TX) * ((p->nzp - p->zbeg + ac2::TZ - 1) / ac2::TZ);
     // shots per group from the shallow variants' widths whatever the ring, so that the ring
     // changes launch widths and stages only, never the results
-    const int blocks = p->elem == 8 ? resident_adj_blocks<double>(false) : resident_adj_blocks<float>(false);
-    const int fblocks = p->elem == 8 ? resident_fwd_blocks<double>(false) : resident_fwd_blocks<float>(false);
-    p->deep = p->elem == 4 && (d.ring_depth == 2 || (d.ring_depth == 0 && p->nxp >= kDeepRingCols));
-    const int run_blocks = p->deep ? resident_adj_blocks<float>(true) : blocks;
-    const int run_fblocks = p->deep ? resident_fwd_blocks<float>(true) : fblocks;
+    const bool f64 = p->elem == 8;
+    const int blocks = f64 ? 1 : resident_adj_blocks(false), fblocks = f64 ? 1 : resident_fwd_blocks(false);
+    p->deep = !f64 && (d.ring_depth == 2 || (d.ring_depth == 0 && p->nxp >= kDeepRingCols));
+    const int run_blocks = p->deep ? resident_adj_blocks(true) : blocks;
+    const int run_fblocks = p->deep ? resident_fwd_blocks(true) : fblocks;
     // shots per group of each model: as a plan of that model alone would choose them, so a
     // model's partial sums (and so its results) do not depend on the other models of a batch
     std::vector<int> Gm(p->nm);
     for (int m = 0; m < p->nm; ++m) {
       const std::vector<int> alone = {0, p->model_shot_beg[m + 1] - p->model_shot_beg[m]};
-      Gm[m] = d.shots_per_block > 0 ? d.shots_per_block : pick_unit_shots(alone, ntiles, fblocks, blocks);
+      if (d.shots_per_block > 0) Gm[m] = d.shots_per_block;
+      else if (f64) Gm[m] = f64_group_shots(alone[1], ac3::tiles(p->L, p->zbeg));
+      else Gm[m] = pick_unit_shots(alone, ntiles, fblocks, blocks);
     }
     build_tiling(p, &p->t2, ac2::TZ, ac2::TX, Gm, rcv_z, rcv_x);
     p->t2.blocks = std::max(1, std::min(run_blocks, p->t2.ntiles * p->t2.ngroups));
     p->t2.fwd_blocks = std::max(1, std::min(run_fblocks, p->t2.ntiles * p->t2.ngroups));
+  }
+  if (p->elem == 8) {
+    p->o_rij = t.size();
+    for (int r = 0; r < d.nr; ++r) t.push_back((rcv_z[r] + d.nabc) << 16 | (rcv_x[r] + d.nabc));
+    p->o_cij = t.size();
+    for (int q = 0; q < p->t2.ncells; ++q) {  // a cell's first receiver tells where it lies
+      const int r = t[p->t2.o_cr + t[p->t2.o_tcr + q]];
+      const int ij = t[p->o_rij + r];
+      t.push_back(ij);
+    }
   }
   plan_resident(p, rcv_z, rcv_x);
   if (t.empty()) t.push_back(0);
