@@ -218,8 +218,12 @@ def thomsen_to_elastic_moduli(alpha_thomsen, beta_thomsen, rho, eps_thomsen, del
     return c11, c13, c33, c44, c66
 
 
-def _zeros21(nz, nx, device, dtype):
-    return [torch.zeros((nz, nx), dtype=dtype).to(device) for _ in range(21)]
+_ZERO_MODULI = (3, 4, 5, 8, 9, 10, 12, 13, 14, 16, 17, 19)  # moduli that are zero in VTI and HTI media
+
+
+def _zero_moduli(nz, nx, device, dtype):
+    """21 places with zeros, made on the device, at those that no modulus takes."""
+    return [torch.zeros((nz, nx), dtype=dtype, device=device) if k in _ZERO_MODULI else None for k in range(21)]
 
 
 def _five_point(a, nz, nx):
@@ -246,7 +250,7 @@ class _ElasticBase(AbstractModel):
         self.mu, self.lamu, self.lam, self.b = vs_vp_to_Lame(self.vp, self.vs, self.rho)
 
     def _parameterization_elastic_moduli(self):
-        CC = _zeros21(self.nz, self.nx, self.device, self.dtype)
+        CC = _zero_moduli(self.nz, self.nx, self.device, self.dtype)
         C11, C13, C33, C44, C66 = thomsen_to_elastic_moduli(self.vp, self.vs, self.rho, self.eps,
                                                             self.delta, self.gamma)
         C12 = (C11 - 2 * C66).clone()

@@ -23,13 +23,15 @@ CUDA device (the parameters' padded coefficients are copied there and the record
 differentiably, so gradients reach the CPU parameters). There is no CPU solver: without a CUDA
 device the constructor raises.
 """
+import ctypes
 from typing import Dict, Optional
 
 import numpy as np
 import torch
 from torch import Tensor
 
-from .acoustic import AcousticPlan, AcousticSolve
+from . import _native as N
+from .acoustic import AcousticPlan, AcousticSolve, dtype_code
 from .boundary import bc_gerjan, bc_pml, bc_pml_xz, bc_sincos
 from .utils import numpy2tensor
 
@@ -42,10 +44,50 @@ def _is_survey(s):
     return hasattr(s, "source") and hasattr(s, "receiver")
 
 
+_PAD_PLANES = 10  # planes of one native call
+
+
+def _native_planes(ts):
+    """Whether the CUDA library pads / folds these planes: plain FP32 or FP64 planes of one device."""
+    return (all(type(t) in (Tensor, torch.nn.Parameter) and t.is_cuda and t.dim() == 2 and t.numel() > 0
+                and t.dtype == ts[0].dtype and t.device == ts[0].device for t in ts)
+            and ts[0].dtype in (torch.float32, torch.float64) and not torch.compiler.is_compiling())
+
+
+def _native_call(fn, src, dst, shapes, pads):
+    """``adfwi_pad_replicate`` / ``adfwi_fold_replicate`` of the planes, a launch for every _PAD_PLANES."""
+    dev = src[0].device
+    call = getattr(N.lib(), fn)
+    code = dtype_code(src[0].dtype)
+    with torch.cuda.device(dev):
+        st = N.stream_handle(dev)
+        for k in range(0, len(src), _PAD_PLANES):
+            a, b, n = src[k:k + _PAD_PLANES], dst[k:k + _PAD_PLANES], min(_PAD_PLANES, len(src) - k)
+            N.check(call(n, code, (ctypes.c_void_p * n)(*[t.data_ptr() for t in a]),
+                         (ctypes.c_void_p * n)(*[t.data_ptr() for t in b]),
+                         (ctypes.c_int32 * (2 * n))(*[d for hw in shapes[k:k + _PAD_PLANES] for d in hw]), *pads, st), fn)
+
+
+def _fold_planes(gs, top, bottom, left, right):
+    """``fold_replicate`` of several planes: one launch for CUDA planes outside a graph of their own."""
+    graph = torch.is_grad_enabled() and any(g.requires_grad for g in gs)
+    if graph or not _native_planes(gs):
+        return [_fold_torch(g, top, bottom, left, right) for g in gs]
+    gs = [g.contiguous() for g in gs]
+    shapes = [(g.shape[0] - top - bottom, g.shape[1] - left - right) for g in gs]
+    outs = [g.new_empty(hw) for g, hw in zip(gs, shapes)]
+    _native_call("adfwi_fold_replicate", gs, outs, shapes, (top, bottom, left, right))
+    return outs
+
+
 def fold_replicate(g, top, bottom, left, right):
     """Adjoint of edge-replicate padding by (top, bottom, left, right) cells: the padded strips
     fold into the edge rows / columns and the corner blocks into the corner cells, with
     fixed-order reductions (the same sums on every run)."""
+    return _fold_planes([g], top, bottom, left, right)[0]
+
+
+def _fold_torch(g, top, bottom, left, right):
     nz, nx = g.shape[0] - top - bottom, g.shape[1] - left - right
     r0, r1, c0, c1 = top, top + nz, left, left + nx
     out = g[r0:r1, c0:c1].clone()
@@ -69,23 +111,41 @@ def fold_replicate(g, top, bottom, left, right):
 
 
 class _PadReplicate(torch.autograd.Function):
-    """Edge-replicate padding with the fold above as its backward (PyTorch's replicate-pad
-    backward accumulates with atomics on CUDA, so its FP32 sums vary from run to run)."""
+    """Edge-replicate padding of several planes with the fold above as its backward (PyTorch's
+    replicate-pad backward accumulates with atomics on CUDA, so its FP32 sums vary from run to
+    run). CUDA planes take one launch each way."""
 
     @staticmethod
-    def forward(ctx, v, top, bottom, left, right):
-        ctx.pads = (top, bottom, left, right)
-        return torch.nn.functional.pad(v[None, None], (left, right, top, bottom), mode="replicate")[0, 0]
+    def forward(ctx, pads, *vs):
+        ctx.pads = pads
+        ctx.set_materialize_grads(False)
+        top, bottom, left, right = pads
+        if not _native_planes(vs):
+            return tuple(torch.nn.functional.pad(v[None, None], (left, right, top, bottom), mode="replicate")[0, 0]
+                         for v in vs)
+        src = [v.contiguous() for v in vs]
+        shapes = [tuple(v.shape) for v in src]
+        outs = [v.new_empty((h + top + bottom, w + left + right)) for v, (h, w) in zip(src, shapes)]
+        _native_call("adfwi_pad_replicate", src, outs, shapes, pads)
+        return tuple(outs)
 
     @staticmethod
-    def backward(ctx, g):
-        return fold_replicate(g, *ctx.pads), None, None, None, None
+    def backward(ctx, *gs):
+        take = [k for k, g in enumerate(gs) if g is not None and ctx.needs_input_grad[1 + k]]
+        out = [None] * len(gs)
+        for k, g in zip(take, _fold_planes([gs[k] for k in take], *ctx.pads) if take else ()):
+            out[k] = g
+        return (None, *out)
+
+
+def _pad_planes(vs, top, bottom, left, right):
+    """Edge-replicate padding of planes (acoustic_kernels.py:16-37, elastic_kernels.py:175-216),
+    differentiable with a deterministic backward."""
+    return _PadReplicate.apply((top, bottom, left, right), *vs)
 
 
 def _pad_replicate(v, top, bottom, left, right):
-    """Edge-replicate padding (acoustic_kernels.py:16-37, elastic_kernels.py:175-216),
-    differentiable with a deterministic backward."""
-    return _PadReplicate.apply(v, top, bottom, left, right)
+    return _pad_planes([v], top, bottom, left, right)[0]
 
 
 class _PropagatorBase(torch.nn.Module):
@@ -217,8 +277,7 @@ class AcousticPropagator(_PropagatorBase):
         """alpha1 = rho c^2 dt/dz and alpha2 = dt/(rho dz) on the padded grid (acoustic_kernels.py:225-260)."""
         model = self.model if model is None else model
         n = self.nabc
-        c = _pad_replicate(model.vp, n, n, n, n)
-        den = _pad_replicate(model.rho, n, n, n, n)
+        c, den = _pad_planes([model.vp, model.rho], n, n, n, n)
         # The divisor is a 0-d tensor on the device: PyTorch's CUDA division by a host scalar
         # multiplies by its reciprocal, which rounds differently from the reference's division
         # (1 ulp on about a quarter of the cells); an elementwise division rounds like the CPU.
@@ -318,9 +377,8 @@ class ElasticPropagator(_PropagatorBase):
         fs_off = fd_order // 2
         n = self.nabc
         top = fs_off if self.free_surface else fs_off + n
-        pad = lambda a: _pad_replicate(a, top, n, n, n)  # noqa: E731
         CC = model.CC
-        coefs = [pad(CC[k]) for k in (0, 2, 4, 11, 13, 18)] + [pad(model.bx), pad(model.bz)]
+        coefs = _pad_planes([CC[k] for k in (0, 2, 4, 11, 13, 18)] + [model.bx, model.bz], top, n, n, n)
         coefs = [c.to(self.dtype) if c.dtype != self.dtype else c for c in coefs]
         bpad = lambda a: _pad_replicate(a, fs_off, 0, 0, 0)  # noqa: E731
         if self.abc_type.lower() == "pml":

@@ -285,6 +285,22 @@ int adfwi_acoustic_forward_noalloc(const adfwi_acoustic_plan* plan, const void* 
 int adfwi_acoustic_noalloc_status(const adfwi_acoustic_plan* plan, int32_t* status, void* stream);
 
 /* ------------------------------------------------------------------------- */
+/* Padding of model planes.                                                  */
+/* ------------------------------------------------------------------------- */
+
+/* Edge-replicate padding of up to ADFWI_PAD_PLANES dense device planes in one launch, and its
+ * adjoint: plane q is shapes[2q] x shapes[2q+1] unpadded and grows by top + bottom rows and
+ * left + right columns. adfwi_pad_replicate writes the padded planes; adfwi_fold_replicate adds
+ * padded planes `src` up to the unpadded `dst` (the padded strips and corner blocks into the edge
+ * cells they were copied from, summed in double precision in a fixed order). dtype: ADFWI_F32 or
+ * ADFWI_F64, of all planes. */
+#define ADFWI_PAD_PLANES 10
+int adfwi_pad_replicate(int32_t n, int32_t dtype, const void* const* src, void* const* dst, const int32_t* shapes,
+                        int32_t top, int32_t bottom, int32_t left, int32_t right, void* stream);
+int adfwi_fold_replicate(int32_t n, int32_t dtype, const void* const* src, void* const* dst, const int32_t* shapes,
+                         int32_t top, int32_t bottom, int32_t left, int32_t right, void* stream);
+
+/* ------------------------------------------------------------------------- */
 /* Errors and build information.                                             */
 /* ------------------------------------------------------------------------- */
 
