@@ -17,6 +17,7 @@ import numpy as np
 import torch
 
 from . import _native as N
+from .acoustic import dtype_code
 
 
 def smooth2d(z, span=10, stream=None):
@@ -84,6 +85,41 @@ class GradProcessor(object):
             self._taper[key] = t
         return t
 
+    def _native(self, nx, nz, vmax, g, forw, thred, dev):
+        """``forward`` with the illumination preconditioner by the CUDA library: plain (nz, nx) planes
+        that no autograd graph follows (otherwise None, and the device operations below run)."""
+        keep = self.grad_mute if self.marine_or_land in ("marine", "offshore") and self.grad_smooth > 0 else 0
+        if not (type(g) is torch.Tensor and type(forw) in (torch.Tensor, torch.nn.Parameter)
+                and tuple(g.shape) == (nz, nx) and tuple(forw.shape) == (nz, nx) and min(nz, nx) >= 2
+                and forw.dtype in (torch.float32, torch.float64) and 0 <= keep < nz
+                and isinstance(self.grad_smooth, int) and not torch.compiler.is_compiling()
+                and not (torch.is_grad_enabled() and (g.requires_grad or forw.requires_grad))):
+            return None
+        taper = mask = None
+        if self.grad_mute > 0:
+            taper = self._taper_for(nz, nx, thred, dev)
+        if self.grad_mask is not None:
+            mask = torch.as_tensor(np.asarray(self.grad_mask) if not torch.is_tensor(self.grad_mask) else self.grad_mask,
+                                   device=dev)
+            if tuple(mask.shape) != tuple(g.shape):
+                raise ValueError("Wrong size of grad mask: the size of the mask should be identical to the size of "
+                                 "vp model")
+            mask = mask.double().contiguous()
+        span = 40 if min(nz, nx) > 40 else int(min(nz, nx) / 2)
+        smooth = max(self.grad_smooth, 0)
+        g, forw = g.contiguous(), forw.contiguous()
+        out = torch.empty((nz, nx), dtype=torch.float64, device=dev)
+        lib = N.lib()
+        need = ctypes.c_int64()
+        N.check(lib.adfwi_gradproc_workspace_bytes(nz, nx, span, smooth, ctypes.byref(need)),
+                "adfwi_gradproc_workspace_bytes")
+        ws = torch.empty(need.value, dtype=torch.uint8, device=dev)
+        with torch.cuda.device(dev):
+            N.check(lib.adfwi_gradproc(nz, nx, span, smooth, keep, N.ptr(g), N.ptr(taper), N.ptr(mask),
+                                       dtype_code(forw.dtype), N.ptr(forw), int(bool(self.norm_grad)), float(vmax),
+                                       N.ptr(out), N.ptr(ws), ws.numel(), N.stream_handle(dev)), "adfwi_gradproc")
+        return out
+
     def forward(self, nx, nz, vmax, grad, forw=None):
         numpy_io = not torch.is_tensor(grad)
         if numpy_io:
@@ -100,6 +136,10 @@ class GradProcessor(object):
         else:
             raise ValueError("not supported modeling marine_or_land: %s" % self.marine_or_land)
         g = torch.as_tensor(grad, device=dev).to(torch.float32)
+        if self.forw_illumination and forw is not None:
+            out = self._native(nx, nz, vmax, g, torch.as_tensor(forw, device=dev), thred, dev)
+            if out is not None:
+                return out.cpu().numpy() if numpy_io else out
         if self.grad_mute > 0:  # in place on the float32 gradient
             g = (g.double() * self._taper_for(nz, nx, thred, dev)).float()
         if self.grad_mask is not None:

@@ -257,6 +257,16 @@ int adfwi_smooth2d_workspace_bytes(int32_t nz, int32_t nx, int32_t span, int64_t
 int adfwi_smooth2d(int32_t nz, int32_t nx, int32_t span, const double* in, double* out, void* workspace,
                    int64_t workspace_bytes, void* stream);
 
+/* The gradient processor with the illumination preconditioner in seven launches: grad (FP32) times
+ * taper and mask (FP64, each may be null, each product rounded to FP32), divided by the square of
+ * the illumination smoothed with `span`, scaled to at most 1 and kept above 1e-4; with smooth > 0 the
+ * rows from keep_rows on are smoothed; with norm the result is scaled to an absolute maximum of vmax.
+ * illum is FP32 or FP64, out FP64 (nz, nx). */
+int adfwi_gradproc_workspace_bytes(int32_t nz, int32_t nx, int32_t span, int32_t smooth, int64_t* bytes);
+int adfwi_gradproc(int32_t nz, int32_t nx, int32_t span, int32_t smooth, int32_t keep_rows, const float* grad,
+                   const double* taper, const double* mask, int32_t illum_dtype, const void* illum, int32_t norm,
+                   double vmax, double* out, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* Forward solve that allocates nothing, for callers that cannot call cudaMalloc: hosts whose
  * device memory is entirely owned by another allocator or pool, sandboxed plug-ins that may
  * not grow their footprint after start-up, or code running where an allocation would break
