@@ -225,7 +225,8 @@ struct adfwi_acoustic_plan {
   Tiling t2;             // 16 x 64 tiles of the pipelined forward and adjoint steps
   Resident rf, ra;       // the resident time loop, forward and adjoint, where the grid allows it
   int64_t o_sm = 0;      // tab: the model of each shot
-  int64_t o_rij = 0, o_cij = 0;  // tab: padded cells of the receivers and of the unique receiver cells (FP64)
+  // tab (FP64): padded cells of the receivers and of the unique receiver cells; the latter by tile
+  int64_t o_rij = 0, o_cij = 0, o_ftb = 0, o_ftc = 0;
   int K, nseg;           // snapshot interval and number of segments (gradient mode)
   int last_chunk_start;  // first step of the reference's last checkpoint chunk
   int elem;              // bytes per element
@@ -484,10 +485,10 @@ int launch_adj(const adfwi_acoustic_plan* p, const ac::Geo<float>& g, int it, co
   return kOk;
 }
 
-// The double-precision step (acoustic_f64.cuh): the same arguments.
+// The double-precision steps (acoustic_f64.cuh): the same arguments.
 ac3::Cells f64_cells(const adfwi_acoustic_plan* p, const ac::Geo<double>& g) {
   const int32_t* tb = g.src_z - p->o_srcz;
-  return {tb + p->o_rij, tb + p->o_cij, p->t2.ncells};
+  return {tb + p->o_rij, tb + p->o_cij, tb + p->o_ftb, tb + p->o_ftc, p->t2.ncells};
 }
 unsigned f64_blocks(int64_t n) { return (unsigned)((n + ac3::kThreads - 1) / ac3::kThreads); }
 
@@ -501,33 +502,30 @@ int launch_fwd(const adfwi_acoustic_plan* p, const ac::Geo<double>& g, int it, i
   const unsigned rb = rp != nullptr && p->d.nr > 0 ? f64_blocks(p->d.nr) : 0;
   const dim3 b(ac3::kThreads);
   ADFWI_LAUNCH(kAcFwdStep, st,
-               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::p_step, dim3(nt + (it > 0 ? rb : 0), gy), b, 0, st, g, cells, (int)nt,
-                                                it, cf, cfs, p0, u0, w0, p1, d1, wav, ilp, ru, rw)));
-  ADFWI_LAUNCH(kAcFwdStep, st,
-               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::uw_step, dim3(nt + rb, gy), b, 0, st, g, cells, (int)nt, it, cf, cfs,
-                                                (const double*)p1, u0, w0, u1, w1, accum_u ? ilu : nullptr, rp)));
+               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::fwd_step, dim3(nt + (it > 0 ? rb : 0), gy), b, 0, st, g, cells, (int)nt,
+                                                it, cf, cfs, p0, u0, w0, p1, u1, w1, d1, wav, ilp,
+                                                accum_u ? ilu : nullptr, rp, ru, rw)));
   if (rb && it + 1 == p->d.nt)
-    ADFWI_LAUNCH(kAux, st, ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::record_uw, dim3(rb, gy), b, 0, st, g, cells, it,
-                                                            (const double*)u1, (const double*)w1, ru, rw)));
+    ADFWI_LAUNCH(kAux, st, ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::record_last, dim3(rb, gy), b, 0, st, g, cells, it,
+                                                            (const double*)p1, (const double*)u1, (const double*)w1, rp,
+                                                            ru, rw)));
   return kOk;
 }
 
-// (lambda_u and lambda_w advance in place; qp: one scratch plane per shot, zero above the tiled rows)
-int launch_adj_f64(const adfwi_acoustic_plan* p, const ac::Geo<double>& g, int it, const double* cf, const double* lp0,
-                   double* lp1, double* lu, double* lw, double* qp, const double* ph, const double* dh, const double* gp,
-                   const double* gu, const double* gw, double* g1, double* g2, cudaStream_t st) {
+int launch_adj(const adfwi_acoustic_plan* p, const ac::Geo<double>& g, int it, const double* cf, const double* lp0,
+               const double* lu0, const double* lw0, double* lp1, double* lu1, double* lw1, const double* ph,
+               const double* dh, const double* gp, const double* gu, const double* gw, double* g1, double* g2, int*,
+               cudaStream_t st) {
   const ac3::Cells cells = f64_cells(p, g);
   const int64_t cfs = (int64_t)ac::kNumCoef * p->L.plane;
-  const unsigned nt = ac3::tiles(p->L, p->zbeg), gy = p->t2.ngroups, cb = f64_blocks(cells.ncells);
+  const unsigned nt = ac3::tiles(p->L, p->zbeg), gy = p->t2.ngroups;
   const dim3 b(ac3::kThreads);
   ADFWI_LAUNCH(kAcAdjStep, st,
-               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::adj_p_step, dim3(nt, gy), b, 0, st, g, cf, cfs, lp0, (const double*)lu,
-                                                (const double*)lw, lp1, qp, dh, g1)));
-  ADFWI_LAUNCH(kAcAdjStep, st,
-               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::adj_uw_step, dim3(nt + (gp && it >= 1 ? cb : 0), gy), b, 0, st, g, cells,
-                                                (int)nt, it, cf, cfs, (const double*)qp, lu, lw, ph, g2, gp, lp1)));
+               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::adj_step, dim3(nt, gy), b, 0, st, g, cells, it, cf, cfs, lp0, lu0, lw0,
+                                                lp1, lu1, lw1, ph, dh, g1, g2, gp)));
   if ((gu || gw) && it >= 1 && cells.ncells > 0) {
-    ADFWI_LAUNCH(kAux, st, (ac3::adj_inject_uw<<<dim3(cb, p->d.ns), b, 0, st>>>(g, cells, it - 1, gu, gw, lu, lw)));
+    ADFWI_LAUNCH(kAux, st, (ac3::adj_inject_uw<<<dim3(f64_blocks(cells.ncells), p->d.ns), b, 0, st>>>(g, cells, it - 1, gu,
+                                                                                                       gw, lu1, lw1)));
     ADFWI_CUDA_TRY(cudaGetLastError());
   }
   return kOk;
@@ -953,14 +951,8 @@ int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void*
   T* lnxt = lb;
   // reverse step it on p after it and its divergence
   auto reverse = [&](int it, const T* ph, const T* dh) {
-    int e;
-    if constexpr (sizeof(T) == 8) {  // lambda_u, lambda_w in place in la; q in lb
-      e = launch_adj_f64(p, g2, it, cf, lcur, lnxt, la + ns * pl, la + 2 * ns * pl, lb + ns * pl, ph, dh, gp, gu, gw, g1p,
-                         g2p, st);
-    } else {
-      e = launch_adj(p, g2, it, cf, lcur, lcur + ns * pl, lcur + 2 * ns * pl, lnxt, lnxt + ns * pl, lnxt + 2 * ns * pl, ph,
-                     dh, gp, gu, gw, g1p, g2p, flag, st);
-    }
+    const int e = launch_adj(p, g2, it, cf, lcur, lcur + ns * pl, lcur + 2 * ns * pl, lnxt, lnxt + ns * pl,
+                             lnxt + 2 * ns * pl, ph, dh, gp, gu, gw, g1p, g2p, flag, st);
     std::swap(lcur, lnxt);
     return e;
   };
@@ -1663,6 +1655,20 @@ int plan_create_impl(const adfwi_acoustic_desc* desc, const int32_t* src_z, cons
       const int ij = t[p->o_rij + r];
       t.push_back(ij);
     }
+    const int tx = (p->nxp + ac3::kX - 1) / ac3::kX, nt = ac3::tiles(p->L, p->zbeg);
+    std::vector<int32_t> beg(nt + 1, 0), order(p->t2.ncells);
+    auto tile = [&](int q) {
+      const int ij = t[p->o_cij + q];
+      return ((ij >> 16) - p->zbeg) / ac3::kZ * tx + (ij & 0xffff) / ac3::kX;
+    };
+    for (int q = 0; q < p->t2.ncells; ++q) ++beg[tile(q) + 1];
+    for (int q = 0; q < nt; ++q) beg[q + 1] += beg[q];
+    std::vector<int32_t> at(beg.begin(), beg.end() - 1);
+    for (int q = 0; q < p->t2.ncells; ++q) order[at[tile(q)]++] = q;
+    p->o_ftb = t.size();
+    t.insert(t.end(), beg.begin(), beg.end());
+    p->o_ftc = t.size();
+    t.insert(t.end(), order.begin(), order.end());
   }
   plan_resident(p, rcv_z, rcv_x);
   if (t.empty()) t.push_back(0);
