@@ -292,9 +292,9 @@ class AcousticL2Solve(torch.autograd.Function):
     given, already normalised); the records come back without gradient.
 
     ``adjoint_source``: "array" writes the source as an (ns, nt, nr) array in one
-    bandwidth-bound pass that the adjoint reads (the faster form on GB300); "inject" forms each
-    sample inside the adjoint step as it is injected, with no array (the lanes that inject the
-    receivers then pace their tiles: about 10-15% more time per adjoint step on the 300 x 700,
+    bandwidth-bound pass that the adjoint reads; "inject" needs no array: the resident time loop
+    forms the source of a stretch of steps at a time in its workspace, the per-step kernels form
+    each sample as they inject it (about 10-15% more time per adjoint step on the 300 x 700,
     30-shot workload). Both give the same bits."""
 
     @staticmethod

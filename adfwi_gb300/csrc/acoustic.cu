@@ -1102,8 +1102,9 @@ int resident_fwd_blocks(bool deep) {
                          deep ? ac2::VDEEP : ac2::VMINB);
 }
 
-// Padded grids at least this wide run the deep-ring variants (one more stage, 2 blocks per SM).
-// An empirical rule from per-launch times of both rings (FP32, full history; forward / adjoint
+// Padded grids at least this wide run the deep-ring variants (one more stage, 2 blocks per SM), where
+// the per-step kernels are taken at all (boundary saving, dL/d u- and w-records, grids that do not fit
+// on the chip). An empirical rule from per-launch times of both rings (FP32, full history; forward / adjoint
 // in us, shallow -> deep): 600 x 1600 padded with 4 / 8 / 16 shots 44.1 -> 41.6 / 77.2 -> 69.1,
 // 86.0 -> 73.5 / 130.8 -> 118.0, 161.8 -> 165.8 / 227.6 -> 217.1; every narrower grid measured
 // (300 x 700 with 10 / 30 / 60 shots, 400 x 1000 with 8 / 16 / 30, 200 x 400 with 16 / 64,

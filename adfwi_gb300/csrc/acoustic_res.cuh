@@ -22,7 +22,7 @@
 //
 // What bounds it is the shared-memory pipe: about 90 wavefronts per 128 cells and step of the 130
 // to 190 clocks they take, next to the exchange (1 to 2 us per step, acoustic.cu res_choose).
-// Measured per step of all shots, start -> here, in us: 300 x 700 with 30 shots forward 52 -> 29,
+// Measured per step of all shots, per-step kernels -> here, in us: 300 x 700 with 30 shots forward 52 -> 29,
 // adjoint 80 -> 41; 600 x 1600 with 8 shots 79 -> 54, 120 -> 66; 148 x 260 with 40 shots and a free
 // surface 18.7 -> 7.3, 35 -> 9.4; 200 x 200 with 10 shots (records only) 9.2 -> 3.1.
 // Tried and slower: the state of a thread's cells in registers with shuffles for the horizontal

@@ -310,8 +310,8 @@ class AcousticPropagator(_PropagatorBase):
         (ADFWI/fwi/acoustic_fwi.py:149-150) and its autograd gradient as separate PyTorch passes).
         ``normalise_obs`` divides obs by its trace peaks too; ``silent_rel`` > 0 treats traces
         whose peak is at most that share of their gather's peak as zero (0 = the reference).
-        ``adjoint_source``: "array" (one (ns, nt, nr) source array, the faster form) or "inject"
-        (formed inside the adjoint step, no array); the same bits either way."""
+        ``adjoint_source``: "array" (one (ns, nt, nr) source array) or "inject" (formed as the
+        adjoint goes, no array); the same bits either way."""
         from .acoustic import AcousticL2Solve
         model = self.model if model is None else model
         model.forward()
