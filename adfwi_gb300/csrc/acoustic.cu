@@ -247,8 +247,8 @@ struct adfwi_acoustic_plan {
 namespace {
 
 struct Carve {
-  int64_t coef, fa, fb, ilp, ilu, tab, flag, box;  // forward
-  int64_t snap, snap_scale, bsv, hp, hd, la, lb, g1, g2;  // gradient extras
+  int64_t coef, fa, fb, ilp, ilu, tab, flag, box;  // forward (box: the strips' inboxes)
+  int64_t snap, snap_scale, bsv, hp, hd, la, lb, abox, g1, g2;  // gradient extras (abox: the adjoint's inboxes)
   int64_t mst, mpk, mnorm, mfac;                     // fused misfit: trace stats, gather peaks, norms, factors
   int64_t total;
 };
@@ -261,7 +261,10 @@ int64_t res_box_bytes(const Resident& r);
 // history of that step is kept).
 bool boundary_saving(const adfwi_acoustic_plan* p) { return p->bsave && p->d.nt > 1; }
 
-// (box: with the inboxes of the resident loop's strips)
+// (box: with the inboxes of the resident loop's strips. They lie in planes that the loop leaves unused,
+// the third of each shot in fb and the per-step kernels' illumination sums after it, in lb and the
+// per-step gradient sums after it, where they fit: so that a plan's snapshot interval under a memory
+// budget, which decides what quantised snapshots round, does not depend on them)
 Carve carve(const adfwi_acoustic_plan* p, bool grad, int K, bool box = true) {
   Carve c{};
   const int64_t pl = p->L.plane * p->elem;
@@ -275,7 +278,8 @@ Carve carve(const adfwi_acoustic_plan* p, bool grad, int K, bool box = true) {
   c.ilu = take((int64_t)p->t2.ngroups * pl);
   c.tab = take((int64_t)p->tab.size() * 4);
   c.flag = take(256);
-  if (box) c.box = take(std::max(res_box_bytes(p->rf), grad ? res_box_bytes(p->ra) : (int64_t)0));
+  c.box = c.fb + 2 * ns * pl;
+  if (box && res_box_bytes(p->rf) > c.tab - c.box) c.box = take(res_box_bytes(p->rf));
   if (grad) {
     const int nseg = (p->d.nt + K - 1) / K;
     const bool bs = boundary_saving(p);
@@ -291,6 +295,8 @@ Carve carve(const adfwi_acoustic_plan* p, bool grad, int K, bool box = true) {
     c.lb = take(3 * ns * pl);
     c.g1 = take((int64_t)p->t2.ngroups * pl);
     c.g2 = take((int64_t)p->t2.ngroups * pl);
+    c.abox = c.lb + 2 * ns * pl;
+    if (res_box_bytes(p->ra) > o - c.abox) c.abox = take(res_box_bytes(p->ra));
     const int64_t traces = (int64_t)ns * std::max(1, p->d.nr);
     const bool f64 = p->elem == 8;
     c.mst = take(traces * (f64 ? (int64_t)sizeof(l2::TraceStats<double>) : (int64_t)sizeof(l2::TraceStats<float>)));
@@ -634,7 +640,7 @@ res::ResArgs res_args(const adfwi_acoustic_plan* p, const Resident& r, unsigned 
   a.trid = tb + r.o_ti;
   a.srbeg = tb + r.o_rb;
   a.srcv = tb + r.o_rv;
-  a.box = reinterpret_cast<unsigned long long*>(ws + c.box);
+  a.box = reinterpret_cast<unsigned long long*>(ws + (&r == &p->ra ? c.abox : c.box));
   a.flag = reinterpret_cast<int*>(ws + c.flag);
   a.nz = 0x8000000080000000ull;
   return a;
@@ -1216,9 +1222,20 @@ void build_tiling(adfwi_acoustic_plan* p, Tiling* tl, int tz, int tx, const std:
 }
 
 // Shots per group of the double-precision steps: one while that gives at most 16 blocks of 128 threads
-// per SM (more blocks than are resident), then as many as keep to that; a group has one partial plane
-// per sum.
-int f64_group_shots(int ns, int tiles) { return std::max(1, (int)((int64_t)ns * tiles / (152 * 16))); }
+// per SM (more blocks than are resident), then as many as keep to that. A group has one partial plane
+// per sum, so where memory is short (the allocation-free forward's scratch, a budget below the whole
+// history) groups stay as large as one block per SM of 16 x 64 tiles would make them.
+int f64_group_shots(const adfwi_acoustic_plan* p, const std::vector<int>& alone, int ntiles, int64_t scratch) {
+  const int ns = alone[1], tight = pick_unit_shots(alone, ntiles, 152, 152);
+  const int fine = std::max(1, (int)((int64_t)ns * ac3::tiles(p->L, p->zbeg) / (152 * 16)));
+  auto bytes = [&](int G, int64_t fields) {
+    const int64_t groups = (int64_t)p->nm * ((ns + G - 1) / G);
+    return (ac::kNumCoef * (int64_t)p->nm + fields * p->d.ns + (fields > 6 ? 4 : 2) * groups) * p->L.plane * 8 + (1 << 20);
+  };
+  if (bytes(fine, 6) > scratch && bytes(tight, 6) <= scratch + (2 << 20)) return tight;
+  if (p->d.memory_budget > 0 && bytes(fine, 12 + 2 * (int64_t)p->d.nt) > p->d.memory_budget / 50 * 49) return tight;
+  return fine;
+}
 
 // Shared memory of a configuration, in words.
 // (most, most_rows: receiver cells, and rows holding any, of the strip that has the most)
@@ -1640,7 +1657,7 @@ int plan_create_impl(const adfwi_acoustic_desc* desc, const int32_t* src_z, cons
     for (int m = 0; m < p->nm; ++m) {
       const std::vector<int> alone = {0, p->model_shot_beg[m + 1] - p->model_shot_beg[m]};
       if (d.shots_per_block > 0) Gm[m] = d.shots_per_block;
-      else if (f64) Gm[m] = f64_group_shots(alone[1], ac3::tiles(p->L, p->zbeg));
+      else if (f64) Gm[m] = f64_group_shots(p, alone, ntiles, kStaticScratchBytes);
       else Gm[m] = pick_unit_shots(alone, ntiles, fblocks, blocks);
     }
     build_tiling(p, &p->t2, ac2::TZ, ac2::TX, Gm, rcv_z, rcv_x);
