@@ -1303,10 +1303,16 @@ int resident_clusters(const Resident& r, int n, int dev, ResKernel k) {
 // In us, from sweeps of G and of the variants with per-launch times (300 x 700 padded with 10 and
 // 30 shots, 148 x 260 with 40, 200 x 200 with 10, 600 x 1600 with 8):
 //   exchange: 1.6 through global memory, 0.7 in a cluster (whose shared memory is next door, but
-//     only 7 clusters of 16 blocks, 13 of 10 or 23 of 6 fit the GPU at a time);
-//   per unit, forward / adjoint: 0.065 / 0.09 for 3 rows per thread and 128 registers; the adjoint
+//     only 7 clusters of 16 blocks, 13 of 10 or 23 of 6 fit the GPU at a time), 0.3 without one;
+//   0.6 more in blocks of less than two warps, and in the forward loop with strips of at most 5 rows,
+//     whose few threads wait for both neighbours;
+//   per unit, forward / adjoint: 0.065 / 0.09 for 3 rows per thread and 128 registers (0.06 for 2, forward, which
+//     strips of equal even height take); the adjoint
 //     loses a third at 80 registers (spills), and more rows per thread leave fewer warps;
-//   several blocks per SM run 15 % slower than one that does the same work.
+//   several blocks per SM run 15 % slower than one that does the same work; clusters that do not fit
+//     at one block per SM double up on some SMs while others idle, however few blocks there are in
+//     all (10 shots of 200 x 200: 2.87 us with 15 strips, 2.35 with 10; 20 of 96 x 232: 3.9 with 7, 2.4
+//     with 6; 30 of 100 x 120: 2.7 with 5, 2.1 with 9): forward 0.9, adjoint 0.75 of their number.
 // For example 300 x 700 with 30 shots, us per step: forward 29.2 with 25 strips of 12 rows and
 // 3 rows per thread (35.4 with 6, 43.5 with 38 strips of 8), adjoint 40.8 with 25 strips and 6
 // rows per thread (45.8 with 4, 46.9 with 3, 52.6 with 50 strips of 6).
@@ -1343,6 +1349,7 @@ Resident res_choose(const adfwi_acoustic_plan* p, bool adj, const std::vector<st
         r.RB = v[0];
         r.MT = v[1];
         r.TR = (r.R + r.RB - 1) / r.RB;
+        if (adj && r.RB == 2) continue;
         if (least / r.TR < 2) continue;  // the boundary threads own both rows that cross
         r.T = (r.TR * CG + 31) / 32 * 32;
         if (r.T > r.MT) continue;
@@ -1356,11 +1363,19 @@ Resident res_choose(const adfwi_acoustic_plan* p, bool adj, const std::vector<st
           if (cap < 1) continue;
           r.S = glb ? std::min(ns, cap) : ns;
           const int waves = (ns + cap - 1) / cap;
-          const double load = (double)std::min(ns, cap) * G / sms;
-          const double units = r.R * CG / 32.0 * (load > 1.0 ? 1.15 * load : 1.0);
+          const int act = std::min(ns, cap);
+          double load = (double)act * G / sms;
+          load = load > 1.0 ? 1.15 * load : 1.0;
+          if (!glb && G > 1) {  // clusters at one block per SM, and how many share an SM beyond that
+            Resident one = r;
+            one.words = max_smem / 4;
+            const int alone = std::max(1, resident_clusters(one, 1, dev, res_kernel(r, adj, true)));
+            load = std::max(std::max(1.0, load), (act > alone ? adj ? 0.75 : 0.9 : 0.0) * ((act + alone - 1) / alone));
+          }
           const double per_unit = adj ? (r.RB == 3 ? (r.MT == 512 ? 0.09 : 0.12) : r.RB == 4 ? (r.MT == 512 ? 0.105 : 0.115) : 0.1)
-                                      : (r.RB == 3 ? 0.065 : r.RB == 4 ? (r.MT == 512 ? 0.09 : 0.076) : 0.084);
-          const double cost = waves * ((glb ? 1.6 : 0.7) + per_unit * units) * (1.0 - 0.01 * kept);
+                                      : (r.RB == 2 ? 0.06 : r.RB == 3 ? 0.065 : r.RB == 4 ? (r.MT == 512 ? 0.09 : 0.076) : 0.084);
+          const double fixed = (glb ? 1.6 : G > 1 ? 0.7 : 0.3) + (r.T < 64 || (!adj && r.R <= 5) ? 0.6 : 0.0);
+          const double cost = waves * (fixed + per_unit * r.R * CG / 32.0 * load) * (1.0 - 0.01 * kept);
           if (cost < best_cost) {
             best_cost = cost;
             best = r;

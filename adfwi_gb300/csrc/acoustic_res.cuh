@@ -24,7 +24,7 @@
 // to 190 clocks they take, next to the exchange (1 to 2 us per step, acoustic.cu res_choose).
 // Measured per step of all shots, per-step kernels -> here, in us: 300 x 700 with 30 shots forward 52 -> 29,
 // adjoint 80 -> 41; 600 x 1600 with 8 shots 79 -> 54, 120 -> 66; 148 x 260 with 40 shots and a free
-// surface 18.7 -> 7.3, 35 -> 9.4; 200 x 200 with 10 shots (records only) 9.2 -> 3.1.
+// surface 18.7 -> 7.3, 35 -> 9.4; 200 x 200 with 10 shots (records only) 9.2 -> 2.4.
 // Tried and slower: the state of a thread's cells in registers with shuffles for the horizontal
 // neighbours (spills; 4.3 against 3.1 us on 20 rows x 256), all coefficients in shared memory with
 // loads lifted across rows (the same or slower), two smaller blocks per SM to hide the exchange
