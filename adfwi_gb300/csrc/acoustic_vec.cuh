@@ -57,28 +57,14 @@ __device__ __forceinline__ void ld4(const float* p, float (&r)[4]) {
   const float4 q = *reinterpret_cast<const float4*>(p);
   r[0] = q.x, r[1] = q.y, r[2] = q.z, r[3] = q.w;
 }
-__device__ __forceinline__ void ld4(const double* p, double (&r)[4]) {
-  const double2 a = *reinterpret_cast<const double2*>(p);
-  const double2 b = *reinterpret_cast<const double2*>(p + 2);
-  r[0] = a.x, r[1] = a.y, r[2] = b.x, r[3] = b.y;
-}
 __device__ __forceinline__ void st4(float* p, const float (&r)[4]) {
   *reinterpret_cast<float4*>(p) = make_float4(r[0], r[1], r[2], r[3]);
-}
-__device__ __forceinline__ void st4(double* p, const double (&r)[4]) {
-  *reinterpret_cast<double2*>(p) = make_double2(r[0], r[1]);
-  *reinterpret_cast<double2*>(p + 2) = make_double2(r[2], r[3]);
 }
 
 // read-only (non-coherent path) loads of data that no thread writes during the launch
 __device__ __forceinline__ void ldg4(const float* p, float (&r)[4]) {
   const float4 q = __ldg(reinterpret_cast<const float4*>(p));
   r[0] = q.x, r[1] = q.y, r[2] = q.z, r[3] = q.w;
-}
-__device__ __forceinline__ void ldg4(const double* p, double (&r)[4]) {
-  const double2 a = __ldg(reinterpret_cast<const double2*>(p));
-  const double2 b = __ldg(reinterpret_cast<const double2*>(p + 2));
-  r[0] = a.x, r[1] = a.y, r[2] = b.x, r[3] = b.y;
 }
 
 // twelve consecutive values (three 16-byte groups)
