@@ -7,6 +7,8 @@ fails, a RuntimeError says why.
 import ctypes
 import os
 
+from torch.autograd import forward_ad
+
 _LIB = None
 
 F32, F64 = 0, 1
@@ -133,6 +135,17 @@ def ptr(t):
     if t is None:
         return None
     return c_void_p(t.data_ptr())
+
+
+def by_address(t):
+    """Whether a kernel may take ``t`` by its address: a tensor with memory of its own (not batched
+    or wrapped by a function transform), not a lazy negation, without a forward-mode tangent."""
+    try:
+        if t.data_ptr() == 0 or t.is_neg():
+            return False
+    except RuntimeError:
+        return False
+    return forward_ad.unpack_dual(t).tangent is None
 
 
 def stream_handle(device):

@@ -93,6 +93,7 @@ class GradProcessor(object):
                 and tuple(g.shape) == (nz, nx) and tuple(forw.shape) == (nz, nx) and min(nz, nx) >= 2
                 and forw.dtype in (torch.float32, torch.float64) and 0 <= keep < nz
                 and isinstance(self.grad_smooth, int) and not torch.compiler.is_compiling()
+                and N.by_address(g) and N.by_address(forw)
                 and not (torch.is_grad_enabled() and (g.requires_grad or forw.requires_grad))):
             return None
         taper = mask = None

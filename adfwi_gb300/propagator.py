@@ -50,7 +50,7 @@ _PAD_PLANES = 10  # planes of one native call
 def _native_planes(ts):
     """Whether the CUDA library pads / folds these planes: plain FP32 or FP64 planes of one device."""
     return (all(type(t) in (Tensor, torch.nn.Parameter) and t.is_cuda and t.dim() == 2 and t.numel() > 0
-                and t.dtype == ts[0].dtype and t.device == ts[0].device for t in ts)
+                and t.dtype == ts[0].dtype and t.device == ts[0].device and N.by_address(t) for t in ts)
             and ts[0].dtype in (torch.float32, torch.float64) and not torch.compiler.is_compiling())
 
 
@@ -120,13 +120,16 @@ class _PadReplicate(torch.autograd.Function):
         ctx.pads = pads
         ctx.set_materialize_grads(False)
         top, bottom, left, right = pads
-        if not _native_planes(vs):
-            return tuple(torch.nn.functional.pad(v[None, None], (left, right, top, bottom), mode="replicate")[0, 0]
-                         for v in vs)
-        src = [v.contiguous() for v in vs]
-        shapes = [tuple(v.shape) for v in src]
-        outs = [v.new_empty((h + top + bottom, w + left + right)) for v, (h, w) in zip(src, shapes)]
-        _native_call("adfwi_pad_replicate", src, outs, shapes, pads)
+        if _native_planes(vs):
+            src = [v.contiguous() for v in vs]
+            shapes = [tuple(v.shape) for v in src]
+            outs = [v.new_empty((h + top + bottom, w + left + right)) for v, (h, w) in zip(src, shapes)]
+            _native_call("adfwi_pad_replicate", src, outs, shapes, pads)
+        else:
+            outs = [torch.nn.functional.pad(v[None, None], (left, right, top, bottom), mode="replicate")[0, 0]
+                    for v in vs]
+        # a plane that needs no gradient stays without one beside planes that do
+        ctx.mark_non_differentiable(*[o for k, o in enumerate(outs) if not ctx.needs_input_grad[1 + k]])
         return tuple(outs)
 
     @staticmethod
