@@ -1308,14 +1308,15 @@ int resident_clusters(const Resident& r, int n, int dev, ResKernel k) {
 //     whose few threads wait for both neighbours;
 //   per unit, forward / adjoint: 0.065 / 0.09 for 3 rows per thread and 128 registers (0.06 for 2, forward, which
 //     strips of equal even height take); the adjoint
-//     loses a third at 80 registers (spills), and more rows per thread leave fewer warps;
+//     loses a third at 80 registers (spills), and more rows per thread leave fewer warps; 6 rows take
+//     168 registers where 384 threads do (at 128 the adjoint through global memory spills 80 B);
 //   several blocks per SM run 15 % slower than one that does the same work; clusters that do not fit
 //     at one block per SM double up on some SMs while others idle, however few blocks there are in
 //     all (10 shots of 200 x 200: 2.87 us with 15 strips, 2.35 with 10; 20 of 96 x 232: 3.9 with 7, 2.4
 //     with 6; 30 of 100 x 120: 2.7 with 5, 2.1 with 9): forward 0.9, adjoint 0.75 of their number.
 // For example 300 x 700 with 30 shots, us per step: forward 29.2 with 25 strips of 12 rows and
-// 3 rows per thread (35.4 with 6, 43.5 with 38 strips of 8), adjoint 40.8 with 25 strips and 6
-// rows per thread (45.8 with 4, 46.9 with 3, 52.6 with 50 strips of 6).
+// 3 rows per thread (35.4 with 6, 43.5 with 38 strips of 8), adjoint 37.2 with 25 strips and 6
+// rows per thread (40.2 at 128 registers; 45.8 with 4 rows, 46.9 with 3, 52.6 with 50 strips of 6).
 Resident res_choose(const adfwi_acoustic_plan* p, bool adj, const std::vector<std::pair<int64_t, int>>& rc, int max_smem,
                     int sms, int dev) {
   const int z0 = p->d.free_surface ? p->fs : 0;
@@ -1349,7 +1350,7 @@ Resident res_choose(const adfwi_acoustic_plan* p, bool adj, const std::vector<st
         r.RB = v[0];
         r.MT = v[1];
         r.TR = (r.R + r.RB - 1) / r.RB;
-        if (adj && r.RB == 2) continue;
+        if (adj ? r.RB == 2 : r.MT == 384) continue;
         if (least / r.TR < 2) continue;  // the boundary threads own both rows that cross
         r.T = (r.TR * CG + 31) / 32 * 32;
         if (r.T > r.MT) continue;
@@ -1372,7 +1373,7 @@ Resident res_choose(const adfwi_acoustic_plan* p, bool adj, const std::vector<st
             const int alone = std::max(1, resident_clusters(one, 1, dev, res_kernel(r, adj, true)));
             load = std::max(std::max(1.0, load), (act > alone ? adj ? 0.75 : 0.9 : 0.0) * ((act + alone - 1) / alone));
           }
-          const double per_unit = adj ? (r.RB == 3 ? (r.MT == 512 ? 0.09 : 0.12) : r.RB == 4 ? (r.MT == 512 ? 0.105 : 0.115) : 0.1)
+          const double per_unit = adj ? (r.RB == 3 ? (r.MT == 512 ? 0.09 : 0.12) : r.RB == 4 ? (r.MT == 512 ? 0.105 : 0.115) : r.MT == 384 ? 0.095 : 0.1)
                                       : (r.RB == 2 ? 0.06 : r.RB == 3 ? 0.065 : r.RB == 4 ? (r.MT == 512 ? 0.09 : 0.076) : 0.084);
           const double fixed = (glb ? 1.6 : G > 1 ? 0.7 : 0.3) + (r.T < 64 || (!adj && r.R <= 5) ? 0.6 : 0.0);
           const double cost = waves * (fixed + per_unit * r.R * CG / 32.0 * load) * (1.0 - 0.01 * kept);

@@ -50,10 +50,11 @@ struct ResArgs {
 
 using ResKernel = void (*)(const ac::Geo<float>, const ResArgs);
 
-// Rows per thread and most threads of a block of each compiled variant (2 rows: the forward loop only).
+// Rows per thread and most threads of a block of each compiled variant (2 rows: the
+// forward loop only; 384 threads, 168 registers each: the adjoint only).
 // (Registers decide: the sums over time take 8 per row beside some 90 of the stencils, and what
 // spills goes to L2, the L1 being shared memory.)
-constexpr int kVariants[][2] = {{2, 512}, {3, 512}, {3, 768}, {4, 512}, {4, 640}, {6, 512}};
+constexpr int kVariants[][2] = {{2, 512}, {3, 512}, {3, 768}, {4, 512}, {4, 640}, {6, 384}, {6, 512}};
 // The variant's kernel (glb: strips of a cooperative launch instead of a cluster; sums: the
 // illumination is summed).
 ResKernel forward_kernel(int rb, int mt, bool sums, bool glb);

@@ -15,7 +15,7 @@ ResKernel pick(bool glb) {
 ResKernel adjoint_kernel(int rb, int mt, bool glb) {
   if (rb == 3) return mt == 512 ? pick<3, 512>(glb) : pick<3, 768>(glb);
   if (rb == 4) return mt == 512 ? pick<4, 512>(glb) : pick<4, 640>(glb);
-  return pick<6, 512>(glb);
+  return mt == 384 ? pick<6, 384>(glb) : pick<6, 512>(glb);
 }
 
 }  // namespace res

@@ -31,6 +31,7 @@ SHAPES = [
     (88, 201, 30, 12, True, "row"),
     (100, 102, 50, 10, False, "column"),
     (120, 420, 40, 9, False, "row"),
+    (200, 600, 50, 6, False, "row"),
     (200, 600, 50, 7, True, "shared"),
     (60, 1500, 20, 3, False, "row"),
 ]
