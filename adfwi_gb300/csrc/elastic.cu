@@ -39,6 +39,45 @@ __device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float rdiv(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __forceinline__ double rdiv(double a, double b) { return __ddiv_rn(a, b); }
+// Division by a number d that many are divided by, correctly rounded (P. Markstein, Computation of elementary
+// functions on the IBM RISC System/6000 processor, 1990): with r = 1 / d rounded and e = 1 / d - r, y = x r + x e
+// is one of the two numbers next to x / d, x - y d is exact, and y + (x - y d) r rounds to x / d. A numerator
+// below `low`, where these would underflow, is scaled up first (tiny); zero needs nothing. It replaces the
+// division because that takes a path of tens of instructions for numerators near zero, which some
+// warp of every launch has at the front of a wave (300 steps of a shot on a 122 x 140 grid: 2.2 ms, with
+// divisions 3.0).
+template <typename T>
+struct Divisor {
+  static constexpr bool kF = sizeof(T) == 4;
+  static constexpr T low = kF ? T(0x1p-95) : T(0x1p-900), most = kF ? T(0x1p90) : T(0x1p900), range = T(0x1p20);
+  static constexpr T up = kF ? T(0x1p100) : T(0x1p900), down = T(1) / up;
+  static constexpr T tie = kF ? T(0x1p-50) : T(0x1p-175);  // half of the least number, scaled up
+  T d, r, e;
+  T hi;  // numerators up to this; -1: the divisor is out of range and none is
+  Divisor() = default;
+  __host__ __device__ __forceinline__ explicit Divisor(T d_) : d(d_) {
+    r = T(1) / d;
+    e = fma(-r, d, T(1)) * r;
+    hi = d >= T(1) / range && d <= range ? most : T(-1);
+  }
+  __device__ __forceinline__ bool takes(T x) const { return fabs(x) <= hi; }
+  static __device__ __forceinline__ bool small(T x) { return fabs(x) < low && x != T(0); }
+  __device__ __forceinline__ T of(T x) const {
+    const T y = fma(x, r, x * e);
+    return fma(fma(-y, d, x), r, y);
+  }
+  // Numerators of any size that is taken. Scaling a subnormal quotient back rounds a second time: half
+  // way between two numbers, the remainder of the first rounding decides.
+  __device__ __forceinline__ T tiny(T x) const {
+    const bool s = fabs(x) < low;
+    x = s ? x * up : x;
+    const T y = of(x), z = s ? y * down : y, rem = fma(-y, d, x);
+    if (s && fabs(y - z * up) == tie && rem != T(0)) return (y + copysign(tie, rem)) * down;
+    return z;
+  }
+};
 
 // Field indices inside the state blocks (each field = ns consecutive planes).
 enum { TXX_X = 0, TXX_Z, TZZ_X, TZZ_Z, TXZ_X, TXZ_Z };  // split stresses (PML)
@@ -54,9 +93,9 @@ struct Geo {
   int fsurf, h;                // free surface; h = NN + 1
   int ilo, ihi, jlo, jhi;      // update region I = [NN, nzp-NN-1] x [NN, nxp-NN-1]
   int top, nabc, nz, nx;       // energy window
-  T dt, dx, dz, dt_dx, dt_dz, hdt;
+  T dt, dt_dx, dt_dz, hdt;
+  Divisor<T> dx, dz;
   T f0, f1, f2;                // staggered coefficients
-  T fx[3], fz[3];              // the same times dt / dx and dt / dz, rounded once
   const int* src_z;
   const int* src_x;
   const T* src_m;              // ns x 3 source weights (xx, zz, xz) already scaled for the mode
@@ -93,10 +132,7 @@ constexpr int kTileX = 32, kTileZ = 8, kTileThreads = kTileX * kTileZ;
   (void)NSP;
 
 // 1 / d of a PML denominator d = 1 + dt/2 d(x): exactly 1 where d is (outside the absorbing frame),
-// so the division runs only inside the frame. Only coefficients are divided: where a wave has not
-// arrived a field is zero or subnormal, and a division of such a value takes a slow path of tens of
-// instructions (two launches of 20 shots on a 242 x 480 grid: 82 us with four divisions of fields a
-// cell, 61 with products).
+// so the division runs only inside the frame.
 template <typename T>
 __device__ __forceinline__ T pml_inv(T d) {
   return d == T(1) ? T(1) : T(1) / d;
@@ -158,12 +194,18 @@ struct Row {
   }
   __device__ __forceinline__ T operator()(int k) const { return v[H + k]; }
 };
-// Half-cell difference (elastic_kernels.py:66-108), the coefficients with or without dt / dx: `at(m)` is the
-// value m cells from the lower of the two middle ones. Differences, coefficient products and sums
-// of the forward kernels are fused multiply-adds, and one sum is added to a total.
+// Half-cell difference (elastic_kernels.py:66-108): `at(m)` is the value m cells from the lower of the two
+// middle ones. `rounded` keeps the reference's operations, each rounded by itself, for the forward
+// kernels; `diff` is contracted to multiply-adds, for the gradients' sums.
 template <typename T>
 struct Fd {
   T f0, f1, f2;
+  template <int NN, typename A>
+  __device__ __forceinline__ T rounded(const A& at) const {
+    T r = radd(rmul(f0, rsub(at(1), at(0))), rmul(f1, rsub(at(2), at(-1))));
+    if (NN == 3) r = radd(r, rmul(f2, rsub(at(3), at(-2))));
+    return r;
+  }
   template <int NN, typename A>
   __device__ __forceinline__ T diff(const A& at) const {
     T r = f0 * (at(1) - at(0)) + f1 * (at(2) - at(-1));
@@ -171,6 +213,39 @@ struct Fd {
     return r;
   }
 };
+// Vectors over their divisors by(k, e).
+template <int N, typename T, typename By>
+__device__ __forceinline__ void divide(Vec<T> (&a)[N], const By& by) {
+  bool taken = true, small = false;
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int e = 0; e < kVW<T>; ++e) {
+      taken = taken && by(k, e).takes(a[k].v[e]);
+      small = small || Divisor<T>::small(a[k].v[e]);
+    }
+  if (!taken) {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int e = 0; e < kVW<T>; ++e) a[k].v[e] = rdiv(a[k].v[e], by(k, e).d);
+  } else if (small) {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int e = 0; e < kVW<T>; ++e) a[k].v[e] = by(k, e).tiny(a[k].v[e]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int e = 0; e < kVW<T>; ++e) a[k].v[e] = by(k, e).of(a[k].v[e]);
+  }
+}
+// the x parts (even planes) over dx, the z parts over dz
+template <int N, typename T>
+__device__ __forceinline__ void over_dx_dz(const Geo<T>& g, Vec<T> (&a)[N]) {
+  divide(a, [&](int k, int) -> const Divisor<T>& { return k & 1 ? g.dz : g.dx; });
+}
 template <typename T>
 __host__ __device__ __forceinline__ int vec_tiles(const Layout& L) {
   return ((L.nxp + kVecX - 1) / kVecX) * ((L.nzp + kVecRows<T> - 1) / kVecRows<T>);
@@ -270,7 +345,11 @@ __device__ __forceinline__ void store_stress(const Geo<T>& g, int i, int64_t o, 
 // thread that takes 96 registers, five blocks per SM (six and eight spill and measured 7 and 30 %
 // slower). 300 steps of one shot on a 122 x 140 grid: 4.56 -> 3.0 ms; 200 steps of 20 shots on a
 // 242 x 480 grid: 16.3 -> 10.5 ms, against one cell and two shots per thread with scalar loads and
-// exact divisions by dx.
+// divisions by dx.
+//
+// Every operation is the reference's, rounded by itself and in its order. Products and sums fused, with
+// dt / dx rounded into the difference coefficients, took as long (2.2 to 2.3 ms for the 300 steps either way)
+// and left the energy maps of some short solves two to four times further from 64 bits.
 //
 // Cells that keep split fields: outside the update region, where a PML factor differs from 1,
 // and in the surface rows that mirror others or are mirrored (h-3 .. h) plus one. Every other cell
@@ -367,35 +446,42 @@ __global__ void __launch_bounds__(kVecThreads, 5)
         stv(v + VZ * NSP + o - 2 * P, az);
       }
     }
-    const Fd<T> fx{g.fx[0], g.fx[1], g.fx[2]}, fz{g.fz[0], g.fz[1], g.fz[2]};
-    Vec<T> a[6];  // the increments of the split parts xx_x, xx_z, zz_x, zz_z, xz_x, xz_z
+    const Fd<T> fd{g.f0, g.f1, g.f2};
+    // the increments of the split parts xx_x, xx_z, zz_x, zz_z, xz_x, xz_z: times dt / dx or dt / dz with
+    // PML, as sums of coefficient and difference products otherwise
+    Vec<T> a[6];
 #pragma unroll
     for (int e = 0; e < W; ++e) {
       auto zx = [&](int m) { return m == 0 ? x(e) : rx[NN + m].v[e]; };
       auto zz = [&](int m) { return m == 0 ? z(e) : rz[NN + m].v[e]; };
-      const T dxbm_vx = fx.template diff<NN>([&](int m) { return x(e - 1 + m); });
-      const T dxbm_vz = fx.template diff<NN>([&](int m) { return z(e - 1 + m); });
-      const T dzbm_vx = fz.template diff<NN>([&](int m) { return zx(m - 1); });
-      const T dzbm_vz = fz.template diff<NN>([&](int m) { return zz(m - 1); });
-      const T dxfm_vx = fx.template diff<NN>([&](int m) { return x(e + m); });
-      const T dxfm_vz = fx.template diff<NN>([&](int m) { return z(e + m); });
-      const T dzfm_vx = fz.template diff<NN>(zx);
-      const T dzfm_vz = fz.template diff<NN>(zz);
+      const T dxbm_vx = fd.template rounded<NN>([&](int m) { return x(e - 1 + m); });
+      const T dxbm_vz = fd.template rounded<NN>([&](int m) { return z(e - 1 + m); });
+      const T dzbm_vx = fd.template rounded<NN>([&](int m) { return zx(m - 1); });
+      const T dzbm_vz = fd.template rounded<NN>([&](int m) { return zz(m - 1); });
+      const T dxfm_vx = fd.template rounded<NN>([&](int m) { return x(e + m); });
+      const T dxfm_vz = fd.template rounded<NN>([&](int m) { return z(e + m); });
+      const T dzfm_vx = fd.template rounded<NN>(zx);
+      const T dzfm_vz = fd.template rounded<NN>(zz);
       const T c11 = c[0].v[e], c13 = c[1].v[e], c15 = c[2].v[e], c33 = c[3].v[e], c35 = c[4].v[e], c55 = c[5].v[e];
-      a[0].v[e] = c11 * dxbm_vx + c15 * dxbm_vz;
-      a[1].v[e] = c15 * dzbm_vx + c13 * dzbm_vz;
-      a[2].v[e] = c13 * dxbm_vx + c35 * dxbm_vz;
-      a[3].v[e] = c35 * dzbm_vx + c33 * dzbm_vz;
-      a[4].v[e] = c15 * dxfm_vx + c55 * dxfm_vz;
-      a[5].v[e] = c55 * dzfm_vx + c35 * dzfm_vz;
+      a[0].v[e] = radd(rmul(c11, dxbm_vx), rmul(c15, dxbm_vz));
+      a[1].v[e] = radd(rmul(c15, dzbm_vx), rmul(c13, dzbm_vz));
+      a[2].v[e] = radd(rmul(c13, dxbm_vx), rmul(c35, dxbm_vz));
+      a[3].v[e] = radd(rmul(c35, dzbm_vx), rmul(c33, dzbm_vz));
+      a[4].v[e] = radd(rmul(c15, dxfm_vx), rmul(c55, dxfm_vz));
+      a[5].v[e] = radd(rmul(c55, dzfm_vx), rmul(c35, dzfm_vz));
+      if (PML) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) a[k].v[e] = rmul(k & 1 ? g.dt_dz : g.dt_dx, a[k].v[e]);
+      }
     }
     if (!PML) {
+      over_dx_dz(g, a);
 #pragma unroll
       for (int k = 0; k < 3; ++k)
 #pragma unroll
         for (int e = 0; e < W; ++e) {
-          if (in[e]) t[k].v[e] += a[2 * k].v[e] + a[2 * k + 1].v[e];
-          if (has_src && e == se) t[k].v[e] += w[k];
+          if (in[e]) t[k].v[e] = radd(t[k].v[e], rmul(g.dt, radd(a[2 * k].v[e], a[2 * k + 1].v[e])));
+          if (has_src && e == se) t[k].v[e] = radd(t[k].v[e], w[k]);
         }
     } else {
 #pragma unroll
@@ -403,17 +489,17 @@ __global__ void __launch_bounds__(kVecThreads, 5)
 #pragma unroll
         for (int e = 0; e < W; ++e)
           if (!sp[e]) {
-            t[k].v[e] += a[2 * k].v[e] + a[2 * k + 1].v[e];
-            if (has_src && e == se) t[k].v[e] += T(2) * w[k];  // -MT/2 w on both split parts
+            t[k].v[e] = radd(radd(t[k].v[e], a[2 * k].v[e]), a[2 * k + 1].v[e]);
+            if (has_src && e == se) t[k].v[e] = radd(t[k].v[e], rmul(T(2), w[k]));  // -MT/2 w on both split parts
           }
       if (any) {
         T pxn[W], pxi[W], pzn[W], pzi[W];
 #pragma unroll
         for (int e = 0; e < W; ++e) {
-          pxn[e] = T(1) - g.hdt * bcx.v[e];
-          pzn[e] = T(1) - g.hdt * bcz.v[e];
-          pxi[e] = pml_inv(T(1) + g.hdt * bcx.v[e]);
-          pzi[e] = pml_inv(T(1) + g.hdt * bcz.v[e]);
+          pxn[e] = rsub(T(1), rmul(g.hdt, bcx.v[e]));
+          pzn[e] = rsub(T(1), rmul(g.hdt, bcz.v[e]));
+          pxi[e] = pml_inv(radd(T(1), rmul(g.hdt, bcx.v[e])));
+          pzi[e] = pml_inv(radd(T(1), rmul(g.hdt, bcz.v[e])));
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -421,14 +507,14 @@ __global__ void __launch_bounds__(kVecThreads, 5)
           for (int e = 0; e < W; ++e)
             if (sp[e]) {
               if (in[e]) {
-                px[k].v[e] = (pxn[e] * px[k].v[e] + a[2 * k].v[e]) * pxi[e];
-                pz[k].v[e] = (pzn[e] * pz[k].v[e] + a[2 * k + 1].v[e]) * pzi[e];
+                px[k].v[e] = rmul(radd(rmul(pxn[e], px[k].v[e]), a[2 * k].v[e]), pxi[e]);
+                pz[k].v[e] = rmul(radd(rmul(pzn[e], pz[k].v[e]), a[2 * k + 1].v[e]), pzi[e]);
               }
               if (has_src && e == se) {
-                px[k].v[e] += w[k];
-                pz[k].v[e] += w[k];
+                px[k].v[e] = radd(px[k].v[e], w[k]);
+                pz[k].v[e] = radd(pz[k].v[e], w[k]);
               }
-              t[k].v[e] = px[k].v[e] + pz[k].v[e];
+              t[k].v[e] = radd(px[k].v[e], pz[k].v[e]);
             }
           stv(ts + (2 * k) * NSP + o, px[k]);
           stv(ts + (2 * k + 1) * NSP + o, pz[k]);
@@ -485,50 +571,62 @@ __global__ void __launch_bounds__(kVecThreads, 5)
 #pragma unroll
       for (int k = 0; k < 4; ++k) f[k] = ldv(vs + k * NSP + o);
     }
-    const Fd<T> fx{g.fx[0], g.fx[1], g.fx[2]}, fz{g.fz[0], g.fz[1], g.fz[2]};
-    Vec<T> a[4];  // the increments of the split parts vx_x, vx_z, vz_x, vz_z
+    const Fd<T> fd{g.f0, g.f1, g.f2};
+    // the increments of the split parts vx_x, vx_z, vz_x, vz_z with PML, the differences over dx or dz otherwise
+    Vec<T> a[4];
 #pragma unroll
     for (int e = 0; e < W; ++e) {
-      a[0].v[e] = bx.v[e] * fx.template diff<NN>([&](int m) { return xx(e + m); });
-      a[1].v[e] = bx.v[e] * fz.template diff<NN>([&](int m) { return m == 1 ? xz(e) : rxz[NN + m - 1].v[e]; });
-      a[2].v[e] = bz.v[e] * fx.template diff<NN>([&](int m) { return xz(e - 1 + m); });
-      a[3].v[e] = bz.v[e] * fz.template diff<NN>([&](int m) { return rzz[NN + m - 1].v[e]; });
-    }
-    if (!PML) {
+      a[0].v[e] = fd.template rounded<NN>([&](int m) { return xx(e + m); });
+      a[1].v[e] = fd.template rounded<NN>([&](int m) { return m == 1 ? xz(e) : rxz[NN + m - 1].v[e]; });
+      a[2].v[e] = fd.template rounded<NN>([&](int m) { return xz(e - 1 + m); });
+      a[3].v[e] = fd.template rounded<NN>([&](int m) { return rzz[NN + m - 1].v[e]; });
 #pragma unroll
-      for (int e = 0; e < W; ++e) {
+      for (int k = 0; k < 4; ++k)
+        if (PML) a[k].v[e] = rmul(rmul(g.dt, (k < 2 ? bx : bz).v[e]), a[k].v[e]);
+    }
+    over_dx_dz(g, a);
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      if (!PML) {
         if (in[e]) {
-          nx.v[e] += a[0].v[e] + a[1].v[e];
-          nz.v[e] += a[2].v[e] + a[3].v[e];
+          nx.v[e] = radd(nx.v[e], rmul(rmul(g.dt, bx.v[e]), radd(a[0].v[e], a[1].v[e])));
+          nz.v[e] = radd(nz.v[e], rmul(rmul(g.dt, bz.v[e]), radd(a[2].v[e], a[3].v[e])));
         }
         if (!g.fsurf) {
-          nx.v[e] *= damp.v[e];
-          nz.v[e] *= damp.v[e];
+          nx.v[e] = rmul(nx.v[e], damp.v[e]);
+          nz.v[e] = rmul(nz.v[e], damp.v[e]);
         }
+      } else if (!sp[e]) {
+        nx.v[e] = radd(radd(nx.v[e], a[0].v[e]), a[1].v[e]);
+        nz.v[e] = radd(radd(nz.v[e], a[2].v[e]), a[3].v[e]);
       }
-    } else {
-#pragma unroll
-      for (int e = 0; e < W; ++e) {
-        if (!sp[e]) {
-          nx.v[e] += a[0].v[e] + a[1].v[e];
-          nz.v[e] += a[2].v[e] + a[3].v[e];
-        }
-      }
+    }
+    if (PML) {
       if (any) {
+        Divisor<T> d[2][W];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const Vec<T>& bc = k & 1 ? bcz : bcx;
+        for (int e = 0; e < W; ++e) {
+          d[0][e] = Divisor<T>(radd(T(1), rmul(g.hdt, bcx.v[e])));
+          d[1][e] = Divisor<T>(radd(T(1), rmul(g.hdt, bcz.v[e])));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
 #pragma unroll
           for (int e = 0; e < W; ++e)
-            if (sp[e] && in[e])
-              f[k].v[e] = ((T(1) - g.hdt * bc.v[e]) * f[k].v[e] + a[k].v[e]) * pml_inv(T(1) + g.hdt * bc.v[e]);
+            a[k].v[e] = radd(rmul(rsub(T(1), rmul(g.hdt, (k & 1 ? bcz : bcx).v[e])), f[k].v[e]), a[k].v[e]);
+        divide(a, [&](int k, int e) -> const Divisor<T>& { return d[k & 1][e]; });
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+#pragma unroll
+          for (int e = 0; e < W; ++e)
+            if (sp[e] && in[e]) f[k].v[e] = a[k].v[e];
           stv(vs + k * NSP + o, f[k]);
         }
 #pragma unroll
         for (int e = 0; e < W; ++e)
           if (sp[e]) {
-            nx.v[e] = f[VX_X].v[e] + f[VX_Z].v[e];
-            nz.v[e] = f[VZ_X].v[e] + f[VZ_Z].v[e];
+            nx.v[e] = radd(f[VX_X].v[e], f[VX_Z].v[e]);
+            nz.v[e] = radd(f[VZ_X].v[e], f[VZ_Z].v[e]);
           }
       }
       if (g.fsurf && (i == g.h - 2 || i == g.h - 3)) return;  // the next stress update's
@@ -1506,19 +1604,14 @@ el::Geo<T> egeo(const adfwi_elastic_plan* p, const unsigned char* ws, const ECar
   g.nz = d.nz;
   g.nx = d.nx;
   g.dt = (T)d.dt;
-  g.dx = (T)d.dx;
-  g.dz = (T)d.dz;
+  g.dx = el::Divisor<T>((T)d.dx);
+  g.dz = el::Divisor<T>((T)d.dz);
   g.dt_dx = (T)(d.dt / d.dx);
   g.dt_dz = (T)(d.dt / d.dz);
   g.hdt = (T)(0.5 * d.dt);
   g.f0 = (T)d.fdc[0];
   g.f1 = (T)d.fdc[1];
   g.f2 = (T)(p->NN == 3 ? d.fdc[2] : 0.0);
-  for (int k = 0; k < 3; ++k) {
-    const double f = k < p->NN ? d.fdc[k] : 0.0;
-    g.fx[k] = (T)(f * d.dt / d.dx);
-    g.fz[k] = (T)(f * d.dt / d.dz);
-  }
   const int32_t* tb = reinterpret_cast<const int32_t*>(ws + c.tab);
   g.src_z = tb + p->o_srcz;
   g.src_x = tb + p->o_srcx;
