@@ -90,11 +90,14 @@ __device__ __forceinline__ void griddep_launch_dependents() {
 }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Host: launch `kernel` with programmatic stream serialisation (the kernel must call
-// griddep_wait() before it touches data of the previous launch on the stream).
+// Host: launch `kernel`, with `programmatic` serialised programmatically: the kernel must then call
+// griddep_wait() before it touches data that the previous launch on the stream writes. That holds
+// for any launch before it, also one that signals nothing: blocks may start when its last ones have
+// ended, and see its writes only after griddep_wait(). A kernel that reads ahead of its wait what an
+// earlier step wrote is launched without, where a launch of another kind comes before it.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args&&... args) {
+cudaError_t launch_kernel(bool programmatic, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                          cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -104,8 +107,13 @@ cudaError_t launch_pdl_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = programmatic ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args&&... args) {
+  return launch_kernel(true, kernel, grid, block, smem, st, static_cast<Args&&>(args)...);
 }
 
 }  // namespace adfwi

@@ -377,7 +377,8 @@ __global__ void __launch_bounds__(kVecThreads, 5)
   const int s = blockIdx.y;
   const int64_t so = (int64_t)s * PL, o = so + occ;
   const int src_row = g.src_z[s], src_col = g.src_x[s];
-  // What the launch before this one (the velocity update) does not write is read ahead of its end.
+  // What the launch before this one (the velocity update, or work that the stream has completed) does not
+  // write is read ahead of its end.
   Vec<T> c[6], bcx, bcz, t[3], px[3], pz[3];
 #pragma unroll
   for (int k = 0; k < 6; ++k) c[k] = ldv(cf + (C11 + k) * PL + occ);
@@ -1657,9 +1658,11 @@ int esetup(const adfwi_elastic_plan* p, unsigned char* ws, const ECarve& c, cons
 // One forward step. vin, tprev: velocity and stress totals at the start of the step; vout, tt:
 // where the new totals go (the same memory when they advance in place). rec: records, or null: the
 // velocity records of the step before and the stress records of this one are taken.
-// Programmatically serialised launches: each kernel waits for the previous one's data.
+// Programmatically serialised launches: each kernel waits for the previous one's data. The stress update
+// reads coefficients and previous totals ahead of its wait: `first`, the first step of a loop, follows the
+// launches that write those (packing, a snapshot's restoring) and is ordered by the stream.
 template <typename T, int NN>
-void estep(const adfwi_elastic_plan* p, const el::Geo<T>& g, int it, const T* cf, const T* wav, T* st, T* tt,
+void estep(const adfwi_elastic_plan* p, const el::Geo<T>& g, int it, bool first, const T* cf, const T* wav, T* st, T* tt,
            const T* tprev, T* vin, T* vout, T* rec, cudaStream_t s) {
   const dim3 b(el::kVecThreads);
   const int64_t NSP = (int64_t)p->d.ns * p->L.plane;
@@ -1668,7 +1671,7 @@ void estep(const adfwi_elastic_plan* p, const el::Geo<T>& g, int it, const T* cf
   const dim3 gs(tiles + (it > 0 ? rb : 0), gy), gv(tiles + rb, gy);
   auto stress = p->d.pml ? el::stress_step<T, NN, true> : el::stress_step<T, NN, false>;
   auto vel = p->d.pml ? el::vel_step<T, NN, true> : el::vel_step<T, NN, false>;
-  ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(stress, gs, b, 0, s, g, it, cf, vin, st, tt, tprev, wav, rec));
+  ADFWI_LAUNCH(kElFwdStep, s, (void)launch_kernel(!first, stress, gs, b, 0, s, g, it, cf, vin, st, tt, tprev, wav, rec));
   ADFWI_LAUNCH(kElFwdStep, s, (void)launch_pdl_kernel(vel, gv, b, 0, s, g, it, cf, (const T*)tt,
                                                       p->d.pml ? st + 6 * NSP : nullptr, vout, (const T*)vin, rec));
   if (!p->d.pml && p->d.free_surface) {
@@ -1746,7 +1749,7 @@ int eforward(const adfwi_elastic_plan* p, const void* const* coef, const int32_t
       tt = ht + (int64_t)it * 3 * NSP;
       if (it > 0) tprev = ht + (int64_t)(it - 1) * 3 * NSP;
     }
-    estep<T, NN>(p, g, it, cf, wav, stt, tt, tprev, vin, vout, static_cast<T*>(rec), s);
+    estep<T, NN>(p, g, it, it == 0, cf, wav, stt, tt, tprev, vin, vout, static_cast<T*>(rec), s);
     if (rec && p->d.nr > 0 && it + 1 == nt) {
       dim3 gr((unsigned)((p->d.nr + 127) / 128), p->d.ns);
       ADFWI_LAUNCH(kAux, s, (void)launch_pdl_kernel(el::record_v<T>, gr, dim3(128), 0, s, g, it, (const T*)vout,
@@ -1820,7 +1823,7 @@ int ebackward(const adfwi_elastic_plan* p, const void* wavelet, const void* grec
         T* vout = k + 1 < K && it + 1 < t1 ? hv + (int64_t)(k + 1) * 2 * NSP : v0;
         T* tt = ht + (int64_t)k * 3 * NSP;
         const T* tprev = k > 0 ? ht + (int64_t)(k - 1) * 3 * NSP : tt0;
-        estep<T, NN>(p, g, it, cf, wav, stt, tt, tprev, vin, vout, (T*)nullptr, s);
+        estep<T, NN>(p, g, it, k == 0, cf, wav, stt, tt, tprev, vin, vout, (T*)nullptr, s);
       }
     }
     for (int it = t1 - 1; it >= t0; --it) {
