@@ -507,10 +507,11 @@ int launch_fwd(const adfwi_acoustic_plan* p, const ac::Geo<double>& g, int it, i
   const unsigned nt = ac3::tiles(p->L, p->zbeg), gy = p->t2.ngroups;
   const unsigned rb = rp != nullptr && p->d.nr > 0 ? f64_blocks(p->d.nr) : 0;
   const dim3 b(ac3::kThreads);
+  // (the step reads coefficients ahead of its wait: the first one of a solve follows the kernel that writes them)
   ADFWI_LAUNCH(kAcFwdStep, st,
-               ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::fwd_step, dim3(nt + (it > 0 ? rb : 0), gy), b, 0, st, g, cells, (int)nt,
-                                                it, cf, cfs, p0, u0, w0, p1, u1, w1, d1, wav, ilp,
-                                                accum_u ? ilu : nullptr, rp, ru, rw)));
+               ADFWI_CUDA_TRY(launch_kernel(it > 0, ac3::fwd_step, dim3(nt + (it > 0 ? rb : 0), gy), b, 0, st, g, cells,
+                                            (int)nt, it, cf, cfs, p0, u0, w0, p1, u1, w1, d1, wav, ilp,
+                                            accum_u ? ilu : nullptr, rp, ru, rw)));
   if (rb && it + 1 == p->d.nt)
     ADFWI_LAUNCH(kAux, st, ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::record_last, dim3(rb, gy), b, 0, st, g, cells, it,
                                                             (const double*)p1, (const double*)u1, (const double*)w1, rp,

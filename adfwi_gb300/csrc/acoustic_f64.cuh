@@ -9,8 +9,9 @@
 // kept 96 of the 152 SMs busy. 300 forward and reverse steps of those shots: 29.0 -> 10.8 ms (14.8 with
 // p and u, w in two launches, which forms nothing twice but waits for its loads twice).
 //
-// Launches are programmatically serialised: a kernel reads coefficients and dL/d records ahead of the
-// end of the launch before it. The records of a step are taken by extra blocks of the
+// Launches are programmatically serialised, but for the first step of a solve, which follows the kernel that
+// writes the coefficients: a kernel reads coefficients and dL/d records ahead of the end of the launch
+// before it. The records of a step are taken by extra blocks of the
 // next, which reads them.
 #pragma once
 #include "acoustic_geo.cuh"
