@@ -225,8 +225,8 @@ struct adfwi_acoustic_plan {
   Tiling t2;             // 16 x 64 tiles of the pipelined forward and adjoint steps
   Resident rf, ra;       // the resident time loop, forward and adjoint, where the grid allows it
   int64_t o_sm = 0;      // tab: the model of each shot
-  // tab (FP64): padded cells of the receivers and of the unique receiver cells; the latter by tile
-  int64_t o_rij = 0, o_cij = 0, o_ftb = 0, o_ftc = 0;
+  // tab (FP64): padded rows and columns of the receivers and of the unique receiver cells; the latter by tile
+  int64_t o_rz = 0, o_rx = 0, o_cz = 0, o_cx = 0, o_ftb = 0, o_ftc = 0;
   int K, nseg;           // snapshot interval and number of segments (gradient mode)
   int last_chunk_start;  // first step of the reference's last checkpoint chunk
   int elem;              // bytes per element
@@ -494,7 +494,7 @@ int launch_adj(const adfwi_acoustic_plan* p, const ac::Geo<float>& g, int it, co
 // The double-precision steps (acoustic_f64.cuh): the same arguments.
 ac3::Cells f64_cells(const adfwi_acoustic_plan* p, const ac::Geo<double>& g) {
   const int32_t* tb = g.src_z - p->o_srcz;
-  return {tb + p->o_rij, tb + p->o_cij, tb + p->o_ftb, tb + p->o_ftc, p->t2.ncells};
+  return {tb + p->o_rz, tb + p->o_rx, tb + p->o_cz, tb + p->o_cx, tb + p->o_ftb, tb + p->o_ftc, p->t2.ncells};
 }
 unsigned f64_blocks(int64_t n) { return (unsigned)((n + ac3::kThreads - 1) / ac3::kThreads); }
 
@@ -1324,7 +1324,7 @@ Resident res_choose(const adfwi_acoustic_plan* p, bool adj, const std::vector<st
   const int NR = p->nzp - z0, CG = (p->nxp + 3) / 4, ns = p->d.ns;
   std::vector<int> cells(NR + 1, 0);  // receiver cells of the rows before each row
   for (size_t q = 0; q < rc.size(); ++q)
-    if (q == 0 || rc[q].first != rc[q - 1].first) cells[(rc[q].first >> 16) + 1]++;
+    if (q == 0 || rc[q].first != rc[q - 1].first) cells[(rc[q].first >> 32) + 1]++;
   std::vector<int> held(NR + 1, 0);   // rows before each row that hold any
   for (int r = 0; r < NR; ++r) {
     held[r + 1] = held[r] + (cells[r + 1] > 0);
@@ -1418,7 +1418,7 @@ void plan_resident(adfwi_acoustic_plan* p, const int32_t* rcv_z, const int32_t* 
   bool above = false;
   for (int r = 0; r < d.nr; ++r) {
     const int z = rcv_z[r] + d.nabc - z0, x = rcv_x[r] + d.nabc;
-    rc[r] = {((int64_t)z << 16) | x, r};
+    rc[r] = {((int64_t)z << 32) | x, r};
     above = above || z < 0;
   }
   if (above) return;
@@ -1438,7 +1438,7 @@ void plan_resident(adfwi_acoustic_plan* p, const int32_t* rcv_z, const int32_t* 
     const int sb = res::kGrp * (r->CG + 1);
     int strip = 0, last = -1, nslot = 0;
     for (size_t q = 0; q < rc.size(); ++q) {
-      const int z = (int)(rc[q].first >> 16), x = (int)(rc[q].first & 0xffff);
+      const int z = (int)(rc[q].first >> 32), x = (int)(rc[q].first & 0xffffffff);
       while (z >= (int)((int64_t)(strip + 1) * NR / r->G)) ++strip, nslot = 0;
       if (z != last) slot[z] = ++nslot;
       last = z;
@@ -1682,20 +1682,18 @@ int plan_create_impl(const adfwi_acoustic_desc* desc, const int32_t* src_z, cons
     p->t2.fwd_blocks = std::max(1, std::min(run_fblocks, p->t2.ntiles * p->t2.ngroups));
   }
   if (p->elem == 8) {
-    p->o_rij = t.size();
-    for (int r = 0; r < d.nr; ++r) t.push_back((rcv_z[r] + d.nabc) << 16 | (rcv_x[r] + d.nabc));
-    p->o_cij = t.size();
-    for (int q = 0; q < p->t2.ncells; ++q) {  // a cell's first receiver tells where it lies
-      const int r = t[p->t2.o_cr + t[p->t2.o_tcr + q]];
-      const int ij = t[p->o_rij + r];
-      t.push_back(ij);
-    }
+    p->o_rz = t.size();
+    for (int r = 0; r < d.nr; ++r) t.push_back(rcv_z[r] + d.nabc);
+    p->o_rx = t.size();
+    for (int r = 0; r < d.nr; ++r) t.push_back(rcv_x[r] + d.nabc);
+    auto first_at = [&](int q) { return t[p->t2.o_cr + t[p->t2.o_tcr + q]]; };  // a cell lies where its first receiver does
+    p->o_cz = t.size();
+    for (int q = 0; q < p->t2.ncells; ++q) t.push_back(rcv_z[first_at(q)] + d.nabc);
+    p->o_cx = t.size();
+    for (int q = 0; q < p->t2.ncells; ++q) t.push_back(rcv_x[first_at(q)] + d.nabc);
     const int tx = (p->nxp + ac3::kX - 1) / ac3::kX, nt = ac3::tiles(p->L, p->zbeg);
     std::vector<int32_t> beg(nt + 1, 0), order(p->t2.ncells);
-    auto tile = [&](int q) {
-      const int ij = t[p->o_cij + q];
-      return ((ij >> 16) - p->zbeg) / ac3::kZ * tx + (ij & 0xffff) / ac3::kX;
-    };
+    auto tile = [&](int q) { return (t[p->o_cz + q] - p->zbeg) / ac3::kZ * tx + t[p->o_cx + q] / ac3::kX; };
     for (int q = 0; q < p->t2.ncells; ++q) ++beg[tile(q) + 1];
     for (int q = 0; q < nt; ++q) beg[q + 1] += beg[q];
     std::vector<int32_t> at(beg.begin(), beg.end() - 1);

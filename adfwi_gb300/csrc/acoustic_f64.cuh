@@ -26,11 +26,11 @@ using ac::rsub;
 
 constexpr int kX = 32, kThreads = 128, kLanes = kX / 2, kZ = kThreads / kLanes;
 
-// Padded cells (i << 16 | j) of the receivers and of the unique receiver cells (in the order of
+// Padded rows and columns of the receivers and of the unique receiver cells (in the order of
 // Geo's tcell_rbeg); the unique cells' indices in the order of this file's tiles.
 struct Cells {
-  const int* rcv;
-  const int* cell;
+  const int *rcv_z, *rcv_x;
+  const int *cell_z, *cell_x;
   const int* tile_beg;
   const int* tile_cell;
   int ncells;
@@ -72,7 +72,7 @@ __device__ __forceinline__ void record(const ac::Geo<double>& g, const Cells& c,
                                        const double* u, const double* w, double* rp, double* ru, double* rw) {
   const int r = ((int)blockIdx.x - first) * kThreads + (int)threadIdx.x;
   if (r >= g.nr) return;
-  const int64_t oc = g.L.off(c.rcv[r] >> 16, c.rcv[r] & 0xffff);
+  const int64_t oc = g.L.off(c.rcv_z[r], c.rcv_x[r]);
   for (int s = g.grp_beg[blockIdx.y]; s < g.grp_beg[blockIdx.y + 1]; ++s) {
     const int64_t o = (int64_t)s * g.L.plane + oc, e = ((int64_t)s * g.nt + it) * g.nr + r;
     rp[e] = p[o];
@@ -260,11 +260,11 @@ __global__ void __launch_bounds__(kThreads)
       st(si + 2 * threadIdx.x, 0.0, 0.0);
       __syncthreads();
       for (int k = cb + (int)threadIdx.x; k < ce; k += kThreads) {
-        const int c = cells.tile_cell[k], zx = cells.cell[c];
+        const int c = cells.tile_cell[k];
         double ap = 0.0;
         for (int m = g.tcell_rbeg[c]; m < g.tcell_rbeg[c + 1]; ++m)
           ap += ac::grad_rec_p(g, gp, s, it - 1, g.cell_rcv[m], gmul);
-        si[((zx >> 16) - q.i0) * kX + (zx & 0xffff) - q.j0] = ap;
+        si[(cells.cell_z[c] - q.i0) * kX + cells.cell_x[c] - q.j0] = ap;
       }
     }
     if (s == s_beg) {
@@ -388,7 +388,7 @@ __global__ void adj_inject_uw(ac::Geo<double> g, Cells cells, int it, const doub
                               double* lw) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cells.ncells) return;
-  const int s = blockIdx.y, zx = cells.cell[k], i = zx >> 16, j = zx & 0xffff;
+  const int s = blockIdx.y, i = cells.cell_z[k], j = cells.cell_x[k];
   double au = 0.0, aw = 0.0;
   for (int m = g.tcell_rbeg[k]; m < g.tcell_rbeg[k + 1]; ++m) {
     const int64_t e = ((int64_t)s * g.nt + it) * g.nr + g.cell_rcv[m];
