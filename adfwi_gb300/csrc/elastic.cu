@@ -101,7 +101,8 @@ struct Geo {
   const T* src_m;              // ns x 3 source weights (xx, zz, xz) already scaled for the mode
   const int* rcv_z;
   const int* rcv_x;
-  const int* ucell_zx;         // unique receiver cells (i << 16 | j)
+  const int* ucell_z;          // rows and columns of the unique receiver cells
+  const int* ucell_x;
   const int* ucell_beg;        // ncells+1 offsets into ucell_rcv
   const int* ucell_rcv;
   const int* tile_beg;         // first unique receiver cell of each tile of the reverse kernels, and the end
@@ -705,8 +706,7 @@ __global__ void adj_inject(Geo<T> g, int it, const T* __restrict__ grec, T* lv) 
   if (q >= g.ncells) return;
   const int s = blockIdx.y;
   const int64_t NSP = (int64_t)g.ns * g.L.plane;
-  const int cell = g.ucell_zx[q];
-  const int64_t o = (int64_t)s * g.L.plane + g.L.off(cell >> 16, cell & 0xffff);
+  const int64_t o = (int64_t)s * g.L.plane + g.L.off(g.ucell_z[q], g.ucell_x[q]);
   const int64_t RS = (int64_t)g.ns * g.nt * g.nr, base = ((int64_t)s * g.nt + it) * g.nr;
   for (int c = 0; c < 2; ++c) {
     T a = T(0);
@@ -950,8 +950,7 @@ struct Inject {
     if (beg < end) take(g, beg);
   }
   __device__ __forceinline__ void take(const Geo<T>& g, int q) {
-    const int zx = g.ucell_zx[q];
-    cell = (zx >> 16) % kAR * kVecX + (zx & 0xffff) % kVecX;
+    cell = g.ucell_z[q] % kAR * kVecX + g.ucell_x[q] % kVecX;
     m0 = g.ucell_beg[q];
     m1 = g.ucell_beg[q + 1];
   }
@@ -1499,7 +1498,7 @@ struct adfwi_elastic_plan {
   std::vector<int32_t> tab;
   std::vector<unsigned char> srcm;  // ns x 3 source weights (xx, zz, xz) in the solve's dtype
   PinnedBytes tab_pin, srcm_pin;    // page-locked copies of tab and srcm, the sources of each upload
-  int64_t o_srcz, o_srcx, o_rcvz, o_rcvx, o_uzx, o_ubeg, o_urcv, o_tbeg;
+  int64_t o_srcz, o_srcx, o_rcvz, o_rcvx, o_uz, o_ux, o_ubeg, o_urcv, o_tbeg;
   int ncells;
   std::vector<int> chunk_end;  // last step of each reference checkpoint chunk
 };
@@ -1619,7 +1618,8 @@ el::Geo<T> egeo(const adfwi_elastic_plan* p, const unsigned char* ws, const ECar
   g.src_m = reinterpret_cast<const T*>(ws + c.srcm);
   g.rcv_z = tb + p->o_rcvz;
   g.rcv_x = tb + p->o_rcvx;
-  g.ucell_zx = tb + p->o_uzx;
+  g.ucell_z = tb + p->o_uz;
+  g.ucell_x = tb + p->o_ux;
   g.ucell_beg = tb + p->o_ubeg;
   g.ucell_rcv = tb + p->o_urcv;
   g.tile_beg = tb + p->o_tbeg;
@@ -1945,20 +1945,22 @@ int adfwi_elastic_plan_create(const adfwi_elastic_desc* desc, const int32_t* src
   // unique receiver cells
   // in the order of the reverse kernels' tiles
   struct Cell {
-    int tile, zx, r;
-    bool operator<(const Cell& o) const { return tile != o.tile ? tile < o.tile : zx < o.zx; }
+    int tile, z, x, r;
+    bool same(const Cell& o) const { return z == o.z && x == o.x; }
+    bool operator<(const Cell& o) const { return tile != o.tile ? tile < o.tile : z != o.z ? z < o.z : x < o.x; }
   };
   const int tiles_x = (p->nxp + el::kVecX - 1) / el::kVecX, tiles = adj_tiles(p);
   std::vector<Cell> cells(d.nr);
   for (int r = 0; r < d.nr; ++r) {
     const int z = rcv_z[r] + p->top, x = rcv_x[r] + d.nabc;
-    cells[r] = {z / el::kAR * tiles_x + x / el::kVecX, (z << 16) | x, r};
+    cells[r] = {z / el::kAR * tiles_x + x / el::kVecX, z, x, r};
   }
   std::stable_sort(cells.begin(), cells.end());
-  std::vector<int32_t> uzx, ubeg, urcv, tbeg(tiles + 1, 0);
+  std::vector<int32_t> uz, ux, ubeg, urcv, tbeg(tiles + 1, 0);
   for (int q = 0; q < d.nr; ++q) {
-    if (q == 0 || cells[q].zx != cells[q - 1].zx) {
-      uzx.push_back(cells[q].zx);
+    if (q == 0 || !cells[q].same(cells[q - 1])) {
+      uz.push_back(cells[q].z);
+      ux.push_back(cells[q].x);
       ubeg.push_back((int32_t)urcv.size());
       ++tbeg[cells[q].tile + 1];
     }
@@ -1966,9 +1968,11 @@ int adfwi_elastic_plan_create(const adfwi_elastic_desc* desc, const int32_t* src
   }
   for (int t = 0; t < tiles; ++t) tbeg[t + 1] += tbeg[t];
   ubeg.push_back((int32_t)urcv.size());
-  p->ncells = (int)uzx.size();
-  p->o_uzx = t.size();
-  t.insert(t.end(), uzx.begin(), uzx.end());
+  p->ncells = (int)uz.size();
+  p->o_uz = t.size();
+  t.insert(t.end(), uz.begin(), uz.end());
+  p->o_ux = t.size();
+  t.insert(t.end(), ux.begin(), ux.end());
   p->o_ubeg = t.size();
   t.insert(t.end(), ubeg.begin(), ubeg.end());
   p->o_urcv = t.size();

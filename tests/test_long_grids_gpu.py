@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import adfwi_gb300 as A
-from _cases import acoustic_problem, oracle_acoustic, rel
+from _cases import ELASTIC_KEYS, acoustic_problem, elastic_problem, oracle_acoustic, oracle_elastic, rel
 
 pytestmark = pytest.mark.gpu
 TOL = {torch.float64: (1e-12, 1e-9), torch.float32: (1e-5, 1e-4)}
@@ -45,3 +45,23 @@ def test_acoustic_long_grids(nz, nx, dtype):
     sum((ref[k] * w[k]).sum() for k in "puw").backward()
     for got, want in ((model.vp.grad, vp.grad), (model.rho.grad, rho.grad)):
         assert rel(got, want) <= TOL[dtype][1]
+
+
+@pytest.mark.parametrize("nz,nx", SHAPES[:2])
+@pytest.mark.parametrize("abc_type,free_surface", [("PML", True), ("gerjan", False)])
+def test_elastic_long_grids(nz, nx, abc_type, free_surface):
+    nt = 8
+    kw = dict(nabc=4, nt=nt, ns=1, nr=3, dtype=torch.float64, abc_type=abc_type, free_surface=free_surface)
+    model, survey, prop = elastic_problem(A, nz=nz, nx=nx, **kw)
+    survey, nr = survey_at_the_far_end(survey, nz, nx, nt)
+    prop = A.ElasticPropagator(model, survey, device="cuda:0", dtype=torch.float64)
+    rec = prop.forward(fd_order=4)
+    ref, pars = oracle_elastic(prop, model, fd_order=4)
+    w = {k: torch.randn((1, nt, nr), generator=torch.Generator().manual_seed(3), dtype=torch.float64) for k in ELASTIC_KEYS}
+    for k in ELASTIC_KEYS:
+        assert float(ref[k].detach()[:, :, :11].abs().max()) > 0
+        assert rel(rec[k].detach(), ref[k].detach()) <= 1e-12, k
+    sum((rec[k] * w[k].cuda()).sum() for k in ELASTIC_KEYS).backward()
+    sum((ref[k] * w[k]).sum() for k in ELASTIC_KEYS).backward()
+    for p in ("vp", "vs", "rho", "eps", "delta"):
+        assert rel(getattr(model, p).grad, pars[p].grad) <= 1e-9, p
