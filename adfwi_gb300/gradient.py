@@ -117,8 +117,9 @@ class GradProcessor(object):
         ws = torch.empty(need.value, dtype=torch.uint8, device=dev)
         with torch.cuda.device(dev):
             N.check(lib.adfwi_gradproc(nz, nx, span, smooth, keep, N.ptr(g), N.ptr(taper), N.ptr(mask),
-                                       dtype_code(forw.dtype), N.ptr(forw), int(bool(self.norm_grad)), float(vmax),
-                                       N.ptr(out), N.ptr(ws), ws.numel(), N.stream_handle(dev)), "adfwi_gradproc")
+                                       dtype_code(forw.dtype), N.ptr(forw), int(bool(self.norm_grad)),
+                                       float(vmax) if self.norm_grad else 0.0, N.ptr(out), N.ptr(ws), ws.numel(),
+                                       N.stream_handle(dev)), "adfwi_gradproc")
         return out
 
     def forward(self, nx, nz, vmax, grad, forw=None):
