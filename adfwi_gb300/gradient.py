@@ -96,6 +96,10 @@ class GradProcessor(object):
                 and N.by_address(g) and N.by_address(forw)
                 and not (torch.is_grad_enabled() and (g.requires_grad or forw.requires_grad))):
             return None
+        m = self.grad_mask
+        if torch.is_tensor(m) and not (type(m) in (torch.Tensor, torch.nn.Parameter) and N.by_address(m)
+                                       and not (torch.is_grad_enabled() and m.requires_grad)):
+            return None
         taper = mask = None
         if self.grad_mute > 0:
             taper = self._taper_for(nz, nx, thred, dev)

@@ -20,3 +20,10 @@ def test_no_maximum_velocity_without_scaling():
     q._native = lambda *a: None
     out, ref = (r.forward(nx=45, nz=30, vmax=None, grad=g, forw=f) for r in (p, q))
     assert float((out - ref).abs().max()) <= 1e-13 * float(ref.abs().max())
+
+
+def test_a_mask_with_a_gradient_keeps_it():
+    g, f = planes()
+    mask = torch.rand((30, 45), device="cuda:0").requires_grad_()
+    GradProcessor(grad_mask=mask).forward(nx=45, nz=30, vmax=3000.0, grad=g, forw=f).sum().backward()
+    assert float(mask.grad.abs().max()) > 0
