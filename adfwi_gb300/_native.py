@@ -69,6 +69,7 @@ def _bind(lib):
         "adfwi_acoustic_noalloc_status": (c_int32, [P, ctypes.POINTER(c_int32), P]),
         "adfwi_last_error": (c_int32, [ctypes.c_char_p, ctypes.c_size_t]),
         "adfwi_wait_selftest": (c_int32, [c_int64, P, P]),
+        "adfwi_row_wait_selftest": (c_int32, [c_int64, P, P, P]),
         "adfwi_profile_start": (c_int32, [c_int32]),
         "adfwi_profile_stop": (c_int32, [ctypes.POINTER(KernelStat), c_int32, ctypes.POINTER(c_int32)]),
         "adfwi_launch_count": (c_int64, []),
@@ -175,3 +176,10 @@ def wait_selftest(limit_ns, flag, stream=None):
     1 once a wait that nothing completes has run out after `limit_ns`."""
     st = ctypes.c_void_p(stream) if stream is not None else stream_handle(flag.device)
     check(lib().adfwi_wait_selftest(int(limit_ns), ptr(flag), st), "adfwi_wait_selftest")
+
+
+def row_wait_selftest(limit_ns, flag, row, stream=None):
+    """The same for the wait of a strip on its neighbour's rows, in global and in shared memory; `row`
+    (8 float32) receives what the two waits left."""
+    st = ctypes.c_void_p(stream) if stream is not None else stream_handle(flag.device)
+    check(lib().adfwi_row_wait_selftest(int(limit_ns), ptr(flag), ptr(row), st), "adfwi_row_wait_selftest")

@@ -1759,6 +1759,12 @@ int adfwi_acoustic_workspace_bytes(const adfwi_acoustic_plan* p, int32_t with_gr
   return kOk;
 }
 
+int adfwi_row_wait_selftest(int64_t limit_ns, int32_t* flag, float* row, void* stream) {
+  ADFWI_CHECK_ARG(flag != nullptr && row != nullptr, "null flag or row");
+  ADFWI_CHECK_ARG(limit_ns > 0 && limit_ns <= 2000000000ll, "limit_ns must be in (0, 2 s]");
+  return res::row_wait_selftest(limit_ns, reinterpret_cast<int*>(flag), row, static_cast<cudaStream_t>(stream));
+}
+
 int adfwi_acoustic_snapshot_every(const adfwi_acoustic_plan* p, int32_t* steps) {
   ADFWI_CHECK_ARG(p && steps, "null plan or output pointer");
   *steps = p->bsave ? ADFWI_SNAP_EVERY_BOUNDARY : p->K;

@@ -173,7 +173,8 @@ __device__ __forceinline__ void put_row(f2* box, int rank, unsigned tag, const f
 // raises the device flag and the block's `dead` mark: from then on nothing waits, and every
 // block runs to its end.
 template <bool GLB>
-__device__ __forceinline__ void take_row(const f2* box, unsigned tag, float* dst, int* flag, volatile int* dead) {
+__device__ __forceinline__ void take_row(const f2* box, unsigned tag, float* dst, int* flag, volatile int* dead,
+                                         unsigned long long limit_ns = kWaitNs) {
   f2 a, b, c, d;
   unsigned long long t0 = 0;
   for (unsigned n = 0;; ++n) {
@@ -190,7 +191,7 @@ __device__ __forceinline__ void take_row(const f2* box, unsigned tag, float* dst
       if (*dead) break;
       const unsigned long long t = global_ns();
       if (t0 == 0) t0 = t;
-      if (t - t0 > kWaitNs || *(volatile int*)flag != 0) {
+      if (t - t0 > limit_ns || *(volatile int*)flag != 0) {
         raise_flag(flag, kErrWaitTimeout);
         *dead = 1;
       }

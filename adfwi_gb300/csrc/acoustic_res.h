@@ -59,6 +59,7 @@ constexpr int kVariants[][2] = {{2, 512}, {3, 512}, {3, 768}, {4, 512}, {4, 640}
 // illumination is summed).
 ResKernel forward_kernel(int rb, int mt, bool sums, bool glb);
 ResKernel adjoint_kernel(int rb, int mt, bool glb);
+int row_wait_selftest(int64_t limit_ns, int* flag, float* row, cudaStream_t st);
 
 }  // namespace res
 }  // namespace adfwi

@@ -223,6 +223,12 @@ int adfwi_acoustic_status(const adfwi_acoustic_plan* plan, const void* workspace
  * usable. Stream-ordered; the caller zeroes *flag first. */
 int adfwi_wait_selftest(int64_t limit_ns, int32_t* flag, void* stream);
 
+/* The same for the resident loop's wait of a strip on its neighbour's rows: words that nothing writes
+ * are waited for in global memory until limit_ns have passed, then in shared memory, where the
+ * raised flag ends the wait at once. DEVICE float row[8] receives what the two waits left (the
+ * words' zeroes; -1 where a wait did not mark its block as having given up). */
+int adfwi_row_wait_selftest(int64_t limit_ns, int32_t* flag, float* row, void* stream);
+
 /* ------------------------------------------------------------------------- */
 /* Normalised L2 trace misfit and its adjoint source.                          */
 /* ------------------------------------------------------------------------- */
