@@ -617,7 +617,6 @@ res::ResArgs res_args(const adfwi_acoustic_plan* p, const Resident& r, unsigned 
   a.S = r.S;
   a.z0 = p->d.free_surface ? p->fs : 0;
   a.NR = p->nzp - a.z0;
-  a.R = r.R;
   a.TR = r.TR;
   a.CG = r.CG;
   a.oS = r.oS;
@@ -1225,7 +1224,9 @@ void build_tiling(adfwi_acoustic_plan* p, Tiling* tl, int tz, int tx, const std:
 // Shots per group of the double-precision steps: one while that gives at most 16 blocks of 128 threads
 // per SM (more blocks than are resident), then as many as keep to that. A group has one partial plane
 // per sum, so where memory is short (the allocation-free forward's scratch, a budget below the whole
-// history) groups stay as large as one block per SM of 16 x 64 tiles would make them.
+// history) groups stay as large as one block per SM of 16 x 64 tiles would make them. Short is what the whole
+// batch takes: there a model's shots may be grouped otherwise than in a plan of its own, and its FP64
+// sums rounded in another order.
 int f64_group_shots(const adfwi_acoustic_plan* p, const std::vector<int>& alone, int ntiles, int64_t scratch) {
   const int ns = alone[1], tight = pick_unit_shots(alone, ntiles, 152, 152);
   const int fine = std::max(1, (int)((int64_t)ns * ac3::tiles(p->L, p->zbeg) / (152 * 16)));

@@ -23,7 +23,7 @@
 // What bounds it is the shared-memory pipe: about 90 wavefronts per 128 cells and step of the 130
 // to 190 clocks they take, next to the exchange (1 to 2 us per step, acoustic.cu res_choose).
 // Measured per step of all shots, per-step kernels -> here, in us: 300 x 700 with 30 shots forward 52 -> 29,
-// adjoint 80 -> 41; 600 x 1600 with 8 shots 79 -> 54, 120 -> 66; 148 x 260 with 40 shots and a free
+// adjoint 80 -> 37; 600 x 1600 with 8 shots 79 -> 54, 120 -> 66; 148 x 260 with 40 shots and a free
 // surface 18.7 -> 7.3, 35 -> 9.4; 200 x 200 with 10 shots (records only) 9.2 -> 2.4.
 // Tried and slower: the state of a thread's cells in registers with shuffles for the horizontal
 // neighbours (spills; 4.3 against 3.1 us on 20 rows x 256), all coefficients in shared memory with
@@ -39,7 +39,9 @@
 //   dL/d alpha1 = - sum V div(u, w) / alpha1,   dL/d alpha2 = - sum (U dp/dx + W dp/dz) / alpha2,
 // so no neighbour's coefficient is needed. Cells of an update region whose alpha is zero carry
 // the unscaled lambda in the global state planes instead (V, U, W are zero there). No result
-// depends on G, R, the variant or how the steps are split into launches.
+// depends on G, R or the variant. Nor does it on how the steps are split into launches, but for the
+// gradients of the four columns of a thread that hold such a cell: their sums begin anew in every launch and
+// are added up at its end.
 #pragma once
 #include "acoustic_res.h"
 #include "tma.cuh"

@@ -17,7 +17,7 @@ constexpr int kHeadWords = 16;        // two mbarriers and the block's give-up m
 constexpr int kGrp = 12, kW = 4, kP = 8;
 
 struct ResArgs {
-  int G, S, NR, z0, R, TR, CG;  // blocks per shot, shots at a time, rows and the first of them, most rows per strip, thread rows, column groups
+  int G, S, NR, z0, TR, CG;  // blocks per shot, shots at a time, rows and the first of them, thread rows, column groups
   int oS, oA1, oA2, oPH, oDH, oBox, oInj, injw, injg, oRow, oT;  // shared memory, in words (oA1, oA2: 0 = not kept)
   int t0, t1;                 // steps t0 .. t1-1 (the adjoint runs them downwards)
   int h0;                     // step of history slot 0

@@ -11,11 +11,11 @@
 //   ADFWI/propagator/elastic_kernels.py:709-774   absorbing-layer step (unsplit, -MT/3 source, v *= damp)
 //   ADFWI/propagator/elastic_kernels.py:917-1037  padding, index shifts, chunked loop, record dict
 //
-// One time step is a short sequence of launches, each a pointwise or gather stencil over
-// (cell, shot): the split fields are updated in place (every update reads only its own
-// cell of the field it writes), totals and free-surface rows are rebuilt from the split
-// fields. Gradient kernels handle one cell for every shot in a loop, so the coefficient
-// gradients are summed over shots in a fixed order (deterministic, no atomics). The
+// One time step is two launches over (cell, shot), stresses and velocities (four with an absorbing layer
+// under a free surface). Split fields are kept where the scheme needs them and updated in place, every
+// other cell advances its totals; free-surface rows are written with the rows they mirror. A reverse
+// step is two launches over tiles and groups of shots (three there): a block takes the shots of its group one
+// after another and sums their coefficient gradients in a fixed order (deterministic, no atomics). The
 // forward arithmetic uses explicitly rounded operations in the reference's order.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -153,7 +153,6 @@ __device__ __forceinline__ T pml_inv(T d) {
 // same bytes with twice the instructions, four leave too few warps: 12.1, 10.5 and 12.7 ms for 200
 // forward steps of 20 shots on a 242 x 480 grid with 1, 2 and 4.
 constexpr int kVecThreads = 128, kVecX = 32;
-template <typename T>
 constexpr int kVW = 2;
 template <int B>
 struct Bytes;
@@ -166,12 +165,12 @@ struct Bytes<16> {
   using t = int4;
 };
 template <typename T>
-using VecBits = typename Bytes<kVW<T> * (int)sizeof(T)>::t;
+using VecBits = typename Bytes<kVW * (int)sizeof(T)>::t;
 template <typename T>
-constexpr int kVecRows = kVecThreads * kVW<T> / kVecX;
+constexpr int kVecRows = kVecThreads * kVW / kVecX;
 template <typename T>
 struct Vec {
-  T v[kVW<T>];
+  T v[kVW];
 };
 template <typename T>
 __device__ __forceinline__ Vec<T> ldv(const T* p) {
@@ -186,11 +185,11 @@ __device__ __forceinline__ void stv(T* p, const Vec<T>& x) {
 // The vector at p of a row with the whole vectors that hold its NN neighbours on each side.
 template <typename T, int NN>
 struct Row {
-  static constexpr int H = (NN + kVW<T> - 1) / kVW<T> * kVW<T>;
-  T v[kVW<T> + 2 * H];
+  static constexpr int H = (NN + kVW - 1) / kVW * kVW;
+  T v[kVW + 2 * H];
   __device__ __forceinline__ explicit Row(const T* p) {
 #pragma unroll
-    for (int k = 0; k < kVW<T> + 2 * H; k += kVW<T>)
+    for (int k = 0; k < kVW + 2 * H; k += kVW)
       *reinterpret_cast<VecBits<T>*>(v + k) = *reinterpret_cast<const VecBits<T>*>(p - H + k);
   }
   __device__ __forceinline__ T operator()(int k) const { return v[H + k]; }
@@ -221,7 +220,7 @@ __device__ __forceinline__ void divide(Vec<T> (&a)[N], const By& by) {
 #pragma unroll
   for (int k = 0; k < N; ++k)
 #pragma unroll
-    for (int e = 0; e < kVW<T>; ++e) {
+    for (int e = 0; e < kVW; ++e) {
       taken = taken && by(k, e).takes(a[k].v[e]);
       small = small || Divisor<T>::small(a[k].v[e]);
     }
@@ -229,17 +228,17 @@ __device__ __forceinline__ void divide(Vec<T> (&a)[N], const By& by) {
 #pragma unroll
     for (int k = 0; k < N; ++k)
 #pragma unroll
-      for (int e = 0; e < kVW<T>; ++e) a[k].v[e] = rdiv(a[k].v[e], by(k, e).d);
+      for (int e = 0; e < kVW; ++e) a[k].v[e] = rdiv(a[k].v[e], by(k, e).d);
   } else if (small) {
 #pragma unroll
     for (int k = 0; k < N; ++k)
 #pragma unroll
-      for (int e = 0; e < kVW<T>; ++e) a[k].v[e] = by(k, e).tiny(a[k].v[e]);
+      for (int e = 0; e < kVW; ++e) a[k].v[e] = by(k, e).tiny(a[k].v[e]);
   } else {
 #pragma unroll
     for (int k = 0; k < N; ++k)
 #pragma unroll
-      for (int e = 0; e < kVW<T>; ++e) a[k].v[e] = by(k, e).of(a[k].v[e]);
+      for (int e = 0; e < kVW; ++e) a[k].v[e] = by(k, e).of(a[k].v[e]);
   }
 }
 // the x parts (even planes) over dx, the z parts over dz
@@ -253,7 +252,7 @@ __host__ __device__ __forceinline__ int vec_tiles(const Layout& L) {
 }
 // this thread's row i and first column j
 #define EL_VEC_IJ                                                               \
-  constexpr int W = kVW<T>;                                                     \
+  constexpr int W = kVW;                                                     \
   const int tiles_x_ = (g.L.nxp + kVecX - 1) / kVecX;                           \
   const int ti_ = (int)blockIdx.x / tiles_x_, tj_ = (int)blockIdx.x - ti_ * tiles_x_; \
   const int i = ti_ * kVecRows<T> + (int)threadIdx.x / (kVecX / W);             \
@@ -319,7 +318,7 @@ __device__ __forceinline__ void store_stress(const Geo<T>& g, int i, int64_t o, 
   }
   Vec<T> nz, nx;
 #pragma unroll
-  for (int e = 0; e < kVW<T>; ++e) {
+  for (int e = 0; e < kVW; ++e) {
     if (i == h - 1) zz.v[e] = T(0);
     nz.v[e] = -zz.v[e];
     nx.v[e] = -xz.v[e];
@@ -788,7 +787,7 @@ __device__ __forceinline__ void tfs_adjoint(const Geo<T>& g, const T* lzz, const
 // every cell, tiles of 8 rows, and two launches for the dL/d records).
 constexpr int kAR = 16;
 template <typename T>
-constexpr int kAdjThreads = kAR * kVecX / kVW<T>;
+constexpr int kAdjThreads = kAR * kVecX / kVW;
 constexpr int kAXW = kVecX + 8;                             // an x plane's row: columns j0-4 .. j0+35
 constexpr int kAX = kAR * kAXW, kAZ = (kAR + 6) * kVecX;  // x plane: tile rows; z plane: rows i0-3 ..
 constexpr int kAH = (kAR + 6) * kAXW;                       // a history plane: z plane's rows, x plane's columns
@@ -809,7 +808,7 @@ __device__ __forceinline__ T diff_t(const Geo<T>& g, const A& at) {
 // A thread's vector of the tile and the vector of the tile's halo that it also forms sources for.
 template <typename T, int NN>
 struct AdjTile {
-  static constexpr int W = kVW<T>, NX = kAR * 8 / W, NZ = 2 * NN * kVecX / W;  // halo vectors beside, above and below
+  static constexpr int W = kVW, NX = kAR * 8 / W, NZ = 2 * NN * kVecX / W;  // halo vectors beside, above and below
   static_assert(NX + NZ <= kAdjThreads<T>, "one halo vector per thread");
   int i0, j0;            // the tile's first cell
   int i, j, px, pz, ph, pi;  // own vector; its place in an x, a z and a history plane and in the tile
@@ -877,17 +876,17 @@ __device__ __forceinline__ void stage_full(const Geo<T>& g, T* dst, const T* src
 // unit: bit e set where cell e keeps no split fields (only cells of I can); in: cells of I.
 template <typename T, bool PML>
 struct AdjFactors {
-  T kx[kVW<T>], kz[kVW<T>], sx[kVW<T>], sz[kVW<T>];
+  T kx[kVW], kz[kVW], sx[kVW], sz[kVW];
   unsigned in = 0, unit = 0;
   __device__ __forceinline__ AdjFactors(const Geo<T>& g, const T* cf, int i, int j) {
     Vec<T> bx, bz;
-    const bool near = i >= g.ilo && i <= g.ihi && j + kVW<T> > g.jlo && j <= g.jhi;
+    const bool near = i >= g.ilo && i <= g.ihi && j + kVW > g.jlo && j <= g.jhi;
     if (PML && near) {
       bx = ldv(cf + BCX * g.L.plane + g.L.off(i, j));
       bz = ldv(cf + BCZ * g.L.plane + g.L.off(i, j));
     }
 #pragma unroll
-    for (int e = 0; e < kVW<T>; ++e) {
+    for (int e = 0; e < kVW; ++e) {
       const bool ok = in_I(g, i, j + e);
       kx[e] = ok ? g.dt_dx : T(0);
       kz[e] = ok ? g.dt_dz : T(0);
@@ -902,7 +901,7 @@ struct AdjFactors {
         if (!keeps_split(g, i, bx.v[e], bz.v[e])) unit |= 1u << e;
       }
     }
-    if (!PML) unit = (1u << kVW<T>) - 1u;
+    if (!PML) unit = (1u << kVW) - 1u;
   }
   __device__ __forceinline__ bool split() const { return PML && (in & ~unit) != 0u; }
 };
@@ -917,7 +916,7 @@ __device__ __forceinline__ void adj_vel_totals(const Geo<T>& g, const T* cf, con
   az = ldv(l + VZ * kAH + ph);
   if (!PML) {
 #pragma unroll
-    for (int e = 0; e < kVW<T>; ++e) {
+    for (int e = 0; e < kVW; ++e) {
       ax.v[e] *= d.v[e];
       az.v[e] *= d.v[e];
     }
@@ -928,7 +927,7 @@ __device__ __forceinline__ void adj_vel_totals(const Geo<T>& g, const T* cf, con
       return PML ? v : cf[DAMP * g.L.plane + g.L.off(ii, jj)] * v;
     };
 #pragma unroll
-    for (int e = 0; e < kVW<T>; ++e) vfs_adjoint(g, i, j + e, at, ax.v[e], az.v[e]);
+    for (int e = 0; e < kVW; ++e) vfs_adjoint(g, i, j + e, at, ax.v[e], az.v[e]);
   }
 }
 
@@ -989,7 +988,7 @@ __global__ void __launch_bounds__(kAdjThreads<T>, sizeof(T) == 4 ? (PML ? 3 : 2)
                const T* __restrict__ lvs_in, T* __restrict__ lvs_out, T* lt, const T* __restrict__ tt_hist,
                const T* __restrict__ grec, T* gpart, int eg) {
   extern __shared__ __align__(16) unsigned char el_smem[];
-  constexpr int W = kVW<T>;
+  constexpr int W = kVW;
   const AdjTile<T, NN> p(g.L);
   const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL;
   const int64_t oc = g.L.off(p.i, p.j), oh = g.L.off(p.hi, p.hj);
@@ -1195,7 +1194,7 @@ __global__ void __launch_bounds__(kAdjThreads<T>, sizeof(T) == 4 ? 2 : 1)
                T* __restrict__ lts_out, T* lv, const T* __restrict__ v_hist, const T* __restrict__ grec, T* gpart,
                int eg) {
   extern __shared__ __align__(16) unsigned char el_smem[];
-  constexpr int W = kVW<T>;
+  constexpr int W = kVW;
   const AdjTile<T, NN> p(g.L);
   const int64_t PL = g.L.plane, NSP = (int64_t)g.ns * PL;
   const int64_t oc = g.L.off(p.i, p.j), oh = g.L.off(p.hi, p.hj);
@@ -1800,7 +1799,7 @@ int ebackward(const adfwi_elastic_plan* p, const void* wavelet, const void* grec
   const dim3 ga(adj_tiles(p), egr), ba(el::kAdjThreads<T>);
   auto adj_t = p->d.pml ? el::adj_t_step<T, NN, true> : el::adj_t_step<T, NN, false>;
   auto adj_v = p->d.pml ? el::adj_v_step<T, NN, true> : el::adj_v_step<T, NN, false>;
-  // shared memory of the reverse kernels (above the 48 KB default in double precision)
+  // shared memory of the reverse kernels (75 and 91 KB, twice that in double precision: above the 48 KB default)
   const int smem_t = el::kAdjT * (int)sizeof(T), smem_v = el::kAdjV * (int)sizeof(T);
   ADFWI_CUDA_TRY(cudaFuncSetAttribute(adj_t, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
   ADFWI_CUDA_TRY(cudaFuncSetAttribute(adj_v, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_v));
