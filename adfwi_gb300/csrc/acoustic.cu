@@ -78,6 +78,17 @@ __global__ void adj_seed(Geo<T> g, int ntiles, int tz, int tx, const T* __restri
   }
 }
 
+// The adjoint of w[fs-1] = w[fs] (acoustic_kernels.py:163-164), which closes the last step, on the seed: the
+// reverse steps fold what they inject themselves.
+template <typename T>
+__global__ void fold_mirrored_w(Geo<T> g, T* lw) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= g.L.nxp) return;
+  T* up = lw + (int64_t)blockIdx.y * g.L.plane + g.L.off(g.fs - 1, j);
+  up[g.L.pitch] += *up;
+  *up = T(0);
+}
+
 // Copy a dense (h, w) array into a pitched plane at cell (0, 0) (ghosts untouched).
 template <typename T>
 __global__ void pack_plane(Layout L, int h, int w, const T* __restrict__ src, T* __restrict__ dst) {
@@ -222,6 +233,7 @@ struct Resident {
 struct adfwi_acoustic_plan {
   adfwi_acoustic_desc d;
   int nzp, nxp, fs, zbeg;
+  bool rcv_above = false;  // receivers on the mirrored row above a free surface
   Tiling t2;             // 16 x 64 tiles of the pipelined forward and adjoint steps
   Resident rf, ra;       // the resident time loop, forward and adjoint, where the grid allows it
   int64_t o_sm = 0;      // tab: the model of each shot
@@ -952,6 +964,9 @@ int backward_impl(const adfwi_acoustic_plan* p, const void* wavelet, const void*
     dim3 sg(std::max(1, std::min(64, (p->t2.ncells + 127) / 128)), p->d.ns);
     ADFWI_LAUNCH(kAux, st, (ac::adj_seed<T><<<sg, 128, 0, st>>>(g2, p->t2.ntiles, ac2::TZ, ac2::TX, gp, gu, gw, la,
                                                                    la + ns * pl, la + 2 * ns * pl)));
+    if (gw && p->rcv_above)
+      ADFWI_LAUNCH(kAux, st, (ac::fold_mirrored_w<T><<<dim3((p->nxp + 127) / 128, p->d.ns), 128, 0, st>>>(
+                                 g2, la + 2 * ns * pl)));
   }
   T* lcur = la;
   T* lnxt = lb;
@@ -1658,6 +1673,7 @@ int plan_create_impl(const adfwi_acoustic_desc* desc, const int32_t* src_z, cons
       delete p;
       return kBadGeometry;
     }
+    p->rcv_above = p->rcv_above || (d.free_surface && z < p->fs);
   }
   // 16 x 64 tiles: units of G shots spread over the resident blocks of the pipelined steps.
   {
