@@ -543,8 +543,9 @@ int launch_adj(const adfwi_acoustic_plan* p, const ac::Geo<double>& g, int it, c
                ADFWI_CUDA_TRY(launch_pdl_kernel(ac3::adj_step, dim3(nt, gy), b, 0, st, g, cells, it, cf, cfs, lp0, lu0, lw0,
                                                 lp1, lu1, lw1, ph, dh, g1, g2, gp)));
   if ((gu || gw) && it >= 1 && cells.ncells > 0) {
-    ADFWI_LAUNCH(kAux, st, (ac3::adj_inject_uw<<<dim3(f64_blocks(cells.ncells), p->d.ns), b, 0, st>>>(g, cells, it - 1, gu,
-                                                                                                       gw, lu1, lw1)));
+    for (int mirrored = 0; mirrored <= (p->rcv_above ? 1 : 0); ++mirrored)
+      ADFWI_LAUNCH(kAux, st, (ac3::adj_inject_uw<<<dim3(f64_blocks(cells.ncells), p->d.ns), b, 0, st>>>(
+                                 g, cells, it - 1, mirrored != 0, gu, gw, lu1, lw1)));
     ADFWI_CUDA_TRY(cudaGetLastError());
   }
   return kOk;

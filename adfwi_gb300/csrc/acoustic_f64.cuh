@@ -383,12 +383,15 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// dL/d u- and w-records of step it into lambda_u and lambda_w, with the adjoint of w[fs-1] = w[fs].
-__global__ void adj_inject_uw(ac::Geo<double> g, Cells cells, int it, const double* gu, const double* gw, double* lu,
-                              double* lw) {
+// dL/d u- and w-records of step it into lambda_u and lambda_w, with the adjoint of w[fs-1] = w[fs]: at the
+// receiver cells of row fs-1 (mirrored) or at all others. Two cells of a column can meet on row fs, so the
+// two kinds take a launch each: the sums have one order.
+__global__ void adj_inject_uw(ac::Geo<double> g, Cells cells, int it, bool mirrored, const double* gu, const double* gw,
+                              double* lu, double* lw) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cells.ncells) return;
   const int s = blockIdx.y, i = cells.cell_z[k], j = cells.cell_x[k];
+  if ((g.fsurf && i == g.fs - 1) != mirrored) return;
   double au = 0.0, aw = 0.0;
   for (int m = g.tcell_rbeg[k]; m < g.tcell_rbeg[k + 1]; ++m) {
     const int64_t e = ((int64_t)s * g.nt + it) * g.nr + g.cell_rcv[m];
@@ -397,8 +400,7 @@ __global__ void adj_inject_uw(ac::Geo<double> g, Cells cells, int it, const doub
   }
   const int64_t so = s * g.L.plane;
   lu[so + g.L.off(i, j)] += au;
-  // two receiver cells can meet on row fs
-  atomicAdd(lw + so + g.L.off(g.fsurf && i == g.fs - 1 ? g.fs : i, j), aw);
+  lw[so + g.L.off(mirrored ? g.fs : i, j)] += aw;
 }
 
 }  // namespace ac3
